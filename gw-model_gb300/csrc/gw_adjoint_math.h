@@ -21,6 +21,7 @@
 
 #include <cmath>
 
+#include "gw_div64.cuh"
 #include "gw_internal.h"
 
 #ifdef __CUDACC__
@@ -831,14 +832,13 @@ GW_HD void cru_substep(CruCont &s, double h, const CruIn &in, const CruPar &P, d
     for (int j = 0; j < 4; ++j) jxf[j] = P.rxfer * (s.c[j] - in.Cai);
     double cn[4];
     for (int j = 0; j < 4; ++j) {
-        const double x = s.c[j];
-        const double beta = 1.0 / (1.0 + (P.BSR_const / ((P.KBSR + x) * (P.KBSR + x))) +
-                                   (P.BSL_const / ((P.KBSL + x) * (P.KBSL + x))));
+        const double x = s.c[j], u = P.KBSR + x, v = P.KBSL + x;
+        const double beta = div_rn(1.0, 1.0 + div_rn(P.BSR_const, u * u) + div_rn(P.BSL_const, v * v));
         cn[j] = x + h * (s.L[j] + s.rel[j] - jxf[j] + jiss[j]) * beta;
     }
     {
         const double x = s.J;
-        const double beta = 1.0 / (1.0 + P.CSQN_const / ((P.KCSQN + x) * (P.KCSQN + x)));
+        const double beta = div_rn(1.0, 1.0 + div_rn(P.CSQN_const, (P.KCSQN + x) * (P.KCSQN + x)));
         s.J += h * beta * (jtr - P.VSS_VJSR * (s.rel[0] + s.rel[1] + s.rel[2] + s.rel[3]));
     }
     for (int j = 0; j < 4; ++j) s.c[j] = cn[j];
@@ -898,7 +898,7 @@ GW_HD void cru_substep_adj(const CruCont &s0, double h, const CruIn &in, const C
         // over the common denominator (one division; the adjoint need not round as the forward)
         const double x = s0.c[j];
         const double uR = P.KBSR + x, uL = P.KBSL + x, A2 = uR * uR, B2 = uL * uL;
-        const double r = 1.0 / (A2 * B2 + P.BSR_const * B2 + P.BSL_const * A2);
+        const double r = div_rn(1.0, A2 * B2 + P.BSR_const * B2 + P.BSL_const * A2);
         const double beta = A2 * B2 * r;
         const double dbeta = 2.0 * uR * uL * (P.BSR_const * uL * B2 + P.BSL_const * uR * A2) * r * r;
         const double A = s0.L[j] + s0.rel[j] - jxf[j] + jiss[j];
@@ -915,7 +915,7 @@ GW_HD void cru_substep_adj(const CruCont &s0, double h, const CruIn &in, const C
         // beta = u^2 / (u^2 + CSQN), d beta/dx = 2 u CSQN / (u^2 + CSQN)^2,
         // d beta/dCSQN = -u^2 / (u^2 + CSQN)^2
         const double x = s0.J, u = P.KCSQN + x, U2 = u * u;
-        const double r = 1.0 / (U2 + P.CSQN_const);
+        const double r = div_rn(1.0, U2 + P.CSQN_const);
         const double beta = U2 * r;
         const double G = jtr - P.VSS_VJSR * (s0.rel[0] + s0.rel[1] + s0.rel[2] + s0.rel[3]);
         const double lJn = la.J;

@@ -228,7 +228,7 @@ __device__ __noinline__ void ode_phase(const OdeOffsets o, int q, int regime, in
         case OK_EXP: v = GW_ARG(0) * o_exp(GW_ARG(1) * GW_ARG(2) + GW_ARG(3), M); break;
         case OK_AFF: v = GW_ARG(0) * GW_ARG(1) + GW_ARG(2) * GW_ARG(3) + GW_ARG(4) * GW_ARG(5) + GW_ARG(6); break;
         case OK_REC:
-            v = (T)1 / (GW_ARG(0) + GW_ARG(1) * GW_ARG(2) + GW_ARG(3) * GW_ARG(4) + GW_ARG(5) * GW_ARG(6) * GW_ARG(7));
+            v = quot((T)1, GW_ARG(0) + GW_ARG(1) * GW_ARG(2) + GW_ARG(3) * GW_ARG(4) + GW_ARG(5) * GW_ARG(6) * GW_ARG(7));
             break;
         case OK_PROD: v = GW_ARG(0) * GW_ARG(1) * GW_ARG(2) * GW_ARG(3) * GW_ARG(4) * GW_ARG(5) * GW_ARG(6); break;
         case OK_SUM:
