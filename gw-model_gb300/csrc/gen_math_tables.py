@@ -1,62 +1,56 @@
-"""Generates gw_math_tables.h: the tables of the engine's FP64 exp and log (gw_math64.cuh).
+"""Generates gw_math_tables.h: the constants of the engine's FP64 exp and log (gw_math64.cuh), which
+run in 64-bit integer arithmetic.
 
-exp (Tang, ACM TOMS 15(2), 1989): 2^(j/64), j = 0..63, each as a lead double (the value rounded
-to nearest) and a trail double (the rounding error of the lead), plus ln2/64 split the same way.
-log (Tang, ACM TOMS 16(4), 1990): for j = 0..127, F_j = 1 + (j + 1/2)/128, invF_j = 1/F_j rounded
-to nearest double, and -log(invF_j) as lead + trail doubles, plus ln2 split into lead + trail.
-All values come from 60-digit decimal arithmetic (Python's decimal module).
+exp: 2^(j/256), j = 0..255, as integers of 63 fractional bits, 1/ln2 and the Taylor coefficients
+ln2^k / k! of 2^t.
+log: for j = 0..127, c_j = 2^16 / F_j rounded to an integer, F_j = 1 + (j + 1/2)/128, and
+-log(c_j / 2^16) with 64 fractional bits; ln2; the coefficients (-1)^(k-1) / k of log(1 + u).
+All values come from 80-digit decimal arithmetic (Python's decimal module).
 
 Usage: python gen_math_tables.py > gw_math_tables.h
 """
-from decimal import Decimal, getcontext
+from decimal import ROUND_HALF_EVEN, Decimal, getcontext
 
-getcontext().prec = 60
-
-
-def dbl(d: Decimal) -> float:
-    return float(d)  # correctly rounded decimal -> double
+getcontext().prec = 80
 
 
-def split(d: Decimal):
-    lead = dbl(d)
-    trail = dbl(d - Decimal(lead))
-    return lead, trail
+def fixed(d: Decimal, bits: int) -> int:
+    return int((d * Decimal(2) ** bits).to_integral_value(rounding=ROUND_HALF_EVEN))
 
 
 def main():
     ln2 = Decimal(2).ln()
-    out = []
-    out.append("// gw_math_tables.h -- generated by gen_math_tables.py; do not edit.")
-    out.append("#pragma once")
-    out.append("namespace gw {")
-    out.append("namespace math64 {")
-    l_hi, l_lo = split(ln2 / 64)
-    out.append(f"constexpr double kLn2By64Hi = {l_hi.hex()};  // ln2/64, lead")
-    out.append(f"constexpr double kLn2By64Lo = {l_lo.hex()};  // ln2/64 - lead")
-    out.append(f"constexpr double k64ByLn2 = {dbl(64 / ln2).hex()};")
-    n_hi, n_lo = split(ln2)
-    out.append(f"constexpr double kLn2Hi = {n_hi.hex()};")
-    out.append(f"constexpr double kLn2Lo = {n_lo.hex()};")
-    out.append("// 2^(j/64): {lead, trail}")
-    out.append("#define GW_EXP2_TABLE \\")
-    out.append("    { \\")
-    for j in range(64):
-        v = (Decimal(j) / 64 * ln2).exp()
-        a, b = split(v)
-        out.append(f"        {{{a.hex()}, {b.hex()}}}, \\")
-    out.append("    }")
-    out.append("// j = 0..127: {invF_j, lead(-log(invF_j)), trail}, F_j = 1 + (j + 1/2)/128")
-    out.append("#define GW_LOG_TABLE \\")
-    out.append("    { \\")
-    for j in range(128):
-        F = 1 + (Decimal(j) + Decimal("0.5")) / 128
-        inv = dbl(1 / F)
-        L = -(Decimal(inv).ln())
-        a, b = split(L)
-        out.append(f"        {{{inv.hex()}, {a.hex()}, {b.hex()}}}, \\")
-    out.append("    }")
-    out.append("}  // namespace math64")
-    out.append("}  // namespace gw")
+    out = ["// gw_math_tables.h -- generated by gen_math_tables.py; do not edit.", "#pragma once", "namespace gw {",
+           "namespace math64 {"]
+    out.append(f"constexpr unsigned long long kLog2e63 = {fixed(1 / ln2, 63):#x}ull;  // 1/ln2, 63 fractional bits")
+    out.append(f"constexpr unsigned long long kLn2 = {fixed(ln2, 64):#x}ull;      // ln2, 64 fractional bits")
+    bias = 2048 * fixed(ln2, 64)
+    out.append("// 2048 times that, as two words")
+    out.append(f"constexpr unsigned long long kLn2BiasHi = {bias >> 64:#x}ull, kLn2BiasLo = {bias & (2**64 - 1):#x}ull;")
+    f = Decimal(1)
+    for k in range(1, 6):
+        f *= ln2 / k
+        if k <= 3:
+            out.append(f"constexpr unsigned long long kExp{k} = {fixed(f, 64):#x}ull;  // ln2^{k}/{k}!, 64 fractional bits")
+        else:
+            out.append(f"constexpr unsigned int kExp{k} = {fixed(f, 32):#x}u;  // ln2^{k}/{k}!, 32 fractional bits")
+    for k in range(1, 8):
+        v = Decimal(1 if k % 2 else -1) / k
+        if k <= 3:
+            out.append(f"constexpr long long kLog{k} = {fixed(v, 62)}ll;  // (-1)^{k - 1}/{k}, 62 fractional bits")
+        else:
+            out.append(f"constexpr int kLog{k} = {fixed(v, 30)};  // (-1)^{k - 1}/{k}, 30 fractional bits")
+    out += ["// 2^(j/256), 63 fractional bits", "#define GW_EXP2_TABLE \\", "    { \\"]
+    for j in range(0, 256, 4):
+        out.append("        " + " ".join(f"{fixed((Decimal(j + i) / 256 * ln2).exp(), 63):#x}ull," for i in range(4)) + " \\")
+    out += ["    }", "// {c_j, -log(c_j / 2^16) with 64 fractional bits}", "#define GW_LOG_TABLE \\", "    { \\"]
+    for j in range(0, 128, 2):
+        row = []
+        for i in range(2):
+            c = fixed(1 / (1 + (Decimal(j + i) + Decimal("0.5")) / 128), 16)
+            row.append(f"{{{c}ull, {fixed(-(Decimal(c) / 65536).ln(), 64):#x}ull}},")
+        out.append("        " + " ".join(row) + " \\")
+    out += ["    }", "}  // namespace math64", "}  // namespace gw"]
     print("\n".join(out))
 
 

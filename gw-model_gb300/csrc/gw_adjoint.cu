@@ -147,7 +147,7 @@ struct AdjArgs {
 __device__ __forceinline__ double pulse_at(double t, const double *s) {
     double tb = __dsub_rn(t, s[0]);
     if (tb >= 0.0) {
-        if (s[1] > 0.0) tb = __dsub_rn(tb, __dmul_rn(s[1], trunc(__ddiv_rn(tb, s[1]))));
+        if (s[1] > 0.0 && tb >= s[1]) tb = __dsub_rn(tb, __dmul_rn(s[1], trunc(div_rn(tb, s[1]))));
         if (tb < s[2]) return s[3];
     }
     return 0.0;
@@ -489,45 +489,26 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
     }
 }
 
-// Shared-memory layout of k_global: the engine's global-step data (OdeShared, the lane program, its
-// slot array, the exp/log tables, the staging row of the SSA values), as ode_phase addresses them.
-struct GlobalLayout {
-    uint32_t ode, prog, x, math, stage, total;
+// Shared-memory layout of k_global: the engine's global-step data (OdeShared, the lane program's slot
+// array, the exp/log tables, the staging row of the SSA values), as OdeLane uses them.
+struct GlobalSmem {
+    double X[kOdeMaxSlots];
+    double stage[kSvCount];
+    dev::OdeShared os;
+    math64::Tables tables;
+    double sums[4];
 };
-__host__ __device__ inline GlobalLayout global_layout() {
-    auto a16 = [](size_t n) { return (uint32_t)((n + 15) & ~(size_t)15); };
-    GlobalLayout L;
-    uint32_t o = 0;
-    L.ode = o;
-    o += a16(sizeof(dev::OdeShared));
-    L.prog = o;
-    o += a16(sizeof(OdeProgram));
-    L.x = o;
-    o += a16(kOdeMaxSlots * sizeof(double));
-    L.math = o;
-    o += a16(sizeof(math64::Tables));
-    L.stage = o;
-    o += a16(kSvCount * sizeof(double));
-    L.total = o;
-    return L;
-}
 
 // The cell's flux sums of the step (its blocks' partial sums, in block order) and its global step,
 // one block of the engine's kOdeLanes threads per cell running the engine's lane program
-// (gw_ode_program.h): every warp holds one op kind per phase, so a phase costs about one op.  The
-// program's transcendental phases of the step's state run first (the engine keeps them from the
-// previous step; a block here starts from the recorded globals), then the increments with the
-// update, then the phases up to the SSA values of the new state, which are staged as the engine
-// pushes them.
+// (gw_ode_program.h, OdeLane): every warp holds one op kind per phase, so a phase costs about one op.
+// The program's phases of the step's state run first (the engine keeps them from the previous step; a
+// block here starts from the recorded globals), then the increments with the update, then the phases of
+// the new state, whose SSA values are staged as the engine pushes them.
 __global__ void __launch_bounds__(kOdeLanes) k_global(const GradArgs a, int64_t step, int slot, int use_var) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double sums[4];
-    const GlobalLayout L = global_layout();
-    dev::OdeShared &os = *reinterpret_cast<dev::OdeShared *>(smem + L.ode);
-    OdeProgram &P = *reinterpret_cast<OdeProgram *>(smem + L.prog);
-    double *X = reinterpret_cast<double *>(smem + L.x);
-    double *stage = reinterpret_cast<double *>(smem + L.stage);
-    const dev::OdeOffsets off{L.prog, L.x, L.ode, L.math, L.stage};
+    __shared__ __align__(16) GlobalSmem sm;
+    double *X = sm.X;
+    dev::OdeShared &os = sm.os;
     const int cell = blockIdx.x;
     if (a.status[cell] != 0) return;  // the same for the whole block
     const int t = (int)threadIdx.x;
@@ -535,18 +516,13 @@ __global__ void __launch_bounds__(kOdeLanes) k_global(const GradArgs a, int64_t 
     double *g = a.G + (int64_t)kNumGlobals * cell;
     double *cy = a.carry + 4 * (int64_t)cell;
     double *svo = (use_var ? const_cast<double *>(a.var_sv) : a.sv) + (int64_t)kSvCount * cell;
-    {
-        const int4 *src = reinterpret_cast<const int4 *>(a.prog);
-        int4 *dst = reinterpret_cast<int4 *>(&P);
-        for (int i = t; i < (int)(sizeof(OdeProgram) / 16); i += kOdeLanes) dst[i] = src[i];
-    }
-    math64::load_tables(*reinterpret_cast<math64::Tables *>(smem + L.math), t, kOdeLanes);
+    math64::load_tables(sm.tables, t, kOdeLanes);
     for (int i = t; i < kOdeMaxSlots; i += kOdeLanes) X[i] = 0.0;
     if (t < 4) {
         const double *pp = use_var ? a.var_part : a.part;
         double v = 0.0;
         for (int b = a.blk0[cell]; b < a.blk0[cell + 1]; ++b) v += pp[4 * (int64_t)b + t];
-        sums[t] = v;
+        sm.sums[t] = v;
     }
     // the step's record (before anything of it is overwritten)
     if (a.seg_G) {
@@ -567,43 +543,55 @@ __global__ void __launch_bounds__(kOdeLanes) k_global(const GradArgs a, int64_t 
     }
     if (t < kNumGlobals) {
         os.g[t] = g[t];
-        X[XS_G + t] = X[XS_GN + t] = g[t];
+        X[XS_G + t] = g[t];
     }
     for (int i = t; i < kOdeConstCap; i += kOdeLanes) X[XS_FIRST_FREE + i] = C.ode_consts[i];
     __syncthreads();
-    const int reg = dev::v_regime(os.g[0]);
-    for (int q = P.upd_phase + 1; q < P.n_phases; ++q) {
-        dev::ode_phase<double, double>(off, q, reg, t);
+    dev::OdeLane<double, double> L;
+    L.X = reinterpret_cast<unsigned char *>(X);
+    L.stage = sm.stage;
+    L.os = &os;
+    L.M = &sm.tables;
+    L.P = a.prog;
+    L.t = t;
+    L.reg = dev::v_regime(os.g[0]);
+    L.load_all();
+    const bool powers = L.has_powers();
+    auto phases = [&]() {
+        L.terms();
         __syncthreads();
-    }
+        if (powers) {
+            L.powers();
+            __syncthreads();
+        }
+        L.quotients();
+        __syncthreads();
+    };
+    phases();
     const bool nernst = dev::not_positive(os.g[1]) || dev::not_positive(os.g[2]);
-    for (int q = 0; q <= P.upd_phase; ++q) {
-        dev::ode_phase<double, double>(off, q, reg, t);
-        __syncthreads();
-    }
+    const double dv = L.increments();
+    __syncthreads();
+    L.update(dv);
+    __syncthreads();
     // the SSA values of the new state: the constant ones from their slots, the others from the
-    // program's phases up to the push, Cai and CaNSR from the new globals
+    // program's phases, Cai and CaNSR from the new globals
     if (t < kSvCount && t != SV_CAI && t != SV_CANSR && t != SV_CAI_LO && t != SV_CANSR_LO &&
-        P.sv_src[t] < XS_FIRST_FREE + kOdeMaxConsts)
-        stage[t] = X[P.sv_src[t]];
-    const int reg2 = dev::v_regime(os.g[0]);
-    for (int q = P.upd_phase + 1; q <= P.push_phase; ++q) {
-        dev::ode_phase<double, double>(off, q, reg2, t);
-        __syncthreads();
-    }
+        a.prog->sv_src[t] < XS_FIRST_FREE + kOdeMaxConsts)
+        sm.stage[t] = X[a.prog->sv_src[t]];
+    if (t == 64) dev::stage_pair(sm.stage, SV_CAI, SV_CAI_LO, os.g[3]);
+    if (t == 65) dev::stage_pair(sm.stage, SV_CANSR, SV_CANSR_LO, os.g[4]);
+    phases();
     if (t == 0) {
-        dev::stage_pair(stage, SV_CAI, SV_CAI_LO, os.g[3]);
-        dev::stage_pair(stage, SV_CANSR, SV_CANSR_LO, os.g[4]);
         if (nernst) {
             a.status[cell] = GW_ERR_NERNST;
         } else if (os.status != 0) {
             a.status[cell] = os.status;
         } else {
             // carry order {JLCC, ClCh, Jtr, Jxfer} from the per-CRU {JLCC, Jxfer, Jtr, ClCh}
-            cy[0] = sums[0];
-            cy[1] = sums[3];
-            cy[2] = sums[2];
-            cy[3] = sums[1];
+            cy[0] = sm.sums[0];
+            cy[1] = sm.sums[3];
+            cy[2] = sm.sums[2];
+            cy[3] = sm.sums[1];
             a.t[cell] += a.dt;
             if (a.V && (step + 1) % a.sample_every == 0) {
                 const int64_t si = (step + 1) / a.sample_every - 1;
@@ -611,10 +599,9 @@ __global__ void __launch_bounds__(kOdeLanes) k_global(const GradArgs a, int64_t 
             }
         }
     }
-    __syncthreads();
     if (nernst || os.status != 0) return;
     if (t < kNumGlobals) g[t] = os.g[t];
-    if (t < kSvCount) svo[t] = stage[t];
+    if (t < kSvCount) svo[t] = sm.stage[t];
 }
 
 // The adjoint state of CRU i after its step (its lam_x row, and the carry adjoints: the step's
@@ -1278,7 +1265,7 @@ int gw_grad_forward(gw_grad *g, double *V_samples) {
     for (int64_t s = 0; s < g->n_steps; ++s) {
         if (s % g->ck_every == 0 && (rc = g->save(s / g->ck_every))) return rc;
         k_ssa<false><<<g->n_blocks, kBlk, 0, g->stream>>>(a, s, 0);
-        k_global<<<g->n_cells, kOdeLanes, global_layout().total, g->stream>>>(a, s, 0, 0);
+        k_global<<<g->n_cells, kOdeLanes, 0, g->stream>>>(a, s, 0, 0);
     }
     cudaEventRecord(g->ev1, g->stream);
     if ((rc = g->cuda(cudaGetLastError(), "gw_grad_forward launch"))) return rc;
@@ -1334,7 +1321,7 @@ int gw_grad_backward(gw_grad *g, const double *dL_dV, double *sens) {
         if ((rc = g->cuda(cudaMemsetAsync(g->busy_n.p, 0, g->busy_n.n, g->stream), "gw_grad_backward"))) return rc;
         for (int64_t s = s0; s < s1; ++s) {
             k_ssa<false><<<g->n_blocks, kBlk, 0, g->stream>>>(a, s, (int)(s - s0));
-            k_global<<<g->n_cells, kOdeLanes, global_layout().total, g->stream>>>(a, s, (int)(s - s0), 0);
+            k_global<<<g->n_cells, kOdeLanes, 0, g->stream>>>(a, s, (int)(s - s0), 0);
         }
         for (int64_t s = s1 - 1; s >= s0; --s) {
             k_cru_busy<<<bgrid, kBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
@@ -1513,8 +1500,8 @@ int gw_grad_replay(gw_grad *g, int n_var, const int32_t *src_cell, const gw_para
     cudaEventRecord(g->ev0, g->stream);
     for (int64_t s = 0; s < g->n_steps; ++s) {
         k_ssa<true><<<nb, kBlk, 0, g->stream>>>(a, s, 0);
-        k_global<<<n_var, kOdeLanes, global_layout().total, g->stream>>>(a, s, 0, 0);
-        k_global<<<n_var, kOdeLanes, global_layout().total, g->stream>>>(va, s, 0, 1);
+        k_global<<<n_var, kOdeLanes, 0, g->stream>>>(a, s, 0, 0);
+        k_global<<<n_var, kOdeLanes, 0, g->stream>>>(va, s, 0, 1);
     }
     cudaEventRecord(g->ev1, g->stream);
     if ((rc = g->cuda(cudaGetLastError(), "gw_grad_replay launch"))) return rc;

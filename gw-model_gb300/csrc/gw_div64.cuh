@@ -1,4 +1,4 @@
-// gw_div64.cuh -- correctly rounded FP64 division on the integer and FP32 pipes.
+// gw_div64.cuh -- correctly rounded FP64 division and square root on the integer and FP32 pipes.
 //
 // GB300's FP64 pipe takes one warp instruction per ~64 cycles per SM sub-partition; a division through
 // it is about ten of them.  This one is long division on the 53-bit significands: a reciprocal
@@ -11,8 +11,14 @@
 //
 // What it is bound by: ~60 integer and FP32 instructions.  Measured on GB300, dependent divisions by one
 // warp: 235 cycles each (a / b: 600); with 16 warps per SM ~55 cycles of a sub-partition each (565).
+//
+// The square root goes the same way: the root's leading 20 bits from an FP32 reciprocal square root
+// (relative error within 2^-21 with its argument's truncation), two signed digits of 16 bits from the
+// exact remainder x - s^2, the last remainder rounding to nearest (the root of a 53-bit significand is
+// never halfway either).  ~55 instructions.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 namespace gw {
@@ -64,9 +70,41 @@ __device__ __forceinline__ double div_rn(double a, double b) {
     return __longlong_as_double((long long)(N + ((unsigned long long)top << 32)));
 }
 
+// Negative, zero, subnormal, infinite or NaN arguments.
+static __device__ __noinline__ double sqrt_special(double x) { return sqrt(x); }
+
+__device__ __forceinline__ double sqrt_rn(double x) {
+    const uint32_t xh = (uint32_t)__double2hiint(x), xl = (uint32_t)__double2loint(x);
+    const uint32_t ex = xh >> 20;  // with the sign, so that a negative x is out of range
+    if (ex - 1u >= 2046u) return sqrt_special(x);
+    const uint32_t odd = (ex & 1u) ^ 1u;  // an odd exponent of x doubles the significand
+    const uint32_t Xh = (xh & 0xFFFFFu) | 0x100000u;
+    const float v = __uint_as_float(((__funnelshift_l(xl, xh, 3) & 0x7FFFFFu) | 0x3F800000u) + (odd << 23));
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+    const float y4 = y * 0.0625f;
+    // root s1 in units of 2^-20, remainder in units of 2^-52
+    const int s1 = __float_as_int(__fmaf_rn(v * y, 1048576.f, 12582912.f)) - 0x4B400000;
+    unsigned long long r = ((unsigned long long)__funnelshift_l(xl, Xh, odd) << 32) | (xl << odd);
+    r -= (unsigned long long)((long long)s1 * (long long)s1) << 12;
+    float f = __int_as_float(0x4B400000 + (int)((long long)r >> 13)) - 12582912.f;
+    const int d2 = __float_as_int(__fmaf_rn(f, y4, 12582912.f)) - 0x4B400000;
+    r = (r << 20) - ((unsigned long long)((long long)s1 * (long long)d2) << 17) -
+        (unsigned long long)((long long)d2 * (long long)d2);  // units of 2^-72
+    f = __int_as_float(0x4B400000 + (int)((long long)r >> 17)) - 12582912.f;
+    const int d3 = __float_as_int(__fmaf_rn(f, y4, 12582912.f)) - 0x4B400000;
+    const long long s2 = ((long long)s1 << 16) + d2;  // units of 2^-36
+    r = (r << 32) - (((unsigned long long)s2 * (unsigned long long)(long long)d3) << 17) -
+        (unsigned long long)((long long)d3 * (long long)d3);  // units of 2^-104
+    const long long S = (s2 << 16) + d3, R = (long long)r;
+    const long long root = S + (R > S ? 1 : 0) - (R <= -S ? 1 : 0);
+    return __longlong_as_double(root + ((long long)(((ex + 1023u - odd) >> 1) - 1u) << 52));
+}
+
 #else
 
 inline double div_rn(double a, double b) { return a / b; }
+inline double sqrt_rn(double x) { return std::sqrt(x); }
 
 #endif
 

@@ -25,18 +25,22 @@
 namespace gw {
 namespace dev {
 
-// Flux partial of a warp or a CTA, 32 bytes in both precisions:
-//   FP32: {JLCC hi, lo, Jxfer hi, lo, Jtr hi, lo, ClCh count, 0} (float pairs, TwoSum-compensated)
-//   FP64: {JLCC, Jxfer, Jtr, ClCh count}
-struct Partial {
+// Flux partial of a warp: the sums over its CRUs of JLCC, Jxfer, Jtr and the open ClCh count.
+template <bool FP64>
+struct alignas(16) Partial;
+template <>
+struct alignas(16) Partial<true> {
     double v[4];
+};
+template <>
+struct alignas(16) Partial<false> {
+    float j, x, t;
+    int cl;
 };
 
 struct OdeShared {
     double g[kNumGlobals];  // the cell's globals (FP64 state)
-    double t;               // accumulated time
     double sums[4];         // JLCC, ClCh, Jtr, Jxfer sums of the last reduced step (FP64)
-    double stim[2];         // stimulus of step s in slot s & 1, from the leader's SSA warps
     int status;
     int pad;
 };
@@ -46,7 +50,7 @@ constexpr int kMaxThreadsFp64 = 256;  // FP64 instance: at most 4 SSA warps, up 
 constexpr int kMaxWarps = kMaxThreads / 32;
 
 struct SmemLayout {
-    size_t cc, sv, ode, prog, x, math, svs, rtab, part, mbar, fq, tile, total;
+    size_t cc, sv, ode, x, math, svs, rtab, part, mbar, fq, tile, total;
 };
 
 // FP64: CRUs of a CTA whose first iteration of a step waits for the four-lane pass (the queue
@@ -65,8 +69,6 @@ __host__ __device__ inline SmemLayout smem_layout(int tile_cap, int max_cta_cell
     o += align16(2 * kSvCount * sizeof(R));
     L.ode = o;
     o += align16(sizeof(OdeShared));
-    L.prog = o;
-    o += align16(sizeof(OdeProgram));
     L.x = o;
     o += align16(kOdeMaxSlots * sizeof(T));
     L.math = o;  // exp / log tables of the FP64 global step
@@ -76,7 +78,7 @@ __host__ __device__ inline SmemLayout smem_layout(int tile_cap, int max_cta_cell
     L.rtab = o;  // the CTA's subunit rate tables (FP32 SSA), one per step parity
     o += align16((size_t)2 * kRateTab * sizeof(float2));
     L.part = o;  // [parity][rank in cell][warp]: warp partials (written by the cell's CTAs)
-    o += align16((size_t)2 * max_cta_cell * kMaxWarps * sizeof(Partial));
+    o += (size_t)2 * max_cta_cell * kMaxWarps * sizeof(Partial<sizeof(R) == 8>);
     L.mbar = o;  // mbarriers: the warp partials of steps of parity 0 and 1 (leader CTA), then the
     o += 32;     // per-step SSA values of parity 0 and 1 (every CTA)
     L.fq = o;    // FP64: the queue's two counters (by step parity), then kEngQCap tile indices
@@ -85,16 +87,6 @@ __host__ __device__ inline SmemLayout smem_layout(int tile_cap, int max_cta_cell
     o += align16((size_t)tile_cap * sizeof(TileRec<R>));
     L.total = o;
     return L;
-}
-
-// double-float accumulate: (hi, lo) += (bh, bl)
-__device__ __forceinline__ void df_add(float &hi, float &lo, float bh, float bl) {
-    const float s = hi + bh;
-    const float bb = s - hi;
-    float e = (hi - (s - bb)) + (bh - bb);
-    e += lo + bl;
-    hi = s + e;
-    lo = e - (hi - s);
 }
 
 __device__ __forceinline__ bool finite_bits(double x) {
@@ -129,20 +121,31 @@ __device__ __forceinline__ bool bar_or(int id, int n, bool v) {
     return r != 0;
 }
 
-// Stimulus of step ri at time t (pulse train or per-step samples).  Uses explicit round-to-nearest
-// operations so the host's evaluation of the same pulse train gives the same values.
-__device__ __forceinline__ double stimulus(const CellDyn &d, double t, int64_t ri) {
-    if (d.stim_mode == STIM_SAMPLES) return (ri >= 0 && ri < d.stim_n) ? d.stim_samples[ri] : 0.0;
-    if (d.stim_mode == STIM_PULSE) {
-        double tb = __dsub_rn(t, d.stim_start);
-        if (tb >= 0.0) {
-            if (d.stim_period > 0.0)
-                tb = __dsub_rn(tb, __dmul_rn(d.stim_period, trunc(__ddiv_rn(tb, d.stim_period))));
-            if (tb < d.stim_dur) return d.stim_amp;
-        }
+// A cell's stimulus protocol in registers.
+struct Stim {
+    int mode;
+    double start, period, dur, amp;
+    const double *samples;
+    int64_t n;
+    __device__ __forceinline__ explicit Stim(const CellDyn &d)
+        : mode(d.stim_mode), start(d.stim_start), period(d.stim_period), dur(d.stim_dur), amp(d.stim_amp),
+          samples(d.stim_samples), n(d.stim_n) {}
+    __device__ __forceinline__ double sample(int64_t ri) const {
+        return mode == STIM_SAMPLES && ri >= 0 && ri < n ? samples[ri] : 0.0;
     }
-    return 0.0;
-}
+    // Pulse train at time t.  Uses explicit round-to-nearest operations so the host's evaluation of the
+    // same pulse train gives the same values (within the first period the quotient truncates to 0).
+    __device__ __forceinline__ double pulse(double t) const {
+        if (mode == STIM_PULSE) {
+            double tb = __dsub_rn(t, start);
+            if (tb >= 0.0) {
+                if (period > 0.0 && tb >= period) tb = __dsub_rn(tb, __dmul_rn(period, trunc(div_rn(tb, period))));
+                if (tb < dur) return amp;
+            }
+        }
+        return 0.0;
+    }
+};
 
 // Branch of the gate rates (common.hpp:176-218): 0 for V >= -40, 2 for V == -47.13, 1 otherwise
 // (NaN included), from integer compares on the bit pattern (no FP64 issue slots).
@@ -164,17 +167,15 @@ __device__ __forceinline__ double o_exp(double x, const math64::Tables &M) { ret
 __device__ __forceinline__ float o_exp(float x, const math64::Tables &) { return expf(x); }
 __device__ __forceinline__ double o_log(double x, const math64::Tables &M) { return math64::log(x, M); }
 __device__ __forceinline__ float o_log(float x, const math64::Tables &) { return logf(x); }
-
-__device__ __forceinline__ double t_sqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ float t_sqrt(float x) { return sqrtf(x); }
-
-// Shared-memory offsets of the global step's data, passed to ode_phase in place of pointers: the
-// function is out of line, and pointer arguments would turn every operand, program and table
-// read into a generic load; addresses formed from the shared-memory symbol inside the function
-// stay shared-memory loads.
-struct OdeOffsets {
-    uint32_t prog, x, ode, math, stage;
-};
+__device__ __forceinline__ double o_sqrt(double x) { return sqrt_rn(x); }
+__device__ __forceinline__ float o_sqrt(float x) { return sqrtf(x); }
+__device__ __forceinline__ double o_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float o_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// x with its sign flipped where bit 31 of w is set
+__device__ __forceinline__ double flip(double x, uint32_t w) {
+    return __hiloint2double(__double2hiint(x) ^ (int)(w & 0x80000000u), __double2loint(x));
+}
+__device__ __forceinline__ float flip(float x, uint32_t w) { return __uint_as_float(__float_as_uint(x) ^ (w & 0x80000000u)); }
 
 // The FP32 pair (hi, lo) of an FP64 value for the SSA: hi = (float)d, lo = (float)(d - hi); for an
 // FP64 SSA the value itself and 0.
@@ -188,147 +189,244 @@ __device__ __forceinline__ void stage_pair(double *st, int ihi, int ilo, double 
     st[ilo] = 0.0;
 }
 
-// One phase of the lane program by the kOdeLanes ODE threads (t = 0 .. kOdeLanes-1): thread t runs
-// op t of the phase.  Every warp holds one op kind per phase (P.wkind), so the switch does not
-// diverge; lanes without an op skip the arithmetic.  Kept out of line: inlined into the engine
-// kernel's loop, its shuffle tree measured 4x slower (2.2k vs 0.5k cycles per SUM phase).
-// An op whose output is a per-step SSA value also writes it, in the SSA's precision, to the push
-// staging row (P.sv_stage); Cai and CaNSR are staged by the caller (ode_warps).
+// One op of the lane program in registers: the operand slots as byte offsets into X (a sign bit on
+// top of 15 bits), so that a step spends no loads on the program.
+struct LaneOp {
+    uint32_t w[7];   // a[0..13], two to a word
+    uint32_t meta;   // kind | width << 8 | output slot (byte offset; a global's index for OK_DOT) << 16
+    int stage;       // 1 + the sv index an op's output is staged to, or 0
+    __device__ __forceinline__ int kind() const { return (int)(meta & 0xFFu); }
+    __device__ __forceinline__ int width() const { return (int)((meta >> 8) & 0xFFu); }
+    __device__ __forceinline__ uint32_t out() const { return meta >> 16; }
+    __device__ __forceinline__ uint32_t off(int k) const { return (w[k >> 1] >> (16 * (k & 1))) & 0x7FFFu; }
+    __device__ __forceinline__ uint32_t sign(int k) const { return (k & 1) ? w[k >> 1] : w[k >> 1] << 16; }
+};
+
+// The cell's global step by the kOdeLanes ODE threads (t = 0 .. kOdeLanes-1), thread t running op t
+// of each phase.  Every warp holds one op kind per phase, so the kinds do not diverge.
+//   increments()  phase E up to the flux sums: this thread's row sum (rows of up to 8 lanes, shuffles
+//                 in the first warp only)
+//   update()      after a barrier: the flux-sum terms and the Euler update by the rows' first lanes
+//   terms()       phase A of the new state (reloads the ops where V changed its regime)
+//   powers()      phase P (general Jup exponents only)
+//   quotients()   phase B
+// Each is followed by a barrier of the ODE threads (after powers() only when has_powers()).  An op
+// whose output is a per-step SSA value also writes it, in the SSA's precision, to the staging row;
+// Cai and CaNSR are staged by the caller.
+// What bounds it: the latency of three phases, each one op: 4 FP64 instructions (64 cycles each) and
+// a three-level shuffle tree, an integer exp / log / square root between two FP64 instructions
+// (gw_math64.cuh, gw_div64.cuh), and an integer division behind three FP64 instructions.
 template <typename T, typename R>
-__device__ __noinline__ void ode_phase(const OdeOffsets o, int q, int regime, int t) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    R *stage = reinterpret_cast<R *>(smem + o.stage);
-    const OdeProgram &P = *reinterpret_cast<const OdeProgram *>(smem + o.prog);
-    T *X = reinterpret_cast<T *>(smem + o.x);
-    OdeShared &os = *reinterpret_cast<OdeShared *>(smem + o.ode);
-    double *g = os.g;
-    const math64::Tables &M = *reinterpret_cast<const math64::Tables *>(smem + o.math);
-    const int wk = P.wkind[q][t >> 5];
-    if (wk == OK_NOP) return;
-    const int lane = t & 31;
-    const int b0 = P.phase_begin[q];
-    const bool live = t < P.phase_begin[q + 1] - b0;
-    const OdeOp *op = &P.ops[b0 + (live ? t : 0)];
-    if (live && regime > 0) {
-        const int ai = P.alt_idx[b0 + t];
-        if (ai != 255) op = &P.alt[regime - 1][ai];
+struct OdeLane {
+    unsigned char *X;
+    R *stage;
+    OdeShared *os;
+    const math64::Tables *M;
+    const OdeProgram *P;  // global memory
+    int t, reg;
+    LaneOp e, a, b;
+
+    __device__ __forceinline__ T &x(uint32_t off) const { return *reinterpret_cast<T *>(X + off); }
+    __device__ __forceinline__ T arg(const LaneOp &o, int k) const { return x(o.off(k)); }
+    __device__ __forceinline__ T *slots() const { return reinterpret_cast<T *>(X); }
+    __device__ __forceinline__ bool has_powers() const { return P->n_phases == 4; }
+
+    __device__ __forceinline__ void load(LaneOp &o, int q) const {
+        const int b0 = P->phase_begin[q];
+        o = LaneOp{};
+        if (t >= P->phase_begin[q + 1] - b0) return;
+        const int i = b0 + t, ai = P->alt_idx[i];
+        const OdeOp *op = reg > 0 && ai != 255 ? &P->alt[reg - 1][ai] : &P->ops[i];
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(op);
+        const uint32_t m = src[0];
+        const bool dot = (m & 0xFFu) == (uint32_t)OK_DOT;
+        o.meta = (m & 0xFFFFu) | ((m >> 16) * (dot ? 1u : (uint32_t)sizeof(T)) << 16);
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            const uint32_t v = src[1 + k];
+            o.w[k] = (v & 0x80008000u) | ((v & 0x7FFF7FFFu) * (uint32_t)sizeof(T));
+        }
+        o.stage = P->sv_stage[i];
     }
-    // the 32-byte op in two 16-byte loads: consecutive lanes read consecutive ops, so the loads do
-    // not conflict on shared-memory banks (field-by-field loads at a 32-byte stride would)
-    const uint4 w0 = reinterpret_cast<const uint4 *>(op)[0], w1 = reinterpret_cast<const uint4 *>(op)[1];
-    const int kind = live ? (int)(w0.x & 0xFFu) : (int)OK_NOP;
-    const int out = (int)(w0.x >> 16);
-    const uint32_t pw[7] = {w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#define GW_ARG(k) (X[(pw[(k) >> 1] >> (16 * ((k) & 1))) & 0xFFFFu])
-    T v = (T)0;
-    if (kind != OK_NOP) {
-        switch (wk) {
-        case OK_LOG: v = o_log(GW_ARG(0) + GW_ARG(1) * GW_ARG(2), M); break;
-        case OK_SQRT: v = GW_ARG(0) * GW_ARG(1) * t_sqrt(GW_ARG(2) * GW_ARG(3)); break;
-        case OK_EXP: v = GW_ARG(0) * o_exp(GW_ARG(1) * GW_ARG(2) + GW_ARG(3), M); break;
-        case OK_AFF: v = GW_ARG(0) * GW_ARG(1) + GW_ARG(2) * GW_ARG(3) + GW_ARG(4) * GW_ARG(5) + GW_ARG(6); break;
-        case OK_REC:
-            v = quot((T)1, GW_ARG(0) + GW_ARG(1) * GW_ARG(2) + GW_ARG(3) * GW_ARG(4) + GW_ARG(5) * GW_ARG(6) * GW_ARG(7));
+    __device__ __forceinline__ void load_all() {
+        load(e, 0);
+        load(a, 1);
+        load(b, P->push_phase);
+    }
+
+    __device__ __forceinline__ T increments() const {
+        T v = (T)0;
+        if (t >= 64) return v;
+        v = flip(arg(e, 1), e.sign(1)) * arg(e, 2);
+        v = o_fma(flip(arg(e, 3), e.sign(3)), arg(e, 4), v);
+        v = o_fma(flip(arg(e, 5), e.sign(5)), arg(e, 6), v);
+        v = o_fma(flip(arg(e, 7), e.sign(7)), arg(e, 8), v);
+        if (t < 32) {
+            // rows of `width` lanes (a power of two, rows aligned to it): tree over offsets 1, 2, 4
+            const int wm = e.kind() == OK_DOT ? e.width() - 1 : 0;
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) {
+                const T o = __shfl_down_sync(0xffffffffu, v, off);
+                if ((t & wm) + off <= wm && (t & (2 * off - 1)) == 0) v += o;
+            }
+        }
+        return v;
+    }
+    __device__ __forceinline__ void update(T v) const {
+        if (t >= 64 || e.kind() != OK_DOT || (t & (e.width() - 1))) return;
+        if (t < 32) v = o_fma(arg(e, 11), arg(e, 12), o_fma(arg(e, 9), arg(e, 10), v));
+        const int out = (int)e.out();
+        const double ng = sizeof(T) == 8 ? __fma_rn((double)arg(e, 0), (double)v, os->g[out])
+                                         : os->g[out] + (double)(arg(e, 0) * v);
+        os->g[out] = ng;
+        slots()[XS_G + out] = (T)ng;
+        if (!finite_bits(ng)) atomicCAS(&os->status, 0, (int)GW_ERR_NONFINITE);  // first error of the cell
+    }
+    __device__ __forceinline__ void put(const LaneOp &o, T v) const {
+        x(o.out()) = v;
+        if (o.stage) stage[o.stage - 1] = (R)v;
+    }
+    __device__ __forceinline__ void exp_op(const LaneOp &o) const {
+        put(o, o_fma(arg(o, 0), o_exp(o_fma(arg(o, 1), arg(o, 2), arg(o, 3)), *M), arg(o, 4)));
+    }
+    __device__ __forceinline__ void terms() {
+        const int r = v_regime(os->g[0]);
+        if (r != reg) {
+            reg = r;
+            load_all();
+        }
+        switch (a.kind()) {
+        case OK_EXP: exp_op(a); break;
+        case OK_LOG:
+            put(a, o_fma(arg(a, 4), o_log(o_fma(arg(a, 1), arg(a, 5), arg(a, 0)), *M), arg(a, 2) + arg(a, 3)));
             break;
-        case OK_PROD: v = GW_ARG(0) * GW_ARG(1) * GW_ARG(2) * GW_ARG(3) * GW_ARG(4) * GW_ARG(5) * GW_ARG(6); break;
-        case OK_SUM:
-        case OK_SUMU:
-            v = GW_ARG(2) * GW_ARG(3) * GW_ARG(4) + GW_ARG(5) * GW_ARG(6) * GW_ARG(7) + GW_ARG(8) * GW_ARG(9) * GW_ARG(10) +
-                GW_ARG(11) * GW_ARG(12) * GW_ARG(13);
+        case OK_POW: {
+            const T s = o_sqrt(arg(a, 2) * arg(a, 3));
+            const T c = arg(a, 0) * arg(a, 1);
+            put(a, o_fma(c, a.width() == 2 ? s * o_sqrt(s) : s, arg(a, 4)));
             break;
+        }
         default: break;
         }
     }
-    if (wk == OK_SUM || wk == OK_SUMU) {
-        // rows of `width` lanes (a power of two, rows aligned to it): tree over offsets 1, 2, 4
-        const bool row = kind == OK_SUM || kind == OK_SUMU;
-        const int wm = row ? (int)((w0.x >> 8) & 0xFFu) - 1 : 0;
+    __device__ __forceinline__ void powers() const {
+        LaneOp o;
+        load(o, 2);
+        if (o.kind() == OK_EXP) exp_op(o);
+    }
+    __device__ __forceinline__ void quotients() const {
+        if (b.kind() == OK_QUOT)
+            put(b, quot(arg(b, 0) * o_fma(arg(b, 2), arg(b, 3), arg(b, 1)), o_fma(arg(b, 5), arg(b, 6), arg(b, 4))));
+        else if (b.kind() == OK_SUM3)
+            put(b, o_fma(arg(b, 4), arg(b, 5), o_fma(arg(b, 2), arg(b, 3), arg(b, 0) * arg(b, 1))));
+    }
+};
+
+// Sums {JLCC, ClCh, Jtr, Jxfer} of the n warp partials of one slot (n <= 16 CTAs x kMaxWarps) by two
+// warps of the ODE threads: half 0 JLCC and ClCh, half 1 Jtr and Jxfer.  The result does not depend on
+// the order of the partials in either precision's slots beyond their fixed positions.
+constexpr int kSlotsPerLane = 16 * kMaxWarps / 32;
+
+// FP32: each quantity's partials on one fixed-point scale, 2^-54 of the largest's power of two, summed
+// exactly in 64-bit integers (the lanes' sums through REDUX in three pieces) and rounded once to FP64.
+// (A tree of compensated float pairs took ~700 cycles, this ~250.)  A NaN or infinity, which has no
+// scale, makes the sum NaN.
+__device__ __forceinline__ double fixed_sum(const float (&f)[kSlotsPerLane], int nk) {
+    uint32_t top = 0u;
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) {
-            const T o = __shfl_down_sync(0xffffffffu, v, off);
-            if (row && (lane & wm) + off <= wm && (lane & (2 * off - 1)) == 0) v += o;
+    for (int k = 0; k < kSlotsPerLane; ++k)
+        if (k < nk) top = max(top, __float_as_uint(f[k]) & 0x7FFFFFFFu);
+    top = __reduce_max_sync(0xffffffffu, top);
+    const int em = max((int)(top >> 23), 1);
+    long long s = 0;
+#pragma unroll
+    for (int k = 0; k < kSlotsPerLane; ++k)
+        if (k < nk) {
+            const uint32_t b = __float_as_uint(f[k]);
+            const int ex = (int)((b >> 23) & 0xFFu);
+            const unsigned long long m = (unsigned long long)((b & 0x7FFFFFu) | (ex ? 0x800000u : 0u)) << 30;
+            const long long v = (long long)(m >> min(em - max(ex, 1), 63));
+            s += (b >> 31) ? -v : v;
         }
-        if (row && (lane & wm) == 0) {
-            const T r = GW_ARG(0) * GW_ARG(1) * v;
-            if (kind == OK_SUMU) {
-                // Euler update of global `out` (FP64 state); every row of the phase reads the old
-                // values at XS_G, the new one goes to XS_GN for the phases that follow
-                const double ng = g[out] + (double)r;
-                g[out] = ng;
-                X[XS_GN + out] = (T)ng;
-                if (!finite_bits(ng)) atomicCAS(&os.status, 0, (int)GW_ERR_NONFINITE);  // first error of the cell
-            } else {
-                X[out] = r;
-                const int sv = P.sv_stage[b0 + t];
-                if (sv) stage[sv - 1] = (R)r;
-            }
-        }
-        return;
-    }
-#undef GW_ARG
-    if (kind != OK_NOP) {
-        X[out] = v;
-        const int sv = P.sv_stage[b0 + t];
-        if (sv) stage[sv - 1] = (R)v;
-    }
+    const int h = __reduce_add_sync(0xffffffffu, (int)(s >> 32));
+    const uint32_t lo = (uint32_t)s;
+    const uint32_t l1 = __reduce_add_sync(0xffffffffu, lo >> 16), l0 = __reduce_add_sync(0xffffffffu, lo & 0xFFFFu);
+    s = ((long long)h << 32) + ((long long)l1 << 16) + (long long)l0;
+    if (top >= 0x7F800000u) return __longlong_as_double(0x7FF8000000000000ll);
+    if (s == 0) return 0.0;
+    const unsigned long long u = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
+    const int z = __clzll((long long)u);
+    // u 2^(em - 127 - 23 - 30), leading bit at 63 - z
+    const unsigned long long d = math64::pack(u << z, 63 - z + em - 180);
+    return __longlong_as_double((long long)(s < 0 ? d | 0x8000000000000000ull : d));
 }
 
-// Sums {JLCC, ClCh, Jtr, Jxfer} of the cell's CTA partials of one slot; ODE warp w reduces
-// quantity w.  Writes the FP64 sums to out[] (shared) from lane 0 of each warp.  A lane takes the
-// slots lane, lane + 32, ... (at most kSlotsPerLane): all its loads are issued first and summed in
-// a pairwise tree, so the lane's part costs one load latency and three dependent additions.
-constexpr int kSlotsPerLane = 16 * kMaxWarps / 32;  // up to 16 CTAs per cell
-template <bool FP64, typename T>
-__device__ __forceinline__ void reduce_partials(const Partial *slot, int n, int warp, int lane, double *out, T *X) {
-    if (warp >= 4) return;
-    double r;
-    if (FP64) {
-        const int src = warp == 0 ? 0 : (warp == 1 ? 3 : (warp == 2 ? 2 : 1));  // JLCC, ClCh, Jtr, Jxfer
-        double a[kSlotsPerLane];
+template <typename T>
+__device__ __forceinline__ void reduce_partials(const Partial<false> *slot, int n, int half, int lane, double *out, T *X) {
+    const int nk = (n + 31) >> 5;
+    double r0, r1;
+    if (half == 0) {
+        float f[kSlotsPerLane];
+        int cl = 0;
 #pragma unroll
         for (int k = 0; k < kSlotsPerLane; ++k) {
             const int i = lane + 32 * k;
-            a[k] = i < n ? slot[i].v[src] : 0.0;
+            f[k] = 0.f;
+            if (k < nk && i < n) {
+                f[k] = slot[i].j;
+                cl += slot[i].cl;
+            }
         }
-#pragma unroll
-        for (int w = kSlotsPerLane / 2; w > 0; w >>= 1)
-#pragma unroll
-            for (int k = 0; k < w; ++k) a[k] += a[k + w];
-        double acc = a[0];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        r = acc;
+        cl = (int)__reduce_add_sync(0xffffffffu, (unsigned)cl);
+        r0 = fixed_sum(f, nk);
+        r1 = (double)cl;
     } else {
-        // float fields: 0,1 JLCC; 2,3 Jxfer; 4,5 Jtr; 6 ClCh
-        const int src = warp == 0 ? 0 : (warp == 1 ? 6 : (warp == 2 ? 4 : 2));
-        float h[kSlotsPerLane], l[kSlotsPerLane];
+        float f[kSlotsPerLane], g[kSlotsPerLane];
 #pragma unroll
         for (int k = 0; k < kSlotsPerLane; ++k) {
             const int i = lane + 32 * k;
-            const float *f = reinterpret_cast<const float *>(slot[i < n ? i : 0].v);
-            h[k] = i < n ? f[src] : 0.f;
-            l[k] = i < n && warp != 1 ? f[src + 1] : 0.f;
+            f[k] = g[k] = 0.f;
+            if (k < nk && i < n) {
+                f[k] = slot[i].t;
+                g[k] = slot[i].x;
+            }
         }
-#pragma unroll
-        for (int w = kSlotsPerLane / 2; w > 0; w >>= 1)
-#pragma unroll
-            for (int k = 0; k < w; ++k) df_add(h[k], l[k], h[k + w], l[k + w]);
-        float hi = h[0], lo = l[0];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float a0 = __shfl_xor_sync(0xffffffffu, hi, o), a1 = __shfl_xor_sync(0xffffffffu, lo, o);
-            df_add(hi, lo, a0, a1);
-        }
-        r = (double)hi + (double)lo;
+        r0 = fixed_sum(f, nk);
+        r1 = fixed_sum(g, nk);
     }
-    if (lane == 0) {
-        out[warp] = r;
-        X[XS_SUMS + warp] = (T)r;
+    if (lane < 2) {
+        const double r = lane ? r1 : r0;
+        out[2 * half + lane] = r;
+        X[XS_SUMS + 2 * half + lane] = (T)r;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void reduce_partials(const Partial<true> *slot, int n, int half, int lane, double *out, T *X) {
+    const int nk = (n + 31) >> 5;
+    // {JLCC, Jxfer, Jtr, ClCh} of a slot
+    const int s0 = half == 0 ? 0 : 2, s1 = half == 0 ? 3 : 1;
+    double a = 0.0, b = 0.0;
+    for (int k = 0; k < nk; ++k) {
+        const int i = lane + 32 * k;
+        if (i < n) {
+            a += slot[i].v[s0];
+            b += slot[i].v[s1];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane < 2) {
+        const double r = lane ? b : a;
+        out[2 * half + lane] = r;
+        X[XS_SUMS + 2 * half + lane] = (T)r;
     }
 }
 
 // Per-step SSA values of the new state to every CTA of the cell: the staging row (written by the
-// ops that produce the values, see ode_phase, and visible after the phase's barrier) pushed in
+// ops that produce the values, see OdeLane, and visible after the phase's barrier) pushed in
 // 16-byte words (CTA, word) by all kOdeLanes threads, as asynchronous stores that count themselves
 // off the receiving CTA's mbarrier of this slot (local shared address mbar_slot in every CTA).
 template <bool FP64>
@@ -439,12 +537,11 @@ __device__ __forceinline__ void record_pass(const KernelArgs &a, const CtaWork &
 // Per-lane flux accumulators and their warp sum as a Partial (all lanes hold it).
 template <bool FP64>
 struct FluxAcc {
-    float jh = 0, jl = 0, xh = 0, xl = 0, th = 0, tl = 0;  // FP32: (hi, lo) pairs
-    double dj = 0, dx = 0, dtr = 0;                       // FP64
+    float jh = 0, xh = 0, th = 0;    // FP32
+    double dj = 0, dx = 0, dtr = 0;  // FP64
     int acl = 0;
     // FP32: a lane's own CRUs (one to a few per step) add up in FP32, the lane sums in a plain
-    // FP32 tree (warp_total); the cell's warp partials are then combined with compensation
-    // (reduce_partials).
+    // FP32 tree (warp_total); the cell's warp partials are then combined exactly (reduce_partials).
     __device__ __forceinline__ void add(float j, float x, float t, int cl) {
         jh += j;
         xh += x;
@@ -457,9 +554,9 @@ struct FluxAcc {
         dtr += t;
         acl += cl;
     }
-    __device__ __forceinline__ Partial warp_total() {
-        Partial pv;
-        if (FP64) {
+    __device__ __forceinline__ Partial<FP64> warp_total() {
+        Partial<FP64> pv;
+        if constexpr (FP64) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 dj += __shfl_xor_sync(0xffffffffu, dj, o);
@@ -472,22 +569,20 @@ struct FluxAcc {
             pv.v[2] = dtr;
             pv.v[3] = (double)acl;
         } else {
-            // FP32: a plain tree over the 32 lane sums (each covers one to a few CRUs; the
-            // compensated sums start where most terms meet, across the warp partials of a CTA and
-            // the CTA partials of a cell), and one REDUX for the ClCh count.  The per-step tree ran
-            // on every lane of every warp: with compensation it was ~150 instructions per CRU-step
-            // of a 12,500-CRU cell.
+            // FP32: a plain tree over the 32 lane sums (each covers a few CRUs; the exact sums start
+            // where most terms meet, across the cell's warp partials), and one REDUX for the ClCh
+            // count.  The per-step tree runs on every lane of every warp: with compensation it was
+            // ~150 instructions per CRU-step of a 12,500-CRU cell.
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 jh += __shfl_xor_sync(0xffffffffu, jh, o);
                 xh += __shfl_xor_sync(0xffffffffu, xh, o);
                 th += __shfl_xor_sync(0xffffffffu, th, o);
             }
-            acl = (int)__reduce_add_sync(0xffffffffu, (unsigned)acl);
-            float *f = reinterpret_cast<float *>(pv.v);
-            f[0] = jh; f[1] = 0.f; f[2] = xh; f[3] = 0.f; f[4] = th; f[5] = 0.f;
-            f[6] = (float)acl;
-            f[7] = 0.f;
+            pv.j = jh;
+            pv.x = xh;
+            pv.t = th;
+            pv.cl = (int)__reduce_add_sync(0xffffffffu, (unsigned)acl);
         }
         return pv;
     }
@@ -505,17 +600,15 @@ struct CtaView {
     SsaConsts<R> *cc;
     R *svbuf;
     OdeShared *os;
-    OdeProgram *P;
     T *X;
     math64::Tables *M;
     void *svstage;
-    Partial *part;
+    Partial<FP64> *part;
     float2 *rtab;
     int *fq;        // FP64: queue counters [2] (+2 unused), then the queue
     uint32_t mbar;  // shared address of the partials' mbarrier of parity 0 (parity 1 at +8); the
                     // SSA values' mbarriers of parity 0 and 1 at +16 and +24
     TileRec<R> *tile;
-    OdeOffsets off;  // for ode_phase
 
     __device__ __forceinline__ explicit CtaView(const KernelArgs &a) {
         extern __shared__ __align__(16) unsigned char smem[];
@@ -532,102 +625,105 @@ struct CtaView {
         cc = reinterpret_cast<SsaConsts<R> *>(smem + L.cc);
         svbuf = reinterpret_cast<R *>(smem + L.sv);
         os = reinterpret_cast<OdeShared *>(smem + L.ode);
-        P = reinterpret_cast<OdeProgram *>(smem + L.prog);
         X = reinterpret_cast<T *>(smem + L.x);
         M = reinterpret_cast<math64::Tables *>(smem + L.math);
         svstage = smem + L.svs;
-        part = reinterpret_cast<Partial *>(smem + L.part);
+        part = reinterpret_cast<Partial<FP64> *>(smem + L.part);
         rtab = reinterpret_cast<float2 *>(smem + L.rtab);
         fq = reinterpret_cast<int *>(smem + L.fq);
         mbar = smem_addr(smem + L.mbar);
         tile = reinterpret_cast<TileRec<R> *>(smem + L.tile);
-        off = OdeOffsets{(uint32_t)L.prog, (uint32_t)L.x, (uint32_t)L.ode, (uint32_t)L.math, (uint32_t)L.svs};
     }
 };
 
 // The leader CTA's ODE warps over a launch: the transcendental phases of the initial state and
-// the push of sv[0], then per global step s the wait for and reduction of the warp partials of
-// step s-1, the global step s -> s+1 and the push of sv[(s+1)&1], and the carry back to the cell
-// block at the end.  A function of its own (not inlined into the kernel), so that its register allocation and
-// schedule do not depend on the SSA code.
+// the push of sv[0], then per global step s the increments on two warps beside the wait for and the
+// reduction of the warp partials of step s-1 on the other two, the global step s -> s+1 and the push
+// of sv[(s+1)&1], and the carry back to the cell block at the end.  A function of its own (not inlined
+// into the kernel), so that its register allocation and schedule do not depend on the SSA code.
 template <bool FP64, bool ODE64>
 __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
     using T = typename std::conditional<ODE64, double, float>::type;
     using R = typename std::conditional<FP64, double, float>::type;
     const CtaView<FP64, ODE64> v(a);
-    const OdeProgram &P = *v.P;
     OdeShared &os = *v.os;
     T *X = v.X;
-    const math64::Tables &M = *v.M;
-    const int ot = v.ot, lane = v.lane, cell = v.w.cell;
+    const int ot = v.ot, lane = v.lane, cell = v.w.cell, warp = ot >> 5;
     const int pslot = a.max_cta_cell * kMaxWarps;  // warp partials per parity slot
-    {
-        // program, constants and state of the cell
-        const int4 *src = reinterpret_cast<const int4 *>(a.prog);
-        int4 *dst = reinterpret_cast<int4 *>(v.P);
-        for (int i = ot; i < (int)(sizeof(OdeProgram) / 16); i += kOdeLanes) dst[i] = src[i];
+    R *stage = reinterpret_cast<R *>(v.svstage);
+    const CellStatic &C = a.cs[cell];
+    const CellDyn &d0 = a.dyn[cell];
+    const Stim stim(d0);
+    OdeLane<T, R> L;
+    L.X = reinterpret_cast<unsigned char *>(X);
+    L.stage = stage;
+    L.os = &os;
+    L.M = v.M;
+    L.P = a.prog;
+    L.t = ot;
+    for (int i = ot; i < kOdeMaxSlots; i += kOdeLanes) X[i] = (T)0;
+    math64::load_tables(*v.M, ot, kOdeLanes);
+    ode_bar();
+    if (ot == 0) {
+        X[XS_ONE] = (T)1;
+        X[XS_MONE] = (T)-1;
+        os.sums[0] = d0.sum_jlcc;
+        os.sums[1] = d0.sum_clch;
+        os.sums[2] = d0.sum_jtr;
+        os.sums[3] = d0.sum_jxfer;
+        os.status = 0;
+        X[XS_DT] = (T)a.dt;
+        for (int i = 0; i < 4; ++i) X[XS_SUMS + i] = (T)os.sums[i];
     }
-    {
-        const CellStatic &C = a.cs[cell];
-        const CellDyn &d = a.dyn[cell];
-        for (int i = ot; i < kOdeMaxSlots; i += kOdeLanes) X[i] = (T)0;
-        math64::load_tables(*v.M, ot, kOdeLanes);
-        ode_bar();
-        if (ot == 0) {
-            X[XS_ONE] = (T)1;
-            X[XS_MONE] = (T)-1;
-            os.t = d.t;
-            os.sums[0] = d.sum_jlcc;
-            os.sums[1] = d.sum_clch;
-            os.sums[2] = d.sum_jtr;
-            os.sums[3] = d.sum_jxfer;
-            os.status = 0;
-            X[XS_DT] = (T)a.dt;
-            X[XS_ISTIM] = (T)stimulus(d, d.t, a.run_step0);
-            for (int i = 0; i < 4; ++i) X[XS_SUMS + i] = (T)os.sums[i];
-        }
-        for (int i = ot; i < kNumGlobals; i += kOdeLanes) {
-            os.g[i] = d.g[i];
-            X[XS_G + i] = X[XS_GN + i] = (T)d.g[i];
-        }
-        for (int i = ot; i < kOdeConstCap; i += kOdeLanes) X[XS_FIRST_FREE + i] = (T)C.ode_consts[i];
-        ode_bar();
-        // staging row: the constant SSA values once per launch, Cai and CaNSR of the initial state
-        // (the other values are staged by the phases that compute them)
-        R *stage = reinterpret_cast<R *>(v.svstage);
-        if (ot < kSvCount && ot != SV_CAI && ot != SV_CANSR && ot != SV_CAI_LO && ot != SV_CANSR_LO &&
-            P.sv_src[ot] < XS_FIRST_FREE + kOdeMaxConsts)
-            stage[ot] = (R)X[P.sv_src[ot]];
-        if (ot == 0) stage_pair(stage, SV_CAI, SV_CAI_LO, os.g[3]);
-        if (ot == 1) stage_pair(stage, SV_CANSR, SV_CANSR_LO, os.g[4]);
+    for (int i = ot; i < kNumGlobals; i += kOdeLanes) {
+        os.g[i] = d0.g[i];
+        X[XS_G + i] = (T)d0.g[i];
     }
-    // The next step's stimulus is formed by lane 0 of a warp without ops in the update phase (its
-    // t_{s+1} is os.t + dt, the same addition as the update's), else of one idle in the push
-    // phase (os.t is then t_{s+1}), else by thread 0 before the push.
-    int stim_q = -1, stim_warp = 0;
-    for (int w = kOdeWarps - 1; w >= 0; --w)
-        if (stim_q < 0 && P.wkind[P.upd_phase][w] == OK_NOP) stim_q = P.upd_phase, stim_warp = w;
-    for (int w = kOdeWarps - 1; w >= 0; --w)
-        if (stim_q < 0 && P.push_phase > P.upd_phase && P.wkind[P.push_phase][w] == OK_NOP)
-            stim_q = P.push_phase, stim_warp = w;
-    // transcendental phases of the initial state, push sv[0]
-    {
-        const int reg = v_regime(os.g[0]);
-        for (int q = P.upd_phase + 1; q <= P.push_phase; ++q) {
-            ode_phase<T, R>(v.off, q, reg, ot);
+    for (int i = ot; i < kOdeConstCap; i += kOdeLanes) X[XS_FIRST_FREE + i] = (T)C.ode_consts[i];
+    // The accumulated time, and the stimulus of the next step, by a lane of a warp with little to do in
+    // phase B (t_{s+1} = t_s + dt, as the reference accumulates it).
+    const bool clock = ot == 2 * 32;
+    // A sampled stimulus is read a step before its use.
+    double time = d0.t, ahead = 0.0;
+    auto set_stim = [&](int64_t ri) {
+        X[XS_ISTIM] = (T)(stim.mode == STIM_SAMPLES ? ahead : stim.pulse(time));
+        ahead = stim.sample(ri + 1);
+    };
+    if (clock) {
+        ahead = stim.sample(a.run_step0);
+        set_stim(a.run_step0);
+    }
+    ode_bar();
+    // staging row: the constant SSA values once per launch, Cai and CaNSR of the initial state
+    // (the other values are staged by the ops that compute them)
+    if (ot < kSvCount && ot != SV_CAI && ot != SV_CANSR && ot != SV_CAI_LO && ot != SV_CANSR_LO) {
+        const int src = a.prog->sv_src[ot];
+        if (src < XS_FIRST_FREE + kOdeMaxConsts) stage[ot] = (R)X[src];
+    }
+    L.reg = v_regime(os.g[0]);
+    L.load_all();
+    const bool powers = L.has_powers();
+    // Cai and CaNSR of the state with their FP32 remainders, by two lanes of the last warp in phase B
+    const int pair = ot == kOdeLanes - 1 ? 0 : (ot == kOdeLanes - 2 ? 1 : -1);
+    auto phases = [&]() {  // the new state's phases, each with its barrier
+        L.terms();
+        ode_bar();
+        if (powers) {
+            L.powers();
             ode_bar();
         }
-        // (the SSA warps wait for these bytes in step 0: the host launches 1..steps_per_launch
-        // steps, never 0, so no CTA exits while they may be in flight)
-        push_sv<FP64>(v.svbuf, v.svstage, 0, v.mbar + 16u, v.w, ot);
-        for (int q = P.push_phase + 1; q < P.n_phases; ++q) {
-            ode_phase<T, R>(v.off, q, reg, ot);
-            ode_bar();
-        }
-    }
-    // bytes of the cell's warp partials per step (every SSA warp of the cell pushes 32 B)
+        L.quotients();
+        if (pair == 0) stage_pair(stage, SV_CAI, SV_CAI_LO, os.g[3]);
+        if (pair == 1) stage_pair(stage, SV_CANSR, SV_CANSR_LO, os.g[4]);
+    };
+    phases();
+    ode_bar();
+    // (the SSA warps wait for these bytes in step 0: the host launches 1..steps_per_launch
+    // steps, never 0, so no CTA exits while they may be in flight)
+    push_sv<FP64>(v.svbuf, v.svstage, 0, v.mbar + 16u, v.w, ot);
+    // bytes of the cell's warp partials per step
     const uint32_t part_bytes =
-        (uint32_t)sizeof(Partial) * (uint32_t)(v.nw + (v.w.n_cta_cell - 1) * (v.nw + kOdeWarps));
+        (uint32_t)sizeof(Partial<FP64>) * (uint32_t)(v.nw + (v.w.n_cta_cell - 1) * (v.nw + kOdeWarps));
     bool stopped = false;  // a wait ran out (the same on every ODE thread)
     int s_stop = -1;       // the step whose wait (for the partials of step s_stop - 1) ran out
     for (int s = 0; s < a.n_steps; ++s) {
@@ -641,63 +737,43 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         // launch ends within about a second per CTA and few stray bytes land on any mbarrier.
         if (stopped) continue;
         // the partials of step s will complete the next phase of mbarrier par (the previous one,
-        // step s-2's, completed before this thread's wait in step s-1)
+        // step s-2's, completed before the wait of step s-1)
         if (ot == 0)
             mbar_arrive_expect_tx(v.mbar + 8u * (uint32_t)par,
                                   part_bytes + (s == a.n_steps - 1 ? (uint32_t)a.test_extra_tx : 0u));
-        // fluxes of step s-1 (or the carry), then the global step s -> s+1
         if (ot == 0 && (not_positive(os.g[1]) || not_positive(os.g[2])) && os.status == 0)
             os.status = GW_ERR_NERNST;
-        if (s > 0) {
-            const bool ok = mbar_wait(v.mbar + 8u * (uint32_t)(par ^ 1), (uint32_t)((s - 1) >> 1) & 1u);
-            if (bar_or(1, kOdeLanes, !ok)) {  // the same decision on all ODE threads
-                if (ot == 0) atomicCAS(&os.status, 0, (int)GW_ERR_SYNC_TIMEOUT);
-                stopped = true;
-                s_stop = s;
-                continue;
-            }
+        // the increments up to the flux sums (warps 0 and 1), and the sums of step s-1 (warps 2 and 3;
+        // step 0 uses the carry)
+        const T dv = L.increments();
+        bool ok = true;
+        if (s > 0 && warp >= 2) {
+            ok = mbar_wait(v.mbar + 8u * (uint32_t)(par ^ 1), (uint32_t)((s - 1) >> 1) & 1u);
+            // (a warp's lanes may find different outcomes; whatever is summed after a wait that ran out
+            // is not used)
+            reduce_partials(v.part + (par ^ 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp - 2, lane, os.sums, X);
         }
-        if (s > 0) reduce_partials<FP64, T>(v.part + (par ^ 1) * pslot, v.w.n_cta_cell * kMaxWarps, ot >> 5, lane, os.sums, X);
-        if (s > 0 && ot == 0) X[XS_ISTIM] = (T)os.stim[par];  // formed in step s-1 (below)
+        if (bar_or(1, kOdeLanes, !ok)) {  // the same decision on all ODE threads
+            if (ot == 0) atomicCAS(&os.status, 0, (int)GW_ERR_SYNC_TIMEOUT);
+            stopped = true;
+            s_stop = s;
+            continue;
+        }
+        L.update(dv);
         ode_bar();
-        const int reg_n = v_regime(os.g[0]);
-        for (int q = 0; q <= P.upd_phase; ++q) {
-            if (q == stim_q && lane == 0 && (ot >> 5) == stim_warp)
-                os.stim[par ^ 1] = stimulus(a.dyn[cell], os.t + a.dt, ri + 1);
-            ode_phase<T, R>(v.off, q, reg_n, ot);
-            ode_bar();
-        }
-        if (ot == 0) os.t += a.dt;
+        if (clock) time += a.dt;
         if (rec_ok) {
             double *dst = a.tr_glob + ((int64_t)cell * a.rec_cap + r_idx) * kNumGlobals;
             for (int i = ot; i < kNumGlobals; i += kOdeLanes) dst[i] = os.g[i];
-            if (ot == 0 && (cell == 0 || (a.tr_cell >= 0 && cell == a.tr_cell))) a.tr_t[r_idx] = os.t;
+            if (clock && (cell == 0 || (a.tr_cell >= 0 && cell == a.tr_cell))) a.tr_t[r_idx] = time;
         }
-        const int reg = v_regime(os.g[0]);
-        // Cai and CaNSR of the new state with their FP32 remainders, staged for the push by two
-        // lanes of the last ODE warp, whose ops in the next phase finish early
-        if (ot == kOdeLanes - 1) stage_pair(reinterpret_cast<R *>(v.svstage), SV_CAI, SV_CAI_LO, os.g[3]);
-        if (ot == kOdeLanes - 2) stage_pair(reinterpret_cast<R *>(v.svstage), SV_CANSR, SV_CANSR_LO, os.g[4]);
-        for (int q = P.upd_phase + 1; q <= P.push_phase; ++q) {
-            if (q == stim_q && lane == 0 && (ot >> 5) == stim_warp)
-                os.stim[par ^ 1] = stimulus(a.dyn[cell], os.t, ri + 1);
-            ode_phase<T, R>(v.off, q, reg, ot);
-            ode_bar();
-        }
-        // (no warp idle in either phase: the stimulus formed here)
-        if (stim_q < 0 && ot == 0) os.stim[par ^ 1] = stimulus(a.dyn[cell], os.t, ri + 1);
+        phases();
+        if (clock) set_stim(ri + 1);
+        ode_bar();
         // (no push after the launch's last step: no one would wait for those bytes, and a CTA
         // must not exit while stores into its shared memory may still be in flight)
         if (s + 1 < a.n_steps)
             push_sv<FP64>(v.svbuf, v.svstage, par ^ 1, v.mbar + 16u + 8u * (uint32_t)(par ^ 1), v.w, ot);
-        // the new globals become the old ones of the next step's increments (read after the
-        // next step's ode_bar; no phase after this point reads XS_G)
-        if (ot < kNumGlobals) X[XS_G + ot] = X[XS_GN + ot];
-        // off the critical path: the phases the SSA does not need
-        for (int q = P.push_phase + 1; q < P.n_phases; ++q) {
-            ode_phase<T, R>(v.off, q, reg, ot);
-            ode_bar();
-        }
     }
     // carry of the last step's fluxes, globals and counters back to the cell block
     if (a.n_steps > 0 && !stopped) {
@@ -714,17 +790,17 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         mbar_wait(v.mbar + 8u * (uint32_t)((s_stop - 1) & 1), (uint32_t)((s_stop - 1) >> 1) & 1u);
         mbar_wait(v.mbar + 8u * (uint32_t)(s_stop & 1), (uint32_t)(s_stop >> 1) & 1u);
     }
-    if (a.n_steps > 0)
-        reduce_partials<FP64, T>(v.part + ((a.n_steps - 1) & 1) * pslot, v.w.n_cta_cell * kMaxWarps, ot >> 5, lane, os.sums, X);
+    if (a.n_steps > 0 && warp >= 2)
+        reduce_partials(v.part + ((a.n_steps - 1) & 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp - 2, lane, os.sums, X);
     ode_bar();
     CellDyn &d = a.dyn[cell];
     for (int i = ot; i < kNumGlobals; i += kOdeLanes) d.g[i] = os.g[i];
+    if (clock) d.t = time;
     if (ot == 0) {
         d.sum_jlcc = os.sums[0];
         d.sum_clch = os.sums[1];
         d.sum_jtr = os.sums[2];
         d.sum_jxfer = os.sums[3];
-        d.t = os.t;
         d.step = step0 + (uint64_t)a.n_steps;
         if (os.status != 0) atomicCAS(&a.status[cell], 0, os.status);
     }
@@ -952,15 +1028,19 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                 record_pass<R>(a, w, cell, r_idx, beg, end, lane, tile);
             // The warp partial, pushed straight into the leader's slot (rank, warp): the leader
             // sums the cell's warp partials in slot order (no reduction on this side).
-            const Partial pv = acc.warp_total();
+            const Partial<FP64> pv = acc.warp_total();
             if (lane == 0) {
-                // two 16-byte asynchronous stores that count themselves off the leader's mbarrier
-                // of this parity (the warp goes on without waiting for them to land)
-                Partial *dst = v.part + par * pslot + w.rank_in_cell * kMaxWarps + warp;
+                // 16-byte asynchronous stores that count themselves off the leader's mbarrier of this
+                // parity (the warp goes on without waiting for them to land)
+                Partial<FP64> *dst = v.part + par * pslot + w.rank_in_cell * kMaxWarps + warp;
                 const uint32_t rd = map_rank(dst, (uint32_t)w.first);
                 const uint32_t rm = map_rank_addr(v.mbar + 8u * (uint32_t)par, (uint32_t)w.first);
-                st_async(rd, make_uint4(lo_of(pv.v[0]), hi_of(pv.v[0]), lo_of(pv.v[1]), hi_of(pv.v[1])), rm);
-                st_async(rd + 16u, make_uint4(lo_of(pv.v[2]), hi_of(pv.v[2]), lo_of(pv.v[3]), hi_of(pv.v[3])), rm);
+                if constexpr (FP64) {
+                    st_async(rd, make_uint4(lo_of(pv.v[0]), hi_of(pv.v[0]), lo_of(pv.v[1]), hi_of(pv.v[1])), rm);
+                    st_async(rd + 16u, make_uint4(lo_of(pv.v[2]), hi_of(pv.v[2]), lo_of(pv.v[3]), hi_of(pv.v[3])), rm);
+                } else {
+                    st_async(rd, make_uint4(__float_as_uint(pv.j), __float_as_uint(pv.x), __float_as_uint(pv.t), (uint32_t)pv.cl), rm);
+                }
             }
         }
     }
@@ -1049,9 +1129,9 @@ __global__ void __launch_bounds__(FP64 ? kMaxThreadsFp64 : kMaxThreads, 1) engin
         // The leader's warp-partial slots start at zero (slots of warps a CTA does not have stay
         // so); the cell's CTAs write them only after the first cluster barrier of the steps.
         if (v.leader) {
-            double *pz = &v.part[0].v[0];
-            const int nz = 2 * a.max_cta_cell * kMaxWarps * 4;
-            for (int i = (int)threadIdx.x; i < nz; i += (int)blockDim.x) pz[i] = 0.0;
+            uint4 *pz = reinterpret_cast<uint4 *>(v.part);
+            const int nz = 2 * a.max_cta_cell * kMaxWarps * (int)(sizeof(Partial<FP64>) / 16);
+            for (int i = (int)threadIdx.x; i < nz; i += (int)blockDim.x) pz[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         step0 = a.dyn[cell].step;
         if (!v.ode_thread) {

@@ -40,7 +40,7 @@ enum SvIndex {
 
 // Per-cell constant block: the parameters and the reference's Constants (GW_utils.tpp:67-116),
 // computed on the host in FP64 exactly as the reference does.
-constexpr int kOdeConstCap = 256;  // per-cell constants of the global-step lane program
+constexpr int kOdeConstCap = 320;  // per-cell constants of the global-step lane program
 
 struct CellStatic {
     gw_params p;

@@ -158,18 +158,6 @@ __device__ __forceinline__ uint32_t map_rank_addr(uint32_t a, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_remote(uint32_t addr, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-__device__ __forceinline__ void st_remote(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_remote(uint32_t addr, uint4 v) {  // addr 16-byte aligned
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z),
-                 "r"(v.w)
-                 : "memory");
-}
-
 // mbarriers (shared-memory arrival/transaction barriers) and asynchronous remote stores.  An
 // st.async writes 16 bytes into a CTA of the cluster and, once the bytes are there, counts them off
 // that CTA's mbarrier (complete_tx); the issuing thread does not wait for it, and a later fence

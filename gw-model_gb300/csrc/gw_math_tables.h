@@ -2,210 +2,157 @@
 #pragma once
 namespace gw {
 namespace math64 {
-constexpr double kLn2By64Hi = 0x1.62e42fefa39efp-7;  // ln2/64, lead
-constexpr double kLn2By64Lo = 0x1.abc9e3b39803fp-62;  // ln2/64 - lead
-constexpr double k64ByLn2 = 0x1.71547652b82fep+6;
-constexpr double kLn2Hi = 0x1.62e42fefa39efp-1;
-constexpr double kLn2Lo = 0x1.abc9e3b39803fp-56;
-// 2^(j/64): {lead, trail}
+constexpr unsigned long long kLog2e63 = 0xb8aa3b295c17f0bcull;  // 1/ln2, 63 fractional bits
+constexpr unsigned long long kLn2 = 0xb17217f7d1cf79acull;      // ln2, 64 fractional bits
+// 2048 times that, as two words
+constexpr unsigned long long kLn2BiasHi = 0x58bull, kLn2BiasLo = 0x90bfbe8e7bcd6000ull;
+constexpr unsigned long long kExp1 = 0xb17217f7d1cf79acull;  // ln2^1/1!, 64 fractional bits
+constexpr unsigned long long kExp2 = 0x3d7f7bff058b1d51ull;  // ln2^2/2!, 64 fractional bits
+constexpr unsigned long long kExp3 = 0xe35846b82505fc6ull;  // ln2^3/3!, 64 fractional bits
+constexpr unsigned int kExp4 = 0x276556eu;  // ln2^4/4!, 32 fractional bits
+constexpr unsigned int kExp5 = 0x576200u;  // ln2^5/5!, 32 fractional bits
+constexpr long long kLog1 = 4611686018427387904ll;  // (-1)^0/1, 62 fractional bits
+constexpr long long kLog2 = -2305843009213693952ll;  // (-1)^1/2, 62 fractional bits
+constexpr long long kLog3 = 1537228672809129301ll;  // (-1)^2/3, 62 fractional bits
+constexpr int kLog4 = -268435456;  // (-1)^3/4, 30 fractional bits
+constexpr int kLog5 = 214748365;  // (-1)^4/5, 30 fractional bits
+constexpr int kLog6 = -178956971;  // (-1)^5/6, 30 fractional bits
+constexpr int kLog7 = 153391689;  // (-1)^6/7, 30 fractional bits
+// 2^(j/256), 63 fractional bits
 #define GW_EXP2_TABLE \
     { \
-        {0x1.0000000000000p+0, 0x0.0p+0}, \
-        {0x1.02c9a3e778061p+0, -0x1.19083535b085dp-56}, \
-        {0x1.059b0d3158574p+0, 0x1.d73e2a475b465p-55}, \
-        {0x1.0874518759bc8p+0, 0x1.186be4bb284ffp-57}, \
-        {0x1.0b5586cf9890fp+0, 0x1.8a62e4adc610bp-54}, \
-        {0x1.0e3ec32d3d1a2p+0, 0x1.03a1727c57b53p-59}, \
-        {0x1.11301d0125b51p+0, -0x1.6c51039449b3ap-54}, \
-        {0x1.1429aaea92de0p+0, -0x1.32fbf9af1369ep-54}, \
-        {0x1.172b83c7d517bp+0, -0x1.19041b9d78a76p-55}, \
-        {0x1.1a35beb6fcb75p+0, 0x1.e5b4c7b4968e4p-55}, \
-        {0x1.1d4873168b9aap+0, 0x1.e016e00a2643cp-54}, \
-        {0x1.2063b88628cd6p+0, 0x1.dc775814a8495p-55}, \
-        {0x1.2387a6e756238p+0, 0x1.9b07eb6c70573p-54}, \
-        {0x1.26b4565e27cddp+0, 0x1.2bd339940e9d9p-55}, \
-        {0x1.29e9df51fdee1p+0, 0x1.612e8afad1255p-55}, \
-        {0x1.2d285a6e4030bp+0, 0x1.0024754db41d5p-54}, \
-        {0x1.306fe0a31b715p+0, 0x1.6f46ad23182e4p-55}, \
-        {0x1.33c08b26416ffp+0, 0x1.32721843659a6p-54}, \
-        {0x1.371a7373aa9cbp+0, -0x1.63aeabf42eae2p-54}, \
-        {0x1.3a7db34e59ff7p+0, -0x1.5e436d661f5e3p-56}, \
-        {0x1.3dea64c123422p+0, 0x1.ada0911f09ebcp-55}, \
-        {0x1.4160a21f72e2ap+0, -0x1.ef3691c309278p-58}, \
-        {0x1.44e086061892dp+0, 0x1.89b7a04ef80d0p-59}, \
-        {0x1.486a2b5c13cd0p+0, 0x1.3c1a3b69062f0p-56}, \
-        {0x1.4bfdad5362a27p+0, 0x1.d4397afec42e2p-56}, \
-        {0x1.4f9b2769d2ca7p+0, -0x1.4b309d25957e3p-54}, \
-        {0x1.5342b569d4f82p+0, -0x1.07abe1db13cadp-55}, \
-        {0x1.56f4736b527dap+0, 0x1.9bb2c011d93adp-54}, \
-        {0x1.5ab07dd485429p+0, 0x1.6324c054647adp-54}, \
-        {0x1.5e76f15ad2148p+0, 0x1.ba6f93080e65ep-54}, \
-        {0x1.6247eb03a5585p+0, -0x1.383c17e40b497p-54}, \
-        {0x1.6623882552225p+0, -0x1.bb60987591c34p-54}, \
-        {0x1.6a09e667f3bcdp+0, -0x1.bdd3413b26456p-54}, \
-        {0x1.6dfb23c651a2fp+0, -0x1.bbe3a683c88abp-57}, \
-        {0x1.71f75e8ec5f74p+0, -0x1.16e4786887a99p-55}, \
-        {0x1.75feb564267c9p+0, -0x1.0245957316dd3p-54}, \
-        {0x1.7a11473eb0187p+0, -0x1.41577ee04992fp-55}, \
-        {0x1.7e2f336cf4e62p+0, 0x1.05d02ba15797ep-56}, \
-        {0x1.82589994cce13p+0, -0x1.d4c1dd41532d8p-54}, \
-        {0x1.868d99b4492edp+0, -0x1.fc6f89bd4f6bap-54}, \
-        {0x1.8ace5422aa0dbp+0, 0x1.6e9f156864b27p-54}, \
-        {0x1.8f1ae99157736p+0, 0x1.5cc13a2e3976cp-55}, \
-        {0x1.93737b0cdc5e5p+0, -0x1.75fc781b57ebcp-57}, \
-        {0x1.97d829fde4e50p+0, -0x1.d185b7c1b85d1p-54}, \
-        {0x1.9c49182a3f090p+0, 0x1.c7c46b071f2bep-56}, \
-        {0x1.a0c667b5de565p+0, -0x1.359495d1cd533p-54}, \
-        {0x1.a5503b23e255dp+0, -0x1.d2f6edb8d41e1p-54}, \
-        {0x1.a9e6b5579fdbfp+0, 0x1.0fac90ef7fd31p-54}, \
-        {0x1.ae89f995ad3adp+0, 0x1.7a1cd345dcc81p-54}, \
-        {0x1.b33a2b84f15fbp+0, -0x1.2805e3084d708p-57}, \
-        {0x1.b7f76f2fb5e47p+0, -0x1.5584f7e54ac3bp-56}, \
-        {0x1.bcc1e904bc1d2p+0, 0x1.23dd07a2d9e84p-55}, \
-        {0x1.c199bdd85529cp+0, 0x1.11065895048ddp-55}, \
-        {0x1.c67f12e57d14bp+0, 0x1.2884dff483cadp-54}, \
-        {0x1.cb720dcef9069p+0, 0x1.503cbd1e949dbp-56}, \
-        {0x1.d072d4a07897cp+0, -0x1.cbc3743797a9cp-54}, \
-        {0x1.d5818dcfba487p+0, 0x1.2ed02d75b3707p-55}, \
-        {0x1.da9e603db3285p+0, 0x1.c2300696db532p-54}, \
-        {0x1.dfc97337b9b5fp+0, -0x1.1a5cd4f184b5cp-54}, \
-        {0x1.e502ee78b3ff6p+0, 0x1.39e8980a9cc8fp-55}, \
-        {0x1.ea4afa2a490dap+0, -0x1.e9c23179c2893p-54}, \
-        {0x1.efa1bee615a27p+0, 0x1.dc7f486a4b6b0p-54}, \
-        {0x1.f50765b6e4540p+0, 0x1.9d3e12dd8a18bp-54}, \
-        {0x1.fa7c1819e90d8p+0, 0x1.74853f3a5931ep-55}, \
+        0x8000000000000000ull, 0x8058d7d2d5e5f6b1ull, 0x80b1ed4fd999ab6cull, 0x810b40a1d81406d4ull, \
+        0x8164d1f3bc030773ull, 0x81bea1708dde6056ull, 0x8218af4373fc25ecull, 0x8272fb97b2a5894cull, \
+        0x82cd8698ac2ba1d7ull, 0x83285071e0fc4547ull, 0x8383594eefb6ee37ull, 0x83dea15b9541b132ull, \
+        0x843a28c3acde4046ull, 0x8495efb3303efd30ull, 0x84f1f656379c1a29ull, 0x854e3cd8f9c8c95dull, \
+        0x85aac367cc487b15ull, 0x86078a2f23642a9full, 0x8664915b923fba04ull, 0x86c1d919caef5c88ull, \
+        0x871f61969e8d1010ull, 0x877d2afefd4e256cull, 0x87db357ff698d792ull, 0x88398146b919f1d4ull, \
+        0x88980e8092da8527ull, 0x88f6dd5af155ac6bull, 0x8955ee03618e5fddull, 0x89b540a7902557a4ull, \
+        0x8a14d575496efd9aull, 0x8a74ac9a79896e47ull, 0x8ad4c6452c728924ull, 0x8b3522a38e1e1032ull, \
+        0x8b95c1e3ea8bd6e7ull, 0x8bf6a434adde0085ull, 0x8c57c9c4646f4ddeull, 0x8cb932c1bae97a95ull, \
+        0x8d1adf5b7e5ba9e6ull, 0x8d7ccfc09c50e2f8ull, 0x8ddf042022e69cd6ull, 0x8e417ca940e35a01ull, \
+        0x8ea4398b45cd53c0ull, 0x8f073af5a2013520ull, 0x8f6a8117e6c8e5c4ull, 0x8fce0c21c6726481ull, \
+        0x9031dc431466b1dcull, 0x9095f1abc540ca6bull, 0x90fa4c8beee4b12bull, 0x915eed13c89689d3ull, \
+        0x91c3d373ab11c336ull, 0x9228ffdc10a051adull, 0x928e727d9531f9acull, 0x92f42b88f673aa7cull, \
+        0x935a2b2f13e6e92cull, 0x93c071a0eef94bc1ull, 0x9426ff0fab1c04b6ull, 0x948dd3ac8ddb7ed3ull, \
+        0x94f4efa8fef70961ull, 0x955c5336887894d5ull, 0x95c3fe86d6cc7fefull, 0x962bf1cbb8d97560ull, \
+        0x96942d3720185a00ull, 0x96fcb0fb20ac4ba3ull, 0x97657d49f17ab08eull, 0x97ce9255ec4357abull, \
+        0x9837f0518db8a96full, 0x98a1976f7597e996ull, 0x990b87e266c189aaull, 0x9975c1dd47518c77ull, \
+        0x99e0459320b7fa65ull, 0x9a4b13371fd166caull, 0x9ab62afc94ff864aull, 0x9b218d16f441d63dull, \
+        0x9b8d39b9d54e5539ull, 0x9bf93118f3aa4cc1ull, 0x9c6573682ec32c2dull, 0x9cd200db8a0774cbull, \
+        0x9d3ed9a72cffb751ull, 0x9dabfdff6367a2aaull, 0x9e196e189d472420ull, 0x9e872a276f0b98ffull, \
+        0x9ef5326091a111aeull, 0x9f6386f8e28ba651ull, 0x9fd228256400dd06ull, 0xa041161b3d0121beull, \
+        0xa0b0510fb9714fc2ull, 0xa11fd9384a344cf7ull, 0xa18faeca8544b6e4ull, 0xa1ffd1fc25cea188ull, \
+        0xa27043030c496819ull, 0xa2e102153e918f9eull, 0xa3520f68e802bb93ull, 0xa3c36b345991b47cull, \
+        0xa43515ae09e6809eull, 0xa4a70f0c95768ec5ull, 0xa5195786be9ef339ull, 0xa58bef536dbeb6eeull, \
+        0xa5fed6a9b15138eaull, 0xa6720dc0be08a20cull, 0xa6e594cfeee86b1eull, 0xa7596c0ec55ff55bull, \
+        0xa7cd93b4e965356aull, 0xa8420bfa298f70d1ull, 0xa8b6d5167b320e09ull, 0xa92bef41fa77771bull, \
+        0xa9a15ab4ea7c0ef8ull, 0xaa1717a7b5693979ull, 0xaa8d2652ec907629ull, 0xab0386ef48868de1ull, \
+        0xab7a39b5a93ed337ull, 0xabf13edf162675e9ull, 0xac6896a4be3fe929ull, 0xace0413ff83e5d04ull, \
+        0xad583eea42a14ac6ull, 0xadd08fdd43d01491ull, 0xae493452ca35b80eull, 0xaec22c84cc5c9465ull, \
+        0xaf3b78ad690a4375ull, 0xafb51906e75b8661ull, 0xb02f0dcbb6e04584ull, 0xb0a957366fb7a3c9ull, \
+        0xb123f581d2ac2590ull, 0xb19ee8e8c94feb09ull, 0xb21a31a66618fe3bull, 0xb295cff5e47db4a4ull, \
+        0xb311c412a9112489ull, 0xb38e0e38419fae18ull, 0xb40aaea2654b9841ull, 0xb487a58cf4a9c180ull, \
+        0xb504f333f9de6484ull, 0xb58297d3a8b9f0d2ull, 0xb60093a85ed5f76cull, 0xb67ee6eea3b22b8full, \
+        0xb6fd91e328d17791ull, 0xb77c94c2c9d725e9ull, 0xb7fbefca8ca41e7cull, 0xb87ba337a1743834ull, \
+        0xb8fbaf4762fb9ee9ull, 0xb97c143756844dbfull, 0xb9fcd2452c0b9debull, 0xba7de9aebe5fea09ull, \
+        0xbaff5ab2133e45fbull, 0xbb81258d5b704b6full, 0xbc034a7ef2e9fb0dull, 0xbc85c9c560e7b269ull, \
+        0xbd08a39f580c36bfull, 0xbd8bd84bb67ed483ull, 0xbe0f6809860993e2ull, 0xbe935317fc378238ull, \
+        0xbf1799b67a731083ull, 0xbf9c3c248e2486f8ull, 0xc0213aa1f0d08db0ull, 0xc0a6956e8836ca8dull, \
+        0xc12c4cca66709456ull, 0xc1b260f5ca0fbb33ull, 0xc238d2311e3d6673ull, 0xc2bfa0bcfad907c9ull, \
+        0xc346ccda24976407ull, 0xc3ce56c98d21b15dull, 0xc4563ecc5334cb33ull, 0xc4de8523c2c07baaull, \
+        0xc5672a115506daddull, 0xc5f02dd6b0bbc3d9ull, 0xc67990b5aa245f79ull, 0xc70352f04336c51eull, \
+        0xc78d74c8abb9b15dull, 0xc817f681416452b2ull, 0xc8a2d85c8ffe2c45ull, 0xc92e1a9d517f0eccull, \
+        0xc9b9bd866e2f27a3ull, 0xca45c15afcc72624ull, 0xcad2265e4290774eull, 0xcb5eecd3b38597c9ull, \
+        0xcbec14fef2727c5dull, 0xcc799f23d11510e5ull, 0xcd078b86503dcdd2ull, 0xcd95da6a9ff06445ull, \
+        0xce248c151f8480e4ull, 0xceb3a0ca5dc6a55dull, 0xcf4318cf191918c1ull, 0xcfd2f4683f94eeb5ull, \
+        0xd06333daef2b2595ull, 0xd0f3d76c75c5db8dull, 0xd184df6251699ac6ull, 0xd2164c023056bcabull, \
+        0xd2a81d91f12ae45aull, 0xd33a5457a3029054ull, 0xd3ccf099859ac379ull, 0xd45ff29e0972c561ull, \
+        0xd4f35aabcfedfa1full, 0xd5872909ab75d18aull, 0xd61b5dfe9f9bce07ull, 0xd6aff9d1e13ba2feull, \
+        0xd744fccad69d6af4ull, 0xd7da67311797f56aull, 0xd870394c6db32c84ull, 0xd9067364d44a929cull, \
+        0xd99d15c278afd7b6ull, 0xda3420adba4d8704ull, 0xdacb946f2ac9cc72ull, 0xdb63714f8e295255ull, \
+        0xdbfbb797daf23755ull, 0xdc9467913a4f1c92ull, 0xdd2d818508324c20ull, 0xddc705bcd378f7f0ull, \
+        0xde60f4825e0e9124ull, 0xdefb4e1f9d1037f2ull, 0xdf9612deb8f04420ull, 0xe031430a0d99e627ull, \
+        0xe0ccdeec2a94e111ull, 0xe168e6cfd3295d23ull, 0xe2055afffe83d369ull, 0xe2a23bc7d7d91226ull, \
+        0xe33f8972be8a5a51ull, 0xe3dd444c46499619ull, 0xe47b6ca0373da88dull, 0xe51a02ba8e26d681ull, \
+        0xe5b906e77c8348a8ull, 0xe658797368b3a717ull, 0xe6f85aaaee1fce22ull, 0xe798aadadd5b9cbfull, \
+        0xe8396a503c4bdc68ull, 0xe8da9958464b42abull, 0xe97c38406c4f8c57ull, 0xea1e4756550eb27bull, \
+        0xeac0c6e7dd24392full, 0xeb63b74317369840ull, 0xec0718b64c1cbddcull, 0xecaaeb8ffb03ab41ull, \
+        0xed4f301ed9942b84ull, 0xedf3e6b1d418a491ull, 0xee990f980da3025bull, 0xef3eab20e032bc6bull, \
+        0xefe4b99bdcdaf5cbull, 0xf08b3b58cbe8b76aull, 0xf13230a7ad094509ull, 0xf1d999d8b7708cc1ull, \
+        0xf281773c59ffb13aull, 0xf329c9233b6bae9cull, 0xf3d28fde3a641a5bull, 0xf47bcbbe6db9fddfull, \
+        0xf5257d152486cc2cull, 0xf5cfa433e6537290ull, 0xf67a416c733f846eull, 0xf7255510c4288239ull, \
+        0xf7d0df730ad13bb9ull, 0xf87ce0e5b2094d9cull, 0xf92959bb5dd4ba74ull, 0xf9d64a46eb939f35ull, \
+        0xfa83b2db722a033aull, 0xfb3193cc4227c3f4ull, 0xfbdfed6ce5f09c49ull, 0xfc8ec01121e447bbull, \
+        0xfd3e0c0cf486c175ull, 0xfdedd1b496a89f35ull, 0xfe9e115c7b8f884cull, 0xff4ecb59511ec8a5ull, \
     }
-// j = 0..127: {invF_j, lead(-log(invF_j)), trail}, F_j = 1 + (j + 1/2)/128
+// {c_j, -log(c_j / 2^16) with 64 fractional bits}
 #define GW_LOG_TABLE \
     { \
-        {0x1.fe01fe01fe020p-1, 0x1.ff00aa2b10ba0p-9, 0x1.2821ad5a6d357p-63}, \
-        {0x1.fa11caa01fa12p-1, 0x1.7dc475f810a69p-7, 0x1.74944bc161072p-61}, \
-        {0x1.f6310aca0dbb5p-1, 0x1.3cea44346a584p-6, -0x1.865ad48159d00p-61}, \
-        {0x1.f25f644230ab5p-1, 0x1.b9fc027af919ap-6, -0x1.90ae69229dc86p-60}, \
-        {0x1.ee9c7f8458e02p-1, 0x1.1b0d98923d97fp-5, -0x1.74d7444dd6241p-59}, \
-        {0x1.eae807aba01ebp-1, 0x1.58a5bafc8e4d3p-5, -0x1.cab8569c56e40p-64}, \
-        {0x1.e741aa59750e4p-1, 0x1.95c830ec8e3f2p-5, 0x1.eb41d00a417e9p-60}, \
-        {0x1.e3a9179dc1a73p-1, 0x1.d276b8adb0b56p-5, 0x1.078f14c95ff53p-59}, \
-        {0x1.e01e01e01e01ep-1, 0x1.075983598e471p-4, 0x1.006d2999e22dcp-58}, \
-        {0x1.dca01dca01dcap-1, 0x1.253f62f0a1417p-4, 0x1.1f6d34e01d981p-61}, \
-        {0x1.d92f2231e7f8ap-1, 0x1.42edcbea646eep-4, -0x1.511583653349bp-58}, \
-        {0x1.d5cac807572b2p-1, 0x1.60658a93750c4p-4, -0x1.f108b1d8436d3p-59}, \
-        {0x1.d272ca3fc5b1ap-1, 0x1.7da766d7b12d0p-4, 0x1.a2240644d7da2p-59}, \
-        {0x1.cf26e5c44bfc6p-1, 0x1.9ab42462033aep-4, -0x1.a099e1c184e8ep-59}, \
-        {0x1.cbe6d9601cbe7p-1, 0x1.b78c82bb0eda0p-4, -0x1.3ef0e61f9b03cp-58}, \
-        {0x1.c8b265afb8a42p-1, 0x1.d4313d66cb35dp-4, 0x1.b90dd951d90fap-58}, \
-        {0x1.c5894d10d4986p-1, 0x1.f0a30c01162a4p-4, 0x1.8be64b8b7759bp-59}, \
-        {0x1.c26b5392ea01cp-1, 0x1.0671512ca596fp-3, -0x1.2f39b81479b67p-58}, \
-        {0x1.bf583ee868d8bp-1, 0x1.14785846742acp-3, 0x1.94409f1d3f83ap-60}, \
-        {0x1.bc4fd65883e7bp-1, 0x1.2266f190a5acdp-3, -0x1.dab840e7f6177p-57}, \
-        {0x1.b951e2b18ff23p-1, 0x1.303d718e47fd5p-3, -0x1.b5ae71f658247p-57}, \
-        {0x1.b65e2e3beee05p-1, 0x1.3dfc2b0ecc62ap-3, 0x1.ba62b8c13f7f4p-57}, \
-        {0x1.b37484ad806cep-1, 0x1.4ba36f39a55e5p-3, -0x1.f767e433c98aap-57}, \
-        {0x1.b094b31d922a4p-1, 0x1.59338d9982085p-3, 0x1.8d16eaaba9419p-57}, \
-        {0x1.adbe87f94905ep-1, 0x1.66acd4272ad51p-3, -0x1.9201c9c3d5165p-59}, \
-        {0x1.aaf1d2f87ebfdp-1, 0x1.740f8f54037a3p-3, 0x1.6d9bf9d57b326p-58}, \
-        {0x1.a82e65130e159p-1, 0x1.815c0a14357e9p-3, 0x1.141b7f8c5fa9ep-58}, \
-        {0x1.a574107688a4ap-1, 0x1.8e928de886d41p-3, 0x1.2589eb96a6240p-59}, \
-        {0x1.a2c2a87c51ca0p-1, 0x1.9bb362e7dfb85p-3, -0x1.51439c1ff83e7p-58}, \
-        {0x1.a01a01a01a01ap-1, 0x1.a8becfc882f19p-3, -0x1.a8c37918c39ebp-58}, \
-        {0x1.9d79f176b682dp-1, 0x1.b5b519e8fb5a6p-3, -0x1.d5d8023e61e5fp-57}, \
-        {0x1.9ae24ea5510dap-1, 0x1.c2968558c18c2p-3, 0x1.6108e3ae024acp-60}, \
-        {0x1.9852f0d8ec0ffp-1, 0x1.cf6354e09c5ddp-3, 0x1.339a07d55b696p-57}, \
-        {0x1.95cbb0be377aep-1, 0x1.dc1bca0abec7bp-3, 0x1.c698a33316dfbp-58}, \
-        {0x1.934c67f9b2ce6p-1, 0x1.e8c0252aa5a60p-3, -0x1.dc074737f9135p-60}, \
-        {0x1.90d4f120190d5p-1, 0x1.f550a564b7b37p-3, -0x1.13a09202fe73dp-57}, \
-        {0x1.8e6527af1373fp-1, 0x1.00e6c45ad501dp-2, -0x1.3b9568ff6feadp-57}, \
-        {0x1.8bfce8062ff3ap-1, 0x1.071b85fcd590dp-2, 0x1.08b83fcbdef40p-57}, \
-        {0x1.899c0f601899cp-1, 0x1.0d46b579ab74bp-2, 0x1.21f640e1e5ec9p-56}, \
-        {0x1.87427bcc092b9p-1, 0x1.136870293a8b0p-2, 0x1.86cc531dba494p-57}, \
-        {0x1.84f00c2780614p-1, 0x1.1980d2dd4236fp-2, -0x1.02c2e4f1b2eb9p-56}, \
-        {0x1.82a4a0182a4a0p-1, 0x1.1f8ff9e48a2f3p-2, -0x1.93fbf3418960dp-57}, \
-        {0x1.8060180601806p-1, 0x1.2596010df763ap-2, -0x1.9eed8ae0ebd3cp-59}, \
-        {0x1.7e225515a4f1dp-1, 0x1.2b9303ab89d25p-2, -0x1.85ad7f614ab51p-58}, \
-        {0x1.7beb3922e017cp-1, 0x1.31871c9544185p-2, -0x1.ea3598981366fp-57}, \
-        {0x1.79baa6bb6398bp-1, 0x1.3772662bfd85cp-2, 0x1.02a7589fba088p-57}, \
-        {0x1.77908119ac60dp-1, 0x1.3d54fa5c1f710p-2, 0x1.53668e578d9cdp-58}, \
-        {0x1.756cac201756dp-1, 0x1.432ef2a04e813p-2, -0x1.83262e2b59206p-57}, \
-        {0x1.734f0c541fe8dp-1, 0x1.49006804009d0p-2, -0x1.bff0d07c5df6dp-59}, \
-        {0x1.713786d9c7c09p-1, 0x1.4ec9732600269p-2, -0x1.1aa87d977dc5ep-56}, \
-        {0x1.6f26016f26017p-1, 0x1.548a2c3add263p-2, -0x1.58ce7bf1846eep-56}, \
-        {0x1.6d1a62681c861p-1, 0x1.5a42ab0f4cfe2p-2, -0x1.c6bcb7dee9a3dp-56}, \
-        {0x1.6b1490aa31a3dp-1, 0x1.5ff3070a793d4p-2, -0x1.063077d7e37b7p-56}, \
-        {0x1.691473a88d0c0p-1, 0x1.659b57303e1f2p-2, 0x1.db0af8efb83c7p-62}, \
-        {0x1.6719f3601671ap-1, 0x1.6b3bb2235943dp-2, 0x1.957a93326784dp-56}, \
-        {0x1.6524f853b4aa3p-1, 0x1.70d42e2789236p-2, 0x1.ee99bf7143954p-56}, \
-        {0x1.63356b88ac0dep-1, 0x1.7664e1239dbcfp-2, -0x1.d6d5d64f5daf8p-57}, \
-        {0x1.614b36831ae94p-1, 0x1.7bede0a37afbfp-2, -0x1.6783cb9801a5bp-56}, \
-        {0x1.5f66434292dfcp-1, 0x1.816f41da0d495p-2, 0x1.76dc35fb48fe4p-56}, \
-        {0x1.5d867c3ece2a5p-1, 0x1.86e919a330ba1p-2, -0x1.700c9d2029045p-56}, \
-        {0x1.5babcc647fa91p-1, 0x1.8c5b7c858b48bp-2, 0x1.d754b0205fa6cp-56}, \
-        {0x1.59d61f123ccaap-1, 0x1.91c67eb45a83ep-2, 0x1.5e3ea3b96a3dfp-57}, \
-        {0x1.5805601580560p-1, 0x1.972a341135159p-2, -0x1.5a3f62db48f27p-56}, \
-        {0x1.56397ba7c52e2p-1, 0x1.9c86b02dc0862p-2, 0x1.7e81149622bdfp-56}, \
-        {0x1.54725e6bb82fep-1, 0x1.a1dc064d5b995p-2, 0x1.a0128698ba0b8p-56}, \
-        {0x1.52aff56a8054bp-1, 0x1.a72a4966bd9e9p-2, 0x1.529dac69f61f1p-56}, \
-        {0x1.50f22e111c4c5p-1, 0x1.ac718c258b0e5p-2, 0x1.682c7ade8dee3p-56}, \
-        {0x1.4f38f62dd4c9bp-1, 0x1.b1b1e0ebdfc5ap-2, -0x1.0ee1a7dd74ea6p-58}, \
-        {0x1.4d843bedc2c4cp-1, 0x1.b6eb59d3cf35cp-2, 0x1.1524332cd95c4p-56}, \
-        {0x1.4bd3edda68fe1p-1, 0x1.bc1e08b0dad0ap-2, -0x1.385e3e3ea99a8p-58}, \
-        {0x1.4a27fad76014ap-1, 0x1.c149ff115f027p-2, 0x1.46868de7f39f6p-57}, \
-        {0x1.4880522014880p-1, 0x1.c66f4e3ff6ff9p-2, -0x1.82947258b6889p-58}, \
-        {0x1.46dce34596066p-1, 0x1.cb8e0744d7acap-2, 0x1.c5bbc32ef5aebp-56}, \
-        {0x1.453d9e2c776cap-1, 0x1.d0a63ae721e64p-2, 0x1.4acce112c40f2p-57}, \
-        {0x1.43a2730abee4dp-1, 0x1.d5b7f9ae2c684p-2, 0x1.4841807b53f96p-57}, \
-        {0x1.420b5265e5951p-1, 0x1.dac353e2c5955p-2, -0x1.abc65a3f2f204p-56}, \
-        {0x1.40782d10e6566p-1, 0x1.dfc859906d5b5p-2, 0x1.51e1399f96398p-56}, \
-        {0x1.3ee8f42a5af07p-1, 0x1.e4c71a8687704p-2, -0x1.34c36e0f052b9p-56}, \
-        {0x1.3d5d991aa75c6p-1, 0x1.e9bfa659861f5p-2, -0x1.de45038241ecfp-56}, \
-        {0x1.3bd60d9232955p-1, 0x1.eeb20c640ddf3p-2, -0x1.81e47141b8404p-56}, \
-        {0x1.3a524387ac822p-1, 0x1.f39e5bc811e5dp-2, 0x1.200e221139873p-59}, \
-        {0x1.38d22d366088ep-1, 0x1.f884a36fe9ec1p-2, 0x1.618ae4f008400p-56}, \
-        {0x1.3755bd1c945eep-1, 0x1.fd64f20f61571p-2, -0x1.b615859d5a349p-62}, \
-        {0x1.35dce5f9f2af8p-1, 0x1.011fab125ff8ap-1, 0x1.4043750211778p-55}, \
-        {0x1.34679ace01346p-1, 0x1.0389eefce633cp-1, 0x1.8aae29a41ba4ap-59}, \
-        {0x1.32f5ced6a1dfap-1, 0x1.05f14bd26459cp-1, 0x1.935b8ee4f9efep-58}, \
-        {0x1.3187758e9ebb6p-1, 0x1.0855c884b450ep-1, 0x1.785826e49f318p-55}, \
-        {0x1.301c82ac40260p-1, 0x1.0ab76bece14d2p-1, 0x1.02936cabac09ap-56}, \
-        {0x1.2eb4ea1fed14bp-1, 0x1.0d163ccb9d6b8p-1, 0x1.6119595d0f3c3p-59}, \
-        {0x1.2d50a012d50a0p-1, 0x1.0f7241c9b497dp-1, 0x1.ba8443b9db19dp-55}, \
-        {0x1.2bef98e5a3711p-1, 0x1.11cb81787ccf8p-1, 0x1.dc70f563f9920p-56}, \
-        {0x1.2a91c92f3c105p-1, 0x1.1422025243d45p-1, 0x1.7e5e3b6a496ecp-55}, \
-        {0x1.293725bb804a5p-1, 0x1.1675cababa60ep-1, -0x1.cb19c15477c8ep-56}, \
-        {0x1.27dfa38a1ce4dp-1, 0x1.18c6e0ff5cf07p-1, -0x1.9a6baf4f4e637p-56}, \
-        {0x1.268b37cd60127p-1, 0x1.1b154b57da29ep-1, 0x1.2770a5c124ab5p-56}, \
-        {0x1.2539d7e9177b2p-1, 0x1.1d610fe677003p-1, 0x1.d27563647963dp-56}, \
-        {0x1.23eb79717605bp-1, 0x1.1faa34b87094cp-1, 0x1.c42f71ef43276p-55}, \
-        {0x1.22a0122a0122ap-1, 0x1.21f0bfc65beecp-1, -0x1.c24f0c9187c92p-57}, \
-        {0x1.21579804855e6p-1, 0x1.2434b6f483934p-1, -0x1.bebb8cf0f6d11p-57}, \
-        {0x1.2012012012012p-1, 0x1.26762013430e0p-1, -0x1.86a95781c6727p-56}, \
-        {0x1.1ecf43c7fb84cp-1, 0x1.28b500df60783p-1, 0x1.813f3f4aaa9a3p-60}, \
-        {0x1.1d8f5672e4abdp-1, 0x1.2af15f02640acp-1, 0x1.ed8322925675ap-56}, \
-        {0x1.1c522fc1ce059p-1, 0x1.2d2b4012edc9dp-1, 0x1.9ae9d3664e355p-55}, \
-        {0x1.1b17c67f2bae3p-1, 0x1.2f62a99509546p-1, -0x1.7dcbcc6300133p-55}, \
-        {0x1.19e0119e0119ep-1, 0x1.3197a0fa7fe6ap-1, 0x1.f6348fb97128fp-57}, \
-        {0x1.18ab083902bdbp-1, 0x1.33ca2ba328994p-1, 0x1.1c6ba66fd0910p-55}, \
-        {0x1.1778a191bd684p-1, 0x1.35fa4edd36ea0p-1, 0x1.727d468096436p-56}, \
-        {0x1.1648d50fc3201p-1, 0x1.38280fe58797fp-1, -0x1.756f4d8a9b974p-57}, \
-        {0x1.151b9a3fdd5c9p-1, 0x1.3a5373e7ebdf9p-1, 0x1.5ce11148e1124p-56}, \
-        {0x1.13f0e8d344724p-1, 0x1.3c7c7fff73206p-1, -0x1.e80db7025bed1p-60}, \
-        {0x1.12c8b89edc0acp-1, 0x1.3ea33936b2f5bp-1, 0x1.f66e975ec9f52p-59}, \
-        {0x1.11a3019a74826p-1, 0x1.40c7a4880dceap-1, 0x1.13c8b79ff2789p-58}, \
-        {0x1.107fbbe011080p-1, 0x1.42e9c6ddf80bfp-1, -0x1.4d411c2cd7cf1p-55}, \
-        {0x1.0f5edfab325a2p-1, 0x1.4509a5133bb0ap-1, -0x1.5701d7ad284a5p-55}, \
-        {0x1.0e40655826011p-1, 0x1.472743f33aaadp-1, -0x1.a930fed5d6b7ep-60}, \
-        {0x1.0d24456359e3ap-1, 0x1.4942a83a2fc07p-1, 0x1.2a18a88ca56b5p-56}, \
-        {0x1.0c0a7868b4171p-1, 0x1.4b5bd6956e273p-1, -0x1.2c7a06beea772p-55}, \
-        {0x1.0af2f722eecb5p-1, 0x1.4d72d3a39fd01p-1, 0x1.01a9a829c011bp-56}, \
-        {0x1.09ddba6af8360p-1, 0x1.4f87a3f5026e9p-1, -0x1.68ca8b1bcea9dp-55}, \
-        {0x1.08cabb37565e2p-1, 0x1.519a4c0ba3446p-1, 0x1.a332128e4a77fp-55}, \
-        {0x1.07b9f29b8eae2p-1, 0x1.53aad05b99b7cp-1, -0x1.7722c14b894e2p-57}, \
-        {0x1.06ab59c7912fbp-1, 0x1.55b9354b40bcep-1, -0x1.1f342e541a63dp-59}, \
-        {0x1.059eea0727586p-1, 0x1.57c57f336f191p-1, 0x1.1eac5c4377e6ep-55}, \
-        {0x1.04949cc1664c5p-1, 0x1.59cfb25fae87fp-1, -0x1.bb94822ace357p-57}, \
-        {0x1.038c6b78247fcp-1, 0x1.5bd7d30e71c73p-1, -0x1.c9649352e8e44p-67}, \
-        {0x1.02864fc7729e9p-1, 0x1.5ddde57149923p-1, 0x1.0fa37d75ef285p-59}, \
-        {0x1.0182436517a37p-1, 0x1.5fe1edad18919p-1, 0x1.92e93de3ce483p-56}, \
-        {0x1.0080402010080p-1, 0x1.61e3efda46467p-1, 0x1.7923604841473p-57}, \
+        {65281ull, 0xff7f551588de02ull}, {64777ull, 0x2fb6debf18dcec2ull}, \
+        {64281ull, 0x4f32c10f02dd34dull}, {63792ull, 0x6e7a009f8646364ull}, \
+        {63310ull, 0x8d8aec49a6ec158ull}, {62836ull, 0xac531d7e47a6a46ull}, \
+        {62369ull, 0xcae148768667548ull}, {61909ull, 0xe933ac58b121f92ull}, \
+        {61455ull, 0x1075993598e4f130ull}, {61008ull, 0x1254062f0a9416feull}, \
+        {60568ull, 0x142e64bec266e772ull}, {60133ull, 0x1606c5a94e854a48ull}, \
+        {59705ull, 0x17dae56d93235379ull}, {59283ull, 0x19abc1463fb43747ull}, \
+        {58867ull, 0x1b79412bcd862a0bull}, {58457ull, 0x1d434cd6730bde4full}, \
+        {58053ull, 0x1f09cbc0254f2124ull}, {57654ull, 0x20cdc825a774d78bull}, \
+        {57260ull, 0x228f2f08d10d590eull}, {56872ull, 0x244cc63215d596e9ull}, \
+        {56489ull, 0x26079d31c99025f7ull}, {56111ull, 0x27bfa061daf8d3afull}, \
+        {55738ull, 0x2974bbe7408dcd1eull}, {55370ull, 0x2b26dbb3463311b5ull}, \
+        {55007ull, 0x2cd5eb84f22b2472ull}, {54649ull, 0x2e81d6ea81dbc97aull}, \
+        {54295ull, 0x302bbe428df456d5ull}, {53946ull, 0x31d25bbd110c8156ull}, \
+        {53601ull, 0x3376d35d10af8c3bull}, {53261ull, 0x3517daf9105eb186ull}, \
+        {52925ull, 0x36b69a3d1f93c8dcull}, {52593ull, 0x385301ab1ce201dfull}, \
+        {52265ull, 0x39ed019c40144a15ull}, {51942ull, 0x3b8347415cbafa1full}, \
+        {51622ull, 0x3d1846a55d36c149ull}, {51306ull, 0x3eaaaeacc54880a2ull}, \
+        {50995ull, 0x40392616dafce571ull}, {50686ull, 0x41c7777f6156459full}, \
+        {50382ull, 0x4351b75e6b0f2c83ull}, {50081ull, 0x44da6d0a5b73442full}, \
+        {49784ull, 0x46603cb750adbd9eull}, {49490ull, 0x47e46879387dd045ull}, \
+        {49200ull, 0x496590437e58e7c1ull}, {48913ull, 0x4ae4f9eae8cd1368ull}, \
+        {48630ull, 0x4c614125741807aeull}, {48349ull, 0x4ddd0a8b1851f320ull}, \
+        {48072ull, 0x4f55969716fc4194ull}, {47798ull, 0x50cc32a82ed25732ull}, \
+        {47528ull, 0x523f720137472b12ull}, {47260ull, 0x53b208c98dd1a3baull}, \
+        {46995ull, 0x55228c0eb74a0b3full}, {46733ull, 0x5690efc3dc8c081dull}, \
+        {46474ull, 0x57fd27c2b2a15488ull}, {46218ull, 0x596727cc1ca9ccd5ull}, \
+        {45965ull, 0x5acee388d6797625ull}, {45714ull, 0x5c35bd8a202af406ull}, \
+        {45467ull, 0x5d98cd48fdcbb4c9ull}, {45222ull, 0x5efae6290860eea4ull}, \
+        {44979ull, 0x605c01768802d770ull}, {44739ull, 0x61baa168dc5b03fdull}, \
+        {44502ull, 0x6316b92165a429d8ull}, {44267ull, 0x6471b6ad17a9762full}, \
+        {44035ull, 0x65ca160468edd914ull}, {43805ull, 0x6721490b8346057full}, \
+        {43577ull, 0x6877489360bed762ull}, {43352ull, 0x69ca8a59af87a85aull}, \
+        {43129ull, 0x6b1c860965281068ull}, {42908ull, 0x6c6d343b3cf98f70ull}, \
+        {42690ull, 0x6dbb0474f7ef76f4ull}, {42474ull, 0x6f07742c37162906ull}, \
+        {42260ull, 0x70527bc457c89ab3ull}, {42048ull, 0x719c139005bfe0f5ull}, \
+        {41838ull, 0x72e433d173cd44a5ull}, {41631ull, 0x742941b9d40e0e43ull}, \
+        {41425ull, 0x756e596b9b469301ull}, {41222ull, 0x76b04af8d697432eull}, \
+        {41020ull, 0x77f23a641dded53full}, {40820ull, 0x79328aa1ece436ffull}, \
+        {40623ull, 0x7a6f96966efc52a9ull}, {40427ull, 0x7bac8e1903b450d8ull}, \
+        {40233ull, 0x7ce7cdf20a61f00dull}, {40041ull, 0x7e214ddbfd2788f3ull}, \
+        {39851ull, 0x7f590583de3e4651ull}, {39662ull, 0x80909389767e73a4ull}, \
+        {39476ull, 0x81c4a37e80e1d6deull}, {39291ull, 0x82f87ce935755ffbull}, \
+        {39108ull, 0x842a704274706af0ull}, {38926ull, 0x855c23f6884894c8ull}, \
+        {38746ull, 0x868be4661b47e680ull}, {38568ull, 0x87b9a8e4fe6bf740ull}, \
+        {38392ull, 0x88e568bc4d87be8dull}, {38217ull, 0x8a10d229263aa70eull}, \
+        {38044ull, 0x8b3a295da2384e51ull}, {37872ull, 0x8c63207fbaf82dc3ull}, \
+        {37702ull, 0x8d89f7ac2836dcb4ull}, {37533ull, 0x8eb064f33de4980bull}, \
+        {37366ull, 0x8fd4a45c537c5805ull}, {37200ull, 0x90f86fe32e775f14ull}, \
+        {37036ull, 0x9219ff7a52519b1bull}, {36873ull, 0x933b1109a1877e69ull}, \
+        {36712ull, 0x9459d86fe75bfd5aull}, {36552ull, 0x957817815f255709ull}, \
+        {36393ull, 0x9695cb097a816dc5ull}, {36236ull, 0x97b120ca89f230b5ull}, \
+        {36080ull, 0x98cbe07d407350f0ull}, {35926ull, 0x99e433d1f80e6b8bull}, \
+        {35772ull, 0x9afdbb6ec63d1090ull}, {35620ull, 0x9c14cbf30ed41c49ull}, \
+        {35470ull, 0x9d295bf40731c82bull}, {35320ull, 0x9e3f180014b06184ull}, \
+        {35172ull, 0x9f52489b9342f600ull}, {35026ull, 0xa062e44475890483ull}, \
+        {34880ull, 0xa174a36f0405f810ull}, {34735ull, 0xa285a589f4cd024aull}, \
+        {34592ull, 0xa39401f9af556e0dull}, {34450ull, 0xa4a1961d20623d50ull}, \
+        {34309ull, 0xa5ae5e4ad0e8242bull}, {34169ull, 0xa6ba56d23d9cc5efull}, \
+        {34031ull, 0xa7c38efa89fbc2a7ull}, {33893ull, 0xa8cddb06119ed15full}, \
+        {33757ull, 0xa9d55b2dcd306552ull}, {33622ull, 0xaadbf8a5d3a05444ull}, \
+        {33487ull, 0xabe3a49a1df94142ull}, {33354ull, 0xace873300596024eull}, \
+        {33222ull, 0xadec53874ed59eefull}, {33091ull, 0xaeef41b8b0f99e3cull}, \
+        {32961ull, 0xaff139d6950d45f3ull}, {32832ull, 0xb0f237ed2b233612ull}, \
     }
 }  // namespace math64
 }  // namespace gw

@@ -5,10 +5,11 @@
 // reference's ~1400 scalar FP64 operations per step cannot be run by one thread.  The step is
 // instead split into dependency phases; every op of a phase evaluates the same formula shape on
 // operands picked from a slot array X[] by per-op indices, one op per lane (128 lanes = 4 warps).
-// The reference's currents are rewritten as products of factors (PROD) whose linear combinations
-// are formed by SUM rows; transcendental terms are evaluated in uniform LOG / SQRT / EXP / REC
-// passes.  Reassociation changes results at the level of a few ulp, far inside the 1e-12 relative
-// FP64 parity bound.
+// Three phases: the increments with the Euler update, the transcendental terms of the new state, and
+// quotients and rate sums of those; an increment is a sum of products of two slots, so that the
+// product of two quotients, or of a quotient and a driving force, needs no phase of its own.
+// Reassociation changes results at the level of a few ulp, far inside the 1e-12 relative FP64 parity
+// bound.
 #pragma once
 
 #include <cstdint>
@@ -19,21 +20,21 @@ namespace gw {
 
 enum OdeKind : uint8_t {
     OK_NOP = 0,
-    OK_LOG,   // out = log(X[a0] + X[a1]*X[a2])
-    OK_SQRT,  // out = X[a0]*X[a1]*sqrt(X[a2]*X[a3])
-    OK_EXP,   // out = X[a0]*exp(X[a1]*X[a2] + X[a3])
-    OK_AFF,   // out = X[a0]*X[a1] + X[a2]*X[a3] + X[a4]*X[a5] + X[a6]
-    OK_REC,   // out = 1 / (X[a0] + X[a1]*X[a2] + X[a3]*X[a4] + X[a5]*X[a6]*X[a7])
-    OK_PROD,  // out = X[a0]*X[a1]*X[a2]*X[a3]*X[a4]*X[a5]*X[a6]
-    OK_SUM,   // row of `width` lanes: out = X[a0]*X[a1] * sum over lanes and t<4 of
-              //                             X[a2+3t]*X[a3+3t]*X[a4+3t]
-    OK_SUMU,  // SUM row whose result is the increment of global `out`: g[out] += result (FP64
-              // state) by the row's first lane, the new value to X[XS_GN + out]
+    OK_LOG,   // out = (X[a2] + X[a3]) + X[a4] * log(X[a0] + X[a1]*X[a5])
+    OK_EXP,   // out = X[a4] + X[a0] * exp(X[a1]*X[a2] + X[a3])
+    OK_POW,   // out = X[a4] + X[a0]*X[a1] * (X[a2]*X[a3])^(1/2), or ^(3/4) when width = 2
+    OK_QUOT,  // out = X[a0] * (X[a1] + X[a2]*X[a3]) / (X[a4] + X[a5]*X[a6])
+    OK_SUM3,  // out = X[a0]*X[a1] + X[a2]*X[a3] + X[a4]*X[a5]
+    OK_DOT,   // row of `width` lanes: the increment of global `out` is X[a0] times the sum over lanes and
+              // t < 4 of s_t X[a(1+2t)] X[a(2+2t)], s_t = -1 where bit 15 of a(1+2t) is set; the row's
+              // first lane adds X[a9]*X[a10] + X[a11]*X[a12] (the flux sums) and, once every row has
+              // read the old globals, updates g[out] (FP64 state) and X[XS_G + out]
 };
+constexpr uint16_t kOdeNeg = 0x8000;  // sign bit of an OK_DOT factor
 
 struct OdeOp {
     uint8_t kind;
-    uint8_t width;   // OK_SUM: lanes in the row (1, 2, 4 or 8); the row's first lane writes
+    uint8_t width;   // OK_DOT: lanes in the row (1, 2, 4 or 8), the row's first lane writes; OK_POW: see there
     uint16_t out;
     uint16_t a[14];
 };
@@ -52,10 +53,8 @@ enum OdeSlot : uint16_t {
     XS_ZERO = 0,
     XS_ONE = 1,
     XS_MONE = 2,
-    XS_G = 3,                        // 36 globals (gw_globals order), read by the increments
-    XS_GN = XS_G + kNumGlobals,      // the updated globals, read by the phases after the update
-                                     // (copied to XS_G after the push phase)
-    XS_SUMS = XS_GN + kNumGlobals,   // JLCC, ClCh, Jtr, Jxfer sums of the previous step
+    XS_G = 3,                        // 36 globals (gw_globals order)
+    XS_SUMS = XS_G + kNumGlobals,    // JLCC, ClCh, Jtr, Jxfer sums of the previous step
     XS_ISTIM = XS_SUMS + 4,
     XS_DT = XS_ISTIM + 1,
     XS_FIRST_FREE = XS_DT + 1,
@@ -65,8 +64,8 @@ enum OdeSlot : uint16_t {
 struct alignas(16) OdeProgram {
     int n_phases;
     int phase_begin[kOdeMaxPhases + 1];  // ops [phase_begin[p], phase_begin[p+1]) of phase p (<= 128)
-    int upd_phase;                       // phase of the increments and the update (OK_SUMU rows)
-    int push_phase;                      // sv are pushed after this phase
+    int upd_phase;                       // phase of the increments and the update (OK_DOT rows): 0
+    int push_phase;                      // sv are pushed after this phase (the last one)
     int n_slots;
     int const_begin, n_consts;           // per-cell constants occupy X[const_begin, +n_consts)
     int n_alt;
@@ -80,7 +79,8 @@ struct alignas(16) OdeProgram {
 static_assert(sizeof(OdeProgram) % 16 == 0, "OdeProgram is copied in 16-byte words");
 
 // Builds the program shared by all cells (pow_fast: all cells have Hf == Hr == 0.75, so the
-// Jup powers are taken with square roots) and the per-cell constant values.
+// Jup powers are taken with square roots; else a fourth phase exponentiates their logarithms) and the
+// per-cell constant values.
 bool ode_program_build(const CellStatic &cs, bool pow_fast, OdeProgram *prog, double *consts);
 
 // Host evaluation of one global step (FP64) in the device's operation order.
