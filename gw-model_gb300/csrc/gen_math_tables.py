@@ -3,13 +3,13 @@ run in 64-bit integer arithmetic.
 
 exp: 2^(j/256), j = 0..255, as integers of 63 fractional bits, 1/ln2 and the Taylor coefficients
 ln2^k / k! of 2^t.
-log: for j = 0..127, c_j = 2^16 / F_j rounded to an integer, F_j = 1 + (j + 1/2)/128, and
--log(c_j / 2^16) with 64 fractional bits; ln2; the coefficients (-1)^(k-1) / k of log(1 + u).
+log: for j = 0..255, c_j = 2^16 / (1 + j/256) rounded up to an integer, and -log(c_j / 2^16) with 64
+fractional bits; ln2; the magnitudes 1 / k of the coefficients of log(1 + u).
 All values come from 80-digit decimal arithmetic (Python's decimal module).
 
 Usage: python gen_math_tables.py > gw_math_tables.h
 """
-from decimal import ROUND_HALF_EVEN, Decimal, getcontext
+from decimal import ROUND_CEILING, ROUND_HALF_EVEN, Decimal, getcontext
 
 getcontext().prec = 80
 
@@ -34,20 +34,19 @@ def main():
             out.append(f"constexpr unsigned long long kExp{k} = {fixed(f, 64):#x}ull;  // ln2^{k}/{k}!, 64 fractional bits")
         else:
             out.append(f"constexpr unsigned int kExp{k} = {fixed(f, 32):#x}u;  // ln2^{k}/{k}!, 32 fractional bits")
-    for k in range(1, 8):
-        v = Decimal(1 if k % 2 else -1) / k
+    for k in range(2, 8):
         if k <= 3:
-            out.append(f"constexpr long long kLog{k} = {fixed(v, 62)}ll;  // (-1)^{k - 1}/{k}, 62 fractional bits")
+            out.append(f"constexpr unsigned long long kLog{k} = {fixed(Decimal(1) / k, 64):#x}ull;  // 1/{k}, 64 fractional bits")
         else:
-            out.append(f"constexpr int kLog{k} = {fixed(v, 30)};  // (-1)^{k - 1}/{k}, 30 fractional bits")
+            out.append(f"constexpr unsigned int kLog{k} = {fixed(Decimal(1) / k, 32):#x}u;  // 1/{k}, 32 fractional bits")
     out += ["// 2^(j/256), 63 fractional bits", "#define GW_EXP2_TABLE \\", "    { \\"]
     for j in range(0, 256, 4):
         out.append("        " + " ".join(f"{fixed((Decimal(j + i) / 256 * ln2).exp(), 63):#x}ull," for i in range(4)) + " \\")
     out += ["    }", "// {c_j, -log(c_j / 2^16) with 64 fractional bits}", "#define GW_LOG_TABLE \\", "    { \\"]
-    for j in range(0, 128, 2):
+    for j in range(0, 256, 2):
         row = []
         for i in range(2):
-            c = fixed(1 / (1 + (Decimal(j + i) + Decimal("0.5")) / 128), 16)
+            c = int((65536 / (1 + Decimal(j + i) / 256)).to_integral_value(rounding=ROUND_CEILING))
             row.append(f"{{{c}ull, {fixed(-(Decimal(c) / 65536).ln(), 64):#x}ull}},")
         out.append("        " + " ".join(row) + " \\")
     out += ["    }", "}  // namespace math64", "}  // namespace gw"]

@@ -396,26 +396,22 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
                 if (need) {
                     const int nm = qc + __popc(need & ((1u << base) - 1u));
                     qc += __popc(need);
-                    if (m == -1) {
-                        if (nm < qe) {
-                            m = q[nm];
-                            fetch(m, false);
-                            first = true;
-                        } else {
-                            m = -2;
-                        }
+                    if (m == -1) {  // (a group without one holds the range's last)
+                        const int mq = q[min(nm, qe - 1)];
+                        fetch(mq, false);
+                        first = true;
+                        m = nm < qe ? mq : -2;
                     }
                 }
                 if (!__any_sync(0xffffffffu, m >= 0)) break;
+                // (a group that ended its CRU with finish(), or has none, computes along)
+                bool done = m >= 0 && !first && L.surely_last(c, cc, sk, svf, rng, a.dt);
+                if (done) L.finish(c, cc, sv, rng, a.dt);
+                const bool more = m >= 0 && !done;
+                if (__any_sync(0xffffffffu, more))
+                    done |= L.iterate_group(more, c, cc, sv, rng, a.dt, a.event_cap, err) && more;
+                first = false;
                 if (m >= 0) {
-                    bool done;
-                    if (!first && L.surely_last(c, cc, sk, svf, rng, a.dt)) {
-                        L.finish(c, cc, sv, rng, a.dt);
-                        done = true;
-                    } else {
-                        done = L.iterate_group(c, cc, sv, rng, a.dt, a.event_cap, err);
-                    }
-                    first = false;
                     if (done) {
                         if (j == 0) after(m, dev::IterInfo<double>{}, 0u, 0u, true);
                         m = -1;
@@ -569,9 +565,9 @@ __global__ void __launch_bounds__(kOdeLanes) k_global(const GradArgs a, int64_t 
     };
     phases();
     const bool nernst = dev::not_positive(os.g[1]) || dev::not_positive(os.g[2]);
-    const double dv = L.increments();
+    const auto row = L.increments();
     __syncthreads();
-    L.update(dv);
+    L.update(row);
     __syncthreads();
     // the SSA values of the new state: the constant ones from their slots, the others from the
     // program's phases, Cai and CaNSR from the new globals

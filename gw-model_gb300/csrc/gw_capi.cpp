@@ -190,10 +190,10 @@ int byte_of(int v) { return v & 0xFF; }
 
 // Launch shape: cluster size C, CRU tile per CTA and SSA warps per CTA.  A cell needs
 // ceil(ncru / tile) <= C CTAs.
-// The size rule: cluster size C and CTA capacity (tile) for cells of at most max_n CRUs, from the
-// requested values (0 = derive).  Depends on nothing else, so contexts holding shares of an
-// ensemble reach the whole ensemble's shape when given its max_n.
-void shape_rule(int precision, int max_n, int cluster_req, int tile_req, int &C, int &tile) {
+// The size rule: cluster size C and CTA capacity (tile) for n_cells cells of at most max_n CRUs, from the
+// requested values (0 = derive).
+constexpr int kSpreadCtas = 112;
+void shape_rule(int precision, int n_cells, int max_n, int cluster_req, int tile_req, int &C, int &tile) {
     C = cluster_req > 0 ? cluster_req : 0;
     tile = tile_req > 0 ? tile_req : 0;
     if (C == 0 && tile == 0 && precision == GW_PRECISION_FP64) {
@@ -203,9 +203,15 @@ void shape_rule(int precision, int max_n, int cluster_req, int tile_req, int &C,
         C = std::min(kMaxClusterCtas, std::max(1, (max_n + 95) / 96));
         tile = (max_n + C - 1) / C;
     } else if (C == 0 && tile == 0) {
-        // Default: one CRU per SSA thread where possible, at most 16 CTAs per cell.
+        // Default FP32: one CRU per SSA thread where possible, at most 16 CTAs per cell.
         C = 1;
         while (C < kMaxClusterCtas && (max_n + C - 1) / C > 32 * kMaxSsaWarps) C *= 2;
+        // Cells that leave SMs idle are spread further, down to 64 CRUs per CTA beside the leader's:
+        // with one CRU per four lanes in one pass (kGroupCrus) the step is the global step's.  Clusters of
+        // any size are all resident up to 112 CTAs (7 clusters of 16, 14 of 8, 64 of 2).  us per step of
+        // one cell of 200 CRUs over 1, 3, 5 CTAs: 4.5, 3.1, 3.1; of 777 over 4, 9, 16: 4.6, 3.2, 3.2;
+        // of 3,000 over 8, 16: 5.4, 4.8; 16 cells of 777 over 4 and 8: 4.6, 7.0 (two rounds).
+        C = std::max(C, std::min({kMaxClusterCtas, (max_n + 63) / 64 + 1, kSpreadCtas / n_cells}));
         tile = (max_n + C - 1) / C;
     } else if (C == 0) {
         C = std::max(1, (max_n + tile - 1) / tile);
@@ -218,13 +224,15 @@ void shape_rule(int precision, int max_n, int cluster_req, int tile_req, int &C,
 int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
     const int max_n = *std::max_element(c->ncru.begin(), c->ncru.end());
     int C = 0, tile = 0;
-    shape_rule(c->precision, max_n, cluster_req, tile_req, C, tile);
+    shape_rule(c->precision, c->n_cells, max_n, cluster_req, tile_req, C, tile);
     if (C > kMaxClusterCtas || C < 1) return fail(c, GW_ERR_UNSUPPORTED, "cluster size %d not in [1,16]", C);
     const int need = (max_n + tile - 1) / tile;
     if (need > C)
         return fail(c, GW_ERR_UNSUPPORTED, "a cell of %d CRUs needs %d CTAs of %d CRUs but the cluster has %d",
                     max_n, need, tile, C);
-    c->ssa_warps = std::min(c->precision == GW_PRECISION_FP64 ? kMaxSsaWarpsFp64 : kMaxSsaWarps, tile / 32);
+    const bool fp64 = c->precision == GW_PRECISION_FP64;
+    // (FP32: down to one warp for eight CRUs, which take four lanes each)
+    c->ssa_warps = fp64 ? std::min(kMaxSsaWarpsFp64, tile / 32) : std::min(kMaxSsaWarps, tile / 8);
     c->tile_cap = tile;
     // Pack cells (first-fit decreasing on CTA count) into clusters of C CTAs.
     std::vector<int> order(c->n_cells);
@@ -250,11 +258,11 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
     c->work.assign((size_t)c->n_clusters * C, CtaWork{-1, 0, 0, 0, 0, 0, 0, 0});
     // A cell's CRUs are split in proportion to the CTAs' SSA warps that take CRUs: the others have
     // ssa_warps + kOdeWarps, the leader ssa_warps, or none when the cell is spread over several
-    // CTAs of under kLeaderFreeCrus CRUs each: the global step (~12 k cycles, on the leader's SM)
-    // then sets the step, and it runs ~10 % faster without SSA warps beside it (measured on one
-    // 12,500-CRU cell over 16 CTAs: 6.75 -> 6.15 us per step early in the beat, 7.52 -> 7.32 at
-    // 60-160 ms).  Larger CTA loads are SSA-bound and keep the leader's share.
-    constexpr int64_t kLeaderFreeCrus = 1024;
+    // CTAs of under kLeaderFreeCrus CRUs each: the global step on the leader's SM then sets the step and
+    // runs faster without SSA warps beside it.  (One 12,500-CRU cell over 16 CTAs, 782 CRUs each, line
+    // at 1024 and 300: 7.94 and 7.61 ms per 1,000 steps at rest, 10.7 and 10.5 amid the release; 24
+    // cells of 500 to 3,000: line at 500 and 300: 14.0 and 13.7; 200: the same.)
+    constexpr int64_t kLeaderFreeCrus = 300;
     const int64_t wo = c->ssa_warps + kOdeWarps;
     int max_count = 0;
     for (int q = 0; q < c->n_clusters; ++q) {
@@ -656,7 +664,7 @@ int gw_default_shape(const gw_ensemble_desc *d, int *cluster_ctas, int *cta_crus
         if (d->ncru[i] <= 0) return fail(nullptr, GW_ERR_INVALID_ARGUMENT, "cell %d: nCRU must be > 0", i);
         max_n = std::max(max_n, (int)d->ncru[i]);
     }
-    shape_rule(d->precision, max_n, d->cluster_ctas, d->cta_crus, *cluster_ctas, *cta_crus);
+    shape_rule(d->precision, d->n_cells, max_n, d->cluster_ctas, d->cta_crus, *cluster_ctas, *cta_crus);
     return GW_OK;
 }
 

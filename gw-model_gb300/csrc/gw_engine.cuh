@@ -5,11 +5,10 @@
 // global step as the lane program of gw_ode_program.h; in the other CTAs of the cell every warp
 // runs SSA.  The CTAs of a cell are held together only by their data, which travel by st.async
 // and complete per-parity mbarriers of the receiver (no cluster barrier inside the launch):
-//   SSA warps : wait for sv[s&1] (the CTA's mbarrier), then each warp runs the SSA of step s on a
-//               contiguous range of the CTA's CRU tile, one CRU per lane at a time; a lane whose
-//               CRU has finished its step takes the warp's next CRU, so lanes with pending SSA
-//               events do not hold the others back.  Each warp pushes its flux partial into its
-//               slot in the leader's shared memory.
+//   SSA warps : wait for sv[s&1] (the CTA's mbarrier), run the SSA of step s on the CTA's CRU tile, and
+//               push their flux partials into their slots in the leader's shared memory.  FP64: one
+//               CRU per lane at a time, the ones with events on four lanes each.  FP32: group_steps
+//               (few CRUs) or split_steps.
 //   ODE warps : wait for the warp partials of step s-1 (the leader's mbarrier), reduce them,
 //               increments and Euler update (globals s -> s+1), transcendental phases of the new
 //               state (an idle lane forms the stimulus of step s+1), push sv[(s+1)&1]; phases the
@@ -32,11 +31,18 @@ template <>
 struct alignas(16) Partial<true> {
     double v[4];
 };
+// FP32: each sum in two integers, hi and lo 2^-23 of a unit (FluxUnit) below it; or, with flag set, three
+// floats in the hi fields.
 template <>
 struct alignas(16) Partial<false> {
-    float j, x, t;
-    int cl;
+    int jh, jl, xh, xl;
+    int th, tl, cl, flag;
 };
+// The units of the FP32 sums' hi parts: powers of two, 2^21 of them bound a CRU's term (1024, 256 and
+// 16 mM/ms for JLCC, Jxfer and Jtr; the model's terms stay below 100, 100 and 1).  kMaxSumCrus terms
+// fit 32 bits.
+constexpr int kUnitJ = -11, kUnitX = -13, kUnitT = -17;
+constexpr int kMaxSumCrus = 500;
 
 struct OdeShared {
     double g[kNumGlobals];  // the cell's globals (FP64 state)
@@ -80,9 +86,11 @@ __host__ __device__ inline SmemLayout smem_layout(int tile_cap, int max_cta_cell
     L.part = o;  // [parity][rank in cell][warp]: warp partials (written by the cell's CTAs)
     o += (size_t)2 * max_cta_cell * kMaxWarps * sizeof(Partial<sizeof(R) == 8>);
     L.mbar = o;  // mbarriers: the warp partials of steps of parity 0 and 1 (leader CTA), then the
-    o += 32;     // per-step SSA values of parity 0 and 1 (every CTA)
-    L.fq = o;    // FP64: the queue's two counters (by step parity), then kEngQCap tile indices
-    o += sizeof(R) == 8 ? align16((size_t)(4 + kEngQCap) * sizeof(int)) : 0;
+    o += 80;     // per-step SSA values of parity 0 and 1 (every CTA); FP32: the quiet warps', the event
+                 // warps' and the queue's of parity 0 and 1
+    L.fq = o;    // the event queue: FP64: four counters, then kEngQCap tile indices; FP32: eight counters,
+                 // then three queues of a 16-bit tile index for every CRU of the CTA
+    o += sizeof(R) == 8 ? align16((size_t)(4 + kEngQCap) * sizeof(int)) : align16(32 + (size_t)6 * tile_cap);
     L.tile = o;  // TileRec<R> per CRU
     o += align16((size_t)tile_cap * sizeof(TileRec<R>));
     L.total = o;
@@ -178,11 +186,28 @@ __device__ __forceinline__ double flip(double x, uint32_t w) {
 __device__ __forceinline__ float flip(float x, uint32_t w) { return __uint_as_float(__float_as_uint(x) ^ (w & 0x80000000u)); }
 
 // The FP32 pair (hi, lo) of an FP64 value for the SSA: hi = (float)d, lo = (float)(d - hi); for an
-// FP64 SSA the value itself and 0.
+// FP64 SSA the value itself and 0.  By integer operations where hi and lo are normal (the two
+// conversions and the subtraction would take the FP64 pipe, of every warp that meets them predicated).
 __device__ __forceinline__ void stage_pair(float *st, int ihi, int ilo, double d) {
-    const float hi = (float)d;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+    const uint32_t e = (uint32_t)(b >> 52) & 0x7FFu, sign = (uint32_t)(b >> 32) & 0x80000000u;
+    float hi, lo;
+    if (e - 960u < 180u) {
+        // significand 2^52 + f: its upper 24 bits rounded to nearest even, the rest a signed 30-bit integer
+        const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+        const unsigned long long r = m + 0x0FFFFFFFull + ((m >> 29) & 1ull);
+        const uint32_t h = (uint32_t)(r >> 29);  // 2^23 .. 2^24
+        const int rest = (int)((long long)m - (long long)((unsigned long long)h << 29));
+        hi = __uint_as_float(sign | (((e - 897u) << 23) + h));
+        // rest 2^(e - 1075): rounded to 24 bits by the conversion, then scaled by a normal power of two
+        const float l = __fmul_rn((float)rest, __uint_as_float((e - 948u) << 23));
+        lo = __uint_as_float(__float_as_uint(l) ^ sign);
+    } else {
+        hi = (float)d;
+        lo = (float)(d - (double)hi);
+    }
     st[ihi] = hi;
-    st[ilo] = (float)(d - (double)hi);
+    st[ilo] = lo;
 }
 __device__ __forceinline__ void stage_pair(double *st, int ihi, int ilo, double d) {
     st[ihi] = d;
@@ -205,7 +230,7 @@ struct LaneOp {
 // The cell's global step by the kOdeLanes ODE threads (t = 0 .. kOdeLanes-1), thread t running op t
 // of each phase.  Every warp holds one op kind per phase, so the kinds do not diverge.
 //   increments()  phase E up to the flux sums: this thread's row sum (rows of up to 8 lanes, shuffles
-//                 in the first warp only)
+//                 in the first warp only), with update()'s other operands already loaded
 //   update()      after a barrier: the flux-sum terms and the Euler update by the rows' first lanes
 //   terms()       phase A of the new state (reloads the ops where V changed its regime)
 //   powers()      phase P (general Jup exponents only)
@@ -254,10 +279,17 @@ struct OdeLane {
         load(b, P->push_phase);
     }
 
-    __device__ __forceinline__ T increments() const {
-        T v = (T)0;
-        if (t >= 64) return v;
-        v = flip(arg(e, 1), e.sign(1)) * arg(e, 2);
+    // A row's first lane after increments(): its sum, and what update() will need that does not depend
+    // on the flux sums.
+    struct Row {
+        T v, s, c0, c1;
+        double g;
+        bool first;
+    };
+    __device__ __forceinline__ Row increments() const {
+        Row r{};
+        if (t >= 64) return r;
+        T v = flip(arg(e, 1), e.sign(1)) * arg(e, 2);
         v = o_fma(flip(arg(e, 3), e.sign(3)), arg(e, 4), v);
         v = o_fma(flip(arg(e, 5), e.sign(5)), arg(e, 6), v);
         v = o_fma(flip(arg(e, 7), e.sign(7)), arg(e, 8), v);
@@ -270,14 +302,20 @@ struct OdeLane {
                 if ((t & wm) + off <= wm && (t & (2 * off - 1)) == 0) v += o;
             }
         }
-        return v;
+        r.first = e.kind() == OK_DOT && (t & (e.width() - 1)) == 0;
+        r.v = v;
+        r.s = arg(e, 0);
+        r.c0 = arg(e, 9);
+        r.c1 = arg(e, 11);
+        r.g = os->g[r.first ? e.out() : 0u];
+        return r;
     }
-    __device__ __forceinline__ void update(T v) const {
-        if (t >= 64 || e.kind() != OK_DOT || (t & (e.width() - 1))) return;
-        if (t < 32) v = o_fma(arg(e, 11), arg(e, 12), o_fma(arg(e, 9), arg(e, 10), v));
+    __device__ __forceinline__ void update(const Row &r) const {
+        if (!r.first) return;
+        T v = r.v;
+        if (t < 32) v = o_fma(r.c1, arg(e, 12), o_fma(r.c0, arg(e, 10), v));
         const int out = (int)e.out();
-        const double ng = sizeof(T) == 8 ? __fma_rn((double)arg(e, 0), (double)v, os->g[out])
-                                         : os->g[out] + (double)(arg(e, 0) * v);
+        const double ng = sizeof(T) == 8 ? __fma_rn((double)r.s, (double)v, r.g) : r.g + (double)(r.s * v);
         os->g[out] = ng;
         slots()[XS_G + out] = (T)ng;
         if (!finite_bits(ng)) atomicCAS(&os->status, 0, (int)GW_ERR_NONFINITE);  // first error of the cell
@@ -301,9 +339,8 @@ struct OdeLane {
             put(a, o_fma(arg(a, 4), o_log(o_fma(arg(a, 1), arg(a, 5), arg(a, 0)), *M), arg(a, 2) + arg(a, 3)));
             break;
         case OK_POW: {
-            const T s = o_sqrt(arg(a, 2) * arg(a, 3));
-            const T c = arg(a, 0) * arg(a, 1);
-            put(a, o_fma(c, a.width() == 2 ? s * o_sqrt(s) : s, arg(a, 4)));
+            const T s = o_sqrt(arg(a, 2)), c = arg(a, 0) * arg(a, 1);
+            put(a, o_fma(c, a.width() == 2 ? s * o_sqrt(s) : s, arg(a, 3)));
             break;
         }
         default: break;
@@ -322,128 +359,113 @@ struct OdeLane {
     }
 };
 
-// Sums {JLCC, ClCh, Jtr, Jxfer} of the n warp partials of one slot (n <= 16 CTAs x kMaxWarps) by two
-// warps of the ODE threads: half 0 JLCC and ClCh, half 1 Jtr and Jxfer.  The result does not depend on
-// the order of the partials in either precision's slots beyond their fixed positions.
+// Sums {JLCC, ClCh, Jtr, Jxfer} of the n warp partials of one slot (n <= 16 CTAs x kMaxWarps), quantity
+// `warp` by ODE warp `warp`.
 constexpr int kSlotsPerLane = 16 * kMaxWarps / 32;
-
-// FP32: each quantity's partials on one fixed-point scale, 2^-54 of the largest's power of two, summed
-// exactly in 64-bit integers (the lanes' sums through REDUX in three pieces) and rounded once to FP64.
-// (A tree of compensated float pairs took ~700 cycles, this ~250.)  A NaN or infinity, which has no
-// scale, makes the sum NaN.
-__device__ __forceinline__ double fixed_sum(const float (&f)[kSlotsPerLane], int nk) {
-    uint32_t top = 0u;
-#pragma unroll
-    for (int k = 0; k < kSlotsPerLane; ++k)
-        if (k < nk) top = max(top, __float_as_uint(f[k]) & 0x7FFFFFFFu);
-    top = __reduce_max_sync(0xffffffffu, top);
-    const int em = max((int)(top >> 23), 1);
-    long long s = 0;
-#pragma unroll
-    for (int k = 0; k < kSlotsPerLane; ++k)
-        if (k < nk) {
-            const uint32_t b = __float_as_uint(f[k]);
-            const int ex = (int)((b >> 23) & 0xFFu);
-            const unsigned long long m = (unsigned long long)((b & 0x7FFFFFu) | (ex ? 0x800000u : 0u)) << 30;
-            const long long v = (long long)(m >> min(em - max(ex, 1), 63));
-            s += (b >> 31) ? -v : v;
-        }
-    const int h = __reduce_add_sync(0xffffffffu, (int)(s >> 32));
+// FP32: 64-bit integer sums, the lanes' through REDUX in three pieces, hence exact, and rounded once to
+// FP64; u is the exponent of their unit.
+__device__ __forceinline__ double fixed_total(long long s, int u) {
     const uint32_t lo = (uint32_t)s;
+    const int h = __reduce_add_sync(0xffffffffu, (int)(s >> 32));
     const uint32_t l1 = __reduce_add_sync(0xffffffffu, lo >> 16), l0 = __reduce_add_sync(0xffffffffu, lo & 0xFFFFu);
     s = ((long long)h << 32) + ((long long)l1 << 16) + (long long)l0;
-    if (top >= 0x7F800000u) return __longlong_as_double(0x7FF8000000000000ll);
-    if (s == 0) return 0.0;
-    const unsigned long long u = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
-    const int z = __clzll((long long)u);
-    // u 2^(em - 127 - 23 - 30), leading bit at 63 - z
-    const unsigned long long d = math64::pack(u << z, 63 - z + em - 180);
+    const unsigned long long m = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
+    if (m == 0ull) return 0.0;
+    const uint32_t mh = (uint32_t)(m >> 32);
+    const int z = mh ? __clz((int)mh) : 32 + __clz((int)(uint32_t)m);
+    const unsigned long long d = math64::pack(m << z, 63 - z + u);
     return __longlong_as_double((long long)(s < 0 ? d | 0x8000000000000000ull : d));
 }
-
 template <typename T>
-__device__ __forceinline__ void reduce_partials(const Partial<false> *slot, int n, int half, int lane, double *out, T *X) {
-    const int nk = (n + 31) >> 5;
-    double r0, r1;
-    if (half == 0) {
-        float f[kSlotsPerLane];
-        int cl = 0;
+__device__ __forceinline__ void reduce_partials(const Partial<false> *slot, int n, int warp, int lane, double *out, T *X) {
+    // field of {jh, jl, xh, xl, th, tl, cl, flag}, and its unit
+    const int at = warp == 0 ? 0 : (warp == 1 ? 6 : (warp == 2 ? 4 : 2));
+    const int unit = warp == 0 ? kUnitJ : (warp == 2 ? kUnitT : kUnitX);
+    int hi[kSlotsPerLane], lo[kSlotsPerLane], flag = 0;
 #pragma unroll
-        for (int k = 0; k < kSlotsPerLane; ++k) {
-            const int i = lane + 32 * k;
-            f[k] = 0.f;
-            if (k < nk && i < n) {
-                f[k] = slot[i].j;
-                cl += slot[i].cl;
-            }
-        }
-        cl = (int)__reduce_add_sync(0xffffffffu, (unsigned)cl);
-        r0 = fixed_sum(f, nk);
-        r1 = (double)cl;
-    } else {
-        float f[kSlotsPerLane], g[kSlotsPerLane];
-#pragma unroll
-        for (int k = 0; k < kSlotsPerLane; ++k) {
-            const int i = lane + 32 * k;
-            f[k] = g[k] = 0.f;
-            if (k < nk && i < n) {
-                f[k] = slot[i].t;
-                g[k] = slot[i].x;
-            }
-        }
-        r0 = fixed_sum(f, nk);
-        r1 = fixed_sum(g, nk);
+    for (int k = 0; k < kSlotsPerLane; ++k) {
+        const int i = lane + 32 * k;
+        const int *f = reinterpret_cast<const int *>(slot + (i < n ? i : 0));
+        hi[k] = i < n ? f[at] : 0;
+        lo[k] = i < n && warp != 1 ? f[at + 1] : 0;
+        flag |= i < n ? f[7] : 0;
     }
-    if (lane < 2) {
-        const double r = lane ? r1 : r0;
-        out[2 * half + lane] = r;
-        X[XS_SUMS + 2 * half + lane] = (T)r;
+    double r;
+    if (!__any_sync(0xffffffffu, flag)) {
+        long long s = 0;
+        const int up = warp == 1 ? 0 : 23;
+#pragma unroll
+        for (int k = 0; k < kSlotsPerLane; ++k) s += ((long long)hi[k] << up) + lo[k];
+        r = fixed_total(s, warp == 1 ? 0 : unit - 23);
+    } else {
+        // some warp had a term beyond the fixed-point range (or a NaN): its sums are floats
+        r = 0.0;
+        for (int k = 0; k < kSlotsPerLane; ++k) {
+            const int i = lane + 32 * k;
+            if (i >= n) continue;
+            if (warp == 1)
+                r += (double)hi[k];
+            else
+                r += slot[i].flag ? (double)__int_as_float(hi[k])
+                                  : (double)(((long long)hi[k] << 23) + lo[k]) * ldexp(1.0, unit - 23);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    }
+    if (lane == 0) {
+        out[warp] = r;
+        X[XS_SUMS + warp] = (T)r;
     }
 }
 template <typename T>
-__device__ __forceinline__ void reduce_partials(const Partial<true> *slot, int n, int half, int lane, double *out, T *X) {
+__device__ __forceinline__ void reduce_partials(const Partial<true> *slot, int n, int warp, int lane, double *out, T *X) {
+    const int src = warp == 0 ? 0 : (warp == 1 ? 3 : (warp == 2 ? 2 : 1));  // of {JLCC, Jxfer, Jtr, ClCh}
     const int nk = (n + 31) >> 5;
-    // {JLCC, Jxfer, Jtr, ClCh} of a slot
-    const int s0 = half == 0 ? 0 : 2, s1 = half == 0 ? 3 : 1;
-    double a = 0.0, b = 0.0;
+    double a = 0.0;
     for (int k = 0; k < nk; ++k) {
         const int i = lane + 32 * k;
-        if (i < n) {
-            a += slot[i].v[s0];
-            b += slot[i].v[s1];
-        }
+        if (i < n) a += slot[i].v[src];
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (lane < 2) {
-        const double r = lane ? b : a;
-        out[2 * half + lane] = r;
-        X[XS_SUMS + 2 * half + lane] = (T)r;
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) {
+        out[warp] = a;
+        X[XS_SUMS + warp] = (T)a;
     }
 }
 
 // Per-step SSA values of the new state to every CTA of the cell: the staging row (written by the
 // ops that produce the values, see OdeLane, and visible after the phase's barrier) pushed in
 // 16-byte words (CTA, word) by all kOdeLanes threads, as asynchronous stores that count themselves
-// off the receiving CTA's mbarrier of this slot (local shared address mbar_slot in every CTA).
+// off the receiving CTA's mbarrier of this slot.  The addresses are formed once per launch.
 template <bool FP64>
-__device__ __forceinline__ void push_sv(void *svbuf, const void *stage, int slot, uint32_t mbar_slot, const CtaWork &w,
-                                        int t) {
+struct SvPush {
     using R = typename std::conditional<FP64, double, float>::type;
-    constexpr int kWords = kSvCount * (int)sizeof(R) / 16;  // 16-byte words of one slot
+    static constexpr int kWords = kSvCount * (int)sizeof(R) / 16;  // 16-byte words of one slot
+    static constexpr int kMost = (kWords * kMaxClusterCtas + kOdeLanes - 1) / kOdeLanes;
     static_assert(kSvCount * sizeof(R) % 16 == 0, "sv slot in 16-byte words");
-    const uint4 *src = reinterpret_cast<const uint4 *>(stage);
-    uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<R *>(svbuf) + slot * kSvCount);
-    const int total = kWords * w.n_cta_cell;
-    for (int idx = t; idx < total; idx += kOdeLanes) {
-        const int r = idx / kWords, i = idx - r * kWords;
-        const uint32_t rank = (uint32_t)(w.first + r);
-        st_async(map_rank(dst + i, rank), src[i], map_rank_addr(mbar_slot, rank));
+    const uint4 *src[kMost];
+    uint32_t dst[kMost], bar[kMost];  // of slot 0 (slot 1: kSvCount values and 8 bytes on); dst 0: none
+    __device__ __forceinline__ SvPush(void *svbuf, const void *stage, uint32_t mbar, const CtaWork &w, int t) {
+#pragma unroll
+        for (int k = 0; k < kMost; ++k) {
+            const int idx = t + k * kOdeLanes, r = idx / kWords, i = idx - r * kWords;
+            src[k] = reinterpret_cast<const uint4 *>(stage) + i;
+            dst[k] = bar[k] = 0u;
+            if (r < w.n_cta_cell) {
+                const uint32_t rank = (uint32_t)(w.first + r);
+                dst[k] = map_rank(reinterpret_cast<uint4 *>(svbuf) + i, rank);
+                bar[k] = map_rank_addr(mbar, rank);
+            }
+        }
     }
-}
+    __device__ __forceinline__ void operator()(int slot) const {
+#pragma unroll
+        for (int k = 0; k < kMost; ++k)
+            if (bar[k])
+                st_async(dst[k] + (uint32_t)slot * (uint32_t)(kSvCount * sizeof(R)), *src[k], bar[k] + 8u * (uint32_t)slot);
+    }
+};
 
 // Ca in 2^-40 mM fixed point (exact, order-independent sums of the record-time CRU sums).
 __device__ __forceinline__ long long fix40(float x) { return __float2ll_rn(x * 0x1p40f); }
@@ -536,53 +558,85 @@ __device__ __forceinline__ void record_pass(const KernelArgs &a, const CtaWork &
 
 // Per-lane flux accumulators and their warp sum as a Partial (all lanes hold it).
 template <bool FP64>
-struct FluxAcc {
-    float jh = 0, xh = 0, th = 0;    // FP32
-    double dj = 0, dx = 0, dtr = 0;  // FP64
+struct FluxAcc;
+template <>
+struct FluxAcc<true> {
+    double dj = 0, dx = 0, dtr = 0;
     int acl = 0;
-    // FP32: a lane's own CRUs (one to a few per step) add up in FP32, the lane sums in a plain
-    // FP32 tree (warp_total); the cell's warp partials are then combined exactly (reduce_partials).
-    __device__ __forceinline__ void add(float j, float x, float t, int cl) {
-        jh += j;
-        xh += x;
-        th += t;
-        acl += cl;
-    }
     __device__ __forceinline__ void add(double j, double x, double t, int cl) {
         dj += j;
         dx += x;
         dtr += t;
         acl += cl;
     }
-    __device__ __forceinline__ Partial<FP64> warp_total() {
-        Partial<FP64> pv;
-        if constexpr (FP64) {
+    __device__ __forceinline__ Partial<true> warp_total() {
+        Partial<true> pv;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            dj += __shfl_xor_sync(0xffffffffu, dj, o);
+            dx += __shfl_xor_sync(0xffffffffu, dx, o);
+            dtr += __shfl_xor_sync(0xffffffffu, dtr, o);
+            acl += __shfl_xor_sync(0xffffffffu, acl, o);
+        }
+        pv.v[0] = dj;
+        pv.v[1] = dx;
+        pv.v[2] = dtr;
+        pv.v[3] = (double)acl;
+        return pv;
+    }
+};
+// FP32: fixed-point sums, so that they do not depend on which lane of which warp took a CRU, or when (the
+// split between quiet and event warps depends on the launch's start).  A term v is rounded to a multiple
+// of its unit by adding 1.5 * 2^23 units, whose float's low bits are then the multiple (less the
+// constant's); what is left goes the same way to a unit 2^-23 of that.  Two exact subtractions and
+// integer adds; a term's rounding error is at most half the lower unit (2.9e-11, 7.3e-12 and 4.5e-13
+// mM/ms).  Terms out of range, or too many of them, set `big`, and the warp sends plain float sums.
+template <>
+struct FluxAcc<false> {
+    int jh = 0, jl = 0, xh = 0, xl = 0, th = 0, tl = 0, acl = 0;
+    float jf = 0, xf = 0, tf = 0;
+    bool big = false;
+    __device__ __forceinline__ static constexpr float pow2(int e) { return e < 0 ? 1.f / (float)(1ull << -e) : (float)(1ull << e); }
+    template <int UNIT>
+    __device__ __forceinline__ void split(float v, int &hi, int &lo) {
+        constexpr float H = 12582912.f * pow2(UNIT), L = H * pow2(-23);
+        const float t = __fadd_rn(v, H);
+        const float u = __fadd_rn(__fsub_rn(v, __fsub_rn(t, H)), L);
+        hi += __float_as_int(t) - (0x4B400000 + UNIT * (1 << 23));
+        lo += __float_as_int(u) - (0x4B400000 + ((UNIT - 23) * (1 << 23)));
+        big |= !(fabsf(v) < 2097152.f * pow2(UNIT));
+    }
+    __device__ __forceinline__ void add(float j, float x, float t, int cl) {
+        split<kUnitJ>(j, jh, jl);
+        split<kUnitX>(x, xh, xl);
+        split<kUnitT>(t, th, tl);
+        jf += j;
+        xf += x;
+        tf += t;
+        acl += cl;
+    }
+    __device__ __forceinline__ Partial<false> warp_total() {
+        Partial<false> pv;
+        pv.cl = __reduce_add_sync(0xffffffffu, acl);
+        pv.flag = __any_sync(0xffffffffu, big) ? 1 : 0;
+        if (pv.flag) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                dj += __shfl_xor_sync(0xffffffffu, dj, o);
-                dx += __shfl_xor_sync(0xffffffffu, dx, o);
-                dtr += __shfl_xor_sync(0xffffffffu, dtr, o);
-                acl += __shfl_xor_sync(0xffffffffu, acl, o);
+                jf += __shfl_xor_sync(0xffffffffu, jf, o);
+                xf += __shfl_xor_sync(0xffffffffu, xf, o);
+                tf += __shfl_xor_sync(0xffffffffu, tf, o);
             }
-            pv.v[0] = dj;
-            pv.v[1] = dx;
-            pv.v[2] = dtr;
-            pv.v[3] = (double)acl;
+            pv.jh = __float_as_int(jf);
+            pv.xh = __float_as_int(xf);
+            pv.th = __float_as_int(tf);
+            pv.jl = pv.xl = pv.tl = 0;
         } else {
-            // FP32: a plain tree over the 32 lane sums (each covers a few CRUs; the exact sums start
-            // where most terms meet, across the cell's warp partials), and one REDUX for the ClCh
-            // count.  The per-step tree runs on every lane of every warp: with compensation it was
-            // ~150 instructions per CRU-step of a 12,500-CRU cell.
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                jh += __shfl_xor_sync(0xffffffffu, jh, o);
-                xh += __shfl_xor_sync(0xffffffffu, xh, o);
-                th += __shfl_xor_sync(0xffffffffu, th, o);
-            }
-            pv.j = jh;
-            pv.x = xh;
-            pv.t = th;
-            pv.cl = (int)__reduce_add_sync(0xffffffffu, (unsigned)acl);
+            pv.jh = __reduce_add_sync(0xffffffffu, jh);
+            pv.jl = __reduce_add_sync(0xffffffffu, jl);
+            pv.xh = __reduce_add_sync(0xffffffffu, xh);
+            pv.xl = __reduce_add_sync(0xffffffffu, xl);
+            pv.th = __reduce_add_sync(0xffffffffu, th);
+            pv.tl = __reduce_add_sync(0xffffffffu, tl);
         }
         return pv;
     }
@@ -605,9 +659,13 @@ struct CtaView {
     void *svstage;
     Partial<FP64> *part;
     float2 *rtab;
-    int *fq;        // FP64: queue counters [2] (+2 unused), then the queue
+    int *fq;        // FP64: by parity, entries queued; FP32: by step mod 3, entries reserved << 16 | written, and
+                    // claimed, then the split by parity; then the queues
     uint32_t mbar;  // shared address of the partials' mbarrier of parity 0 (parity 1 at +8); the
-                    // SSA values' mbarriers of parity 0 and 1 at +16 and +24
+                    // SSA values' mbarriers of parity 0 and 1 at +16 and +24; FP32: the quiet warps'
+                    // at +32 and +40, the event warps' at +48 and +56, the queue's (cleared for the
+                    // step) at +64 and +72
+    bool grouped;   // FP32: few enough CRUs for group_steps
     TileRec<R> *tile;
 
     __device__ __forceinline__ explicit CtaView(const KernelArgs &a) {
@@ -621,6 +679,7 @@ struct CtaView {
         leader = active && w.rank_in_cell == 0;
         ode_thread = leader && warp >= nw;
         n_ssa = (leader ? nw : nw + kOdeWarps) * 32;  // SSA threads of this CTA
+        grouped = !FP64 && w.cru_count <= kGroupCrus * (n_ssa >> 5);
         const SmemLayout L = smem_layout<R, T>(a.tile_cap, a.max_cta_cell);
         cc = reinterpret_cast<SsaConsts<R> *>(smem + L.cc);
         svbuf = reinterpret_cast<R *>(smem + L.sv);
@@ -637,9 +696,9 @@ struct CtaView {
 };
 
 // The leader CTA's ODE warps over a launch: the transcendental phases of the initial state and
-// the push of sv[0], then per global step s the increments on two warps beside the wait for and the
-// reduction of the warp partials of step s-1 on the other two, the global step s -> s+1 and the push
-// of sv[(s+1)&1], and the carry back to the cell block at the end.  A function of its own (not inlined
+// the push of sv[0], then per global step s the increments up to the flux sums, the wait for and the
+// reduction of the warp partials of step s-1 (one quantity per warp), the global step s -> s+1 and the
+// push of sv[(s+1)&1], and the carry back to the cell block at the end.  A function of its own (not inlined
 // into the kernel), so that its register allocation and schedule do not depend on the SSA code.
 template <bool FP64, bool ODE64>
 __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
@@ -680,18 +739,13 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         X[XS_G + i] = (T)d0.g[i];
     }
     for (int i = ot; i < kOdeConstCap; i += kOdeLanes) X[XS_FIRST_FREE + i] = (T)C.ode_consts[i];
-    // The accumulated time, and the stimulus of the next step, by a lane of a warp with little to do in
-    // phase B (t_{s+1} = t_s + dt, as the reference accumulates it).
+    // The accumulated time, and the stimulus of the next step, by a lane that has no increment (t_{s+1} =
+    // t_s + dt, as the reference accumulates it).  A sampled stimulus is read a step before its use.
     const bool clock = ot == 2 * 32;
-    // A sampled stimulus is read a step before its use.
-    double time = d0.t, ahead = 0.0;
-    auto set_stim = [&](int64_t ri) {
-        X[XS_ISTIM] = (T)(stim.mode == STIM_SAMPLES ? ahead : stim.pulse(time));
-        ahead = stim.sample(ri + 1);
-    };
+    double time = d0.t, next_time = d0.t, next_stim = 0.0, ahead = 0.0;
     if (clock) {
-        ahead = stim.sample(a.run_step0);
-        set_stim(a.run_step0);
+        ahead = stim.sample(a.run_step0 + 1);
+        X[XS_ISTIM] = (T)(stim.mode == STIM_SAMPLES ? stim.sample(a.run_step0) : stim.pulse(time));
     }
     ode_bar();
     // staging row: the constant SSA values once per launch, Cai and CaNSR of the initial state
@@ -700,6 +754,7 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         const int src = a.prog->sv_src[ot];
         if (src < XS_FIRST_FREE + kOdeMaxConsts) stage[ot] = (R)X[src];
     }
+    const SvPush<FP64> push(v.svbuf, v.svstage, v.mbar + 16u, v.w, ot);
     L.reg = v_regime(os.g[0]);
     L.load_all();
     const bool powers = L.has_powers();
@@ -720,7 +775,7 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
     ode_bar();
     // (the SSA warps wait for these bytes in step 0: the host launches 1..steps_per_launch
     // steps, never 0, so no CTA exits while they may be in flight)
-    push_sv<FP64>(v.svbuf, v.svstage, 0, v.mbar + 16u, v.w, ot);
+    push(0);
     // bytes of the cell's warp partials per step
     const uint32_t part_bytes =
         (uint32_t)sizeof(Partial<FP64>) * (uint32_t)(v.nw + (v.w.n_cta_cell - 1) * (v.nw + kOdeWarps));
@@ -743,15 +798,21 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
                                   part_bytes + (s == a.n_steps - 1 ? (uint32_t)a.test_extra_tx : 0u));
         if (ot == 0 && (not_positive(os.g[1]) || not_positive(os.g[2])) && os.status == 0)
             os.status = GW_ERR_NERNST;
-        // the increments up to the flux sums (warps 0 and 1), and the sums of step s-1 (warps 2 and 3;
-        // step 0 uses the carry)
-        const T dv = L.increments();
+        // the increments up to the flux sums (warps 0 and 1), the next stimulus (warp 2), and the sums of
+        // step s-1 (step 0 uses the carry)
+        const typename OdeLane<T, R>::Row row = L.increments();
+        if (clock) {
+            next_time = time + a.dt;
+            next_stim = stim.mode == STIM_SAMPLES ? ahead : stim.pulse(next_time);
+            ahead = stim.sample(ri + 2);
+        }
         bool ok = true;
-        if (s > 0 && warp >= 2) {
-            ok = mbar_wait(v.mbar + 8u * (uint32_t)(par ^ 1), (uint32_t)((s - 1) >> 1) & 1u);
+        if (s > 0) {
+            ok = mbar_wait_warp(v.mbar + 8u * (uint32_t)(par ^ 1), (uint32_t)((s - 1) >> 1) & 1u);
+            __syncwarp();
             // (a warp's lanes may find different outcomes; whatever is summed after a wait that ran out
             // is not used)
-            reduce_partials(v.part + (par ^ 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp - 2, lane, os.sums, X);
+            reduce_partials(v.part + (par ^ 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp, lane, os.sums, X);
         }
         if (bar_or(1, kOdeLanes, !ok)) {  // the same decision on all ODE threads
             if (ot == 0) atomicCAS(&os.status, 0, (int)GW_ERR_SYNC_TIMEOUT);
@@ -759,21 +820,23 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
             s_stop = s;
             continue;
         }
-        L.update(dv);
+        L.update(row);
+        if (clock) {
+            time = next_time;
+            X[XS_ISTIM] = (T)next_stim;
+        }
         ode_bar();
-        if (clock) time += a.dt;
         if (rec_ok) {
             double *dst = a.tr_glob + ((int64_t)cell * a.rec_cap + r_idx) * kNumGlobals;
             for (int i = ot; i < kNumGlobals; i += kOdeLanes) dst[i] = os.g[i];
             if (clock && (cell == 0 || (a.tr_cell >= 0 && cell == a.tr_cell))) a.tr_t[r_idx] = time;
         }
         phases();
-        if (clock) set_stim(ri + 1);
         ode_bar();
         // (no push after the launch's last step: no one would wait for those bytes, and a CTA
         // must not exit while stores into its shared memory may still be in flight)
         if (s + 1 < a.n_steps)
-            push_sv<FP64>(v.svbuf, v.svstage, par ^ 1, v.mbar + 16u + 8u * (uint32_t)(par ^ 1), v.w, ot);
+            push(par ^ 1);
     }
     // carry of the last step's fluxes, globals and counters back to the cell block
     if (a.n_steps > 0 && !stopped) {
@@ -790,8 +853,8 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         mbar_wait(v.mbar + 8u * (uint32_t)((s_stop - 1) & 1), (uint32_t)((s_stop - 1) >> 1) & 1u);
         mbar_wait(v.mbar + 8u * (uint32_t)(s_stop & 1), (uint32_t)(s_stop >> 1) & 1u);
     }
-    if (a.n_steps > 0 && warp >= 2)
-        reduce_partials(v.part + ((a.n_steps - 1) & 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp - 2, lane, os.sums, X);
+    if (a.n_steps > 0)
+        reduce_partials(v.part + ((a.n_steps - 1) & 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp, lane, os.sums, X);
     ode_bar();
     CellDyn &d = a.dyn[cell];
     for (int i = ot; i < kNumGlobals; i += kOdeLanes) d.g[i] = os.g[i];
@@ -809,14 +872,338 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
     cluster_wait();
 }
 
+// A warp's flux partial of a step of parity par, pushed by lane 0 straight into the leader's slot (rank,
+// warp) by 16-byte asynchronous stores that count themselves off the leader's mbarrier of this parity
+// (the warp goes on without waiting for them to land); the leader sums the cell's warp partials.
+template <bool FP64, bool ODE64>
+__device__ __forceinline__ void send_partial(const KernelArgs &a, const CtaView<FP64, ODE64> &v, int par, int pslot,
+                                             const Partial<FP64> &pv) {
+    if (v.lane != 0) return;
+    Partial<FP64> *dst = v.part + par * pslot + v.w.rank_in_cell * kMaxWarps + v.warp;
+    const uint32_t rd = map_rank(dst, (uint32_t)v.w.first);
+    const uint32_t rm = map_rank_addr(v.mbar + 8u * (uint32_t)par, (uint32_t)v.w.first);
+    if constexpr (FP64) {
+        st_async(rd, make_uint4(lo_of(pv.v[0]), hi_of(pv.v[0]), lo_of(pv.v[1]), hi_of(pv.v[1])), rm);
+        st_async(rd + 16u, make_uint4(lo_of(pv.v[2]), hi_of(pv.v[2]), lo_of(pv.v[3]), hi_of(pv.v[3])), rm);
+    } else {
+        st_async(rd, make_uint4((uint32_t)pv.jh, (uint32_t)pv.jl, (uint32_t)pv.xh, (uint32_t)pv.xl), rm);
+        st_async(rd + 16u, make_uint4((uint32_t)pv.th, (uint32_t)pv.tl, (uint32_t)pv.cl, (uint32_t)pv.flag), rm);
+    }
+}
+
+// The step of the CRUs held by a warp's eight groups of four lanes (m < 0: none), from begin().
+__device__ __forceinline__ void group_run(const KernelArgs &a, const SsaConsts<float> &cc, TileRec<float> *tile, int m,
+                                          Cru<float> &c, SsaLane<float, false> &sl, Stream &rng, const float *sv,
+                                          const float2 *rtab, uint32_t tag, FluxAcc<false> &acc,
+                                          unsigned long long &my_events, int &my_err) {
+    while (__any_sync(0xffffffffu, m >= 0)) {
+        int err = 0;
+        const bool done = sl.iterate_group(m >= 0, c, cc, sv, rtab, rng, (float)a.dt, a.event_cap, err);
+        if (m >= 0 && done) {
+            if ((threadIdx.x & 3u) == 0u) {
+                tile_put(tile[m], c, tag);
+                my_events += (unsigned long long)sl.ev;
+                my_err |= err;
+                acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
+                        __popc((c.flags >> 4) & 0xFu));
+            }
+            m = -1;
+        }
+    }
+}
+
+// The FP32 SSA of a CTA with few CRUs (v.grouped): every CRU on four lanes, eight per warp at a time, each warp
+// with a contiguous range.  With up to 128 CRUs in a CTA of 16 warps that is one pass, 2.0 k cycles without
+// an event and 5.3 k with one, and the global step beside it sets the time: 3.2 us per step for a cell of
+// 777 CRUs over 9 to 16 CTAs (4.4 with one CRU per lane), 4.6 in split_steps over 4.
+template <bool ODE64>
+__device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<false, ODE64> &v, uint64_t step0,
+                                            unsigned long long &my_events, int &my_err, int &s_stop) {
+    const CtaWork &w = v.w;
+    const int warp = v.warp, lane = v.lane, cell = w.cell;
+    const SsaConsts<float> &cc = *v.cc;
+    TileRec<float> *tile = v.tile;
+    const int pslot = a.max_cta_cell * kMaxWarps;
+    const uint32_t rcell = (uint32_t)(a.cell_base + cell);
+    const int nse = max(1, min(v.leader ? w.lead_warps : v.n_ssa >> 5, (w.cru_count + 7) >> 3));
+    const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
+    const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
+    for (int s = 0; s < a.n_steps; ++s) {
+        const int par = s & 1;
+        const int64_t ri = a.run_step0 + s;
+        const bool rec = a.record_every > 0 && (ri % a.record_every) == 0;
+        const int64_t r_idx = rec ? ri / a.record_every - a.rec_base : -1;
+        const bool rec_ok = rec && r_idx >= 0 && r_idx < a.rec_cap;
+        if (my_err & 2) continue;
+        // (as in split_steps; the first two warps wait, one entry of the rate table per lane)
+        const uint32_t svm = v.mbar + 16u + 8u * (uint32_t)par;
+        if (threadIdx.x == 0) mbar_arrive_expect_tx(svm, (uint32_t)(kSvCount * sizeof(float)));
+        const float *sv = v.svbuf + par * kSvCount;
+        float2 *rtab = v.rtab + par * kRateTab;
+        FluxAcc<false> acc;
+        Cru<float> c;
+        SsaLane<float, false> sl;
+        Stream rng;
+        bool bad = false;
+        __syncwarp();  // (the CRUs of the last step are stored)
+        for (int b = beg;; b += 8) {
+            // (a group without a CRU computes along on the range's last)
+            int m = min(b + (lane >> 2), end - 1);
+            tile_get(c, tile[max(m, 0)]);
+            rng.open(a.seed, rcell, (uint32_t)(w.cru_begin + m), step0 + s, 0);
+            sl.begin(c, cc);
+            if (b + (lane >> 2) >= end) m = -1;
+            if (b == beg) {
+                if (warp < 2) {
+                    bad = !mbar_wait_warp(svm, (uint32_t)(s >> 1) & 1u);
+                    for (int e = (int)threadIdx.x; e < kRateTab; e += 64) build_rate_entry<float>(rtab, cc, sv, e);
+                }
+                bad = bar_or(2, v.n_ssa, bad);
+                if (bad) break;
+            }
+            group_run(a, cc, tile, m, c, sl, rng, sv, rtab, (uint32_t)s + 2u, acc, my_events, my_err);
+            if (b + 8 >= end) break;
+        }
+        if (bad) {
+            my_err |= 2;
+            s_stop = s;
+            continue;
+        }
+        if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr)) {
+            __syncwarp();
+            record_pass<float>(a, w, cell, r_idx, beg, end, lane, tile);
+        }
+        send_partial<false, ODE64>(a, v, par, pslot, acc.warp_total());
+    }
+}
+
+// The FP32 SSA of a CTA with more CRUs, split by the kind of work.
+//
+// Quiet passes, on the first nq warps, in groups of 32 of the CTA's CRUs: every CRU through the step as
+// if it had no jump (SsaLane::quiet), 32 at a time with full lanes.  A CRU that may have a
+// jump is left untouched, tagged with the step and put in the CTA's queue.
+// Events, on the other warps: the queued CRUs through all their iterations, in batches that a warp claims
+// as they are queued: eight, each on four lanes.
+// The split follows the load (quiet_warps): warp 0 sets nq of step s + 1 from the events up to step s - 2.
+//
+// (With both kinds in one loop, one or two lanes of a warp with an event made the other thirty walk
+// through the event code, in most passes: 17 of 32 lanes active during the release.  A pass takes 2.4 k
+// cycles beside eleven others, a batch 5.5 k to 8 k.  us per step, one loop before: a 12,500-CRU cell over 16
+// CTAs 6.7 at rest, 10.6 amid the release, now 5.9 and 8.9; 256 mixed cells amid the release 132, now 113.
+// A queue per warp run at its end costs about as much as one loop, its few lanes' event code being as long
+// as all the quiet passes; one CRU per lane for the events takes twice the latency.)
+//
+// The quiet passes do not wait for the events of the step before: the CRUs of step s's queue are skipped
+// by their tag at step s + 1 and taken last, in the queue's order, once the events of step s are through.
+// Buffers: the SSA values, the rate table and the split of step s are used until the warps send their
+// partials of step s, and rewritten for step s + 2, whose SSA values the leader sends only after those
+// partials.  The queue of step s, one of three, is used until the quiet passes of step s + 1 are through
+// (m_quiet), and cleared for step s + 3 after that.
+// m_quiet(s): every warp arrives when its quiet passes of step s are through, its queue entries written;
+// m_event(s): when it finds no more events of step s.  Two of each, by parity: the phase of step s + 2
+// takes every warp's arrival in step s + 2, so a waiter is at most one phase behind and the parity tells
+// the two apart.
+//
+// The split: of nw warps, as many take events as make the rounds of quiet passes plus the event batches per
+// warp shortest, a batch counting as kBatchCost passes, for load / 8 events; the present one (nq quiet
+// warps) stays unless it is an eighth longer, since a warp that comes back from the events holds the quiet
+// passes up.
+__device__ __forceinline__ int quiet_warps(int nw, int n_crus, int load, int lane, int nq) {
+    const int groups = (n_crus + 31) / 32 + (load + 255) / 256;
+    const int ne = min(lane + 1, nw >> 1);  // one choice per lane
+    const int cost = 8 * ((groups + nw - ne - 1) / (nw - ne)) + kBatchCost * max(8, (load + (load >> 2)) / (8 * ne));
+    const unsigned best = __reduce_min_sync(0xffffffffu, ((unsigned)cost << 5) | (unsigned)ne);
+    const int now = __shfl_sync(0xffffffffu, cost, max(nw - nq - 1, 0));
+    return nq > 0 && now <= (int)(best >> 5) * 9 / 8 ? nq : nw - (int)(best & 31u);
+}
+template <bool ODE64>
+__device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<false, ODE64> &v, uint64_t step0,
+                                            unsigned long long &my_events, int &my_err, int &s_stop) {
+    const CtaWork &w = v.w;
+    const int warp = v.warp, lane = v.lane, cell = w.cell, nw = v.n_ssa >> 5, n_crus = w.cru_count;
+    const SsaConsts<float> &cc = *v.cc;
+    TileRec<float> *tile = v.tile;
+    const int pslot = a.max_cta_cell * kMaxWarps;
+    const float dt = (float)a.dt;
+    const uint32_t rcell = (uint32_t)(a.cell_base + cell);
+    uint16_t *const queues = reinterpret_cast<uint16_t *>(v.fq + 8);
+    int load = n_crus >> 2;  // (warp 0) eight times the recent events per step; until known, one in 32 CRUs
+    int nq = quiet_warps(nw, n_crus, load, lane, 0);
+    bool bad = false;  // a wait ran out
+    int slot = 0;      // s mod 3
+    for (int s = 0; s < a.n_steps; ++s) {
+        const int par = s & 1;
+        const uint32_t ph = (uint32_t)(s >> 1) & 1u, ph_prev = (uint32_t)((s - 1) >> 1) & 1u;
+        const uint32_t bars = v.mbar + 8u * (uint32_t)par, bars_prev = v.mbar + 8u * (uint32_t)(par ^ 1);
+        constexpr uint32_t kSv = 16u, kQuiet = 32u, kEvent = 48u, kClear = 64u;
+        if (my_err & 2) continue;
+        const float *sv = v.svbuf + par * kSvCount;
+        float2 *rtab = v.rtab + par * kRateTab;
+        const uint32_t tag = (uint32_t)s + 2u;
+        const int slot_prev = slot == 0 ? 2 : slot - 1, slot_next = slot == 2 ? 0 : slot + 1;
+        uint16_t *q = queues + slot * a.tile_cap;
+        int *const q_put = v.fq + 2 * slot, *const q_got = q_put + 1;
+        const bool quiet_warp = warp < nq;
+        FluxAcc<false> acc;
+        int taken = 0;
+        int nq_next;
+        if (!quiet_warp) {
+            // (each of these waits for itself: they may be in different steps, the set changing with nq)
+            if (lane == 0) mbar_arrive(bars + kQuiet);
+            bad |= !mbar_wait_warp(bars + kClear, ph);
+            if (bad) {
+                my_err |= 2;  // the leader's wait for this warp's partial runs out in turn
+                continue;
+            }
+            nq_next = v.fq[6 + (par ^ 1)];
+        } else {
+            // The SSA values of step s arrive by st.async from the leader's ODE warps and complete this
+            // CTA's mbarrier of parity par (thread 0 declares the bytes; that mbarrier's previous phase,
+            // step s-2's, completed before this CTA's waits of step s-2).  The quiet warps meet at named
+            // barrier 2 (bar_or below) and take the waits' outcome together: after a wait has run out
+            // the CTA stops for the rest of the launch (no more sends), so that its partners stop too.
+            if (threadIdx.x == 0) mbar_arrive_expect_tx(bars + kSv, (uint32_t)(kSvCount * sizeof(float)));
+            // (the first warp alone waits and builds the rate table: a waiting warp's polling takes issue
+            // slots, a warp at a named barrier none)
+            if (warp == 0) {
+                bad |= !mbar_wait_warp(bars + kSv, ph);
+                // (with the split a group may pass to another warp, and its last one may take events now)
+                if (s > 0) bad |= !mbar_wait_warp(bars_prev + kQuiet, ph_prev);
+                // the split of step s + 1, from the events of step s - 2
+                const int n_events = v.fq[2 * slot_next] & 0xFFFF;
+                load = s < 2 ? load : (s == 2 ? 8 * n_events : load + n_events - (load >> 3));
+                const int nq1 = quiet_warps(nw, n_crus, load, lane, s <= 2 ? 0 : nq);
+                __syncwarp();
+                if (lane == 0) v.fq[6 + (par ^ 1)] = nq1;
+                if (lane == 0) v.fq[2 * slot_next] = v.fq[2 * slot_next + 1] = 0;
+                for (int e = lane; e < kRateTab; e += 32) build_rate_entry<float>(rtab, cc, sv, e);
+            }
+            if (bar_or(2, nq * 32, bad)) {
+                my_err |= 2;
+                s_stop = s;
+                continue;
+            }
+            nq_next = v.fq[6 + (par ^ 1)];
+            if (warp == 0) {
+                if (lane == 0) mbar_arrive(bars + kClear);  // to the event warps
+            }
+            StepDraw draw;
+            draw.open(a.seed, rcell, step0 + s, 0);
+            // The CTA's groups of 32, without the CRUs of step s-1's queue, then the groups of those, in turn
+            // to the quiet warps.
+            const int n_own = (n_crus + 31) >> 5, n_late = s > 0 ? v.fq[2 * slot_prev] & 0xFFFF : 0;
+            const uint16_t *q_prev = queues + slot_prev * a.tile_cap;
+            bool waited = false;
+            for (int g = warp; g < n_own + ((n_late + 31) >> 5); g += nq) {
+                const bool late = g >= n_own;
+                int m = 32 * g + lane;
+                if (late) {
+                    if (!waited) bad |= !mbar_wait_warp(bars_prev + kEvent, ph_prev);
+                    waited = true;
+                    m -= 32 * n_own;
+                    m = m < n_late ? (int)q_prev[m] : -1;
+                } else if (m >= n_crus) {
+                    m = -1;
+                }
+                // (a lane without a CRU computes along on the CTA's first: no branch in the pass)
+                Cru<float> c;
+                SsaLane<float, false> sl;
+                TileRec<float> &rec_m = tile[max(m, 0)];
+                tile_get(c, rec_m);
+                // (its group's pass may reach a CRU of step s-1's queue before or after that was taken here)
+                const bool valid = m >= 0 && (late || tile_tag(rec_m) < tag - 1u);
+                sl.begin(c, cc);
+                const bool quiet = sl.quiet(c, cc, sv, rtab, draw.word((uint32_t)(w.cru_begin + m)), dt);
+                const bool done = valid && quiet, jumps = valid && !quiet;
+                if (done) tile_put_quiet(rec_m, c, late ? tag - 1u : 0u);
+                taken += 32;
+                acc.add(done ? c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3] : 0.f, done ? sl.jxfer_sum : 0.f,
+                        done ? sl.jtr : 0.f, done ? __popc((c.flags >> 4) & 0xFu) : 0);
+                const unsigned em = __ballot_sync(0xffffffffu, jumps);
+                if (em == 0u) continue;
+                // into the queue: slots reserved, written, then counted as written
+                const int ne = __popc(em);
+                int q0 = 0;
+                if (lane == 0) q0 = atomicAdd(q_put, ne << 16) >> 16;
+                q0 = __shfl_sync(0xffffffffu, q0, 0);
+                if (jumps) {
+                    tile_tag(rec_m) = tag;
+                    q[q0 + __popc(em & ((1u << lane) - 1u))] = (uint16_t)m;
+                }
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) atomicAdd(q_put, ne);
+            }
+            // the warp's queue entries and CRUs are stored
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + kQuiet);
+        }
+        while (!quiet_warp) {
+            // The next batch, claimed by lane 0 for the warp (bounded: the quiet warps arrive, or their own
+            // wait ran out).  Every lane polls, with the loop's branches on votes: see mbar_wait_warp.
+            int h = -1, n = 0;
+            const long long t0 = clock64();
+            for (;;) {
+                const bool fin = __all_sync(0xffffffffu, mbar_test(bars + kQuiet, ph));
+                if (lane == 0) {
+                    const int word = *(volatile int *)q_put, head = *(volatile int *)q_got;
+                    const int written = (word & 0xFFFF) == (word >> 16) ? word & 0xFFFF : 0;
+                    n = written - head;
+                    n = n >= 8 || fin ? min(n, 8) : 0;
+                    if (n > 0 && atomicCAS(q_got, head, head + n) == head) h = head;
+                }
+                h = __shfl_sync(0xffffffffu, h, 0);
+                n = __shfl_sync(0xffffffffu, n, 0);
+                if (h >= 0 || (fin && n <= 0)) break;
+                if (n <= 0) __nanosleep(20);
+                if (__any_sync(0xffffffffu, clock64() - t0 > (1ll << 32))) {
+                    bad = true;
+                    break;
+                }
+            }
+            if (h < 0) break;
+            __threadfence_block();
+            taken += n;
+            // (a group without a CRU holds, and computes along on, the batch's last)
+            const int i = lane >> 2;
+            int m = q[h + min(i, n - 1)];
+            Cru<float> c;
+            SsaLane<float, false> sl;
+            Stream rng;
+            tile_get(c, tile[m]);
+            rng.open(a.seed, rcell, (uint32_t)(w.cru_begin + m), step0 + s, 0);
+            sl.begin(c, cc);
+            if (i >= n) m = -1;
+            group_run(a, cc, tile, m, c, sl, rng, sv, rtab, tag, acc, my_events, my_err);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars + kEvent);
+        acc.big |= taken > kMaxSumCrus;
+        const int64_t ri = a.run_step0 + s;
+        if (quiet_warp && a.record_every > 0 && (ri % a.record_every) == 0 && (cell == a.tr_cell || a.tr_sums != nullptr)) {
+            // records of this step, from the warp's part of the tile at the end of the step
+            const int64_t r_idx = ri / a.record_every - a.rec_base;
+            if (r_idx >= 0 && r_idx < a.rec_cap) {
+                bad |= !mbar_wait_warp(bars + kEvent, ph);
+                const int beg = (int)((int64_t)n_crus * warp / nq), end = (int)((int64_t)n_crus * (warp + 1) / nq);
+                record_pass<float>(a, w, cell, r_idx, beg, end, lane, tile);
+                __syncwarp();
+            }
+        }
+        send_partial<false, ODE64>(a, v, par, pslot, acc.warp_total());
+        nq = nq_next;
+        slot = slot_next;
+    }
+    if (bad) my_err |= 2;
+}
+
 // The SSA warps over a launch (every warp of a CTA that is not a leader's ODE warp, and every
 // warp of an idle CTA, which only keeps the closing cluster barrier): per global step the SSA of
-// the warp's CRUs, the record pass and the flux partials, and the tile back to the cell's planes
-// at the end.  Inlined into the kernel (out of line it spills).
+// the warp's CRUs, the record pass and the flux partials (FP32: group_steps or split_steps), and the
+// tile back to the cell's planes at the end.  Inlined into the kernel (out of line it spills).
 template <bool FP64, bool ODE64>
 __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
     using R = typename std::conditional<FP64, double, float>::type;
-    constexpr bool EXACT = FP64;
     const CtaView<FP64, ODE64> v(a);
     const CtaWork &w = v.w;
     const int warp = v.warp, lane = v.lane, cell = w.cell, n_ssa = v.n_ssa;
@@ -827,139 +1214,79 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
     unsigned long long my_events = 0;
     int my_err = 0;  // bit 0: a CRU hit the event cap; bit 1: a wait for the SSA values ran out
     int s_stop = -1;  // the step whose wait ran out
-    for (int s = 0; s < a.n_steps; ++s) {
-        const int par = s & 1;
-        const int64_t ri = a.run_step0 + s;
-        const bool rec = a.record_every > 0 && (ri % a.record_every) == 0;
-        const int64_t r_idx = rec ? ri / a.record_every - a.rec_base : -1;
-        const bool rec_ok = rec && r_idx >= 0 && r_idx < a.rec_cap;
-        if (v.active && !(my_err & 2)) {
-            // The SSA values of step s arrive by st.async from the leader's ODE warps and complete
-            // this CTA's mbarrier of parity par (thread 0 declares the bytes; that mbarrier's
-            // previous phase, step s-2's, completed before this CTA's waits of step s-2).  The
-            // CTA's SSA threads then meet at named barrier 2 (bar_or below; the CTAs of a cell are
-            // held together only by their data) and take the wait's outcome together: after a
-            // wait has run out the CTA stops for the rest of the launch (no more sends), so that
-            // its partners stop too.
-            const uint32_t svm = v.mbar + 16u + 8u * (uint32_t)par;
-            if (threadIdx.x == 0) mbar_arrive_expect_tx(svm, (uint32_t)(kSvCount * sizeof(R)));
-            const bool ok = mbar_wait(svm, (uint32_t)(s >> 1) & 1u);
-            const R *sv = v.svbuf + par * kSvCount;
-            // FP32: the CTA's rate table of this step, entry e by SSA thread e, into the table of
-            // this parity, before bar_or(2) of step s, which publishes it.  No reader of that
-            // table (step s-2's) can remain: every SSA thread passed bar_or of step s-1 after its
-            // last iteration of step s-2.  A warp still in step s-1 reads the other table.
-            float2 *rtab = v.rtab + par * kRateTab;
-            if (!FP64)
-                for (int e = (int)threadIdx.x; e < kRateTab; e += n_ssa) build_rate_entry<R>(rtab, cc, sv, e);
-            // FP64: float copies of the step's SSA values for the screen, in the same place and
-            // under the same rule (floats 0..kSvCount-1 of this parity's table)
-            float *svf = reinterpret_cast<float *>(rtab);
-            const float *sk = reinterpret_cast<const float *>(v.rtab) + 64;
-            if (FP64)
+    if constexpr (FP64) {
+        for (int s = 0; s < a.n_steps; ++s) {
+            const int par = s & 1;
+            const int64_t ri = a.run_step0 + s;
+            const bool rec = a.record_every > 0 && (ri % a.record_every) == 0;
+            const int64_t r_idx = rec ? ri / a.record_every - a.rec_base : -1;
+            const bool rec_ok = rec && r_idx >= 0 && r_idx < a.rec_cap;
+            if (v.active && !(my_err & 2)) {
+                // The SSA values of step s arrive by st.async from the leader's ODE warps and complete
+                // this CTA's mbarrier of parity par (thread 0 declares the bytes; that mbarrier's
+                // previous phase, step s-2's, completed before this CTA's waits of step s-2).  The
+                // CTA's SSA threads then meet at named barrier 2 (bar_or below; the CTAs of a cell are
+                // held together only by their data) and take the wait's outcome together: after a
+                // wait has run out the CTA stops for the rest of the launch (no more sends), so that
+                // its partners stop too.
+                const uint32_t svm = v.mbar + 16u + 8u * (uint32_t)par;
+                if (threadIdx.x == 0) mbar_arrive_expect_tx(svm, (uint32_t)(kSvCount * sizeof(R)));
+                const bool ok = mbar_wait_warp(svm, (uint32_t)(s >> 1) & 1u);
+                const R *sv = v.svbuf + par * kSvCount;
+                // Float copies of the step's SSA values for the screen, in the rate-table area of this
+                // parity (floats 0..kSvCount-1), before bar_or(2) of step s, which publishes them.  No reader
+                // of that area (step s-2's) can remain: every SSA thread passed bar_or of step s-1 after its
+                // last iteration of step s-2.  A warp still in step s-1 reads the other one.
+                float2 *rtab = v.rtab + par * kRateTab;
+                float *svf = reinterpret_cast<float *>(rtab);
+                const float *sk = reinterpret_cast<const float *>(v.rtab) + 64;
                 for (int e = (int)threadIdx.x; e < kSvCount; e += n_ssa) svf[e] = (float)sv[e];
-            if (bar_or(2, n_ssa, !ok)) {
-                my_err |= 2;
-                s_stop = s;
-                continue;
-            }
-            const int nsw = n_ssa >> 5;
-            // This warp's CRUs [cursor, end).  A lane whose CRU has finished its step takes the
-            // next one, so lanes with pending SSA events do not hold the others back.
-            // (a leader takes CRUs on its first lead_warps SSA warps only, possibly none)
-            // FP64: no more working warps than ceil(CRUs / 32).  An FP64 warp instruction takes its
-            // sub-partition's FP64 pipe for ~64 cycles whatever its active lanes, so two warps of
-            // 16 CRUs cost twice one warp of 32; the first warps of a CTA sit on distinct
-            // sub-partitions.
-            int nse = v.leader ? w.lead_warps : nsw;
-            if (FP64) nse = min(nse, (w.cru_count + 31) >> 5);
-            const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
-            const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
-            int cursor = beg;
-            FluxAcc<FP64> acc;
-            Cru<R> c;
-            SsaLane<R, EXACT> sl;
-            Stream rng;
-            int m = -1;  // CRU of this lane; -1 none yet, -2 none left
-            if constexpr (FP64) {
-                // Pass 1: the warp's CRUs, one iteration per lane and pass.  An iteration that the
-                // FP32 screen shows to be the step's last runs without the FP64 rates (finish); a
-                // CRU whose first iteration it declines (an event in the step) goes, untouched in
-                // the tile, to the CTA's queue, and its lane takes the next CRU.
-                int *qn = v.fq + par;
-                int *q = v.fq + 4;
-                if (threadIdx.x == 0) v.fq[par ^ 1] = 0;  // step s-1's count: every reader has passed
-                                                          // bar_or(2) of this step
-                bool fresh = false;
-                for (;;) {
-                    const unsigned need = __ballot_sync(0xffffffffu, m == -1);
-                    if (need) {
-                        const int nm = cursor + __popc(need & ((1u << lane) - 1u));
-                        cursor += __popc(need);
-                        if (m == -1) {
-                            if (nm < end) {
-                                m = nm;
-                                tile_get(c, tile[m]);
-                                rng.open(a.seed, (uint32_t)(a.cell_base + cell), (uint32_t)(w.cru_begin + m),
-                                         step0 + s, 0);
-                                sl.begin(c, cc);
-                                fresh = true;
-                            } else {
-                                m = -2;
-                            }
-                        }
-                    }
-                    if (!__any_sync(0xffffffffu, m >= 0)) break;
-                    if (m >= 0) {
-                        int err = 0;
-                        bool done = false;
-                        if (sl.surely_last(c, cc, sk, svf, rng, dt)) {
-                            sl.finish(c, cc, sv, rng, dt);
-                            done = true;
-                        } else {
-                            const int qs = fresh ? atomicAdd(qn, 1) : kEngQCap;
-                            if (qs < kEngQCap) {
-                                q[qs] = m;
-                                m = -1;
-                            } else {  // the queue is full, or the CRU is past its first iteration
-                                done = sl.iterate(c, cc, sv, rtab, rng, dt, a.event_cap, err);
-                            }
-                        }
-                        fresh = false;
-                        if (done) {
-                            tile_put(tile[m], c);
-                            my_events += (unsigned long long)sl.ev;
-                            my_err |= err;
-                            acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
-                                    __popc((c.flags >> 4) & 0xFu));
-                            m = -1;
-                        }
-                    }
+                if (bar_or(2, n_ssa, !ok)) {
+                    my_err |= 2;
+                    s_stop = s;
+                    continue;
                 }
-                // Pass 2: the queued CRUs on four lanes each (SsaLane::iterate_group: one subunit's
-                // rates per lane), eight per warp at a time, over the CTA's SSA warps.
-                ssa_bar(n_ssa);
-                const int nq = min(*qn, kEngQCap);
-                const int jq = lane & 3, base = lane & ~3;
-                const int nwu = min(nsw, (nq + 7) >> 3);
-                if (warp < nwu) {
-                    int qc = (int)((int64_t)nq * warp / nwu);
-                    const int qe = (int)((int64_t)nq * (warp + 1) / nwu);
-                    m = -1;
-                    bool first = false;
+                const int nsw = n_ssa >> 5;
+                // This warp's CRUs [cursor, end).  A lane whose CRU has finished its step takes the
+                // next one, so lanes with pending SSA events do not hold the others back.
+                // (a leader takes CRUs on its first lead_warps SSA warps only, possibly none)
+                // No more working warps than ceil(CRUs / 32).  An FP64 warp instruction takes its
+                // sub-partition's FP64 pipe for ~64 cycles whatever its active lanes, so two warps of
+                // 16 CRUs cost twice one warp of 32; the first warps of a CTA sit on distinct
+                // sub-partitions.
+                int nse = v.leader ? w.lead_warps : nsw;
+                nse = min(nse, (w.cru_count + 31) >> 5);
+                const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
+                const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
+                int cursor = beg;
+                FluxAcc<FP64> acc;
+                Cru<R> c;
+                SsaLane<R, true> sl;
+                Stream rng;
+                int m = -1;  // CRU of this lane; -1 none yet, -2 none left
+                {
+                    // Pass 1: the warp's CRUs, one iteration per lane and pass.  An iteration that the
+                    // FP32 screen shows to be the step's last runs without the FP64 rates (finish); a
+                    // CRU whose first iteration it declines (an event in the step) goes, untouched in
+                    // the tile, to the CTA's queue, and its lane takes the next CRU.
+                    int *qn = v.fq + par;
+                    int *q = v.fq + 4;
+                    if (threadIdx.x == 0) v.fq[par ^ 1] = 0;  // step s-1's count: every reader has passed
+                                                              // bar_or(2) of this step
+                    bool fresh = false;
                     for (;;) {
-                        const unsigned need = __ballot_sync(0xffffffffu, m == -1 && jq == 0);
+                        const unsigned need = __ballot_sync(0xffffffffu, m == -1);
                         if (need) {
-                            const int nm = qc + __popc(need & ((1u << base) - 1u));
-                            qc += __popc(need);
+                            const int nm = cursor + __popc(need & ((1u << lane) - 1u));
+                            cursor += __popc(need);
                             if (m == -1) {
-                                if (nm < qe) {
-                                    m = q[nm];
+                                if (nm < end) {
+                                    m = nm;
                                     tile_get(c, tile[m]);
                                     rng.open(a.seed, (uint32_t)(a.cell_base + cell), (uint32_t)(w.cru_begin + m),
                                              step0 + s, 0);
                                     sl.begin(c, cc);
-                                    first = true;
+                                    fresh = true;
                                 } else {
                                     m = -2;
                                 }
@@ -968,81 +1295,93 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                         if (!__any_sync(0xffffffffu, m >= 0)) break;
                         if (m >= 0) {
                             int err = 0;
-                            bool done;
-                            if (!first && sl.surely_last(c, cc, sk, svf, rng, dt)) {
+                            bool done = false;
+                            if (sl.surely_last(c, cc, sk, svf, rng, dt)) {
                                 sl.finish(c, cc, sv, rng, dt);
                                 done = true;
                             } else {
-                                done = sl.iterate_group(c, cc, sv, rng, dt, a.event_cap, err);
-                            }
-                            first = false;
-                            if (done) {
-                                if (jq == 0) {
-                                    tile_put(tile[m], c);
-                                    my_events += (unsigned long long)sl.ev;
-                                    my_err |= err;
-                                    acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
-                                            __popc((c.flags >> 4) & 0xFu));
+                                const int qs = fresh ? atomicAdd(qn, 1) : kEngQCap;
+                                if (qs < kEngQCap) {
+                                    q[qs] = m;
+                                    m = -1;
+                                } else {  // the queue is full, or the CRU is past its first iteration
+                                    done = sl.iterate(c, cc, sv, rtab, rng, dt, a.event_cap, err);
                                 }
+                            }
+                            fresh = false;
+                            if (done) {
+                                tile_put(tile[m], c);
+                                my_events += (unsigned long long)sl.ev;
+                                my_err |= err;
+                                acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
+                                        __popc((c.flags >> 4) & 0xFu));
                                 m = -1;
                             }
                         }
                     }
-                }
-                // the records read the warps' tile ranges, which pass 2 may have written elsewhere
-                if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr)) ssa_bar(n_ssa);
-            } else {
-                for (;;) {
-                    const unsigned need = __ballot_sync(0xffffffffu, m == -1);
-                    if (need) {
-                        const int nm = cursor + __popc(need & ((1u << lane) - 1u));
-                        cursor += __popc(need);
-                        if (m == -1) {
-                            if (nm < end) {
-                                m = nm;
-                                tile_get(c, tile[m]);
-                                rng.open(a.seed, (uint32_t)(a.cell_base + cell), (uint32_t)(w.cru_begin + m),
-                                         step0 + s, 0);
-                                sl.begin(c, cc);
-                            } else {
-                                m = -2;
+                    // Pass 2: the queued CRUs on four lanes each (SsaLane::iterate_group: one subunit's
+                    // rates per lane), eight per warp at a time, over the CTA's SSA warps.
+                    ssa_bar(n_ssa);
+                    const int nq = min(*qn, kEngQCap);
+                    const int jq = lane & 3, base = lane & ~3;
+                    const int nwu = min(nsw, (nq + 7) >> 3);
+                    if (warp < nwu) {
+                        int qc = (int)((int64_t)nq * warp / nwu);
+                        const int qe = (int)((int64_t)nq * (warp + 1) / nwu);
+                        m = -1;
+                        bool first = false;
+                        for (;;) {
+                            const unsigned need = __ballot_sync(0xffffffffu, m == -1 && jq == 0);
+                            if (need) {
+                                const int nm = qc + __popc(need & ((1u << base) - 1u));
+                                qc += __popc(need);
+                                if (m == -1) {  // (a group without one holds the range's last)
+                                    const int mq = q[min(nm, qe - 1)];
+                                    tile_get(c, tile[mq]);
+                                    rng.open(a.seed, (uint32_t)(a.cell_base + cell), (uint32_t)(w.cru_begin + mq),
+                                             step0 + s, 0);
+                                    sl.begin(c, cc);
+                                    first = true;
+                                    m = nm < qe ? mq : -2;
+                                }
+                            }
+                            if (!__any_sync(0xffffffffu, m >= 0)) break;
+                            // (a group that ended its CRU with finish(), or has none, computes along)
+                            int err = 0;
+                            bool done = m >= 0 && !first && sl.surely_last(c, cc, sk, svf, rng, dt);
+                            if (done) sl.finish(c, cc, sv, rng, dt);
+                            const bool more = m >= 0 && !done;
+                            if (__any_sync(0xffffffffu, more))
+                                done |= sl.iterate_group(more, c, cc, sv, rng, dt, a.event_cap, err) && more;
+                            first = false;
+                            if (m >= 0) {
+                                if (done) {
+                                    if (jq == 0) {
+                                        tile_put(tile[m], c);
+                                        my_events += (unsigned long long)sl.ev;
+                                        my_err |= err;
+                                        acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
+                                                __popc((c.flags >> 4) & 0xFu));
+                                    }
+                                    m = -1;
+                                }
                             }
                         }
                     }
-                    if (!__any_sync(0xffffffffu, m >= 0)) break;
-                    if (m >= 0) {
-                        int err = 0;
-                        if (sl.iterate(c, cc, sv, rtab, rng, dt, a.event_cap, err)) {
-                            tile_put(tile[m], c);
-                            my_events += (unsigned long long)sl.ev;
-                            my_err |= err;
-                            acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
-                                    __popc((c.flags >> 4) & 0xFu));
-                            m = -1;
-                        }
-                    }
+                    // the records read the warps' tile ranges, which pass 2 may have written elsewhere
+                    if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr)) ssa_bar(n_ssa);
                 }
-            }
-            // Records of this step, from the warp's part of the tile (now at the end of the step)
-            if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr))
-                record_pass<R>(a, w, cell, r_idx, beg, end, lane, tile);
-            // The warp partial, pushed straight into the leader's slot (rank, warp): the leader
-            // sums the cell's warp partials in slot order (no reduction on this side).
-            const Partial<FP64> pv = acc.warp_total();
-            if (lane == 0) {
-                // 16-byte asynchronous stores that count themselves off the leader's mbarrier of this
-                // parity (the warp goes on without waiting for them to land)
-                Partial<FP64> *dst = v.part + par * pslot + w.rank_in_cell * kMaxWarps + warp;
-                const uint32_t rd = map_rank(dst, (uint32_t)w.first);
-                const uint32_t rm = map_rank_addr(v.mbar + 8u * (uint32_t)par, (uint32_t)w.first);
-                if constexpr (FP64) {
-                    st_async(rd, make_uint4(lo_of(pv.v[0]), hi_of(pv.v[0]), lo_of(pv.v[1]), hi_of(pv.v[1])), rm);
-                    st_async(rd + 16u, make_uint4(lo_of(pv.v[2]), hi_of(pv.v[2]), lo_of(pv.v[3]), hi_of(pv.v[3])), rm);
-                } else {
-                    st_async(rd, make_uint4(__float_as_uint(pv.j), __float_as_uint(pv.x), __float_as_uint(pv.t), (uint32_t)pv.cl), rm);
-                }
+                // Records of this step, from the warp's part of the tile (now at the end of the step)
+                if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr))
+                    record_pass<R>(a, w, cell, r_idx, beg, end, lane, tile);
+                send_partial<FP64, ODE64>(a, v, par, pslot, acc.warp_total());
             }
         }
+    } else if (v.active) {
+        if (v.grouped)
+            group_steps<ODE64>(a, v, step0, my_events, my_err, s_stop);
+        else
+            split_steps<ODE64>(a, v, step0, my_events, my_err, s_stop);
     }
     // A CTA that stopped at step s_stop may still receive the SSA values of steps s_stop and
     // s_stop + 1, stores the leader issued before it stopped in turn (it pushes step s + 2 only
@@ -1109,6 +1448,13 @@ __global__ void __launch_bounds__(FP64 ? kMaxThreadsFp64 : kMaxThreads, 1) engin
     // before the cluster barrier that every CTA passes before its first remote write.
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < 4; ++i) mbar_init(v.mbar + 8u * i, 1);
+        if (!FP64) {
+            for (uint32_t i = 0; i < 2; ++i) {
+                mbar_init(v.mbar + 32u + 8u * i, (uint32_t)(v.n_ssa >> 5));
+                mbar_init(v.mbar + 48u + 8u * i, (uint32_t)(v.n_ssa >> 5));
+                mbar_init(v.mbar + 64u + 8u * i, 1);
+            }
+        }
         mbar_fence_init();
     }
     cluster_arrive();
@@ -1126,6 +1472,7 @@ __global__ void __launch_bounds__(FP64 ? kMaxThreadsFp64 : kMaxThreads, 1) engin
                 v.fq[1] = 0;
             }
         }
+        if (!FP64 && threadIdx.x < 8) v.fq[threadIdx.x] = 0;
         // The leader's warp-partial slots start at zero (slots of warps a CTA does not have stay
         // so); the cell's CTAs write them only after the first cluster barrier of the steps.
         if (v.leader) {

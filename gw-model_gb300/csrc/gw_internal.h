@@ -68,6 +68,11 @@ struct CellDyn {
     int64_t stim_n;
 };
 
+// FP32 engine: CTAs with at most this many CRUs per SSA warp run every CRU on four lanes.
+constexpr int kGroupCrus = 16;
+// FP32 engine, larger CTAs: an event batch (eight CRUs) in quiet passes (32 CRUs).
+constexpr int kBatchCost = 4;
+
 // One CTA's share of work: a contiguous CRU range of one cell.  A cell's CTAs are contiguous in
 // its cluster, starting at cluster rank `first`; the first of them (the leader) runs the cell's
 // global ODE.
@@ -78,7 +83,7 @@ struct CtaWork {
     int rank_in_cell;
     int first;
     int n_cta_cell;
-    int lead_warps;  // SSA warps of the cell's leader CTA that take CRUs (0: the leader runs only
+    int lead_warps;  // warps of the cell's leader CTA that take CRUs (0: the leader runs only
                      // the global step, for cells spread thinly enough that it sets the step)
     int pad1;
 };

@@ -20,7 +20,7 @@
 // Precision.  FP64 (EXACT): reference expression order, FP64 everywhere, 53-bit uniforms; with
 // -fmad=false it reproduces the oracle to rounding of the transcendental functions.  FP32: CRU
 // state and propensities in FP32 with 24-bit uniforms, compensated Cai/CaNSR/CaJSR differences,
-// direct RyR totals and zero-weight guards in the transition scans (see ssa_cru).
+// direct RyR totals and zero-weight guards in the transition scans.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,25 +39,28 @@ constexpr double kFaraday = 96.5;  // common.hpp:9
 // Counter-based uniforms: Philox4x32-10 (Salmon et al., SC'11), key {seed_lo, seed_hi},
 // counter {draw >> 1, cru, step, (stream << 28) | cell}; draw k uses 64-bit lane pair k & 1.
 // ------------------------------------------------------------------------------------------
+__device__ __forceinline__ void philox_round(uint32_t (&c)[4], uint32_t k0, uint32_t k1) {
+    const uint32_t hi0 = __umulhi(0xD2511F53u, c[0]), lo0 = 0xD2511F53u * c[0];
+    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c[2]), lo1 = 0xCD9E8D57u * c[2];
+    c[0] = hi1 ^ c[1] ^ k0;
+    c[1] = lo1;
+    c[2] = hi0 ^ c[3] ^ k1;
+    c[3] = lo0;
+}
+// U: rounds unrolled.  The code of an event (draws, selection, re-splits) runs once in a while in every
+// step: what it costs is less its instructions than fetching them, so it takes the rounds in a loop.
+template <int U = 10>
 __device__ __forceinline__ void philox10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
                                          uint32_t k0, uint32_t k1, uint32_t out[4]) {
-#pragma unroll
+    uint32_t c[4] = {c0, c1, c2, c3};
+#pragma unroll U
     for (int r = 0; r < 10; ++r) {
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-        const uint32_t n0 = hi1 ^ c1 ^ k0;
-        const uint32_t n2 = hi0 ^ c3 ^ k1;
-        c0 = n0;
-        c1 = lo1;
-        c2 = n2;
-        c3 = lo0;
+        philox_round(c, k0, k1);
         k0 += 0x9E3779B9u;
         k1 += 0xBB67AE85u;
     }
-    out[0] = c0;
-    out[1] = c1;
-    out[2] = c2;
-    out[3] = c3;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = c[i];
 }
 
 struct Stream {
@@ -73,10 +76,11 @@ struct Stream {
         cellw = (stream << 28) | (cell & 0x0FFFFFFFu);
         blk = 0xFFFFFFFFu;
     }
+    template <int U = 10>
     __device__ __forceinline__ void words(uint32_t k, uint32_t &hi, uint32_t &lo) {
         const uint32_t want = k >> 1;
         if (want != blk) {
-            philox10(want, cru, step, cellw, k0, k1, b);
+            philox10<U>(want, cru, step, cellw, k0, k1, b);
             blk = want;
         }
         const bool h = (k & 1u) != 0;
@@ -84,32 +88,43 @@ struct Stream {
         lo = h ? b[2] : b[0];
     }
     // U53: max(w >> 11, 1) * 2^-53
+    template <int U = 10>
     __device__ __forceinline__ double u53(uint32_t k) {
         uint32_t hi, lo;
-        words(k, hi, lo);
+        words<U>(k, hi, lo);
         unsigned long long m = ((((unsigned long long)hi) << 32) | lo) >> 11;
         if (m == 0ull) m = 1ull;
         return (double)m * 0x1p-53;
     }
     // U24: max(w >> 40, 1) * 2^-24  (exact in float)
+    template <int U = 10>
     __device__ __forceinline__ float u24(uint32_t k) {
         uint32_t hi, lo;
-        words(k, hi, lo);
+        words<U>(k, hi, lo);
         uint32_t m = hi >> 8;
         if (m == 0u) m = 1u;
         return (float)m * 0x1p-24f;
     }
-    template <typename R>
-    __device__ __forceinline__ R uniform(uint32_t k);
+    template <typename R, int U = 2>
+    __device__ __forceinline__ R uniform(uint32_t k) {
+        if constexpr (sizeof(R) == 8) return u53<U>(k);
+        else return u24<U>(k);
+    }
     // U24 draws k, k+1, k+2 (an event selection's draws).  They lie in blocks k >> 1 and
     // (k >> 1) + 1; both are computed without a branch, so that their rounds interleave (the first
     // is often the block already held: recomputing it costs instructions but no latency), and the
     // second is kept for the next draws.
     __device__ __forceinline__ void u24x3(uint32_t k, float &a, float &b2, float &c) {
         const uint32_t B = k >> 1;
-        uint32_t o1[4], o2[4];
-        philox10(B, cru, step, cellw, k0, k1, o1);
-        philox10(B + 1u, cru, step, cellw, k0, k1, o2);
+        uint32_t o1[4] = {B, cru, step, cellw}, o2[4] = {B + 1u, cru, step, cellw};
+        uint32_t a0 = k0, a1 = k1;
+#pragma unroll 2
+        for (int r = 0; r < 10; ++r) {
+            philox_round(o1, a0, a1);
+            philox_round(o2, a0, a1);
+            a0 += 0x9E3779B9u;
+            a1 += 0xBB67AE85u;
+        }
         const bool odd = (k & 1u) != 0u;
         a = u24_of(odd ? o1[3] : o1[1]);
         b2 = u24_of(odd ? o2[1] : o1[3]);
@@ -126,14 +141,51 @@ struct Stream {
         return (float)m * 0x1p-24f;
     }
 };
-template <>
-__device__ __forceinline__ double Stream::uniform<double>(uint32_t k) {
-    return u53(k);
-}
-template <>
-__device__ __forceinline__ float Stream::uniform<float>(uint32_t k) {
-    return u24(k);
-}
+// Draw 0 of every CRU of one (seed, cell, step), for the FP32 lane's quiet pass: the parts of the
+// first three Philox rounds that do not depend on the CRU (the counter is {0, cru, step, cell}, so
+// round 1 multiplies 0 and the step, round 2 the CRU's word and a constant) are formed once per step,
+// and only the word that becomes the uniform is carried through the last two: 14 wide products
+// instead of 20 per CRU-step.
+struct StepDraw {
+    uint32_t k0, k1;  // key of round 4
+    uint32_t x1;      // round 1: word 0 = x1 ^ cru
+    uint32_t y2;      // round 2: word 2 = hi(M0 word 0) ^ y2, word 3 = lo(M0 word 0)
+    uint32_t x3, y3, z3;  // round 3: word 0 = hi(M1 word 2) ^ x3, word 2 = y3 ^ word 3, word 3 = z3
+    __device__ __forceinline__ void open(uint64_t seed, uint32_t cell, uint64_t step, uint32_t stream) {
+        const uint32_t s0 = (uint32_t)seed, s1 = (uint32_t)(seed >> 32);
+        const uint32_t w0 = 0x9E3779B9u, w1 = 0xBB67AE85u;
+        const uint32_t cellw = (stream << 28) | (cell & 0x0FFFFFFFu);
+        x1 = __umulhi(0xCD9E8D57u, (uint32_t)step) ^ s0;
+        const uint32_t l1 = 0xCD9E8D57u * (uint32_t)step, c2 = cellw ^ s1;
+        y2 = s1 + w1;
+        const uint32_t n0 = __umulhi(0xCD9E8D57u, c2) ^ l1 ^ (s0 + w0), n1 = 0xCD9E8D57u * c2;
+        x3 = n1 ^ (s0 + 2u * w0);
+        y3 = __umulhi(0xD2511F53u, n0) ^ (s1 + 2u * w1);
+        z3 = 0xD2511F53u * n0;
+        k0 = s0 + 3u * w0;
+        k1 = s1 + 3u * w1;
+    }
+    // the high word of draw 0 of CRU cru (Stream::u24_of makes the uniform of it)
+    __device__ __forceinline__ uint32_t word(uint32_t cru) const {
+        uint32_t c0 = x1 ^ cru;
+        const uint32_t t2 = __umulhi(0xD2511F53u, c0) ^ y2, t3 = 0xD2511F53u * c0;
+        c0 = __umulhi(0xCD9E8D57u, t2) ^ x3;
+        uint32_t c1 = 0xCD9E8D57u * t2, c2 = t3 ^ y3, c3 = z3;
+        uint32_t a = k0, b = k1;
+#pragma unroll
+        for (int r = 4; r <= 8; ++r) {
+            const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
+            const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
+            c0 = hi1 ^ c1 ^ a;
+            c1 = lo1;
+            c2 = hi0 ^ c3 ^ b;
+            c3 = lo0;
+            a += 0x9E3779B9u;
+            b += 0xBB67AE85u;
+        }
+        return 0xCD9E8D57u * (__umulhi(0xD2511F53u, c0) ^ c3 ^ b);  // rounds 9 and 10
+    }
+};
 
 // ------------------------------------------------------------------------------------------
 // Cluster helpers (inline PTX).
@@ -181,6 +233,24 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t mbar, uint32_t tx
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 %0, [%1], %2;" : "=l"(state) : "r"(mbar), "r"(tx) : "memory");
     (void)state;
 }
+// one arrival on the local mbarrier (release at CTA scope)
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    uint64_t state;
+    asm volatile("mbarrier.arrive.shared::cta.b64 %0, [%1];" : "=l"(state) : "r"(mbar) : "memory");
+    (void)state;
+}
+// whether the phase of the given parity has completed (never suspends); acquire at CTA scope
+__device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return ok != 0u;
+}
 // true once the phase of the given parity has completed; acquire at cluster scope, so the bytes
 // that completed it (written by other CTAs) are visible.  May suspend the thread for a while.
 __device__ __forceinline__ bool mbar_try_wait(uint32_t mbar, uint32_t parity) {
@@ -194,13 +264,43 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t mbar, uint32_t parity) {
         : "memory");
     return ok != 0u;
 }
-// Bounded wait: false if the phase did not complete within 2^31 cycles (about a second).
+// The same without ordering: for polling (one acquire follows the poll that succeeds).
+__device__ __forceinline__ bool mbar_poll(uint32_t mbar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return ok != 0u;
+}
+// Bounded wait: false if the phase did not complete within 2^31 cycles (about a second).  The clock is
+// read every 64th time only: the loop's instructions are issue slots that the SM's other warps lose.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    if (mbar_try_wait(mbar, parity)) return true;
     const long long t0 = clock64();
-    while (!mbar_try_wait(mbar, parity))
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 64; ++i)
+            if (mbar_poll(mbar, parity)) return mbar_try_wait(mbar, parity);
         if (clock64() - t0 > (1ll << 31)) return false;
-    return true;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// mbar_wait by a whole warp, one outcome for its lanes.  Every lane polls, and the loop's branch is on a vote:
+// after a loop that one lane ran for the others the warp went on in parts, every instruction once for each
+// (a batch of events took 17 k cycles instead of 5.5 k).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity) {
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 64; ++i)
+            if (__all_sync(0xffffffffu, mbar_poll(mbar, parity)))
+                return __all_sync(0xffffffffu, mbar_try_wait(mbar, parity));
+        if (__any_sync(0xffffffffu, clock64() - t0 > (1ll << 31))) return false;
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -334,14 +434,23 @@ __device__ __forceinline__ void tile_get(Cru<float> &c, const TileRec<float> &t)
     c.jlcc[2] = __uint_as_float(e.z); c.jlcc[3] = __uint_as_float(e.w);
     c.cajsr = __uint_as_float(f.x); c.cajsr_lo = __uint_as_float(f.y);
 }
-__device__ __forceinline__ void tile_put(TileRec<float> &t, const Cru<float> &c) {
+// Tag of an FP32 record (the third word of its last 16 bytes, free of state): 2 + the launch's step in
+// which the CRU last went to the event warps, 0 after a step without.
+__device__ __forceinline__ uint32_t &tile_tag(TileRec<float> &t) { return t.w[4].z; }
+__device__ __forceinline__ void tile_put(TileRec<float> &t, const Cru<float> &c, uint32_t tag = 0u) {
     t.w[0] = make_uint4(c.lcc, c.flags, c.ryr[0], c.ryr[1]);
     t.w[1] = make_uint4(c.ryr[2], c.ryr[3], c.ryr[4], c.ryr[5]);
     t.w[2] = make_uint4(__float_as_uint(c.cass[0]), __float_as_uint(c.cass[1]), __float_as_uint(c.cass[2]),
                         __float_as_uint(c.cass[3]));
     t.w[3] = make_uint4(__float_as_uint(c.jlcc[0]), __float_as_uint(c.jlcc[1]), __float_as_uint(c.jlcc[2]),
                         __float_as_uint(c.jlcc[3]));
-    t.w[4] = make_uint4(__float_as_uint(c.cajsr), __float_as_uint(c.cajsr_lo), 0u, 0u);
+    t.w[4] = make_uint4(__float_as_uint(c.cajsr), __float_as_uint(c.cajsr_lo), tag, 0u);
+}
+// What a quiet step changes: CaSS and CaJSR.
+__device__ __forceinline__ void tile_put_quiet(TileRec<float> &t, const Cru<float> &c, uint32_t tag) {
+    t.w[2] = make_uint4(__float_as_uint(c.cass[0]), __float_as_uint(c.cass[1]), __float_as_uint(c.cass[2]),
+                        __float_as_uint(c.cass[3]));
+    t.w[4] = make_uint4(__float_as_uint(c.cajsr), __float_as_uint(c.cajsr_lo), tag, 0u);
 }
 __device__ __forceinline__ double dbl_of(uint32_t lo, uint32_t hi) { return __hiloint2double((int)hi, (int)lo); }
 __device__ __forceinline__ uint32_t lo_of(double x) { return (uint32_t)__double2loint(x); }
@@ -585,7 +694,7 @@ __device__ __forceinline__ void resplit_pair(uint32_t &a, uint32_t &b, int j, R 
     if (n > 0) {
         int X = 0;
         for (int i = 0; i < n; ++i)
-            if (rng.uniform<R>(kr++) < p) ++X;
+            if (rng.uniform<R, 1>(kr++) < p) ++X;
         a = byte_set(a, j, X);
         b = byte_set(b, j, n - X);
     } else {
@@ -674,14 +783,21 @@ template <typename R>
 __device__ __forceinline__ void resplit_crossed(Cru<R> &s, const SsaConsts<R> &c, const int (&kind)[4], Stream &rng,
                                                 uint32_t k) {
     uint32_t kr = k + 1u;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if (kind[j] == 0) continue;
-        const R x = s.cass[j];
-        if (kind[j] == 1)
-            resplit_pair<R>(s.ryr[4], s.ryr[5], j, quot(c.k65, c.k65 + c.k56 * (x * x)), rng, kr);
-        else
-            resplit_pair<R>(s.ryr[2], s.ryr[3], j, quot(c.k43, c.k43 + c.k34 * (x * x)), rng, kr);
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {  // (one copy of the code: see philox10)
+        const int kj = pick4(kind, j);
+        if (kj == 0) continue;
+        const R x = pick4(s.cass, j);
+        const R down = kj == 1 ? c.k65 : c.k43, up = kj == 1 ? c.k56 : c.k34;
+        uint32_t a = kj == 1 ? s.ryr[4] : s.ryr[2], b = kj == 1 ? s.ryr[5] : s.ryr[3];
+        resplit_pair<R>(a, b, j, quot(down, down + up * (x * x)), rng, kr);
+        if (kj == 1) {
+            s.ryr[4] = a;
+            s.ryr[5] = b;
+        } else {
+            s.ryr[2] = a;
+            s.ryr[3] = b;
+        }
     }
 }
 
@@ -1030,23 +1146,26 @@ struct SsaLane {
     // CaSS update of subunit j, the group exchanges them by shuffles, and the rest runs on the four
     // lanes alike.  Same expressions in the same order as iterate(), hence the same results on every
     // lane; an FP64 warp instruction costs the same whatever its active lanes, so the iteration takes
-    // about a third of the FP64 instructions of one lane's.  The four lanes must call it together.
-    __device__ __forceinline__ bool iterate_group(Cru<R> &s, const SsaConsts<R> &c, const R *sv, Stream &rng, R dt,
-                                                  int cap, int &err) {
+    // about a third of the FP64 instructions of one lane's.  The whole warp calls it together, and its
+    // shuffles are the whole warp's: (each group's own four lanes as the mask would split the warp).  A group that is not live
+    // computes along and leaves its state as it is.
+    __device__ __forceinline__ bool iterate_group(bool live, Cru<R> &s, const SsaConsts<R> &c, const R *sv,
+                                                  Stream &rng, R dt, int cap, int &err) {
         static_assert(sizeof(R) == 8 && EXACT, "the group iteration is for the FP64 lane");
+        constexpr unsigned kAll = 0xffffffffu;
         const int lane = (int)(threadIdx.x & 31u), j = lane & 3, base = lane & ~3;
-        const unsigned gm = 0xFu << base;
         R jxfer[4], jiss[4];
+        const R jtr0 = jtr;
         fluxes(s, c, sv, jxfer, jiss);
         Rates<R> rj;
         const R sj = subunit_rates<R>(s, j, pick4(s.cass, j), c, sv, rj);
         R sub[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) sub[q] = __shfl_sync(gm, sj, base + q);
+        for (int q = 0; q < 4; ++q) sub[q] = __shfl_sync(kAll, sj, base + q);
         const R total = sub[0] + sub[1] + sub[2] + sub[3];
         const R u0 = rng.uniform<R>(k);
         const R jump = quot(-log(u0), total);
-        const bool last = !(t + jump < dt);
+        const bool last = !live || !(t + jump < dt);
         const R h = last ? (dt - t) : jump;
         R tj;
         int kj;
@@ -1057,26 +1176,32 @@ struct SsaLane {
         uint32_t D = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            tmp[q] = __shfl_sync(gm, tj, base + q);
-            kind[q] = __shfl_sync(gm, kj, base + q);
-            D += __shfl_sync(gm, Dj, base + q);
+            tmp[q] = __shfl_sync(kAll, tj, base + q);
+            kind[q] = __shfl_sync(kAll, kj, base + q);
+            D += __shfl_sync(kAll, Dj, base + q);
         }
         uint32_t kk = k + 1u + D;
         int act = 0, aj = 0, atr = 0;
-        if (!last) {
-            t += jump;
+        if (__any_sync(kAll, !last)) {
             // select_event with the drawn subunit's rates from its lane
-            const R us = rng.uniform<R>(kk++) * total;
-            aj = scan_weights<R, 4, false>(sub, us);
+            if (!last) {
+                t += jump;
+                const R us = rng.uniform<R>(kk++) * total;
+                aj = scan_weights<R, 4, false>(sub, us);
+            }
             const int src = base + aj;
             Rates<R> r;
 #pragma unroll
-            for (int q = 0; q < 3; ++q) r.lcc[q] = __shfl_sync(gm, rj.lcc[q], src);
-            r.inact = __shfl_sync(gm, rj.inact, src);
+            for (int q = 0; q < 3; ++q) r.lcc[q] = __shfl_sync(kAll, rj.lcc[q], src);
+            r.inact = __shfl_sync(kAll, rj.inact, src);
 #pragma unroll
-            for (int q = 0; q < 12; ++q) r.ryr[q] = __shfl_sync(gm, rj.ryr[q], src);
-            r.clch = __shfl_sync(gm, rj.clch, src);
-            select_transition<R, true>(r, pick4(sub, aj), rng, kk, act, atr);
+            for (int q = 0; q < 12; ++q) r.ryr[q] = __shfl_sync(kAll, rj.ryr[q], src);
+            r.clch = __shfl_sync(kAll, rj.clch, src);
+            if (!last) select_transition<R, true>(r, pick4(sub, aj), rng, kk, act, atr);
+        }
+        if (!live) {
+            jtr = jtr0;
+            return false;
         }
         return conclude(s, c, sv, rng, h, last, tmp, kind, D, kk, act, aj, atr, jxfer, cap, err, nullptr);
     }
@@ -1135,7 +1260,8 @@ struct SsaLane {
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// a - b as -1 * b + a, one rounding (the packed add has no negation of its own)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 // x / y as x * rcp.approx(y), the arithmetic of __fdividef without its guard for |y| > 2^126 (the
 // divisors here are rate sums and buffer terms far below that)
 __device__ __forceinline__ float rcp_approx(float y) {
@@ -1196,14 +1322,13 @@ __device__ __forceinline__ void ryr_rates_f32(const Cru<float> &s, int j, float 
 
 // FP32 event selection: select_event's draws and decisions, with the subunit's RyR total taken
 // from the iteration's packed total computation (ryr_sub) and the 12 individual RyR rates formed
-// only when the RyR class is drawn (at rest most events are LCC and gate transitions).  The three
-// draws are formed up front (Stream::u24x3); a selection uses two or three of them, as
-// select_event's sequential draws would.
+// only when the RyR class is drawn (at rest most events are LCC and gate transitions).  ua, ub, uc: draws
+// kk, kk + 1, kk + 2; a selection uses two or three of them, as select_event's sequential draws would,
+// and kk moves on by so many.
 __device__ __forceinline__ void select_event_f32(const Cru<float> &s, const SsaConsts<float> &c, const float *sv,
                                                  const float (&sub)[4], const float (&ryr_sub)[4], float total,
-                                                 Stream &rng, uint32_t &kk, int &act, int &aj, int &atr) {
-    float ua, ub, uc;
-    rng.u24x3(kk, ua, ub, uc);
+                                                 float ua, float ub, float uc, uint32_t &kk, int &act, int &aj,
+                                                 int &atr) {
     const float us = ua * total;
     aj = scan_weights<float, 4, true>(sub, us);
     const float x = pick4(s.cass, aj);
@@ -1264,78 +1389,95 @@ struct SsaLane<float, false> {
         for (int p = 0; p < 2; ++p) {
             const float2 open = add2(counts2(b2, p, K[PK_BIAS]), counts2(b3, p, K[PK_BIAS]));
             const float2 x = make_float2(s.cass[2 * p], s.cass[2 * p + 1]);
-            const float2 jr = mul2(mul2(K[PK_RRYR], open), add2(cj, neg2(x)));
+            const float2 jr = mul2(mul2(K[PK_RRYR], open), sub2(cj, x));
             jrel[2 * p] = jr.x;
             jrel[2 * p + 1] = jr.y;
         }
     }
 
-    __device__ __forceinline__ bool iterate(Cru<float> &s, const SsaConsts<float> &c, const float *sv,
-                                            const float2 *tab, Stream &rng, float dt, int cap, int &err) {
+    // Fluxes (update_fluxes, SSA.tpp:37-45) and subunit totals at the iteration's start: jtr, dss (jiss less
+    // its factor), jx, the totals S with their RyR parts Y, and their sum.  All lanes of the warp call it
+    // together, and it branches on the RyR regimes of all of them at once, once each (a branch per pair of
+    // subunits keeps the pairs' instructions from interleaving).
+    __device__ __forceinline__ float totals(const Cru<float> &s, const SsaConsts<float> &c, const float *sv,
+                                            const float2 *tab, const float2 (&C)[2], float2 (&dss)[2], float2 (&jx)[2],
+                                            float2 (&S)[2], float2 (&Y)[2]) {
         const float2 *K = c.pk;
         const float Cai = sv[SV_CAI], CaNSR = sv[SV_CANSR], Cai_lo = sv[SV_CAI_LO], CaNSR_lo = sv[SV_CANSR_LO];
-        const float2 C[2] = {make_float2(s.cass[0], s.cass[1]), make_float2(s.cass[2], s.cass[3])};
-        // update_fluxes (SSA.tpp:37-45)
         jtr = c.rtr * ((CaNSR - s.cajsr) + (CaNSR_lo - s.cajsr_lo));
         const float2 eo = add2(C[0], C[1]);  // (c0 + c2, c1 + c3)
         const float2 oe = make_float2(eo.y, eo.x);
-        float2 jiss[2], jx[2];
         const float2 ncai = make_float2(-Cai, -Cai), ncailo = make_float2(-Cai_lo, -Cai_lo);
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-            jiss[p] = mul2(K[PK_RISS], fma2(K[PK_M2], C[p], oe));
+            dss[p] = fma2(K[PK_M2], C[p], oe);
             jx[p] = mul2(K[PK_RXFER], add2(add2(C[p], ncai), ncailo));
         }
         // subunit totals (the FP32 regrouping of subunit_total_fast)
         const uint32_t iw = rate_index_word(s.lcc, s.flags);
         const uint32_t b0 = s.ryr[0] ^ 0x80808080u, b1 = s.ryr[1] ^ 0x80808080u, b2 = s.ryr[2] ^ 0x80808080u;
         const uint32_t b3 = s.ryr[3] ^ 0x80808080u, b4 = s.ryr[4] ^ 0x80808080u, b5 = s.ryr[5] ^ 0x80808080u;
-        float2 S[2], Y[2];  // subunit totals, and their RyR parts
+        // RyR states 3/4 are lumped above 3.685e-2, states 5/6 above 1.15e-4
+        const float lo = fminf(fminf(C[0].x, C[0].y), fminf(C[1].x, C[1].y));
+        const float hi = fmaxf(fmaxf(C[0].x, C[0].y), fmaxf(C[1].x, C[1].y));
+        const bool any34 = __any_sync(0xffffffffu, hi > 3.685e-2f);
+        const bool all56 = __all_sync(0xffffffffu, lo > 1.15e-4f);
+        float2 p34[2], p56[2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const float2 X2 = mul2(C[p], C[p]);
+            const float2 R2 = counts2(b2, p, K[PK_BIAS]), R3 = counts2(b3, p, K[PK_BIAS]);
+            p34[p] = fma2(R2, K[PK_K32], fma2(R3, K[PK_K4543], mul2(mul2(X2, R2), K[PK_K34])));
+            const float2 R45 = add2(counts2(b4, p, K[PK_BIAS]), counts2(b5, p, K[PK_BIAS]));
+            const float2 num = mul2(K[PK_K65], fma2(K[PK_K54], X2, K[PK_K52])), den = fma2(K[PK_K56], X2, K[PK_K65]);
+            p56[p] = mul2(R45, div2(num, den));
+        }
+        if (any34) {
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const float2 X2 = mul2(C[p], C[p]);
+                const float2 R23 = add2(counts2(b2, p, K[PK_BIAS]), counts2(b3, p, K[PK_BIAS]));
+                const float2 num = fma2(K[PK_K45K34], X2, K[PK_K32K43]), den = fma2(K[PK_K34], X2, K[PK_K43]);
+                const float2 hv = mul2(R23, div2(num, den));
+                p34[p].x = C[p].x > 3.685e-2f ? hv.x : p34[p].x;
+                p34[p].y = C[p].y > 3.685e-2f ? hv.y : p34[p].y;
+            }
+        }
+        if (!all56) {
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const float2 X2 = mul2(C[p], C[p]);
+                const float2 R4 = counts2(b4, p, K[PK_BIAS]), R5 = counts2(b5, p, K[PK_BIAS]);
+                const float2 u = fma2(R5, K[PK_K65], fma2(R4, K[PK_K52], mul2(mul2(X2, R4), K[PK_K5654])));
+                p56[p].x = C[p].x > 1.15e-4f ? p56[p].x : u.x;
+                p56[p].y = C[p].y > 1.15e-4f ? p56[p].y : u.y;
+            }
+        }
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
             const float2 X = C[p];
             const float2 X2 = mul2(X, X);
             const float2 R0 = counts2(b0, p, K[PK_BIAS]), R1 = counts2(b1, p, K[PK_BIAS]);
             float2 y = fma2(X2, fma2(R1, K[PK_K2325], mul2(R0, K[PK_K12])), mul2(R1, K[PK_K21]));
-            // RyR states 3/4: lumped above 3.685e-2
-            const bool h0 = X.x > 3.685e-2f, h1 = X.y > 3.685e-2f;
-            const float2 R2 = counts2(b2, p, K[PK_BIAS]), R3 = counts2(b3, p, K[PK_BIAS]);
-            float2 p34 = fma2(R2, K[PK_K32], fma2(R3, K[PK_K4543], mul2(mul2(X2, R2), K[PK_K34])));
-            if (h0 || h1) {
-                const float2 num = fma2(K[PK_K45K34], X2, K[PK_K32K43]), den = fma2(K[PK_K34], X2, K[PK_K43]);
-                const float2 hv = mul2(add2(R2, R3), div2(num, den));
-                if (h0) p34.x = hv.x;
-                if (h1) p34.y = hv.y;
-            }
-            y = add2(y, p34);
-            // RyR states 5/6: lumped above 1.15e-4
-            const bool g0 = X.x > 1.15e-4f, g1 = X.y > 1.15e-4f;
-            const float2 R4 = counts2(b4, p, K[PK_BIAS]), R5 = counts2(b5, p, K[PK_BIAS]);
-            float2 p56 = make_float2(0.f, 0.f);
-            if (!(g0 && g1)) p56 = fma2(R5, K[PK_K65], fma2(R4, K[PK_K52], mul2(mul2(X2, R4), K[PK_K5654])));
-            if (g0 || g1) {
-                const float2 num = mul2(K[PK_K65], fma2(K[PK_K54], X2, K[PK_K52])), den = fma2(K[PK_K56], X2, K[PK_K65]);
-                const float2 hv = mul2(add2(R4, R5), div2(num, den));
-                if (g0) p56.x = hv.x;
-                if (g1) p56.y = hv.y;
-            }
-            y = add2(y, p56);
+            y = add2(add2(y, p34[p]), p56[p]);
             // LCC, gate and ClCh rates from the warp's table: base + slope * CaSS
             const float2 ta = tab[(iw >> (16 * p)) & 0x3Fu], tb = tab[(iw >> (16 * p + 8)) & 0x3Fu];
             Y[p] = y;
             S[p] = add2(make_float2(fmaf(ta.y, X.x, ta.x), fmaf(tb.y, X.y, tb.x)), y);
         }
-        const float sub[4] = {S[0].x, S[0].y, S[1].x, S[1].y};
         const float2 st = add2(S[0], S[1]);
-        const float total = st.x + st.y;
-        const float u0 = rng.uniform<float>(k);
-        const float jump = -logf(u0) * rcp_approx(total);
-        const bool last = !(t + jump < dt);
-        const float h = last ? (dt - t) : jump;
+        return st.x + st.y;
+    }
 
-        // update_CaSS (SSA.tpp:87-99), first pass
-        float2 tmp[2];
+    // update_CaSS (SSA.tpp:87-99), first pass, over a sub-step h: the new CaSS, and whether any subunit
+    // fell through a threshold.  Multiply-adds are written as such where iterate_group has to round alike:
+    // left to the compiler, a packed product and sum become one operation and a scalar pair stays two.
+    __device__ __forceinline__ bool cass_step(const Cru<float> &s, const SsaConsts<float> &c, float h,
+                                              const float2 (&C)[2], const float2 (&dss)[2], const float2 (&jx)[2],
+                                              float2 (&tmp)[2]) const {
+        const float2 *K = c.pk;
         const float2 H = make_float2(h, h);
+        bool crossed = false;
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
             const float2 A = add2(K[PK_KBSR], C[p]), B = add2(K[PK_KBSL], C[p]);
@@ -1345,58 +1487,158 @@ struct SsaLane<float, false> {
             const float2 beta = div2(UV, den);
             const float2 jl = make_float2(s.jlcc[2 * p], s.jlcc[2 * p + 1]);
             const float2 jr = make_float2(jrel[2 * p], jrel[2 * p + 1]);
-            const float2 f = add2(add2(add2(jl, jr), neg2(jx[p])), jiss[p]);
-            tmp[p] = add2(C[p], mul2(mul2(H, f), beta));
-        }
-        // Threshold crossings are rare: an exact any-crossing test first, then the kinds and the
-        // re-split draw count only when one occurred (if-converted, the full test per subunit
-        // cost ~120 instructions per CRU-step).
-        bool crossed = false;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
+            const float2 f = fma2(K[PK_RISS], dss[p], sub2(add2(jl, jr), jx[p]));
+            tmp[p] = fma2(mul2(H, f), beta, C[p]);
             crossed |= (C[p].x > 1.15e-4f && tmp[p].x <= 1.15e-4f) || (C[p].x > 0.03685f && tmp[p].x <= 0.03685f);
             crossed |= (C[p].y > 1.15e-4f && tmp[p].y <= 1.15e-4f) || (C[p].y > 0.03685f && tmp[p].y <= 0.03685f);
         }
-        int kind[4] = {0, 0, 0, 0};
+        return crossed;
+    }
+    __device__ __forceinline__ static uint32_t crossing_kinds(const Cru<float> &s, const float2 (&C)[2],
+                                                              const float2 (&tmp)[2], int (&kind)[4]) {
         uint32_t D = 0;
-        if (crossed) {
-            kind[0] = crossing<float>(s, 0, C[0].x, tmp[0].x, D);
-            kind[1] = crossing<float>(s, 1, C[0].y, tmp[0].y, D);
-            kind[2] = crossing<float>(s, 2, C[1].x, tmp[1].x, D);
-            kind[3] = crossing<float>(s, 3, C[1].y, tmp[1].y, D);
-        }
+        kind[0] = crossing<float>(s, 0, C[0].x, tmp[0].x, D);
+        kind[1] = crossing<float>(s, 1, C[0].y, tmp[0].y, D);
+        kind[2] = crossing<float>(s, 2, C[1].x, tmp[1].x, D);
+        kind[3] = crossing<float>(s, 3, C[1].y, tmp[1].y, D);
+        return D;
+    }
 
-        uint32_t kk = k + 1u + D;
-        int act = 0, aj = 0, atr = 0;
-        if (!last) {
-            t += jump;
-            const float ryr_sub[4] = {Y[0].x, Y[0].y, Y[1].x, Y[1].y};
-            select_event_f32(s, c, sv, sub, ryr_sub, total, rng, kk, act, aj, atr);
-        }
-        if (crossed) resplit_crossed<float>(s, c, kind, rng, k);
+    // update_CaJSR (SSA.hpp:68-71) over a sub-step h, Fast2Sum into (hi, lo) as in the generic lane
+    __device__ __forceinline__ void cajsr_step(Cru<float> &s, const SsaConsts<float> &c, float h) const {
+        const float x = s.cajsr;
+        const float u = (c.KCSQN + x) * (c.KCSQN + x);
+        const float beta = u * rcp_approx(u + c.CSQN_const);
+        const float2 jr = add2(make_float2(jrel[0], jrel[1]), make_float2(jrel[2], jrel[3]));
+        const float d = h * beta * (jtr - c.VSS_VJSR * (jr.x + jr.y));
+        const float hi = s.cajsr;
+        const float y = d + s.cajsr_lo;
+        const float sum = hi + y;
+        const float err_ = y - (sum - hi);
+        s.cajsr = sum;
+        s.cajsr_lo = err_;
+    }
+
+    // The step of a CRU without a jump or a threshold crossing in it, from its start: iterate_group()'s only
+    // iteration, with the same results, in s.  False when a jump is possible or CaSS falls through a
+    // threshold; s is then of no use, and the caller leaves the CRU to iterate_group().  The jump passes the end
+    // of the step when -log(u0) / total >= dt, and -log(u0) > 1 - u0, which FP32 holds exactly; so
+    // 1 - u0 >= total dt (1 + 1e-5) with total > 0 suffices, the margin covering the roundings of that
+    // product and of -logf(u0) * rcp(total) (about 1e-6 together).  It spares the quiet CRU the
+    // logarithm and misses only jump times within a factor 1 + total dt / 2 of the step's end.  All lanes
+    // of the warp call it together, and nothing in it depends on the outcome, so that its instructions
+    // interleave freely (one call's latency is what a warp of the quiet pass waits for).
+    __device__ __forceinline__ bool quiet(Cru<float> &s, const SsaConsts<float> &c, const float *sv, const float2 *tab,
+                                          uint32_t draw0, float dt) {
+        const float2 C[2] = {make_float2(s.cass[0], s.cass[1]), make_float2(s.cass[2], s.cass[3])};
+        float2 dss[2], jx[2], S[2], Y[2], tmp[2];
+        const float total = totals(s, c, sv, tab, C, dss, jx, S, Y);
+        const float u0 = Stream::u24_of(draw0);
+        const bool last = total > 0.f && 1.f - u0 >= total * dt * 1.00001f;
+        const bool crossed = cass_step(s, c, dt, C, dss, jx, tmp);
         s.cass[0] = tmp[0].x;
         s.cass[1] = tmp[0].y;
         s.cass[2] = tmp[1].x;
         s.cass[3] = tmp[1].y;
-
-        // update_CaJSR (SSA.hpp:68-71), Fast2Sum into (hi, lo) as in the generic lane
-        {
-            const float x = s.cajsr;
-            const float u = (c.KCSQN + x) * (c.KCSQN + x);
-            const float beta = u * rcp_approx(u + c.CSQN_const);
-            const float2 jr = add2(make_float2(jrel[0], jrel[1]), make_float2(jrel[2], jrel[3]));
-            const float d = h * beta * (jtr - c.VSS_VJSR * (jr.x + jr.y));
-            const float hi = s.cajsr;
-            const float y = d + s.cajsr_lo;
-            const float sum = hi + y;
-            const float err_ = y - (sum - hi);
-            s.cajsr = sum;
-            s.cajsr_lo = err_;
-        }
-
-        if (act != 0) apply_event<float>(s, c, sv, act, aj, atr, jrel);
+        cajsr_step(s, c, dt);
         const float2 jxs = add2(jx[0], jx[1]);
         jxfer_sum = jxs.x + jxs.y;
+        return last && !crossed;
+    }
+
+    // The generic lane's iteration (same draws, same decisions) by the four lanes of a group (lanes 4g ..
+    // 4g+3 of the warp, every one holding the same CRU and lane state): lane j = lane & 3 evaluates subunit
+    // j's total and CaSS update in scalar form (rounding as the packed form of quiet()) and one Philox block
+    // of the next eight draws, the group exchanges them by shuffles, and the rest runs on the four lanes
+    // alike.  It is bound by latency: an iteration without an event takes 2.0 k cycles of a warp, one with an
+    // event about 3 k (1 CRU per lane: 3 k and 5 k, its draws one after the other), which is what a step
+    // waits for.  The whole warp calls it together, and its shuffles are the whole warp's; a group that
+    // is not live computes along and leaves its state as it is.
+    __device__ __forceinline__ bool iterate_group(bool live, Cru<float> &s, const SsaConsts<float> &c,
+                                                  const float *sv, const float2 *tab, Stream &rng, float dt, int cap, int &err) {
+        const int lane = (int)(threadIdx.x & 31u), j = lane & 3, base = lane & ~3;
+        constexpr unsigned kAll = 0xffffffffu;
+        // the draws: lane j has the block of draws 2j and 2j + 1 from k's block on
+        uint32_t blk[4];
+        philox10(k / 2u + (uint32_t)j, rng.cru, rng.step, rng.cellw, rng.k0, rng.k1, blk);
+        auto draw = [&](uint32_t d) {  // draw k + d; the lanes of the group alike
+            const uint32_t i = (k & 1u) + d;
+            return Stream::u24_of(__shfl_sync(kAll, (i & 1u) ? blk[3] : blk[1], base + (int)(i >> 1)));
+        };
+        const float Cai = sv[SV_CAI], CaNSR = sv[SV_CANSR], Cai_lo = sv[SV_CAI_LO], CaNSR_lo = sv[SV_CANSR_LO];
+        jtr = c.rtr * ((CaNSR - s.cajsr) + (CaNSR_lo - s.cajsr_lo));
+        const float x = pick4(s.cass, j), x2 = __fmul_rn(x, x);
+        const float even = __fadd_rn(s.cass[0], s.cass[2]), odd = __fadd_rn(s.cass[1], s.cass[3]);
+        const float dss = __fmaf_rn(-2.f, x, (j & 1) ? even : odd);
+        const float jx = __fmul_rn(c.rxfer, __fadd_rn(__fadd_rn(x, -Cai), -Cai_lo));
+        const float R0 = count_f(s.ryr[0], j), R1 = count_f(s.ryr[1], j), R2 = count_f(s.ryr[2], j);
+        const float R3 = count_f(s.ryr[3], j), R4 = count_f(s.ryr[4], j), R5 = count_f(s.ryr[5], j);
+        float y = __fmaf_rn(x2, __fmaf_rn(R1, c.k2325, __fmul_rn(R0, c.k12)), __fmul_rn(R1, c.k21));
+        float p34 = __fmaf_rn(R2, c.k32, __fmaf_rn(R3, c.k4543, __fmul_rn(__fmul_rn(x2, R2), c.k34)));
+        if (x > 3.685e-2f) {
+            const float num = __fmaf_rn(c.k45k34, x2, c.k32k43), den = __fmaf_rn(c.k34, x2, c.k43);
+            p34 = __fmul_rn(__fadd_rn(R2, R3), __fmul_rn(num, rcp_approx(den)));
+        }
+        float p56;
+        if (x > 1.15e-4f) {
+            const float num = __fmul_rn(c.k65, __fmaf_rn(c.k54, x2, c.k52)), den = __fmaf_rn(c.k56, x2, c.k65);
+            p56 = __fmul_rn(__fadd_rn(R4, R5), __fmul_rn(num, rcp_approx(den)));
+        } else {
+            p56 = __fmaf_rn(R5, c.k65, __fmaf_rn(R4, c.k52, __fmul_rn(__fmul_rn(x2, R4), c.k5654)));
+        }
+        y = __fadd_rn(__fadd_rn(y, p34), p56);
+        const float2 tv = tab[(rate_index_word(s.lcc, s.flags) >> (8 * j)) & 0x3Fu];
+        const float sj = __fadd_rn(__fmaf_rn(tv.y, x, tv.x), y);
+        float sub[4], ryr_sub[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sub[q] = __shfl_sync(kAll, sj, base + q);
+        const float total = __fadd_rn(__fadd_rn(sub[0], sub[2]), __fadd_rn(sub[1], sub[3]));
+        const float u0 = draw(0u);
+        const float jump = -logf(u0) * rcp_approx(total);
+        const bool last = !live || !(t + jump < dt);
+        const float h = last ? (dt - t) : jump;
+        const float A = __fadd_rn(c.KBSR, x), B = __fadd_rn(c.KBSL, x);
+        const float U = __fmul_rn(A, A), V = __fmul_rn(B, B), UV = __fmul_rn(U, V);
+        const float beta = __fmul_rn(UV, rcp_approx(__fmaf_rn(c.BSL_const, U, __fmaf_rn(c.BSR_const, V, UV))));
+        const float f = __fmaf_rn(c.riss, dss, __fsub_rn(__fadd_rn(pick4(s.jlcc, j), pick4(jrel, j)), jx));
+        const float tj = __fmaf_rn(__fmul_rn(h, f), beta, x);
+        uint32_t Dj = 0;
+        const int kj = crossing<float>(s, j, x, tj, Dj);
+        int kind[4] = {0, 0, 0, 0};
+        uint32_t D = 0;
+        if (__any_sync(kAll, kj)) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                kind[q] = __shfl_sync(kAll, kj, base + q);
+                D += __shfl_sync(kAll, Dj, base + q);
+            }
+        }
+        uint32_t kk = k + 1u + D;
+        int act = 0, aj = 0, atr = 0;
+        if (__any_sync(kAll, !last)) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ryr_sub[q] = __shfl_sync(kAll, y, base + q);
+            const uint32_t d = min(D, 3u);  // (draws D + 1 .. D + 3, within the four blocks unless D > 3)
+            float ua = draw(1u + d), ub = draw(2u + d), uc = draw(3u + d);
+            if (!last) {
+                t += jump;
+                if (D > 3u) rng.u24x3(kk, ua, ub, uc);
+                select_event_f32(s, c, sv, sub, ryr_sub, total, ua, ub, uc, kk, act, aj, atr);
+            }
+        }
+        float tmp[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tmp[q] = __shfl_sync(kAll, tj, base + q);
+        // (the packed sum's order: (jx0 + jx2) + (jx1 + jx3))
+        const float jp = __fadd_rn(jx, __shfl_xor_sync(kAll, jx, 2));
+        const float jxs = __fadd_rn(jp, __shfl_xor_sync(kAll, jp, 1));
+        if (!live) return false;
+        jxfer_sum = jxs;
+        if (kind[0] | kind[1] | kind[2] | kind[3]) resplit_crossed<float>(s, c, kind, rng, k);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s.cass[q] = tmp[q];
+        cajsr_step(s, c, h);
+        if (act != 0) apply_event<float>(s, c, sv, act, aj, atr, jrel);
         k = kk;
         if (last) return true;
         if (++ev > cap) {
@@ -1406,19 +1648,6 @@ struct SsaLane<float, false> {
         return false;
     }
 };
-
-template <typename R, bool EXACT>
-__device__ __forceinline__ void ssa_cru(Cru<R> &s, const SsaConsts<R> &c, const R *sv, const float2 *tab, Stream &rng,
-                                        R dt, int cap, R &out_jxfer, R &out_jtr, int &events,
-                                        int &err) {
-    SsaLane<R, EXACT> L;
-    L.begin(s, c);
-    while (!L.iterate(s, c, sv, tab, rng, dt, cap, err)) {
-    }
-    events += L.ev;
-    out_jxfer = L.jxfer_sum;
-    out_jtr = L.jtr;
-}
 
 }  // namespace dev
 }  // namespace gw

@@ -11,13 +11,12 @@ constexpr unsigned long long kExp2 = 0x3d7f7bff058b1d51ull;  // ln2^2/2!, 64 fra
 constexpr unsigned long long kExp3 = 0xe35846b82505fc6ull;  // ln2^3/3!, 64 fractional bits
 constexpr unsigned int kExp4 = 0x276556eu;  // ln2^4/4!, 32 fractional bits
 constexpr unsigned int kExp5 = 0x576200u;  // ln2^5/5!, 32 fractional bits
-constexpr long long kLog1 = 4611686018427387904ll;  // (-1)^0/1, 62 fractional bits
-constexpr long long kLog2 = -2305843009213693952ll;  // (-1)^1/2, 62 fractional bits
-constexpr long long kLog3 = 1537228672809129301ll;  // (-1)^2/3, 62 fractional bits
-constexpr int kLog4 = -268435456;  // (-1)^3/4, 30 fractional bits
-constexpr int kLog5 = 214748365;  // (-1)^4/5, 30 fractional bits
-constexpr int kLog6 = -178956971;  // (-1)^5/6, 30 fractional bits
-constexpr int kLog7 = 153391689;  // (-1)^6/7, 30 fractional bits
+constexpr unsigned long long kLog2 = 0x8000000000000000ull;  // 1/2, 64 fractional bits
+constexpr unsigned long long kLog3 = 0x5555555555555555ull;  // 1/3, 64 fractional bits
+constexpr unsigned int kLog4 = 0x40000000u;  // 1/4, 32 fractional bits
+constexpr unsigned int kLog5 = 0x33333333u;  // 1/5, 32 fractional bits
+constexpr unsigned int kLog6 = 0x2aaaaaabu;  // 1/6, 32 fractional bits
+constexpr unsigned int kLog7 = 0x24924925u;  // 1/7, 32 fractional bits
 // 2^(j/256), 63 fractional bits
 #define GW_EXP2_TABLE \
     { \
@@ -89,70 +88,134 @@ constexpr int kLog7 = 153391689;  // (-1)^6/7, 30 fractional bits
 // {c_j, -log(c_j / 2^16) with 64 fractional bits}
 #define GW_LOG_TABLE \
     { \
-        {65281ull, 0xff7f551588de02ull}, {64777ull, 0x2fb6debf18dcec2ull}, \
-        {64281ull, 0x4f32c10f02dd34dull}, {63792ull, 0x6e7a009f8646364ull}, \
-        {63310ull, 0x8d8aec49a6ec158ull}, {62836ull, 0xac531d7e47a6a46ull}, \
-        {62369ull, 0xcae148768667548ull}, {61909ull, 0xe933ac58b121f92ull}, \
-        {61455ull, 0x1075993598e4f130ull}, {61008ull, 0x1254062f0a9416feull}, \
-        {60568ull, 0x142e64bec266e772ull}, {60133ull, 0x1606c5a94e854a48ull}, \
-        {59705ull, 0x17dae56d93235379ull}, {59283ull, 0x19abc1463fb43747ull}, \
-        {58867ull, 0x1b79412bcd862a0bull}, {58457ull, 0x1d434cd6730bde4full}, \
-        {58053ull, 0x1f09cbc0254f2124ull}, {57654ull, 0x20cdc825a774d78bull}, \
-        {57260ull, 0x228f2f08d10d590eull}, {56872ull, 0x244cc63215d596e9ull}, \
-        {56489ull, 0x26079d31c99025f7ull}, {56111ull, 0x27bfa061daf8d3afull}, \
-        {55738ull, 0x2974bbe7408dcd1eull}, {55370ull, 0x2b26dbb3463311b5ull}, \
-        {55007ull, 0x2cd5eb84f22b2472ull}, {54649ull, 0x2e81d6ea81dbc97aull}, \
-        {54295ull, 0x302bbe428df456d5ull}, {53946ull, 0x31d25bbd110c8156ull}, \
-        {53601ull, 0x3376d35d10af8c3bull}, {53261ull, 0x3517daf9105eb186ull}, \
-        {52925ull, 0x36b69a3d1f93c8dcull}, {52593ull, 0x385301ab1ce201dfull}, \
-        {52265ull, 0x39ed019c40144a15ull}, {51942ull, 0x3b8347415cbafa1full}, \
-        {51622ull, 0x3d1846a55d36c149ull}, {51306ull, 0x3eaaaeacc54880a2ull}, \
-        {50995ull, 0x40392616dafce571ull}, {50686ull, 0x41c7777f6156459full}, \
-        {50382ull, 0x4351b75e6b0f2c83ull}, {50081ull, 0x44da6d0a5b73442full}, \
-        {49784ull, 0x46603cb750adbd9eull}, {49490ull, 0x47e46879387dd045ull}, \
-        {49200ull, 0x496590437e58e7c1ull}, {48913ull, 0x4ae4f9eae8cd1368ull}, \
-        {48630ull, 0x4c614125741807aeull}, {48349ull, 0x4ddd0a8b1851f320ull}, \
-        {48072ull, 0x4f55969716fc4194ull}, {47798ull, 0x50cc32a82ed25732ull}, \
-        {47528ull, 0x523f720137472b12ull}, {47260ull, 0x53b208c98dd1a3baull}, \
-        {46995ull, 0x55228c0eb74a0b3full}, {46733ull, 0x5690efc3dc8c081dull}, \
-        {46474ull, 0x57fd27c2b2a15488ull}, {46218ull, 0x596727cc1ca9ccd5ull}, \
-        {45965ull, 0x5acee388d6797625ull}, {45714ull, 0x5c35bd8a202af406ull}, \
-        {45467ull, 0x5d98cd48fdcbb4c9ull}, {45222ull, 0x5efae6290860eea4ull}, \
-        {44979ull, 0x605c01768802d770ull}, {44739ull, 0x61baa168dc5b03fdull}, \
-        {44502ull, 0x6316b92165a429d8ull}, {44267ull, 0x6471b6ad17a9762full}, \
-        {44035ull, 0x65ca160468edd914ull}, {43805ull, 0x6721490b8346057full}, \
-        {43577ull, 0x6877489360bed762ull}, {43352ull, 0x69ca8a59af87a85aull}, \
-        {43129ull, 0x6b1c860965281068ull}, {42908ull, 0x6c6d343b3cf98f70ull}, \
-        {42690ull, 0x6dbb0474f7ef76f4ull}, {42474ull, 0x6f07742c37162906ull}, \
-        {42260ull, 0x70527bc457c89ab3ull}, {42048ull, 0x719c139005bfe0f5ull}, \
-        {41838ull, 0x72e433d173cd44a5ull}, {41631ull, 0x742941b9d40e0e43ull}, \
-        {41425ull, 0x756e596b9b469301ull}, {41222ull, 0x76b04af8d697432eull}, \
-        {41020ull, 0x77f23a641dded53full}, {40820ull, 0x79328aa1ece436ffull}, \
-        {40623ull, 0x7a6f96966efc52a9ull}, {40427ull, 0x7bac8e1903b450d8ull}, \
-        {40233ull, 0x7ce7cdf20a61f00dull}, {40041ull, 0x7e214ddbfd2788f3ull}, \
-        {39851ull, 0x7f590583de3e4651ull}, {39662ull, 0x80909389767e73a4ull}, \
-        {39476ull, 0x81c4a37e80e1d6deull}, {39291ull, 0x82f87ce935755ffbull}, \
-        {39108ull, 0x842a704274706af0ull}, {38926ull, 0x855c23f6884894c8ull}, \
-        {38746ull, 0x868be4661b47e680ull}, {38568ull, 0x87b9a8e4fe6bf740ull}, \
-        {38392ull, 0x88e568bc4d87be8dull}, {38217ull, 0x8a10d229263aa70eull}, \
-        {38044ull, 0x8b3a295da2384e51ull}, {37872ull, 0x8c63207fbaf82dc3ull}, \
-        {37702ull, 0x8d89f7ac2836dcb4ull}, {37533ull, 0x8eb064f33de4980bull}, \
-        {37366ull, 0x8fd4a45c537c5805ull}, {37200ull, 0x90f86fe32e775f14ull}, \
-        {37036ull, 0x9219ff7a52519b1bull}, {36873ull, 0x933b1109a1877e69ull}, \
-        {36712ull, 0x9459d86fe75bfd5aull}, {36552ull, 0x957817815f255709ull}, \
-        {36393ull, 0x9695cb097a816dc5ull}, {36236ull, 0x97b120ca89f230b5ull}, \
-        {36080ull, 0x98cbe07d407350f0ull}, {35926ull, 0x99e433d1f80e6b8bull}, \
-        {35772ull, 0x9afdbb6ec63d1090ull}, {35620ull, 0x9c14cbf30ed41c49ull}, \
-        {35470ull, 0x9d295bf40731c82bull}, {35320ull, 0x9e3f180014b06184ull}, \
-        {35172ull, 0x9f52489b9342f600ull}, {35026ull, 0xa062e44475890483ull}, \
-        {34880ull, 0xa174a36f0405f810ull}, {34735ull, 0xa285a589f4cd024aull}, \
-        {34592ull, 0xa39401f9af556e0dull}, {34450ull, 0xa4a1961d20623d50ull}, \
-        {34309ull, 0xa5ae5e4ad0e8242bull}, {34169ull, 0xa6ba56d23d9cc5efull}, \
-        {34031ull, 0xa7c38efa89fbc2a7ull}, {33893ull, 0xa8cddb06119ed15full}, \
-        {33757ull, 0xa9d55b2dcd306552ull}, {33622ull, 0xaadbf8a5d3a05444ull}, \
-        {33487ull, 0xabe3a49a1df94142ull}, {33354ull, 0xace873300596024eull}, \
-        {33222ull, 0xadec53874ed59eefull}, {33091ull, 0xaeef41b8b0f99e3cull}, \
-        {32961ull, 0xaff139d6950d45f3ull}, {32832ull, 0xb0f237ed2b233612ull}, \
+        {65536ull, 0x0ull}, {65281ull, 0xff7f551588de02ull}, \
+        {65028ull, 0x1fdfaa6b126788full}, {64777ull, 0x2fb6debf18dcec2ull}, \
+        {64528ull, 0x3f7d51627807b25ull}, {64281ull, 0x4f32c10f02dd34dull}, \
+        {64036ull, 0x5ed6ec2508c1368ull}, {63792ull, 0x6e7a009f8646364ull}, \
+        {63551ull, 0x7dfaec4162c727full}, {63311ull, 0x8d7a5c4df4517ccull}, \
+        {63073ull, 0x9ce79dd4f1085e8ull}, {62837ull, 0xac426d86b8a8dc0ull}, \
+        {62602ull, 0xbb9b47b358e7559ull}, {62369ull, 0xcae148768667548ull}, \
+        {62138ull, 0xda142b89080def2ull}, {61909ull, 0xe933ac58b121f92ull}, \
+        {61681ull, 0xf8508600931532bull}, {61456ull, 0x1074883629640ad6ull}, \
+        {61231ull, 0x1164e8eeaf5cde7eull}, {61009ull, 0x1252f32f8d183e9bull}, \
+        {60788ull, 0x1340c796ac516a38ull}, {60568ull, 0x142e64bec266e772ull}, \
+        {60350ull, 0x151ab33f13e03c65ull}, {60134ull, 0x1605aea96fc2aab5ull}, \
+        {59919ull, 0x16f06a8afa8b45e3ull}, {59706ull, 0x17d9cc6db384b387ull}, \
+        {59494ull, 0x18c2e9d642231d00ull}, {59284ull, 0x19aaa6464fbb998dull}, \
+        {59075ull, 0x1a92193a589d6061ull}, {58868ull, 0x1b78242be5758a99ull}, \
+        {58662ull, 0x1c5de08f760f3b25ull}, {58458ull, 0x1d422dd6d4051f7cull}, \
+        {58255ull, 0x1e26276e8cf2acbfull}, {58053ull, 0x1f09cbc0254f2124ull}, \
+        {57853ull, 0x1febf7320a3ca817ull}, {57654ull, 0x20cdc825a774d78bull}, \
+        {57457ull, 0x21ae18fa06a47685ull}, {57261ull, 0x228e0a094f85827bull}, \
+        {57066ull, 0x236d99aaa3d71e86ull}, {56872ull, 0x244cc63215d596e9ull}, \
+        {56680ull, 0x252a65f047ea4543ull}, {56489ull, 0x26079d31c99025f7ull}, \
+        {56300ull, 0x26e340407f3ec8c8ull}, {56112ull, 0x27be75626a0bed3bull}, \
+        {55925ull, 0x28993ada3481c84eull}, {55739ull, 0x29738ee795cc124dull}, \
+        {55554ull, 0x2a4d6fc753f06b50ull}, {55371ull, 0x2b25acb37c0d64c4ull}, \
+        {55189ull, 0x2bfd70e1bfa76141ull}, {55008ull, 0x2cd4ba85475a6893ull}, \
+        {54828ull, 0x2dab87ce60c4273eull}, {54649ull, 0x2e81d6ea81dbc97aull}, \
+        {54472ull, 0x2f56720453b1fd62ull}, {54296ull, 0x302a8942fecf8819ull}, \
+        {54121ull, 0x30fe1acaea639fe0ull}, {53947ull, 0x31d124bdc1ce76a0ull}, \
+        {53774ull, 0x32a3a53a792d0292ull}, {53602ull, 0x33759a5d5218d791ull}, \
+        {53431ull, 0x3447023fe09cbdd7ull}, {53262ull, 0x35169ff9d0ef940full}, \
+        {53093ull, 0x35e6e69d3b47cbd0ull}, {52925ull, 0x36b69a3d1f93c8dcull}, \
+        {52759ull, 0x37847ae884bb9c80ull}, {52594ull, 0x3851c2aba6931d29ull}, \
+        {52429ull, 0x391faf8f3d344203ull}, {52266ull, 0x39ebc09c4bfd9f95ull}, \
+        {52104ull, 0x3ab732d72ff6bc5dull}, {51942ull, 0x3b8347415cbafa1full}, \
+        {51782ull, 0x3c4d76dc8305b9f7ull}, {51623ull, 0x3d1701a5d7b8e774ull}, \
+        {51464ull, 0x3de12b97bd326c14ull}, {51307ull, 0x3ea967acd16ad3b8ull}, \
+        {51151ull, 0x3f70f8db7a9bbaa1ull}, {50995ull, 0x40392616dafce571ull}, \
+        {50841ull, 0x40ff5c5393d265f5ull}, {50687ull, 0x41c62c7f7560964bull}, \
+        {50534ull, 0x428c4b89d8638b98ull}, {50383ull, 0x43506a5f36a1011dull}, \
+        {50232ull, 0x44151fe749aaee08ull}, {50082ull, 0x44d91e0acca46e22ull}, \
+        {49933ull, 0x459c62af3f17d1b4ull}, {49785ull, 0x465eebb823f5887dull}, \
+        {49637ull, 0x47220905b639e83aull}, {49491ull, 0x47e315798c9409e0ull}, \
+        {49345ull, 0x48a4b3ef4bad9385ull}, {49201ull, 0x49643b444c24b923ull}, \
+        {49057ull, 0x4a245250110c2034ull}, {48914ull, 0x4ae3a2eb82361b7aull}, \
+        {48771ull, 0x4ba382eb8494c270ull}, {48630ull, 0x4c614125741807aeull}, \
+        {48490ull, 0x4d1e326b2efca65bull}, {48350ull, 0x4ddbaf8b6a532a9eull}, \
+        {48211ull, 0x4e985d55fcdf76a6ull}, {48073ull, 0x4f5439978ce863afull}, \
+        {47935ull, 0x5010a01a1ce18ec1ull}, {47799ull, 0x50cad3a87da88e80ull}, \
+        {47663ull, 0x51858f08a37af51full}, {47528ull, 0x523f720137472b12ull}, \
+        {47394ull, 0x52f87a5661ea2a08ull}, {47260ull, 0x53b208c98dd1a3baull}, \
+        {47128ull, 0x5469561da9dfd653ull}, {46996ull, 0x5521270faed0a5c5ull}, \
+        {46864ull, 0x55d97c5d2769acd2ull}, {46734ull, 0x568f88c477810a65ull}, \
+        {46604ull, 0x574616fdc226f018ull}, {46475ull, 0x57fbbec3215376c4ull}, \
+        {46346ull, 0x58b1e7cae9a65481ull}, {46219ull, 0x5965bccca9bfd92dull}, \
+        {46092ull, 0x5a1a107afcd254b7ull}, {45965ull, 0x5acee388d6797625ull}, \
+        {45840ull, 0x5b815aa910875506ull}, {45715ull, 0x5c344e8a280d3500ull}, \
+        {45591ull, 0x5ce64fdb7fbfb419ull}, {45467ull, 0x5d98cd48fdcbb4c9ull}, \
+        {45344ull, 0x5e4a557f7d1e889bull}, {45222ull, 0x5efae6290860eea4ull}, \
+        {45101ull, 0x5faa7cef02462818ull}, {44980ull, 0x605a8c775059a9d9ull}, \
+        {44859ull, 0x610b15687f0e5c82ull}, {44740ull, 0x61b92a6969b60ba6ull}, \
+        {44621ull, 0x6267b61b9e28fb30ull}, {44502ull, 0x6316b92165a429d8ull}, \
+        {44385ull, 0x63c3401d9a1c8082ull}, {44268ull, 0x64703bae0e2810a5ull}, \
+        {44151ull, 0x651dac70b8e3d47aull}, {44035ull, 0x65ca160468edd914ull}, \
+        {43920ull, 0x66757604c181f204ull}, {43805ull, 0x6721490b8346057full}, \
+        {43691ull, 0x67cc0fb31e612520ull}, {43578ull, 0x6875c7941777b819ull}, \
+        {43465ull, 0x691ff044298dc00full}, {43352ull, 0x69ca8a59af87a85aull}, \
+        {43241ull, 0x6a728e6b0ea8a793ull}, {43130ull, 0x6b1b010a5784ae8eull}, \
+        {43019ull, 0x6bc3e2c967638722ull}, {42909ull, 0x6c6bad3b486dc318ull}, \
+        {42800ull, 0x6d125df0523c6a34ull}, {42691ull, 0x6db97b75def921f2ull}, \
+        {42582ull, 0x6e61065a5ccbe970ull}, {42474ull, 0x6f07742c37162906ull}, \
+        {42367ull, 0x6facc276b6b5e7eeull}, {42260ull, 0x70527bc457c89ab3ull}, \
+        {42154ull, 0x70f7129f41fd3393ull}, {42049ull, 0x719a8490d8efa068ull}, \
+        {41944ull, 0x723e5f1f8a6766b2ull}, {41839ull, 0x72e2a2d1970b6f8eull}, \
+        {41735ull, 0x7385be2e95d15a95ull}, {41631ull, 0x742941b9d40e0e43ull}, \
+        {41528ull, 0x74cb99f815af5107ull}, {41426ull, 0x756cc46c4bab71b5ull}, \
+        {41324ull, 0x760e5496fadc45c7ull}, {41222ull, 0x76b04af8d697432eull}, \
+        {41121ull, 0x775110133432711full}, {41021ull, 0x77f0a1652b124d0full}, \
+        {40921ull, 0x7890966b20e1615dull}, {40821ull, 0x7930efa1fc245e27ull}, \
+        {40722ull, 0x79d01187d23dd1faull}, {40623ull, 0x7a6f96966efc52a9ull}, \
+        {40525ull, 0x7b0de1493d44f421ull}, {40428ull, 0x7baaef1a423e8175ull}, \
+        {40330ull, 0x7c49fd7ec41bb178ull}, {40234ull, 0x7ce62cf3046a7dedull}, \
+        {40137ull, 0x7d845de9c584b0e2ull}, {40042ull, 0x7e1faadd177bed2dull}, \
+        {39946ull, 0x7ebcfa3df8ec75aeull}, {39851ull, 0x7f590583de3e4651ull}, \
+        {39757ull, 0x7ff3ca21ce741cc5ull}, {39663ull, 0x808eec899a04906aull}, \
+        {39569ull, 0x812a6d2d31a7f5e2ull}, {39476ull, 0x81c4a37e80e1d6deull}, \
+        {39384ull, 0x825d8cee51b595b6ull}, {39291ull, 0x82f87ce935755ffbull}, \
+        {39200ull, 0x839072e206f8e274ull}, {39108ull, 0x842a704274706af0ull}, \
+        {39017ull, 0x84c31c7acaeb0190ull}, {38927ull, 0x855a74f739e665c7ull}, \
+        {38837ull, 0x85f2272231d3183bull}, {38747ull, 0x868a33663a91fd02ull}, \
+        {38658ull, 0x8720e82f85eb7a3dull}, {38569ull, 0x87b7f5e588e7e280ull}, \
+        {38480ull, 0x884f5cf17264b69aull}, {38392ull, 0x88e568bc4d87be8dull}, \
+        {38305ull, 0x897a16adb0aed884ull}, {38217ull, 0x8a10d229263aa70eull}, \
+        {38131ull, 0x8aa4769905cdc99bull}, {38044ull, 0x8b3a295da2384e51ull}, \
+        {37958ull, 0x8bce79df2354cfd6ull}, {37872ull, 0x8c63207fbaf82dc3ull}, \
+        {37787ull, 0x8cf661a3961345edull}, {37702ull, 0x8d89f7ac2836dcb4ull}, \
+        {37618ull, 0x8e1c24fcd567c232ull}, {37533ull, 0x8eb064f33de4980bull}, \
+        {37450ull, 0x8f417af4a20561f1ull}, {37366ull, 0x8fd4a45c537c5805ull}, \
+        {37283ull, 0x9066608cb86d605eull}, {37201ull, 0x90f6ace49f8a3c67ull}, \
+        {37118ull, 0x91890ebe121a0b4dull}, {37036ull, 0x9219ff7a52519b1bull}, \
+        {36955ull, 0x92a97c75bc7f783eull}, {36874ull, 0x93394a0b34172277ull}, \
+        {36793ull, 0x93c9689579a7a4fcull}, {36712ull, 0x9459d86fe75bfd5aull}, \
+        {36632ull, 0x94e8cff686040ff3ull}, {36552ull, 0x957817815f255709ull}, \
+        {36473ull, 0x9605e36b273b687full}, {36394ull, 0x9693fe0acc2579e6ull}, \
+        {36315ull, 0x972267b7e0a4a48cull}, {36236ull, 0x97b120ca89f230b5ull}, \
+        {36158ull, 0x983e599a8a85ec7eull}, {36081ull, 0x98ca0f7ec9b20486ull}, \
+        {36003ull, 0x9957e3c8d19d6ae7ull}, {35926ull, 0x99e433d1f80e6b8bull}, \
+        {35849ull, 0x9a70d0ed015690c7ull}, {35773ull, 0x9afbe66f64b4d7d7ull}, \
+        {35697ull, 0x9b8747ab4b6ea41bull}, {35621ull, 0x9c12f4f357800c36ull}, \
+        {35545ull, 0x9c9eee9ab270cd3cull}, {35470ull, 0x9d295bf40731c82bull}, \
+        {35395ull, 0x9db4145000431579ull}, {35321ull, 0x9e3d3d003c9455e3ull}, \
+        {35247ull, 0x9ec6af54823eefa6ull}, {35173ull, 0x9f506b9c0f2acbd0ull}, \
+        {35099ull, 0x9fda7226a16c0cccull}, {35026ull, 0xa062e44475890483ull}, \
+        {34953ull, 0xa0eb9f42959539f9ull}, {34880ull, 0xa174a36f0405f810ull}, \
+        {34808ull, 0xa1fc0f183ef2f584ull}, {34736ull, 0xa283c28a2e57ec28ull}, \
+        {34664ull, 0xa30bbe1114f5ff13ull}, {34593ull, 0xa3921cfac4e0be29ull}, \
+        {34522ull, 0xa418c2910eccd714ull}, {34451ull, 0xa49faf1e720b4054ull}, \
+        {34380ull, 0xa526e2ede3f59ee7ull}, {34310ull, 0xa5ac754bc844925bull}, \
+        {34240ull, 0xa6324d7f8770ad8dull}, {34170ull, 0xa6b86bd24de9aee1ull}, \
+        {34101ull, 0xa73ce48f7563605bull}, {34031ull, 0xa7c38efa89fbc2a7ull}, \
+        {33962ull, 0xa84892600b8b5a5cull}, {33894ull, 0xa8cbec06923395c0ull}, \
+        {33826ull, 0xa94f8934a02b24f7ull}, {33757ull, 0xa9d55b2dcd306552ull}, \
+        {33690ull, 0xaa578f3e0b6b6de8ull}, {33622ull, 0xaadbf8a5d3a05444ull}, \
+        {33555ull, 0xab5eb2ae3d245587ull}, {33488ull, 0xabe1af9a480c1dd3ull}, \
+        {33421ull, 0xac64efae8ace3f58ull}, {33355ull, 0xace67c30c5279785ull}, \
+        {33289ull, 0xad684a632717b697ull}, {33223ull, 0xadea5a886fd2d5cbull}, \
+        {33157ull, 0xae6cace3c47ce9b2ull}, {33092ull, 0xaeed46ba0a8f8cf5ull}, \
+        {33027ull, 0xaf6e214b08f92fc2ull}, {32962ull, 0xafef3cd809d90d39ull}, \
+        {32897ull, 0xb07099a2ba4872fbull}, {32833ull, 0xb0f038eea961ee78ull}, \
     }
 }  // namespace math64
 }  // namespace gw

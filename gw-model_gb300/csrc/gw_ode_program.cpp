@@ -255,22 +255,22 @@ void build(Builder &b) {
         while (b.ph[q].size() < 96) b.ph[q].push_back(OdeOp{OK_NOP, 1, 0, {}});
         // (KmNai/Nai)^1.5 = KmNai^1.5 / (Nai sqrt(Nai)); exp(1.5 F/RT (V - EK)) = exp(1.5 F/RT V) *
         // (Ki/Ko)^1.5 (EK = RT/F log(Ko/Ki)); products of two globals through sqrt(1)
-        auto pw = [&](uint16_t out, uint16_t c, uint16_t y, uint16_t x, uint16_t k, int w, uint16_t off) {
-            b.emit(q, OK_POW, out, {c, y, x, k, off});
+        auto pw = [&](uint16_t out, uint16_t c, uint16_t y, uint16_t x, int w, uint16_t off) {
+            b.emit(q, OK_POW, out, {c, y, x, off});
             b.ph[q].back().width = (uint8_t)w;
         };
-        pw(NaS, ONE, Nai, Nai, ONE, 1, ZERO);
-        pw(KiS, K(std::pow(p.Ko, -1.5)), Ki, Ki, ONE, 1, ZERO);
+        pw(NaS, ONE, Nai, Nai, 1, ZERO);
+        pw(KiS, K(std::pow(p.Ko, -1.5)), Ki, Ki, 1, ZERO);
         if (b.fast) {
-            const uint16_t cf = K(1.0 / p.Kmf), cr = K(1.0 / p.Kmr);
-            pw(pf, ONE, ONE, Cai, cf, 2, ZERO);
-            pw(pr, ONE, ONE, NSR, cr, 2, ZERO);
-            pw(opf, ONE, ONE, Cai, cf, 2, ONE);
+            const uint16_t cf = K(std::pow(p.Kmf, -0.75)), cr = K(std::pow(p.Kmr, -0.75));
+            pw(pf, cf, ONE, Cai, 2, ZERO);
+            pw(pr, cr, ONE, NSR, 2, ZERO);
+            pw(opf, cf, ONE, Cai, 2, ONE);
         }
-        pw(Na2, Nai, Nai, ONE, ONE, 1, ZERO);
-        pw(mm, b.G(im), b.G(im), ONE, ONE, 1, ZERO);
-        pw(hj, b.G(ih), b.G(ij), ONE, ONE, 1, ZERO);
-        pw(xKs2, b.G(ixKs), b.G(ixKs), ONE, ONE, 1, ZERO);
+        pw(Na2, Nai, Nai, ONE, 1, ZERO);
+        pw(mm, b.G(im), b.G(im), ONE, 1, ZERO);
+        pw(hj, b.G(ih), b.G(ij), ONE, 1, ZERO);
+        pw(xKs2, b.G(ixKs), b.G(ixKs), ONE, 1, ZERO);
     }
     // ---------------- phase P: general Jup exponents ----------------
     if (!b.fast) {
@@ -579,8 +579,8 @@ void ode_program_step_host(const OdeProgram &P, const double *consts, double *g,
             case OK_LOG: v = (X[a[2]] + X[a[3]]) + X[a[4]] * std::log(X[a[0]] + X[a[1]] * X[a[5]]); break;
             case OK_EXP: v = X[a[4]] + X[a[0]] * std::exp(X[a[1]] * X[a[2]] + X[a[3]]); break;
             case OK_POW: {
-                const double t = std::sqrt(X[a[2]] * X[a[3]]);
-                v = X[a[4]] + X[a[0]] * X[a[1]] * (op->width == 2 ? t * std::sqrt(t) : t);
+                const double t = std::sqrt(X[a[2]]);
+                v = X[a[3]] + X[a[0]] * X[a[1]] * (op->width == 2 ? t * std::sqrt(t) : t);
                 break;
             }
             case OK_QUOT: v = X[a[0]] * (X[a[1]] + X[a[2]] * X[a[3]]) / (X[a[4]] + X[a[5]] * X[a[6]]); break;

@@ -22,7 +22,7 @@ enum OdeKind : uint8_t {
     OK_NOP = 0,
     OK_LOG,   // out = (X[a2] + X[a3]) + X[a4] * log(X[a0] + X[a1]*X[a5])
     OK_EXP,   // out = X[a4] + X[a0] * exp(X[a1]*X[a2] + X[a3])
-    OK_POW,   // out = X[a4] + X[a0]*X[a1] * (X[a2]*X[a3])^(1/2), or ^(3/4) when width = 2
+    OK_POW,   // out = X[a3] + X[a0]*X[a1] * X[a2]^(1/2), or ^(3/4) when width = 2
     OK_QUOT,  // out = X[a0] * (X[a1] + X[a2]*X[a3]) / (X[a4] + X[a5]*X[a6])
     OK_SUM3,  // out = X[a0]*X[a1] + X[a2]*X[a3] + X[a4]*X[a5]
     OK_DOT,   // row of `width` lanes: the increment of global `out` is X[a0] times the sum over lanes and

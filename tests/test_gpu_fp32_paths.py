@@ -1,0 +1,63 @@
+"""FP32 engine: a cell's trajectory does not depend on how its CRUs are spread over CTAs and warps.
+
+A CTA takes its CRUs on four lanes each (few of them), or in quiet passes with the CRUs that may have
+a jump queued for the event warps (the split between both following the events); the flux sums are
+exact.  So every launch shape gives the same bits.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def states(n, busy):
+    from gwgb300 import engine
+
+    rng = np.random.default_rng(n)
+    ryr = np.zeros((n, 4, 6), np.int32)
+    for j in range(4):
+        k = rng.choice(6, (n, 5), p=[0.42, 0.02, 0.02, 0.1, 0.26, 0.18] if busy else [0.609, 0, 0, 0, 0.1955, 0.1955])
+        for q in range(6):
+            ryr[:, j, q] = (k == q).sum(1)
+    lcc = rng.choice([1, 2, 3, 4, 5, 6, 9, 10, 11] if busy else [1, 2, 7], (n, 4)).astype(np.int32)
+    cass = np.exp(rng.uniform(np.log(9e-5), np.log(6e-2), (n, 4))) if busy else np.full((n, 4), 1.4537e-4)
+    return engine.CRUState(CaSS=cass.astype(np.float32).astype(float), LCC=lcc, RyR=ryr,
+                           CaJSR=rng.uniform(0.6, 0.9, n).astype(np.float32).astype(float),
+                           LCC_inactivation=(rng.random((n, 4)) < 0.85).astype(np.int32),
+                           ClCh=(rng.random((n, 4)) < 0.05).astype(np.int32))
+
+
+def simulate(n, busy, **shape):
+    from gwgb300 import engine
+
+    e = engine.Ensemble([n], precision="fp32", seed=5, **shape)
+    if busy:
+        g = e.get_globals(0)
+        g[0], g[3], g[4] = -3.7, 4.0e-4, 0.88
+        e.set_globals(0, g)
+    e.set_crus(0, states(n, busy))
+    e.set_pulse(0.0, 500.0, 0.5, 100.0)
+    e.run(1e-3, 60)
+    s = e.get_crus(0)
+    out = {k: np.array(getattr(s, k)) for k in ("CaSS", "CaJSR", "LCC", "LCC_inactivation", "RyR", "ClCh")}
+    out["globals"] = e.get_globals(0)
+    out["carry"] = np.array(e.get_flux_carry(0))
+    out["events"] = np.array(e.stats()["events"])
+    return out
+
+
+@pytest.mark.parametrize("busy", [False, True])
+@pytest.mark.parametrize("n,shapes", [
+    (5, [(2, 0)]),                          # part of one group of eight
+    (129, [(2, 0), (5, 0)]),                # one more than a pass of 16 warps
+    (257, [(2, 0), (1, 320), (3, 0)]),      # one more than the four-lane CTAs take
+    (1000, [(1, 1024), (2, 0), (4, 0), (9, 0), (16, 0)]),
+    (2080, [(1, 2080), (2, 1056), (3, 0)]),  # many groups per warp, a full queue when busy
+])
+def test_every_shape_gives_the_same_bits(n, shapes, busy):
+    want = simulate(n, busy, cluster_ctas=0)
+    assert not busy or want["events"] > 2 * n
+    for cl, tile in shapes:
+        got = simulate(n, busy, cluster_ctas=cl, cta_crus=tile)
+        for k in want:
+            assert np.array_equal(want[k], got[k]), (k, cl, tile)
