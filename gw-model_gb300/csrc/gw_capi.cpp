@@ -193,6 +193,7 @@ int byte_of(int v) { return v & 0xFF; }
 // The size rule: cluster size C and CTA capacity (tile) for n_cells cells of at most max_n CRUs, from the
 // requested values (0 = derive).
 constexpr int kSpreadCtas = 112;
+constexpr int kSms = 152;
 void shape_rule(int precision, int n_cells, int max_n, int cluster_req, int tile_req, int &C, int &tile) {
     C = cluster_req > 0 ? cluster_req : 0;
     tile = tile_req > 0 ? tile_req : 0;
@@ -230,9 +231,13 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
     if (need > C)
         return fail(c, GW_ERR_UNSUPPORTED, "a cell of %d CRUs needs %d CTAs of %d CRUs but the cluster has %d",
                     max_n, need, tile, C);
+    // SSA warps: one for 32 CRUs; FP32 where there is an SM for every CTA down to one for eight CRUs, which take
+    // four lanes each (a cell of 60 CRUs amid the release 3.8 us per step, with a warp for 32 4.3; but
+    // 256 cells of 100, two CTAs to an SM, 6.9 at rest and 9.9 amid the release against 9.2 and 13.9).
+    int64_t ctas = 0;
+    for (int i = 0; i < c->n_cells; ++i) ctas += (c->ncru[i] + tile - 1) / tile;
     const bool fp64 = c->precision == GW_PRECISION_FP64;
-    // (FP32: down to one warp for eight CRUs, which take four lanes each)
-    c->ssa_warps = fp64 ? std::min(kMaxSsaWarpsFp64, tile / 32) : std::min(kMaxSsaWarps, tile / 8);
+    c->ssa_warps = std::min(fp64 ? kMaxSsaWarpsFp64 : kMaxSsaWarps, tile / (fp64 || ctas > kSms ? 32 : 8));
     c->tile_cap = tile;
     // Pack cells (first-fit decreasing on CTA count) into clusters of C CTAs.
     std::vector<int> order(c->n_cells);

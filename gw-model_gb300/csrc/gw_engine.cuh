@@ -679,7 +679,7 @@ struct CtaView {
         leader = active && w.rank_in_cell == 0;
         ode_thread = leader && warp >= nw;
         n_ssa = (leader ? nw : nw + kOdeWarps) * 32;  // SSA threads of this CTA
-        grouped = !FP64 && w.cru_count <= kGroupCrus * (n_ssa >> 5);
+        grouped = !FP64 && w.cru_count <= (n_ssa == 32 * kMaxWarps ? kGroupCrus : 32) * (n_ssa >> 5);
         const SmemLayout L = smem_layout<R, T>(a.tile_cap, a.max_cta_cell);
         cc = reinterpret_cast<SsaConsts<R> *>(smem + L.cc);
         svbuf = reinterpret_cast<R *>(smem + L.sv);
@@ -912,10 +912,15 @@ __device__ __forceinline__ void group_run(const KernelArgs &a, const SsaConsts<f
     }
 }
 
-// The FP32 SSA of a CTA with few CRUs (v.grouped): every CRU on four lanes, eight per warp at a time, each warp
-// with a contiguous range.  With up to 128 CRUs in a CTA of 16 warps that is one pass, 2.0 k cycles without
-// an event and 5.3 k with one, and the global step beside it sets the time: 3.2 us per step for a cell of
-// 777 CRUs over 9 to 16 CTAs (4.4 with one CRU per lane), 4.6 in split_steps over 4.
+// The FP32 SSA of a CTA with few CRUs (v.grouped), each warp with a contiguous range of them and nothing shared
+// between the warps.  With up to eight to a warp every CRU goes on four lanes at once: one pass, 2.0 k cycles
+// without an event and 5.3 k with one, and the global step beside it sets the time (3.2 us per step at rest
+// for a cell of 777 CRUs over 9 to 16 CTAs; 4.4 with one CRU per lane).  With more, a quiet pass of one CRU
+// per lane (SsaLane::quiet) comes first and those with a possible jump follow, eight at a time.
+// split_steps shares these between warps, which pays from 16 CRUs per warp on in a CTA of 16 warps (us per
+// step of 30 cells of 300 to 1,000 CRUs amid the release, line at 16 and 32: 6.5 and 7.1; at rest 4.6 and
+// 4.4), and not in smaller CTAs, where few warps are left for either part (100 cells of 50 to 200, 12 SSA
+// warps, line at 16 and 32 amid the release: 9.0 and 6.8; 256 of 100, 4 SSA warps: 13.0 and 9.9).
 template <bool ODE64>
 __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<false, ODE64> &v, uint64_t step0,
                                             unsigned long long &my_events, int &my_err, int &s_stop) {
@@ -925,9 +930,13 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
     TileRec<float> *tile = v.tile;
     const int pslot = a.max_cta_cell * kMaxWarps;
     const uint32_t rcell = (uint32_t)(a.cell_base + cell);
-    const int nse = max(1, min(v.leader ? w.lead_warps : v.n_ssa >> 5, (w.cru_count + 7) >> 3));
+    // (a leader takes CRUs on its first lead_warps warps only, possibly none)
+    const int nwu = max(1, v.leader ? w.lead_warps : v.n_ssa >> 5);
+    const bool direct = w.cru_count <= 8 * nwu;
+    const int nse = direct ? max(1, (w.cru_count + 7) >> 3) : nwu;
     const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
     const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
+    uint16_t *const q = reinterpret_cast<uint16_t *>(v.fq + 8) + beg;
     for (int s = 0; s < a.n_steps; ++s) {
         const int par = s & 1;
         const int64_t ri = a.run_step0 + s;
@@ -940,39 +949,58 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
         if (threadIdx.x == 0) mbar_arrive_expect_tx(svm, (uint32_t)(kSvCount * sizeof(float)));
         const float *sv = v.svbuf + par * kSvCount;
         float2 *rtab = v.rtab + par * kRateTab;
-        FluxAcc<false> acc;
-        Cru<float> c;
-        SsaLane<float, false> sl;
-        Stream rng;
         bool bad = false;
-        __syncwarp();  // (the CRUs of the last step are stored)
-        for (int b = beg;; b += 8) {
-            // (a group without a CRU computes along on the range's last)
-            int m = min(b + (lane >> 2), end - 1);
-            tile_get(c, tile[max(m, 0)]);
-            rng.open(a.seed, rcell, (uint32_t)(w.cru_begin + m), step0 + s, 0);
-            sl.begin(c, cc);
-            if (b + (lane >> 2) >= end) m = -1;
-            if (b == beg) {
-                if (warp < 2) {
-                    bad = !mbar_wait_warp(svm, (uint32_t)(s >> 1) & 1u);
-                    for (int e = (int)threadIdx.x; e < kRateTab; e += 64) build_rate_entry<float>(rtab, cc, sv, e);
-                }
-                bad = bar_or(2, v.n_ssa, bad);
-                if (bad) break;
-            }
-            group_run(a, cc, tile, m, c, sl, rng, sv, rtab, (uint32_t)s + 2u, acc, my_events, my_err);
-            if (b + 8 >= end) break;
+        if (warp < 2) {
+            bad = !mbar_wait_warp(svm, (uint32_t)(s >> 1) & 1u);
+            for (int e = (int)threadIdx.x; e < kRateTab; e += 64) build_rate_entry<float>(rtab, cc, sv, e);
         }
-        if (bad) {
+        if (bar_or(2, v.n_ssa, bad)) {
             my_err |= 2;
             s_stop = s;
             continue;
         }
-        if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr)) {
+        FluxAcc<false> acc;
+        acc.big = end - beg > kMaxSumCrus;
+        int n = end - beg;
+        if (!direct) {
+            StepDraw draw;
+            draw.open(a.seed, rcell, step0 + s, 0);
+            n = 0;
+            for (int b = beg; b < end; b += 32) {
+                const int m = b + lane;
+                // (a lane without a CRU computes along on the range's last: no branch in the pass)
+                Cru<float> c;
+                SsaLane<float, false> sl;
+                TileRec<float> &rec_m = tile[min(m, end - 1)];
+                tile_get(c, rec_m);
+                sl.begin(c, cc);
+                const bool quiet = sl.quiet(c, cc, sv, rtab, draw.word((uint32_t)(w.cru_begin + m)), (float)a.dt);
+                const bool done = m < end && quiet, jumps = m < end && !quiet;
+                if (done) tile_put_quiet(rec_m, c, 0u);
+                acc.add(done ? c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3] : 0.f, done ? sl.jxfer_sum : 0.f,
+                        done ? sl.jtr : 0.f, done ? __popc((c.flags >> 4) & 0xFu) : 0);
+                const unsigned em = __ballot_sync(0xffffffffu, jumps);
+                if (jumps) q[n + __popc(em & ((1u << lane) - 1u))] = (uint16_t)m;
+                n += __popc(em);
+            }
             __syncwarp();
-            record_pass<float>(a, w, cell, r_idx, beg, end, lane, tile);
         }
+        for (int h = 0; h < n; h += 8) {
+            // (a group without a CRU holds, and computes along on, the batch's last)
+            const int i = h + (lane >> 2), k = min(i, n - 1);
+            int m = direct ? beg + k : (int)q[k];
+            Cru<float> c;
+            SsaLane<float, false> sl;
+            Stream rng;
+            tile_get(c, tile[m]);
+            rng.open(a.seed, rcell, (uint32_t)(w.cru_begin + m), step0 + s, 0);
+            sl.begin(c, cc);
+            if (i >= n) m = -1;
+            group_run(a, cc, tile, m, c, sl, rng, sv, rtab, 0u, acc, my_events, my_err);
+        }
+        __syncwarp();  // (the CRUs of this step are stored)
+        if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr))
+            record_pass<float>(a, w, cell, r_idx, beg, end, lane, tile);
         send_partial<false, ODE64>(a, v, par, pslot, acc.warp_total());
     }
 }

@@ -1,8 +1,8 @@
 """FP32 engine: a cell's trajectory does not depend on how its CRUs are spread over CTAs and warps.
 
-A CTA takes its CRUs on four lanes each (few of them), or in quiet passes with the CRUs that may have
-a jump queued for the event warps (the split between both following the events); the flux sums are
-exact.  So every launch shape gives the same bits.
+A CTA takes its CRUs on four lanes each (few of them), or in quiet passes followed by the CRUs that may
+have a jump, each warp its own or queued for the event warps (the split between both following the
+events); the flux sums are exact.  So every launch shape gives the same bits.
 """
 import numpy as np
 import pytest
@@ -50,7 +50,8 @@ def simulate(n, busy, **shape):
 @pytest.mark.parametrize("n,shapes", [
     (5, [(2, 0)]),                          # part of one group of eight
     (129, [(2, 0), (5, 0)]),                # one more than a pass of 16 warps
-    (257, [(2, 0), (1, 320), (3, 0)]),      # one more than the four-lane CTAs take
+    (257, [(2, 0), (1, 320), (3, 0)]),      # one more than a CTA of 16 warps takes without a queue
+    (385, [(1, 416), (2, 0), (4, 128)]),    # one more than a CTA of 12 warps does
     (1000, [(1, 1024), (2, 0), (4, 0), (9, 0), (16, 0)]),
     (2080, [(1, 2080), (2, 1056), (3, 0)]),  # many groups per warp, a full queue when busy
 ])
