@@ -405,9 +405,10 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
                 }
                 if (!__any_sync(0xffffffffu, m >= 0)) break;
                 // (a group that ended its CRU with finish(), or has none, computes along)
-                bool done = m >= 0 && !first && L.surely_last(c, cc, sk, svf, rng, a.dt);
-                if (done) L.finish(c, cc, sv, rng, a.dt);
-                const bool more = m >= 0 && !done;
+                const bool last = L.surely_last_group(c, cc, sk, svf, rng, a.dt) && m >= 0 && !first;
+                bool done = last;
+                if (__any_sync(0xffffffffu, last)) L.finish_group(last, c, cc, sv, rng, a.dt);
+                const bool more = m >= 0 && !last;
                 if (__any_sync(0xffffffffu, more))
                     done |= L.iterate_group(more, c, cc, sv, rng, a.dt, a.event_cap, err) && more;
                 first = false;

@@ -199,9 +199,12 @@ void shape_rule(int precision, int n_cells, int max_n, int cluster_req, int tile
     tile = tile_req > 0 ? tile_req : 0;
     if (C == 0 && tile == 0 && precision == GW_PRECISION_FP64) {
         // Default FP64: the SSA is bound by the FP64 pipe (one warp instruction per ~64 cycles per
-        // sub-partition), so a cell is spread over up to 16 CTAs of at most 96 CRUs: three full
-        // warps per CTA on three sub-partitions.
+        // sub-partition), so a cell is spread over up to 16 CTAs of at most 96 CRUs, and where SMs are
+        // idle down to 32, a round of four warps on the four sub-partitions.  us per step at rest of one
+        // cell of 64 CRUs over 1 and 2 CTAs: 21.2, 10.4; of 200 over 3, 8: 18.6, 12.6; of 400 over 6, 16:
+        // 19.0, 13.2; of 1,250 over 12, 16: 25.0, 19.8.
         C = std::min(kMaxClusterCtas, std::max(1, (max_n + 95) / 96));
+        C = std::max(C, std::min({kMaxClusterCtas, (max_n + 31) / 32, kSpreadCtas / n_cells}));
         tile = (max_n + C - 1) / C;
     } else if (C == 0 && tile == 0) {
         // Default FP32: one CRU per SSA thread where possible, at most 16 CTAs per cell.

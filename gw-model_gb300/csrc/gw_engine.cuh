@@ -1275,34 +1275,64 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                     continue;
                 }
                 const int nsw = n_ssa >> 5;
-                // This warp's CRUs [cursor, end).  A lane whose CRU has finished its step takes the
-                // next one, so lanes with pending SSA events do not hold the others back.
+                // This warp's CRUs [beg, end), four lanes each (grouped) or one, on no more warps than these fill.
                 // (a leader takes CRUs on its first lead_warps SSA warps only, possibly none)
-                // No more working warps than ceil(CRUs / 32).  An FP64 warp instruction takes its
-                // sub-partition's FP64 pipe for ~64 cycles whatever its active lanes, so two warps of
-                // 16 CRUs cost twice one warp of 32; the first warps of a CTA sit on distinct
-                // sub-partitions.
-                int nse = v.leader ? w.lead_warps : nsw;
-                nse = min(nse, (w.cru_count + 31) >> 5);
+                const bool grouped = w.cru_count <= kGroupCrusFp64;
+                const int per = grouped ? 8 : 32;
+                const int nse = max(1, min(v.leader ? w.lead_warps : nsw, (w.cru_count + per - 1) / per));
                 const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
                 const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
-                int cursor = beg;
                 FluxAcc<FP64> acc;
                 Cru<R> c;
                 SsaLane<R, true> sl;
                 Stream rng;
-                int m = -1;  // CRU of this lane; -1 none yet, -2 none left
+                const int jq = lane & 3, base = lane & ~3;
+                auto load = [&](int mm) {
+                    tile_get(c, tile[mm]);
+                    rng.open(a.seed, (uint32_t)(a.cell_base + cell), (uint32_t)(w.cru_begin + mm), step0 + s, 0);
+                    sl.begin_group(c, cc);
+                };
+                auto store = [&](int mm, int err) {  // (a group's on its first lane)
+                    tile_put(tile[mm], c);
+                    my_events += (unsigned long long)sl.ev;
+                    my_err |= err;
+                    acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
+                            __popc((c.flags >> 4) & 0xFu));
+                };
                 {
-                    // Pass 1: the warp's CRUs, one iteration per lane and pass.  An iteration that the
-                    // FP32 screen shows to be the step's last runs without the FP64 rates (finish); a
-                    // CRU whose first iteration it declines (an event in the step) goes, untouched in
-                    // the tile, to the CTA's queue, and its lane takes the next CRU.
+                    // Pass 1: the warp's CRUs.  One whose first iteration the FP32 screen shows to be the step's
+                    // last runs without the FP64 rates (finish); the others (an event in the step) go,
+                    // untouched in the tile, to the CTA's queue.
                     int *qn = v.fq + par;
                     int *q = v.fq + 4;
                     if (threadIdx.x == 0) v.fq[par ^ 1] = 0;  // step s-1's count: every reader has passed
                                                               // bar_or(2) of this step
+                    for (int b = beg; grouped && b < end; b += 8) {
+                        // (a group without a CRU holds, and computes along on, the range's last)
+                        const int mb = b + (lane >> 2), m = min(mb, end - 1);
+                        load(m);
+                        const bool last = sl.surely_last_group(c, cc, sk, svf, rng, dt) && mb < end;
+                        sl.finish_group(last, c, cc, sv, rng, dt);
+                        if (last && jq == 0) store(m, 0);
+                        int qs = 0;
+                        if (!last && mb < end && jq == 0) {
+                            qs = atomicAdd(qn, 1);
+                            if (qs < kEngQCap) q[qs] = m;
+                        }
+                        bool more = __shfl_sync(0xffffffffu, qs, base) >= kEngQCap;
+                        while (__any_sync(0xffffffffu, more)) {  // the queue is full
+                            int err = 0;
+                            if (sl.iterate_group(more, c, cc, sv, rng, dt, a.event_cap, err) && more) {
+                                if (jq == 0) store(m, err);
+                                more = false;
+                            }
+                        }
+                    }
+                    // One per lane: a lane whose CRU is done takes the warp's next one.
+                    int m = grouped ? -2 : -1;  // CRU of this lane; -1 none yet, -2 none left
+                    int cursor = beg;
                     bool fresh = false;
-                    for (;;) {
+                    while (!grouped) {
                         const unsigned need = __ballot_sync(0xffffffffu, m == -1);
                         if (need) {
                             const int nm = cursor + __popc(need & ((1u << lane) - 1u));
@@ -1338,61 +1368,52 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                             }
                             fresh = false;
                             if (done) {
-                                tile_put(tile[m], c);
-                                my_events += (unsigned long long)sl.ev;
-                                my_err |= err;
-                                acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
-                                        __popc((c.flags >> 4) & 0xFu));
+                                store(m, err);
                                 m = -1;
                             }
                         }
                     }
-                    // Pass 2: the queued CRUs on four lanes each (SsaLane::iterate_group: one subunit's
-                    // rates per lane), eight per warp at a time, over the CTA's SSA warps.
+                    // Pass 2: the queued CRUs on four lanes each, eight per warp at a time, over the CTA's SSA
+                    // warps.
                     ssa_bar(n_ssa);
                     const int nq = min(*qn, kEngQCap);
-                    const int jq = lane & 3, base = lane & ~3;
                     const int nwu = min(nsw, (nq + 7) >> 3);
                     if (warp < nwu) {
                         int qc = (int)((int64_t)nq * warp / nwu);
                         const int qe = (int)((int64_t)nq * (warp + 1) / nwu);
-                        m = -1;
+                        m = -1;  // the group's CRU
                         bool first = false;
                         for (;;) {
                             const unsigned need = __ballot_sync(0xffffffffu, m == -1 && jq == 0);
                             if (need) {
                                 const int nm = qc + __popc(need & ((1u << base) - 1u));
                                 qc += __popc(need);
-                                if (m == -1) {  // (a group without one holds the range's last)
-                                    const int mq = q[min(nm, qe - 1)];
-                                    tile_get(c, tile[mq]);
-                                    rng.open(a.seed, (uint32_t)(a.cell_base + cell), (uint32_t)(w.cru_begin + mq),
-                                             step0 + s, 0);
-                                    sl.begin(c, cc);
+                                const Cru<R> c0 = c;
+                                const SsaLane<R, true> sl0 = sl;
+                                const Stream rng0 = rng;
+                                const int mq = q[min(nm, qe - 1)];
+                                load(mq);  // (a group without one holds the range's last)
+                                if (m == -1) {
                                     first = true;
                                     m = nm < qe ? mq : -2;
+                                } else {
+                                    c = c0;
+                                    sl = sl0;
+                                    rng = rng0;
                                 }
                             }
                             if (!__any_sync(0xffffffffu, m >= 0)) break;
-                            // (a group that ended its CRU with finish(), or has none, computes along)
                             int err = 0;
-                            bool done = m >= 0 && !first && sl.surely_last(c, cc, sk, svf, rng, dt);
-                            if (done) sl.finish(c, cc, sv, rng, dt);
-                            const bool more = m >= 0 && !done;
+                            const bool last = sl.surely_last_group(c, cc, sk, svf, rng, dt) && m >= 0 && !first;
+                            bool done = last;
+                            if (__any_sync(0xffffffffu, last)) sl.finish_group(last, c, cc, sv, rng, dt);
+                            const bool more = m >= 0 && !last;
                             if (__any_sync(0xffffffffu, more))
                                 done |= sl.iterate_group(more, c, cc, sv, rng, dt, a.event_cap, err) && more;
                             first = false;
-                            if (m >= 0) {
-                                if (done) {
-                                    if (jq == 0) {
-                                        tile_put(tile[m], c);
-                                        my_events += (unsigned long long)sl.ev;
-                                        my_err |= err;
-                                        acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
-                                                __popc((c.flags >> 4) & 0xFu));
-                                    }
-                                    m = -1;
-                                }
+                            if (done) {
+                                if (jq == 0) store(m, err);
+                                m = -1;
                             }
                         }
                     }

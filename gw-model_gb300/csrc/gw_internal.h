@@ -74,6 +74,9 @@ constexpr int kGroupCrus = 16;
 // FP32 engine, larger CTAs: an event batch (eight CRUs) in quiet passes (32 CRUs).
 constexpr int kBatchCost = 4;
 
+// FP64 engine: CTAs with at most this many CRUs run every CRU's step on four lanes.
+constexpr int kGroupCrusFp64 = 384;
+
 // One CTA's share of work: a contiguous CRU range of one cell.  A cell's CTAs are contiguous in
 // its cluster, starting at cluster rank `first`; the first of them (the leader) runs the cell's
 // global ODE.

@@ -1051,9 +1051,8 @@ struct SsaLane {
 
     // update_CaSS (SSA.tpp:87-99), first pass, for subunit j: its new CaSS (tmp_j) and threshold
     // crossing (kind_j; a positive count of the re-split pair adds its draws to D).
-    __device__ __forceinline__ void cass_update(const Cru<R> &s, const SsaConsts<R> &c, int j, R h,
-                                                const R (&jxfer)[4], const R (&jiss)[4], R &tmp_j, int &kind_j,
-                                                uint32_t &D) const {
+    __device__ __forceinline__ void cass_update(const Cru<R> &s, const SsaConsts<R> &c, int j, R h, R jxfer_j, R jiss_j,
+                                                R &tmp_j, int &kind_j, uint32_t &D) const {
         // (pick4: j may be a lane's own subunit, and a register array indexed by a value known only
         // at run time would go to local memory)
         const R x = pick4(s.cass, j);
@@ -1066,7 +1065,7 @@ struct SsaLane {
             const R uv = u * v;
             beta = __fdividef((float)uv, (float)(uv + c.BSR_const * v + c.BSL_const * u));
         }
-        const R d = h * (pick4(s.jlcc, j) + pick4(jrel, j) - pick4(jxfer, j) + pick4(jiss, j)) * beta;
+        const R d = h * (pick4(s.jlcc, j) + pick4(jrel, j) - jxfer_j + jiss_j) * beta;
         tmp_j = x + d;
         kind_j = crossing<R>(s, j, x, tmp_j, D);
     }
@@ -1080,7 +1079,7 @@ struct SsaLane {
         int kind[4];
         uint32_t D = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) cass_update(s, c, j, h, jxfer, jiss, tmp[j], kind[j], D);
+        for (int j = 0; j < 4; ++j) cass_update(s, c, j, h, jxfer[j], jiss[j], tmp[j], kind[j], D);
         // Event selection from the rates of the start of this iteration, draws k+D+1, k+D+2, k+D+3.
         uint32_t kk = k + 1u + D;
         int act = 0, aj = 0, atr = 0;
@@ -1131,32 +1130,81 @@ struct SsaLane {
             info->aj = aj;
             info->atr = atr;
         }
-        jxfer_sum = jxfer[0] + jxfer[1] + jxfer[2] + jxfer[3];
         k = kk;
-        if (last) return true;
-        if (++ev > cap) {
-            err = 1;
-            return true;
-        }
-        return false;
+        const bool over = !last && ++ev > cap;
+        if (over) err = 1;
+        if (last || over) jxfer_sum = jxfer[0] + jxfer[1] + jxfer[2] + jxfer[3];
+        return last || over;
     }
 
-    // iterate() by the four lanes of a group (lanes 4g .. 4g+3 of the warp, every one holding the
-    // same CRU and lane state; EXACT, R = double): lane j = lane & 3 evaluates the 17 rates and the
-    // CaSS update of subunit j, the group exchanges them by shuffles, and the rest runs on the four
-    // lanes alike.  Same expressions in the same order as iterate(), hence the same results on every
-    // lane; an FP64 warp instruction costs the same whatever its active lanes, so the iteration takes
-    // about a third of the FP64 instructions of one lane's.  The whole warp calls it together, and its
-    // shuffles are the whole warp's: (each group's own four lanes as the mask would split the warp).  A group that is not live
+    // The same by the four lanes of a group (lanes 4g .. 4g+3 of the warp, every one holding the same CRU and lane
+    // state; EXACT, R = double): lane j = lane & 3 evaluates subunit j's flux, CaSS update and rates, the
+    // group exchanges them by shuffles, and the rest runs on the four lanes alike.  Same expressions in the
+    // same order as the one-lane functions, hence the same results on every lane; an FP64 warp instruction
+    // takes its sub-partition's pipe for ~64 cycles whatever its active lanes, and a group's step without
+    // an event has about 45 of them on its path where one lane's has 130 (an iteration 130 and 330), at
+    // 1.4 times as many in all per CRU.  The whole warp calls them together, and their shuffles are the whole
+    // warp's (each group's own four lanes as the mask would split the warp).  A group that is not live
     // computes along and leaves its state as it is.
+    __device__ __forceinline__ void begin_group(const Cru<R> &s, const SsaConsts<R> &c) {
+        const int lane = (int)(threadIdx.x & 31u), j = lane & 3, base = lane & ~3;
+        t = (R)0;
+        k = 0;
+        ev = 0;
+        const R r = c.rRyR * count_r<R>(byte_s(s.ryr[2], j) + byte_s(s.ryr[3], j)) * (s.cajsr - pick4(s.cass, j));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) jrel[q] = __shfl_sync(0xffffffffu, r, base + q);
+    }
+    // fluxes() of subunit j alone, and jtr
+    __device__ __forceinline__ R fluxes_group(const Cru<R> &s, const SsaConsts<R> &c, const R *sv, int j, R &jx, R &js) const {
+        const R x = pick4(s.cass, j);
+        const R n0 = (j & 1) ? s.cass[0] : s.cass[1], n1 = (j & 1) ? s.cass[2] : s.cass[3];
+        js = c.riss * minus_twice(n0 + n1, x);
+        jx = c.rxfer * (x - sv[SV_CAI]);
+        return c.rtr * (sv[SV_CANSR] - s.cajsr);
+    }
+    // update_CaSS's first pass, on the group
+    __device__ __forceinline__ void cass_group(const Cru<R> &s, const SsaConsts<R> &c, int j, R h, R jx, R js, R (&tmp)[4],
+                                               int (&kind)[4], uint32_t &D) const {
+        const int base = (int)(threadIdx.x & 28u);
+        R tj;
+        int kj;
+        uint32_t Dj = 0;
+        cass_update(s, c, j, h, jx, js, tj, kj, Dj);
+        D = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            tmp[q] = __shfl_sync(0xffffffffu, tj, base + q);
+            kind[q] = 0;
+        }
+        if (__any_sync(0xffffffffu, kj)) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                kind[q] = __shfl_sync(0xffffffffu, kj, base + q);
+                D += __shfl_sync(0xffffffffu, Dj, base + q);
+            }
+        }
+    }
+    __device__ __forceinline__ void finish_group(bool live, Cru<R> &s, const SsaConsts<R> &c, const R *sv, Stream &rng, R dt) {
+        const int lane = (int)(threadIdx.x & 31u), j = lane & 3, base = lane & ~3;
+        R jx, js, tmp[4], jxfer[4];
+        int kind[4], err = 0;
+        uint32_t D;
+        const R jtr1 = fluxes_group(s, c, sv, j, jx, js);
+        cass_group(s, c, j, dt - t, jx, js, tmp, kind, D);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) jxfer[q] = __shfl_sync(0xffffffffu, jx, base + q);
+        if (!live) return;
+        jtr = jtr1;
+        conclude(s, c, sv, rng, dt - t, true, tmp, kind, D, k + 1u + D, 0, 0, 0, jxfer, 0, err, nullptr);
+    }
     __device__ __forceinline__ bool iterate_group(bool live, Cru<R> &s, const SsaConsts<R> &c, const R *sv,
                                                   Stream &rng, R dt, int cap, int &err) {
         static_assert(sizeof(R) == 8 && EXACT, "the group iteration is for the FP64 lane");
         constexpr unsigned kAll = 0xffffffffu;
         const int lane = (int)(threadIdx.x & 31u), j = lane & 3, base = lane & ~3;
-        R jxfer[4], jiss[4];
-        const R jtr0 = jtr;
-        fluxes(s, c, sv, jxfer, jiss);
+        R jx, js;
+        const R jtr1 = fluxes_group(s, c, sv, j, jx, js);
         Rates<R> rj;
         const R sj = subunit_rates<R>(s, j, pick4(s.cass, j), c, sv, rj);
         R sub[4];
@@ -1167,19 +1215,10 @@ struct SsaLane {
         const R jump = quot(-log(u0), total);
         const bool last = !live || !(t + jump < dt);
         const R h = last ? (dt - t) : jump;
-        R tj;
-        int kj;
-        uint32_t Dj = 0;
-        cass_update(s, c, j, h, jxfer, jiss, tj, kj, Dj);
         R tmp[4];
         int kind[4];
-        uint32_t D = 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            tmp[q] = __shfl_sync(kAll, tj, base + q);
-            kind[q] = __shfl_sync(kAll, kj, base + q);
-            D += __shfl_sync(kAll, Dj, base + q);
-        }
+        uint32_t D;
+        cass_group(s, c, j, h, jx, js, tmp, kind, D);
         uint32_t kk = k + 1u + D;
         int act = 0, aj = 0, atr = 0;
         if (__any_sync(kAll, !last)) {
@@ -1199,10 +1238,11 @@ struct SsaLane {
             r.clch = __shfl_sync(kAll, rj.clch, src);
             if (!last) select_transition<R, true>(r, pick4(sub, aj), rng, kk, act, atr);
         }
-        if (!live) {
-            jtr = jtr0;
-            return false;
-        }
+        R jxfer[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) jxfer[q] = __shfl_sync(kAll, jx, base + q);
+        if (!live) return false;
+        jtr = jtr1;
         return conclude(s, c, sv, rng, h, last, tmp, kind, D, kk, act, aj, atr, jxfer, cap, err, nullptr);
     }
 
@@ -1239,6 +1279,25 @@ struct SsaLane {
             ok &= f32_trunc(s.cass[j], x);
             screen_subunit(s, j, x, xb, c, sk, svf, T, A);
         }
+        return screened(T, A, ok, sk, rng, dt);
+    }
+    // The same on a group's four lanes, a subunit each (the sums' order differs, within the bound above).
+    __device__ __forceinline__ bool surely_last_group(const Cru<R> &s, const SsaConsts<R> &c, const float *sk,
+                                                      const float *svf, Stream &rng, R dt) {
+        const int j = (int)(threadIdx.x & 3u);
+        const R xj = pick4(s.cass, j);
+        float T = 0.f, A = 0.f, x;
+        const bool okj = f32_trunc(xj, x);
+        screen_subunit(s, j, x, __double_as_longlong(xj), c, sk, svf, T, A);
+        if (!okj) T = -1.f, A = 1.f / 0.f;  // (fails the screen for the group)
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            T += __shfl_xor_sync(0xffffffffu, T, o);
+            A += __shfl_xor_sync(0xffffffffu, A, o);
+        }
+        return screened(T, A, true, sk, rng, dt);
+    }
+    __device__ __forceinline__ bool screened(float T, float A, bool ok, const float *sk, Stream &rng, R dt) {
         uint32_t hi, lo;
         rng.words(k, hi, lo);
         const float u_hi = __uint2float_rn((hi >> 8) + 1u) * 0x1p-24f;

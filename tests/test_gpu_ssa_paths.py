@@ -1,8 +1,14 @@
-"""FP32 engine: a cell's trajectory does not depend on how its CRUs are spread over CTAs and warps.
+"""A cell's trajectory does not depend on how its CRUs are spread over CTAs and warps.
+
+FP32 engine.
 
 A CTA takes its CRUs on four lanes each (few of them), or in quiet passes followed by the CRUs that may
 have a jump, each warp its own or queued for the event warps (the split between both following the
 events); the flux sums are exact.  So every launch shape gives the same bits.
+
+FP64 engine.  A CTA takes its CRUs on four lanes each or one, with the CRUs that have an event queued for
+four lanes each (or, the queue full, at once).  The order of the flux sums follows the shape, but the CRUs
+after one step depend on none: every shape gives their same bits.
 """
 import numpy as np
 import pytest
@@ -27,17 +33,17 @@ def states(n, busy):
                            ClCh=(rng.random((n, 4)) < 0.05).astype(np.int32))
 
 
-def simulate(n, busy, **shape):
+def simulate(n, busy, precision="fp32", steps=60, **shape):
     from gwgb300 import engine
 
-    e = engine.Ensemble([n], precision="fp32", seed=5, **shape)
+    e = engine.Ensemble([n], precision=precision, seed=5, **shape)
     if busy:
         g = e.get_globals(0)
         g[0], g[3], g[4] = -3.7, 4.0e-4, 0.88
         e.set_globals(0, g)
     e.set_crus(0, states(n, busy))
     e.set_pulse(0.0, 500.0, 0.5, 100.0)
-    e.run(1e-3, 60)
+    e.run(1e-3, steps)
     s = e.get_crus(0)
     out = {k: np.array(getattr(s, k)) for k in ("CaSS", "CaJSR", "LCC", "LCC_inactivation", "RyR", "ClCh")}
     out["globals"] = e.get_globals(0)
@@ -61,4 +67,19 @@ def test_every_shape_gives_the_same_bits(n, shapes, busy):
     for cl, tile in shapes:
         got = simulate(n, busy, cluster_ctas=cl, cta_crus=tile)
         for k in want:
+            assert np.array_equal(want[k], got[k]), (k, cl, tile)
+
+
+@pytest.mark.parametrize("busy", [False, True])
+@pytest.mark.parametrize("n,shapes", [
+    (7, [(2, 0)]),                          # part of one group of eight
+    (65, [(1, 96), (2, 64)]),               # one more than a pass of eight warps
+    (385, [(1, 416), (2, 0), (4, 0)]),      # one more than the CTAs of four lanes per CRU take
+    (1100, [(1, 1120), (2, 576), (4, 288)]),  # more events than the queue holds when busy
+])
+def test_every_shape_gives_the_same_crus_fp64(n, shapes, busy):
+    want = simulate(n, busy, precision="fp64", steps=1, cluster_ctas=0)
+    for cl, tile in shapes:
+        got = simulate(n, busy, precision="fp64", steps=1, cluster_ctas=cl, cta_crus=tile)
+        for k in ("CaSS", "CaJSR", "LCC", "LCC_inactivation", "RyR", "ClCh", "events"):
             assert np.array_equal(want[k], got[k]), (k, cl, tile)
