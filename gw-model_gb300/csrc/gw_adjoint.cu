@@ -180,12 +180,6 @@ __device__ __forceinline__ void stage_cell(CellStatic &dst, const CellStatic &sr
     for (int i = (int)threadIdx.x; i < (int)(sizeof(CellStatic) / 16); i += (int)blockDim.x) d[i] = s[i];
 }
 
-// The item of thread t when a level's items are dealt round-robin over the block's warps: each item
-// takes its own code path, and a warp runs the paths of its lanes one after the other, so items
-// spread over the four warps (four sub-partitions, four FP64 units) finish about 4x sooner than
-// items packed into the lanes of one or two warps.
-__device__ __forceinline__ int item_of(int t) { return (t & 31) * (kBlk / 32) + (t >> 5); }
-
 __device__ __forceinline__ void open_counts(const CruD &c, int o[4]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) o[j] = dev::byte_s(c.ryr[2], j) + dev::byte_s(c.ryr[3], j);
@@ -760,29 +754,95 @@ __global__ void __launch_bounds__(kBlk) k_cru_busy(const GradArgs a, const AdjAr
 }
 
 // Reverse of the global step `step` (one block per cell): the cell's block sums of the CRU rows, the
-// increment's transcendental terms one per thread, the kAdjParts parts of the increment's adjoint
-// one per thread into rows summed in a fixed order, then the CRU inputs' contributions.
+// increment's transcendental terms, the kAdjParts parts of the increment's adjoint into rows summed in a
+// fixed order, then the CRU inputs' contributions.
+//
+// Bound by the FP64 pipe, which takes ~64 cycles per warp instruction whatever its active lanes: what counts
+// is how many are issued per sub-partition.  So the terms are dealt to warps by function, the argument
+// per lane and one call for all lanes of the warp; each part has a warp of its own, a Kv chain's 26 edges on
+// its lanes; divisions go through the integer pipe; and every output is written by its own thread.  (One
+// part or term per thread over four warps, each with its own calls and the chains' edges one after the
+// other: 55 us per step; now 25.)
 constexpr int kAdjOut = kNumGlobals + 3 + kTheta;  // lam_g, lam_cy, lam_th of one part
-__global__ void __launch_bounds__(kBlk) k_global_adj(const GradArgs a, const AdjArgs b, int64_t step, int slot) {
+constexpr int kGlobAdjBlk = 32 * (kAdjParts + 1);
+// The term of thread t: the exponentials on warps 0, 1, 6 and 7 (one per sub-partition), the logarithms on
+// warp 2, the powers on warp 3, K1's exponential (its argument needs a logarithm) on warp 4.
+__device__ __forceinline__ int term_of(int t) {
+    const int w = t >> 5, l = t & 31;
+    if (w == 2) return l == 0 ? T_LNA : (l == 1 ? T_LK : (l == 2 ? T_LKS : -1));
+    if (w == 3) return l == 0 ? T_PNAK : (l == 1 ? T_FU : (l == 2 ? T_RU : -1));
+    if (w == 4) return l == 0 ? T_K1 : -1;
+    const int q = w < 2 ? w : (w == 6 ? 2 : (w == 7 ? 3 : -1));
+    int k = 4 * l + q;  // among the others, in order: E, E1, ENAK, RKR, KP, then AM on
+    if (q < 0 || k >= kNT - 7) return -1;
+    return k == 0 ? T_E : (k == 1 ? T_E1 : (k == 2 ? T_ENAK : (k == 3 ? T_RKR : (k == 4 ? T_KP : k - 5 + T_AM))));
+}
+// kv_edges' edges: from, to, rate, and coefficient n u / v with u and v from {1, f1..f4, b1..b4}.
+__constant__ unsigned char kKvFrom[26] = {0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 5, 5, 6, 6, 6, 7, 7, 7, 8, 8, 8, 9, 9};
+__constant__ unsigned char kKvTo[26] = {1, 5, 0, 2, 6, 1, 3, 7, 2, 4, 8, 3, 9, 6, 0, 5, 7, 1, 6, 8, 2, 7, 9, 3, 8, 4};
+__constant__ unsigned char kKvRate[26] = {0, 3, 2, 0, 3, 2, 0, 3, 2, 0, 3, 2, 3, 0, 1, 2, 0, 1, 2, 0, 1, 2, 0, 1, 2, 1};
+__constant__ unsigned char kKvN[26] = {4, 1, 1, 3, 1, 2, 2, 1, 3, 1, 1, 4, 1, 4, 1, 1, 3, 1, 2, 2, 1, 3, 1, 1, 4, 1};
+__constant__ unsigned char kKvU[26] = {0, 0, 0, 0, 1, 0, 0, 2, 0, 0, 3, 0, 4, 5, 0, 0, 6, 0, 1, 7, 0, 2, 8, 0, 3, 0};
+__constant__ unsigned char kKvV[26] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 5, 5, 2, 6, 6, 3, 7, 7, 4, 8};
+__constant__ unsigned char kKvFirst[11] = {0, 2, 5, 8, 11, 13, 15, 18, 21, 24, 26};  // edges of each state
+// glob_increment_adj's part AP_KV43 (ch 1) or AP_KV14 (ch 0) by a warp, the same sums in the same order.
+__device__ __forceinline__ void kv_adj_warp(const CellStatic &C, int ch, const double *T, const double *x,
+                                            const double *l, double dt, int lane, double (*sc)[2], double *row, double *lx) {
+    const gw_params &p = C.p;
+    double r[4];
+    kv_rates(p, ch, T, r);
+    const double f1 = ch == 0 ? p.f1Kv14 : p.f1Kv43, f2 = ch == 0 ? p.f2Kv14 : p.f2Kv43;
+    const double f3 = ch == 0 ? p.f3Kv14 : p.f3Kv43, f4 = ch == 0 ? p.f4Kv14 : p.f4Kv43;
+    const double b1 = ch == 0 ? p.b1Kv14 : p.b1Kv43, b2 = ch == 0 ? p.b2Kv14 : p.b2Kv43;
+    const double b3 = ch == 0 ? p.b3Kv14 : p.b3Kv43, b4 = ch == 0 ? p.b4Kv14 : p.b4Kv43;
+    const int k = min(lane, 25), a = kKvFrom[k], b = kKvTo[k];
+    auto par = [&](int i) {
+        return i == 0 ? 1.0 : (i == 1 ? f1 : (i == 2 ? f2 : (i == 3 ? f3 : (i == 4 ? f4 : (i == 5 ? b1 : (i == 6 ? b2 : (i == 7 ? b3 : b4)))))));
+    };
+    const double n = kKvN[k] == 1 ? 1.0 : (kKvN[k] == 2 ? 2.0 : (kKvN[k] == 3 ? 3.0 : 4.0));
+    const double coef = div_rn(n * par(kKvU[k]), par(kKvV[k]));
+    const double qv = coef * dev::pick4(r, kKvRate[k]), w = dt * (l[b] - l[a]);
+    if (lane < 26) {
+        sc[lane][0] = qv * w;
+        sc[lane][1] = coef * x[a] * w;
+    }
+    __syncwarp();
+    double v = 0.0;
+    if (lane < 10) {
+        for (int q = kKvFirst[lane]; q < kKvFirst[lane + 1]; ++q) v += sc[q][0];
+        lx[lane] = v;
+    } else if (lane < 14) {
+        for (int q = 0; q < 26; ++q)
+            if (kKvRate[q] == lane - 10) v += sc[q][1];
+    }
+    double lr[4];
+    for (int q = 0; q < 4; ++q) lr[q] = __shfl_sync(0xffffffffu, v, 10 + q);
+    const double ka = ch == 0 ? p.aaKv14 : p.aaKv43, ki = ch == 0 ? p.aiKv14 : p.aiKv43;
+    const double kb = ch == 0 ? p.baKv14 : p.baKv43, kbi = ch == 0 ? p.biKv14 : p.biKv43;
+    if (lane == 0) row[0] = lr[0] * ka * r[0] - lr[1] * ki * r[1] - lr[2] * kb * r[2] + lr[3] * kbi * r[3];
+}
+__global__ void __launch_bounds__(kGlobAdjBlk) k_global_adj(const GradArgs a, const AdjArgs b, int64_t step, int slot) {
     __shared__ double T[kNT];
     __shared__ double sai[kAdjIn];
     __shared__ double lam[kNumGlobals];
+    __shared__ double gs[kNumGlobals];
     __shared__ double rows[kAdjParts][kAdjOut];
-    __shared__ double tot[kAdjOut];
+    __shared__ double sc[2][26][2];
+    __shared__ double djl[2];
     __shared__ __align__(16) CellStatic C;
     const int cell = blockIdx.x;
-    const int t = (int)threadIdx.x;
+    const int t = (int)threadIdx.x, warp = t >> 5, lane = t & 31;
     stage_cell(C, a.cs[cell]);
-    if (t < kAdjIn) {
-        double v = 0.0;
-        for (int k = a.blk0[cell]; k < a.blk0[cell + 1]; ++k) v += b.ai_part[(int64_t)kAdjIn * k + t];
-        sai[t] = v;
-    }
     const int64_t r = (int64_t)slot * a.n_cells + cell;
     const double *g = a.seg_G + r * kNumGlobals;
-    const double *cyv = a.seg_carry + r * 4;
-    const Carry cy{cyv[0], cyv[1], cyv[2], cyv[3]};
+    const double *sv = a.seg_sv + r * kSvCount;
     double *lgp = b.lam_G + (int64_t)kNumGlobals * cell;
+    if (t >= 64 && t < 64 + kAdjIn) {
+        double v = 0.0;
+#pragma unroll 8
+        for (int k = a.blk0[cell]; k < a.blk0[cell + 1]; ++k) v += b.ai_part[(int64_t)kAdjIn * k + t - 64];
+        sai[t - 64] = v;
+    }
     if (t < kNumGlobals) {
         double v = lgp[t];
         if (t == 0 && (step + 1) % a.sample_every == 0) {
@@ -790,42 +850,55 @@ __global__ void __launch_bounds__(kBlk) k_global_adj(const GradArgs a, const Adj
             if (si < a.n_samples) v += b.dLdV[(int64_t)cell * a.n_samples + si];
         }
         lam[t] = v;
+        gs[t] = g[t];
+    }
+    if (warp < kAdjParts)
+        for (int k = lane; k < kAdjOut; k += 32) rows[warp][k] = 0.0;
+    __syncthreads();
+    const int it = term_of(t);
+    if (it >= 0) {
+        TermKind kind;
+        double y;
+        const double x = glob_arg(C, gs, it, kind, y);
+        if (warp == 2)
+            T[it] = log(x);
+        else if (warp == 3)
+            T[it] = term_pow(x, y);
+        else
+            T[it] = exp(x);
+    }
+    if (warp == kAdjParts && lane == 0) jlcc_factor_derivs(C, gs[0], sv[SV_JEXP], djl[0], djl[1]);
+    __syncthreads();
+    if (warp == AP_KV43 || warp == AP_KV14) {
+        const int ch = warp == AP_KV14 ? 0 : 1, at = ch == 0 ? 26 : 16;
+        kv_adj_warp(C, ch, T, gs + at, lam + at, a.dt, lane, sc[ch], rows[warp], rows[warp] + at);
+    } else if (warp < kAdjParts && lane == 0) {
+        const double *cyv = a.seg_carry + r * 4;
+        const Carry cy{cyv[0], cyv[1], cyv[2], cyv[3]};
+        double *row = rows[warp];
+        glob_increment_adj(C, gs, cy, a.dt, T, lam, warp, row, row + kNumGlobals, row + kNumGlobals + 3);
     }
     __syncthreads();
-    const int it = item_of(t);
-    if (it < kNT) T[it] = glob_term(C, g, it);
-    __syncthreads();
-    if (it < kAdjParts) {
-        double *row = rows[it];
-        for (int k = 0; k < kAdjOut; ++k) row[k] = 0.0;
-        glob_increment_adj(C, g, cy, a.dt, T, lam, it, row, row + kNumGlobals, row + kNumGlobals + 3);
-    }
-    __syncthreads();
-    if (t < kAdjOut) {
-        double v = 0.0;
-        for (int q = 0; q < kAdjParts; ++q) v += rows[q][t];
-        tot[t] = v;
-    }
-    __syncthreads();
-    if (t != 0) return;
-    const double *sv = a.seg_sv + r * kSvCount;
-    double lg[kNumGlobals];
-    for (int k = 0; k < kNumGlobals; ++k) lg[k] = tot[k];
-    double *th = b.lam_th + (int64_t)kTheta * cell;
-    double lth[kTheta];
-    for (int k = 0; k < kTheta; ++k) lth[k] = th[k] + tot[kNumGlobals + 3 + k];
+    if (t >= kAdjOut) return;
+    double v = 0.0;
+    for (int q = 0; q < kAdjParts; ++q) v += rows[q][t];
     // the CRUs' step inputs: Cai, CaNSR and the JLCC factors of V
-    lg[3] += sai[0];
-    lg[4] += sai[1];
-    double dJM, dJE;
-    jlcc_factor_derivs(C, g[0], sv[SV_JEXP], dJM, dJE);
-    lg[0] += sai[2] * dJM + sai[3] * dJE;
-    lth[TH_PCAL] += sai[2] * sv[SV_JMUL];
-    lth[TH_RRYR] += sai[4];
-    lth[TH_CSQNT] += sai[5] * C.CSQN_const;
-    for (int k = 0; k < kNumGlobals; ++k) lgp[k] = lg[k];
-    for (int k = 0; k < 3; ++k) b.lam_cy[3 * (int64_t)cell + k] = tot[kNumGlobals + k];
-    for (int k = 0; k < kTheta; ++k) th[k] = lth[k];
+    if (t < kNumGlobals) {
+        if (t == 0) v += sai[2] * djl[0] + sai[3] * djl[1];
+        if (t == 3) v += sai[0];
+        if (t == 4) v += sai[1];
+        lgp[t] = v;
+    } else if (t < kNumGlobals + 3) {
+        b.lam_cy[3 * (int64_t)cell + t - kNumGlobals] = v;
+    } else {
+        const int k = t - kNumGlobals - 3;
+        double *th = b.lam_th + (int64_t)kTheta * cell + k;
+        v += *th;
+        if (k == TH_PCAL) v += sai[2] * sv[SV_JMUL];
+        if (k == TH_RRYR) v += sai[4];
+        if (k == TH_CSQNT) v += sai[5] * C.CSQN_const;
+        *th = v;
+    }
 }
 
 // SSA constants of every cell, for the kernels whose threads mix cells.
@@ -1323,7 +1396,7 @@ int gw_grad_backward(gw_grad *g, const double *dL_dV, double *sens) {
         for (int64_t s = s1 - 1; s >= s0; --s) {
             k_cru_busy<<<bgrid, kBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
             k_cru_quiet<<<g->n_blocks, kBlk, 0, g->stream>>>(a, b, (int)(s - s0));
-            k_global_adj<<<g->n_cells, kBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
+            k_global_adj<<<g->n_cells, kGlobAdjBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
         }
     }
     cudaEventRecord(g->ev1, g->stream);

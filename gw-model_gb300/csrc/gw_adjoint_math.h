@@ -84,58 +84,74 @@ enum Term {
     kNT = T_KV43 + 4
 };
 
-GW_HD double glob_term(const CellStatic &C, const double *g, int k) {
+enum TermKind { TK_EXP, TK_LOG, TK_POW };
+// Term k is exp(x), log(x) or pow(x, y) of the x returned.
+GW_HD double glob_arg(const CellStatic &C, const double *g, int k, TermKind &kind, double &y) {
     const gw_params &p = C.p;
     const double V = g[0];
+    kind = TK_EXP;
+    y = 0.0;
     switch (k) {
-    case T_E: return exp(-(V * C.F_RT));
-    case T_LNA: return log(p.Nao / g[1]);
-    case T_LK: return log(p.Ko / g[2]);
-    case T_E1: return exp(p.eta * (V * C.F_RT));
-    case T_ENAK: return exp(-0.1 * (V * C.F_RT));
-    case T_PNAK: return pow(p.KmNai / g[1], 1.5);
-    case T_RKR: return exp(0.0446 * V);
-    case T_LKS: return log((p.Ko + 0.01833 * p.Nao) / (g[2] + 0.01833 * g[1]));
+    case T_E: return -(V * C.F_RT);
+    case T_LNA: kind = TK_LOG; return div_rn(p.Nao, g[1]);
+    case T_LK: kind = TK_LOG; return div_rn(p.Ko, g[2]);
+    case T_E1: return p.eta * (V * C.F_RT);
+    case T_ENAK: return -0.1 * (V * C.F_RT);
+    case T_PNAK: kind = TK_POW; y = 1.5; return div_rn(p.KmNai, g[1]);
+    case T_RKR: return 0.0446 * V;
+    case T_LKS: kind = TK_LOG; return div_rn(p.Ko + 0.01833 * p.Nao, g[2] + 0.01833 * g[1]);
     case T_K1: {
-        const double EK = log(p.Ko / g[2]) * C.RT_F / 1.0;
-        return exp(1.5 * (V - EK) * C.F_RT);
+        const double EK = log(div_rn(p.Ko, g[2])) * C.RT_F;
+        return 1.5 * (V - EK) * C.F_RT;
     }
-    case T_KP: return exp((7.488 - V) / 5.98);
-    case T_FU: return pow(g[3] / p.Kmf, p.Hf);
-    case T_RU: return pow(g[4] / p.Kmr, p.Hr);
-    case T_AM: return exp(-0.1 * (V + 47.13));
-    case T_BM: return exp(-V / 11.0);
-    case T_BH_HI: return exp(-(V + 10.66) / 11.1);
-    case T_BJ_HI_Z: return exp(-0.1 * (V + 32.0));
-    case T_BJ_HI_Y: return exp(-2.535e-7 * V);
-    case T_AH_LO: return exp(-(V + 80.0) / 6.8);
-    case T_BH_LO_1: return exp(0.079 * V);
-    case T_BH_LO_2: return exp(0.35 * V);
-    case T_AJ_A: return exp(0.2444 * V);
-    case T_AJ_B: return exp(-0.04391 * V);
-    case T_AJ_D: return exp(0.311 * (V + 79.23));
-    case T_BJ_LO_Z: return exp(-0.1378 * (V + 40.14));
-    case T_BJ_LO_Y: return exp(-0.01052 * V);
-    case T_XINF: return exp(-(V - 24.7) / 13.6);
-    case T_TAU1: return exp(-0.148 * (V - 10.0));
-    case T_TAU2: return exp(0.0687 * (V - 10.0));
-    case T_KR + 0: return exp(0.0272 * V);
-    case T_KR + 1: return exp(-0.0431 * V);
-    case T_KR + 2: return exp(0.0262 * V);
-    case T_KR + 3: return exp(2.71e-6 * V);
-    case T_KR + 4: return exp(-0.0269 * V);
-    case T_KR + 5: return exp(0.0120 * V);
-    case T_KR + 6: return exp(-0.0443 * V);
-    case T_KV14 + 0: return exp(p.aaKv14 * V);
-    case T_KV14 + 1: return exp(-p.aiKv14 * V);
-    case T_KV14 + 2: return exp(-p.baKv14 * V);
-    case T_KV14 + 3: return exp(p.biKv14 * V);
-    case T_KV43 + 0: return exp(p.aaKv43 * V);
-    case T_KV43 + 1: return exp(-p.aiKv43 * V);
-    case T_KV43 + 2: return exp(-p.baKv43 * V);
-    case T_KV43 + 3: return exp(p.biKv43 * V);
+    case T_KP: return div_rn(7.488 - V, 5.98);
+    case T_FU: kind = TK_POW; y = p.Hf; return div_rn(g[3], p.Kmf);
+    case T_RU: kind = TK_POW; y = p.Hr; return div_rn(g[4], p.Kmr);
+    case T_AM: return -0.1 * (V + 47.13);
+    case T_BM: return div_rn(-V, 11.0);
+    case T_BH_HI: return div_rn(-(V + 10.66), 11.1);
+    case T_BJ_HI_Z: return -0.1 * (V + 32.0);
+    case T_BJ_HI_Y: return -2.535e-7 * V;
+    case T_AH_LO: return div_rn(-(V + 80.0), 6.8);
+    case T_BH_LO_1: return 0.079 * V;
+    case T_BH_LO_2: return 0.35 * V;
+    case T_AJ_A: return 0.2444 * V;
+    case T_AJ_B: return -0.04391 * V;
+    case T_AJ_D: return 0.311 * (V + 79.23);
+    case T_BJ_LO_Z: return -0.1378 * (V + 40.14);
+    case T_BJ_LO_Y: return -0.01052 * V;
+    case T_XINF: return div_rn(-(V - 24.7), 13.6);
+    case T_TAU1: return -0.148 * (V - 10.0);
+    case T_TAU2: return 0.0687 * (V - 10.0);
+    case T_KR + 0: return 0.0272 * V;
+    case T_KR + 1: return -0.0431 * V;
+    case T_KR + 2: return 0.0262 * V;
+    case T_KR + 3: return 2.71e-6 * V;
+    case T_KR + 4: return -0.0269 * V;
+    case T_KR + 5: return 0.0120 * V;
+    case T_KR + 6: return -0.0443 * V;
+    case T_KV14 + 0: return p.aaKv14 * V;
+    case T_KV14 + 1: return -p.aiKv14 * V;
+    case T_KV14 + 2: return -p.baKv14 * V;
+    case T_KV14 + 3: return p.biKv14 * V;
+    case T_KV43 + 0: return p.aaKv43 * V;
+    case T_KV43 + 1: return -p.aiKv43 * V;
+    case T_KV43 + 2: return -p.baKv43 * V;
+    case T_KV43 + 3: return p.biKv43 * V;
     default: return 0.0;
     }
+}
+
+// pow(x, y) of those: the model's exponents by square roots (within 1.5 ulp, as pow)
+GW_HD double term_pow(double x, double y) {
+    const double r = sqrt(x);
+    return y == 1.5 ? x * r : (y == 0.75 ? r * sqrt(r) : pow(x, y));
+}
+GW_HD double glob_term(const CellStatic &C, const double *g, int k) {
+    TermKind kind;
+    double y;
+    const double x = glob_arg(C, g, k, kind, y);
+    return kind == TK_EXP ? exp(x) : (kind == TK_LOG ? log(x) : term_pow(x, y));
 }
 
 GW_HD void glob_terms(const CellStatic &C, const double *g, double *T) {
@@ -241,7 +257,7 @@ GW_HD KrQ kr_q(const double *T) {
     q.q32 = 0.0009 * T[T_KR + 4];
     q.q34 = 0.0622 * T[T_KR + 5];
     q.q43 = 0.0059 * T[T_KR + 6];
-    q.q42 = q.q32 * q.q43 * q.q24 / (q.q23 * q.q34);
+    q.q42 = div_rn(q.q32 * q.q43 * q.q24, q.q23 * q.q34);
     return q;
 }
 
@@ -257,46 +273,46 @@ GW_HD Gates gate_rates(double V, bool derivs, const double *T) {
     const bool hi = V >= -40.0;
     {
         const double w = V + 47.13, E = T[T_AM];
-        r.am = (V == -47.13) ? 3.2 : 0.32 * w / (1.0 - E);
-        if (derivs) r.dam = (V == -47.13) ? 0.16 : 0.32 * ((1.0 - E) - w * 0.1 * E) / sqd(1.0 - E);
+        r.am = (V == -47.13) ? 3.2 : div_rn(0.32 * w, 1.0 - E);
+        if (derivs) r.dam = (V == -47.13) ? 0.16 : div_rn(0.32 * ((1.0 - E) - w * 0.1 * E), sqd(1.0 - E));
     }
     r.bm = 0.08 * T[T_BM];
-    r.dbm = -r.bm / 11.0;
+    r.dbm = div_rn(-r.bm, 11.0);
     if (hi) {
         r.ah = 0.0;
         const double X = T[T_BH_HI];
-        r.bh = 1.0 / (0.13 * (1.0 + X));
-        r.dbh = r.bh * X / (11.1 * (1.0 + X));
+        r.bh = div_rn(1.0, 0.13 * (1.0 + X));
+        r.dbh = div_rn(r.bh * X, 11.1 * (1.0 + X));
         r.aj = 0.0;
         const double Z = T[T_BJ_HI_Z], y0 = 0.3 * T[T_BJ_HI_Y];
-        r.bj = y0 / (1.0 + Z);
-        r.dbj = r.bj * (-2.535e-7 + 0.1 * Z / (1.0 + Z));
+        r.bj = div_rn(y0, 1.0 + Z);
+        r.dbj = r.bj * (-2.535e-7 + div_rn(0.1 * Z, 1.0 + Z));
     } else {
         r.ah = 0.135 * T[T_AH_LO];
-        r.dah = -r.ah / 6.8;
+        r.dah = div_rn(-r.ah, 6.8);
         const double e1 = T[T_BH_LO_1], e2 = T[T_BH_LO_2];
         r.bh = 3.56 * e1 + 3.1e5 * e2;
         r.dbh = 3.56 * 0.079 * e1 + 3.1e5 * 0.35 * e2;
         const double ea = T[T_AJ_A], eb = T[T_AJ_B];
         const double P = -127140.0 * ea - 3.474e-5 * eb, Qv = V + 37.78;
         const double D = 1.0 + T[T_AJ_D];
-        r.aj = P * Qv / D;
+        r.aj = div_rn(P * Qv, D);
         const double dP = -127140.0 * 0.2444 * ea + 3.474e-5 * 0.04391 * eb, dD = 0.311 * (D - 1.0);
-        r.daj = (dP * Qv + P) / D - P * Qv * dD / sqd(D);
+        r.daj = div_rn(dP * Qv + P, D) - div_rn(P * Qv * dD, sqd(D));
         const double Z = T[T_BJ_LO_Z], y0 = 0.1212 * T[T_BJ_LO_Y];
-        r.bj = y0 / (1.0 + Z);
-        r.dbj = r.bj * (-0.01052 + 0.1378 * Z / (1.0 + Z));
+        r.bj = div_rn(y0, 1.0 + Z);
+        r.dbj = r.bj * (-0.01052 + div_rn(0.1378 * Z, 1.0 + Z));
     }
     {
         const double X = T[T_XINF];
-        r.xinf = 1.0 / (1.0 + X);
-        r.dxinf = r.xinf * r.xinf * X / 13.6;
+        r.xinf = div_rn(1.0, 1.0 + X);
+        r.dxinf = div_rn(r.xinf * r.xinf * X, 13.6);
     }
     {
         const double u = V - 10.0, E1 = T[T_TAU1], E2 = T[T_TAU2];
-        r.tinv = 0.0000719 * u / (1.0 - E1) + 0.000131 * u / (E2 - 1.0);
-        r.dtinv = 0.0000719 * ((1.0 - E1) - u * 0.148 * E1) / sqd(1.0 - E1) +
-                  0.000131 * ((E2 - 1.0) - u * 0.0687 * E2) / sqd(E2 - 1.0);
+        r.tinv = div_rn(0.0000719 * u, 1.0 - E1) + div_rn(0.000131 * u, E2 - 1.0);
+        r.dtinv = div_rn(0.0000719 * ((1.0 - E1) - u * 0.148 * E1), sqd(1.0 - E1)) +
+                  div_rn(0.000131 * ((E2 - 1.0) - u * 0.0687 * E2), sqd(E2 - 1.0));
     }
     return r;
 }
@@ -553,7 +569,7 @@ GW_HD void step_values(const CellStatic &C, const double *g, double *sv) {
 // dJM/dV and dJE/dV of the JLCC factors: JE = exp(2 V F/RT), JM = JLCC_const V F/RT / (JE - 1).
 GW_HD void jlcc_factor_derivs(const CellStatic &C, double V, double JE, double &dJM, double &dJE) {
     dJE = 2.0 * C.F_RT * JE;
-    dJM = C.JLCC_const * C.F_RT * ((JE - 1.0) - V * dJE) / sqd(JE - 1.0);
+    dJM = div_rn(C.JLCC_const * C.F_RT * ((JE - 1.0) - V * dJE), sqd(JE - 1.0));
 }
 
 // The adjoint of one global increment, in kAdjParts independent parts: with lam = dL/dG[s+1] and
@@ -571,11 +587,11 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
     const double *Kr = g + 11, *Kv43 = g + 16, *Kv14 = g + 26;
     const double F_RT = C.F_RT, RT_F = C.RT_F, CSA = C.CSA_FVcyto;
     const double VF_RT = V * F_RT, e = T[T_E];
-    const double ENa = T[T_LNA] * RT_F, EK = T[T_LK] * RT_F, ECa = T[T_LK] * RT_F / 2.0;
+    const double ENa = T[T_LNA] * RT_F, EK = T[T_LK] * RT_F, ECa = T[T_LK] * RT_F * 0.5;
     // adjoints of the currents: d[0] = dt (Istim - sum I), d[1] and d[2] their Na and K shares, d[3] the
     // buffered cytosolic Ca balance (lQ = lam3 dt beta), d[4] the NSR balance
     const double l0 = -dt * lam[0], l1 = -dt * CSA * lam[1], l2 = -dt * CSA * lam[2];
-    auto beta_cyto = [&]() { return 1.0 / (1.0 + C.CMDN_const / sqd(p.KCMDN + Cai)); };
+    auto beta_cyto = [&]() { return div_rn(1.0, 1.0 + div_rn(C.CMDN_const, sqd(p.KCMDN + Cai))); };
     double lV = 0, lNai = 0, lKi = 0, lCai = 0, lCaNSR = 0, lVF = 0, le = 0, lENa = 0, lEK = 0, lECa = 0;
     switch (part) {
     case AP_NA: {
@@ -590,7 +606,7 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
         lENa -= lINa * p.GNa * m3hj + lINab * p.GNab;
         const double e1 = T[T_E1], e2 = e1 * e;
         const double numNC = e1 * cubed(Nai) * p.Cao - e2 * C.Nao3 * Cai, denNC = 1.0 + p.ksat * e2;
-        const double rden = 1.0 / denNC;
+        const double rden = div_rn(1.0, denNC);
         const double INaCa = C.INaCa_const * numNC * rden;
         const double lnum = lINaCa * C.INaCa_const * rden;
         const double lden = -lINaCa * INaCa * rden;
@@ -606,17 +622,17 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
     case AP_NAK: {
         const double lINaK = l0 + 3 * l1 - 2 * l2, lIKr = l0 + l2, lIKs = l0 + l2;
         const double E1k = T[T_ENAK];
-        const double fNaK = 1.0 / (1.0 + 0.1245 * E1k + 0.0365 * C.sigma * e);
-        const double rq = 1.0 / (1.0 + T[T_PNAK]);
+        const double fNaK = div_rn(1.0, 1.0 + 0.1245 * E1k + 0.0365 * C.sigma * e);
+        const double rq = div_rn(1.0, 1.0 + T[T_PNAK]);
         const double INaK = C.INaK_const * fNaK * rq;
         const double lf = lINaK * C.INaK_const * rq;
         const double lq = -lINaK * INaK * rq;
-        lNai += lq * (-1.5 * T[T_PNAK] / Nai);
+        lNai += lq * div_rn(-1.5 * T[T_PNAK], Nai);
         const double lD = -lf * sqd(fNaK);
         lVF += lD * 0.1245 * (-0.1) * E1k;
         le += lD * 0.0365 * C.sigma;
         lam_th[TH_INAK] += lINaK * INaK;
-        const double ERk = T[T_RKR], RKr = 1.0 / (1.0 + 1.4945 * ERk);
+        const double ERk = T[T_RKR], RKr = div_rn(1.0, 1.0 + 1.4945 * ERk);
         const double k = p.GKr * C.sqrtKo * 0.5;
         lam_g[14] += lIKr * k * RKr * (V - EK);
         const double dRKr = -sqd(RKr) * 1.4945 * 0.0446 * ERk;
@@ -626,7 +642,7 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
         const double sKs = Ki + 0.01833 * Nai, EKs = T[T_LKS] * RT_F;
         lam_g[10] += lIKs * 2 * p.GKs * xKs * (V - EKs);
         lV += lIKs * p.GKs * sqd(xKs);
-        const double lEKs = -lIKs * p.GKs * sqd(xKs), rs = RT_F / sKs;
+        const double lEKs = -lIKs * p.GKs * sqd(xKs), rs = div_rn(RT_F, sKs);
         lKi -= lEKs * rs;
         lNai -= lEKs * 0.01833 * rs;
         lam_th[TH_GKS] += lIKs * (p.GKs * sqd(xKs) * (V - EKs));
@@ -634,7 +650,7 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
     }
     case AP_TO: {
         const double lIto1 = l0 + l2, lIto2 = l0;
-        const double P14 = C.PKv14_Csc * kFaradayA, r1 = 1.0 / (1 - e);
+        const double P14 = C.PKv14_Csc * kFaradayA, r1 = div_rn(1.0, 1 - e);
         const double A14 = (Ki - p.Ko * e) + 0.02 * (Nai - p.Nao * e);
         const double mm = P14 * VF_RT * Kv14[4] * r1;
         const double lmm = lIto1 * A14 * 1.0e9, lA = lIto1 * mm * 1.0e9;
@@ -647,7 +663,7 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
         lam_g[20] += lIto1 * p.GKv43 * (V - EK);
         lV += lIto1 * p.GKv43 * Kv43[4];
         lEK -= lIto1 * p.GKv43 * Kv43[4];
-        const double r2 = 1.0 / (e - 1.0);
+        const double r2 = div_rn(1.0, e - 1.0);
         const double B = (p.Clcyto * e - p.Clo) * r2, k = cy.clch * C.Ito2_const;
         lVF += lIto2 * k * B;
         le += lIto2 * k * VF_RT * (p.Clo - p.Clcyto) * r2 * r2;
@@ -657,31 +673,31 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
         const double lIK1 = l0 + l2, lIKp = l0 + l2;
         const double lQ = lam[3] * dt * beta_cyto();
         const double lICab = l0 - 0.5 * CSA * lQ, lIpCa = l0 - 0.5 * CSA * lQ;
-        const double uK1 = V - EK, EK1 = T[T_K1], K1inf = 1.0 / (2.0 + EK1);
+        const double uK1 = V - EK, EK1 = T[T_K1], K1inf = div_rn(1.0, 2.0 + EK1);
         const double dK1 = -sqd(K1inf) * 1.5 * F_RT * EK1;
         const double dIdu = p.GK1 * C.IK1_const * (K1inf + uK1 * dK1);
         lV += lIK1 * dIdu;
         lEK -= lIK1 * dIdu;
         lam_th[TH_GK1] += lIK1 * (p.GK1 * K1inf * C.IK1_const * uK1);
-        const double EKp = T[T_KP], Kp = 1. / (1. + EKp);
-        const double dKp = sqd(Kp) * EKp / 5.98;
+        const double EKp = T[T_KP], Kp = div_rn(1., 1. + EKp);
+        const double dKp = div_rn(sqd(Kp) * EKp, 5.98);
         lV += lIKp * p.GKp * (Kp + (V - EK) * dKp);
         lEK -= lIKp * p.GKp * Kp;
         lam_cy[0] += l0 * C.ICaL_const;  // ICaL = sum JLCC x ICaL_const
         lV += lICab * p.GCab;
         lECa -= lICab * p.GCab;
-        lCai += lIpCa * p.IpCamax * p.KmpCa / sqd(p.KmpCa + Cai);
+        lCai += div_rn(lIpCa * p.IpCamax * p.KmpCa, sqd(p.KmpCa + Cai));
         break;
     }
     case AP_CA: {
         const double beta = beta_cyto(), lQ = lam[3] * dt * beta;
-        const double fu = T[T_FU], ru = T[T_RU], rd = 1.0 / (1.0 + fu + ru);
+        const double fu = T[T_FU], ru = T[T_RU], rd = div_rn(1.0, 1.0 + fu + ru);
         const double Jup = (p.Vmaxf * fu - p.Vmaxr * ru) * rd;
         const double dLT = p.kLTRPNp * Cai * (p.LTRPNtot - CaLT) - p.kLTRPNm * CaLT;
         const double dHT = p.kHTRPNp * Cai * (p.HTRPNtot - CaHT) - p.kHTRPNm * CaHT;
         const double e1 = T[T_E1], e2 = e1 * e;
-        const double INaCa = C.INaCa_const * (e1 * cubed(Nai) * p.Cao - e2 * C.Nao3 * Cai) / (1.0 + p.ksat * e2);
-        const double ICab = p.GCab * (V - ECa), IpCa = p.IpCamax * (Cai / (p.KmpCa + Cai));
+        const double INaCa = div_rn(C.INaCa_const * (e1 * cubed(Nai) * p.Cao - e2 * C.Nao3 * Cai), 1.0 + p.ksat * e2);
+        const double ICab = p.GCab * (V - ECa), IpCa = p.IpCamax * div_rn(Cai, p.KmpCa + Cai);
         const double Q3 =
             -0.5 * CSA * (ICab + IpCa - 2 * INaCa) + C.VSS_Vcyto * (cy.jxfer * C.CRU_factor) - Jup - (dLT + dHT);
         const double lbeta = lam[3] * dt * Q3;
@@ -689,12 +705,12 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
         const double ldLT = -lQ + dt * lam[5], ldHT = -lQ + dt * lam[6];
         const double dJdf = (p.Vmaxf * (1.0 + ru) + p.Vmaxr * ru) * rd * rd;
         const double dJdr = -(p.Vmaxr * (1.0 + fu) + p.Vmaxf * fu) * rd * rd;
-        lCai += lJup * dJdf * p.Hf * fu / Cai;
-        lCaNSR += lJup * dJdr * p.Hr * ru / CaNSR;
+        lCai += div_rn(lJup * dJdf * p.Hf * fu, Cai);
+        lCaNSR += div_rn(lJup * dJdr * p.Hr * ru, CaNSR);
         lam_th[TH_VMAX] += lJup * Jup;
         lam_cy[1] += -dt * C.VJSR_VNSR * lam[4] * C.CRU_factor;
         lam_cy[2] += C.VSS_Vcyto * lQ * C.CRU_factor;
-        lCai += lbeta * sqd(beta) * 2.0 * C.CMDN_const / cubed(p.KCMDN + Cai);
+        lCai += div_rn(lbeta * sqd(beta) * 2.0 * C.CMDN_const, cubed(p.KCMDN + Cai));
         lCai += ldLT * p.kLTRPNp * (p.LTRPNtot - CaLT) + ldHT * p.kHTRPNp * (p.HTRPNtot - CaHT);
         lam_g[5] += ldLT * (-p.kLTRPNp * Cai - p.kLTRPNm);
         lam_g[6] += ldHT * (-p.kHTRPNp * Cai - p.kHTRPNm);
@@ -738,11 +754,11 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
         edge(4, 3, q.q43, &lq43);
         edge(4, 2, q.q42, &lq42);
         // q42 = q32 q43 q24 / (q23 q34)
-        lq32 += lq42 * q.q42 / q.q32;
-        lq43 += lq42 * q.q42 / q.q43;
-        lq24 += lq42 * q.q42 / q.q24;
-        lq23 -= lq42 * q.q42 / q.q23;
-        lq34 -= lq42 * q.q42 / q.q34;
+        lq32 += div_rn(lq42 * q.q42, q.q32);
+        lq43 += div_rn(lq42 * q.q42, q.q43);
+        lq24 += div_rn(lq42 * q.q42, q.q24);
+        lq23 -= div_rn(lq42 * q.q42, q.q23);
+        lq34 -= div_rn(lq42 * q.q42, q.q34);
         lV += lq01 * 0.0272 * q.q01 + lq10 * (-0.0431) * q.q10 + lq23 * 0.0262 * q.q23 + lq24 * 2.71e-6 * q.q24 +
               lq32 * (-0.0269) * q.q32 + lq34 * 0.0120 * q.q34 + lq43 * (-0.0443) * q.q43;
         break;
@@ -769,8 +785,8 @@ GW_HD void glob_increment_adj(const CellStatic &C, const double *g, const Carry 
     }
     }
     // this part's Nernst potentials, VF_RT and e = exp(-VF_RT) back to the globals
-    if (lENa != 0.0) lNai += lENa * (-RT_F / Nai);
-    if (lEK != 0.0 || lECa != 0.0) lKi += lEK * (-RT_F / Ki) + lECa * (-RT_F / (2.0 * Ki));
+    if (lENa != 0.0) lNai += lENa * div_rn(-RT_F, Nai);
+    if (lEK != 0.0 || lECa != 0.0) lKi += lEK * div_rn(-RT_F, Ki) + lECa * div_rn(-RT_F, 2.0 * Ki);
     lV += F_RT * lVF - F_RT * e * le;
     lam_g[0] += lV;
     lam_g[1] += lNai;
