@@ -58,6 +58,7 @@ namespace {
 constexpr int kBlk = 128;     // threads per block of the CRU kernels (one cell per block)
 constexpr int kSsaBlocksPerSm = 3;  // k_ssa without variants: resident blocks per SM (register cap)
 constexpr int kQCap = 512;    // k_ssa: CRUs per block whose first iteration runs after the block's ranges
+constexpr int kBusyBlk = 32;  // threads of k_busy_rec and k_cru_busy: a warp, for every sub-partition to get its share
 constexpr int kRec = 16;      // sub-steps a CRU keeps per block of its reverse sweep
 constexpr int kAdjIn = 6;     // per-cell CRU adjoints: Cai, CaNSR, JM, JE, rRyR (relative), CSQN_const
 constexpr int kLamX = 9;      // CRU adjoint state: CaSS[4], CaJSR, JLCC[4]
@@ -133,6 +134,7 @@ struct GradArgs {
 };
 
 // Adjoint arrays.
+struct Rec;
 struct AdjArgs {
     double *lam_x;      // [n_crus][9]
     double *lam_G;      // [n_cells][36]
@@ -140,7 +142,11 @@ struct AdjArgs {
     double *lam_th;     // [n_cells][8] relative sensitivities
     double *ai_row;     // [n_crus][kAdjIn] each CRU's adjoints of its step inputs and parameters
     double *ai_part;    // [blocks][kAdjIn] each block's sums of its CRUs' rows
-    const dev::SsaConsts<double> *cc;  // [n_cells] SSA constants (k_cru_busy)
+    const dev::SsaConsts<double> *cc;  // [n_cells] SSA constants (k_busy_rec, k_cru_busy)
+    Rec *pool;   // [pool_cap] the segment's recorded sub-steps, and how many are taken
+    int *pool_n;
+    int pool_cap;
+    int *rec_at;        // [slots][n_crus] where each listed CRU's are, or -1 where they did not fit
     const double *dLdV; // [n_cells][n_samples]
 };
 
@@ -674,6 +680,7 @@ struct Rec {
     CruCont s;
     double h;
     int ev, j, onew;
+    int n;  // of a CRU's first: how many the step has
 };
 
 // Re-runs a CRU's step from x0 and keeps iterations [lo, hi) in rec[k % kRec]; stops after hi
@@ -712,13 +719,40 @@ __device__ int run_rec(const CruD &x0, const dev::SsaConsts<double> &cc, const d
     return k;
 }
 
-// Reverse of step `step` for the CRUs the recompute listed (their step had jumps), one thread per
-// listed CRU: the step is re-run from its stored start state (same draws, same trajectory) to
-// recover the sub-steps, kRec at a time from the last block, and each block is reversed.
-__global__ void __launch_bounds__(kBlk) k_cru_busy(const GradArgs a, const AdjArgs b, int64_t step, int slot) {
+// Before a segment's reverse sweep: the sub-steps of all the CRUs that its steps listed (their step had jumps),
+// one thread per listed CRU, slot0 + blockIdx.y the step's slot.  The step is re-run from its stored start state
+// (same draws, same trajectory); steps do not wait for one another here, as they do in the sweep, where
+// the re-run took two thirds of k_cru_busy's time (84 us per step for three small cells, 165 for 32 x
+// 5,000 CRUs; now 31 and 58, and 3 and 20 here).  A step of more than kRec sub-steps, or one that finds the pool full, is left to
+// the sweep.
+__global__ void __launch_bounds__(kBusyBlk) k_busy_rec(const GradArgs a, const AdjArgs b, int64_t step0, int slot0) {
+    const int slot = slot0 + (int)blockIdx.y, nb = a.busy_n[slot];
+    for (int k = (int)(blockIdx.x * kBusyBlk + threadIdx.x); k < nb; k += (int)(gridDim.x * kBusyBlk)) {
+        const int64_t at = (int64_t)slot * a.n_crus + k, i = a.busy[at];
+        const int cell = a.cru_cell[i];
+        Rec rec[kRec];
+        const int n = run_rec(a.seg_x[(int64_t)slot * a.n_crus + i], b.cc[cell],
+                              a.seg_sv + ((int64_t)slot * a.n_cells + cell) * kSvCount, a.seed,
+                              (uint32_t)a.rng_cell[cell], (uint32_t)(i - a.cru0[cell]), (uint64_t)(step0 + slot), a.dt,
+                              a.event_cap, 0, kRec + 1, rec);
+        int to = -1;
+        if (n <= kRec && *(volatile int *)b.pool_n < b.pool_cap) {
+            to = atomicAdd(b.pool_n, n);
+            if (to > b.pool_cap - n) to = -1;
+        }
+        b.rec_at[at] = to;
+        if (to < 0) continue;
+        rec[0].n = n;
+        for (int q = 0; q < n; ++q) b.pool[to + q] = rec[q];
+    }
+}
+
+// Reverse of step `step` for the CRUs the recompute listed, one thread per listed CRU, from the sub-steps that
+// k_busy_rec recorded; without them the step is re-run here, kRec sub-steps at a time from the last block.
+__global__ void __launch_bounds__(kBusyBlk) k_cru_busy(const GradArgs a, const AdjArgs b, int64_t step, int slot) {
     const int nb = a.busy_n[slot];
-    for (int k = (int)(blockIdx.x * kBlk + threadIdx.x); k < nb; k += (int)(gridDim.x * kBlk)) {
-        const int64_t i = a.busy[(int64_t)slot * a.n_crus + k];
+    for (int k = (int)(blockIdx.x * kBusyBlk + threadIdx.x); k < nb; k += (int)(gridDim.x * kBusyBlk)) {
+        const int64_t at = (int64_t)slot * a.n_crus + k, i = a.busy[at];
         const int cell = a.cru_cell[i];
         const uint32_t m = (uint32_t)(i - a.cru0[cell]);
         const dev::SsaConsts<double> &cc = b.cc[cell];
@@ -732,19 +766,18 @@ __global__ void __launch_bounds__(kBlk) k_cru_busy(const GradArgs a, const AdjAr
         CruAdjIn ai{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         Rec rec[kRec];
         const uint32_t rc = (uint32_t)a.rng_cell[cell];
-        const int n = run_rec(x0, cc, sv, a.seed, rc, m, (uint64_t)step, a.dt, a.event_cap, 0, 1 << 30, rec);
-        for (int blk = (n - 1) / kRec; blk >= 0; --blk) {
-            const int lo = blk * kRec, hi = min(n, lo + kRec);
-            if (blk != (n - 1) / kRec) run_rec(x0, cc, sv, a.seed, rc, m, (uint64_t)step, a.dt, a.event_cap, lo, hi, rec);
-            for (int q = hi - 1; q >= lo; --q) {
-                const Rec &r = rec[q % kRec];
-                CruCont s1 = r.s;
-                double jt, jx;
-                cru_substep(s1, r.h, in, P, jt, jx);
-                cru_event_adj(s1, r.ev, r.j, r.onew, in, P, la, ai);
-                const bool last = q == n - 1;
-                cru_substep_adj(r.s, r.h, in, P, last ? lc[1] : 0.0, last ? lc[2] : 0.0, la, ai);
-            }
+        const Rec *const got = b.rec_at[at] >= 0 ? b.pool + b.rec_at[at] : nullptr;
+        const int n = got ? got->n
+                          : run_rec(x0, cc, sv, a.seed, rc, m, (uint64_t)step, a.dt, a.event_cap, 0, 1 << 30, rec);
+        CruCont s1 = cont_of(x0);  // the state at the sub-step's end (CaSS and CaJSR): the next one's start
+        for (int q = n - 1; q >= 0; --q) {
+            if (!got && q != n - 1 && q % kRec == kRec - 1)
+                run_rec(x0, cc, sv, a.seed, rc, m, (uint64_t)step, a.dt, a.event_cap, q - kRec + 1, q + 1, rec);
+            const Rec &r = got ? got[q] : rec[q % kRec];
+            const bool last = q == n - 1;  // (ends with the step, not with an event)
+            if (!last) cru_event_adj(s1, r.ev, r.j, r.onew, in, P, la, ai);
+            s1 = r.s;
+            cru_substep_adj(s1, r.h, in, P, last ? lc[1] : 0.0, last ? lc[2] : 0.0, la, ai);
         }
         int o[4];
         open_counts(x0, o);
@@ -999,7 +1032,8 @@ struct gw_grad {
     Buf x, out, part, G, carry, t, sv, status, events, V, regime;
     // checkpoints and segment
     Buf ck_x, ck_G, ck_carry, ck_t, ck_sv;
-    Buf seg_x, seg_G, seg_carry, seg_sv, quiet, busy, busy_n;
+    Buf seg_x, seg_G, seg_carry, seg_sv, quiet, busy, busy_n, pool, pool_n, rec_at;
+    int pool_cap = 0;
     // adjoint
     Buf lam_x, lam_G, lam_cy, lam_th, ai_row, ai_part, dLdV;
 
@@ -1061,6 +1095,10 @@ struct gw_grad {
         b.ai_part = ai_part.as<double>();
         b.cc = d_cc.as<dev::SsaConsts<double>>();
         b.dLdV = dLdV.as<double>();
+        b.pool = pool.as<Rec>();
+        b.pool_n = pool_n.as<int>();
+        b.pool_cap = pool_cap;
+        b.rec_at = rec_at.as<int>();
         return b;
     }
     // Restores the state of step s0 = k * ck_every from checkpoint k (k = -1: the initial state).
@@ -1247,6 +1285,8 @@ int gw_grad_create(const gw_grad_desc *d, gw_grad **out) {
     up(g->quiet, nullptr, sizeof(uint8_t) * N * S);
     up(g->busy, nullptr, sizeof(int) * N * S);
     up(g->busy_n, nullptr, sizeof(int) * S);
+    up(g->pool_n, nullptr, sizeof(int));
+    up(g->rec_at, nullptr, sizeof(int) * N * S);
     up(g->lam_x, nullptr, sizeof(double) * kLamX * N);
     up(g->lam_G, nullptr, sizeof(double) * kNumGlobals * C);
     up(g->lam_cy, nullptr, sizeof(double) * 3 * C);
@@ -1267,9 +1307,18 @@ int gw_grad_create(const gw_grad_desc *d, gw_grad **out) {
         delete g;
         return rc;
     }
+    // The pool of recorded sub-steps, for a quarter of the segment's CRU-steps (amid the Ca release six in a
+    // hundred have a jump, and their steps 2.2 sub-steps); without the memory for it the sweep does without.
+    g->pool_cap = (int)std::min<int64_t>(std::max<int64_t>(N * S / 4, 4096), 1 << 26);
+    if (g->pool.alloc(sizeof(Rec) * (size_t)g->pool_cap) != (int)cudaSuccess) {
+        cudaGetLastError();
+        g->pool.n = 0;
+        g->pool_cap = 0;
+    }
     g->stats.checkpoint_bytes = (int64_t)(g->ck_x.n + g->ck_G.n + g->ck_carry.n + g->ck_t.n + g->ck_sv.n);
     g->stats.segment_bytes =
-        (int64_t)(g->seg_x.n + g->seg_G.n + g->seg_carry.n + g->seg_sv.n + g->quiet.n + g->busy.n + g->busy_n.n);
+        (int64_t)(g->seg_x.n + g->seg_G.n + g->seg_carry.n + g->seg_sv.n + g->quiet.n + g->busy.n + g->busy_n.n +
+                  g->pool.n + g->pool_n.n + g->rec_at.n);
     *out = g;
     return GW_OK;
 }
@@ -1383,7 +1432,8 @@ int gw_grad_backward(gw_grad *g, const double *dL_dV, double *sens) {
     a.busy = g->busy.as<int>();
     a.busy_n = g->busy_n.as<int>();
     const AdjArgs b = g->adj_args();
-    const int bgrid = 2 * g->sm_count;
+    const int bgrid = 8 * g->sm_count;
+    const unsigned rgrid = (unsigned)std::min<int64_t>((g->n_crus + kBusyBlk - 1) / kBusyBlk, 256);
     cudaEventRecord(g->ev0, g->stream);
     for (int64_t k = g->n_ck - 1; k >= 0; --k) {
         const int64_t s0 = k * g->ck_every, s1 = std::min(s0 + g->ck_every, g->n_steps);
@@ -1393,8 +1443,12 @@ int gw_grad_backward(gw_grad *g, const double *dL_dV, double *sens) {
             k_ssa<false><<<g->n_blocks, kBlk, 0, g->stream>>>(a, s, (int)(s - s0));
             k_global<<<g->n_cells, kOdeLanes, 0, g->stream>>>(a, s, (int)(s - s0), 0);
         }
+        if ((rc = g->cuda(cudaMemsetAsync(g->pool_n.p, 0, g->pool_n.n, g->stream), "gw_grad_backward"))) return rc;
+        for (int64_t s = s0; s < s1; s += 32768)  // (the grid's y extent)
+            k_busy_rec<<<dim3(rgrid, (unsigned)std::min<int64_t>(s1 - s, 32768)), kBusyBlk, 0, g->stream>>>(a, b, s0,
+                                                                                                        (int)(s - s0));
         for (int64_t s = s1 - 1; s >= s0; --s) {
-            k_cru_busy<<<bgrid, kBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
+            k_cru_busy<<<bgrid, kBusyBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
             k_cru_quiet<<<g->n_blocks, kBlk, 0, g->stream>>>(a, b, (int)(s - s0));
             k_global_adj<<<g->n_cells, kGlobAdjBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
         }
