@@ -90,6 +90,8 @@ struct Buf {
 struct GradArgs {
     const OdeProgram *prog;     // the global step as the engine's lane program (shared by all cells)
     const CellStatic *cs;       // [n_cells] (ode_consts: the program's per-cell constants)
+    const dev::SsaConsts<double> *cc;  // [n_cells] SSA constants and float copies for the screen, or null: from cs
+    const float *sk;            // [n_cells][SK_COUNT]
     const int *blk_cell;        // [blocks] cell of each CRU block
     const int *blk_lo;          // [blocks] first CRU (within the cell) of each block
     const int *blk_hi;          // [blocks] end of the block's CRU range (within the cell)
@@ -240,11 +242,15 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
     __shared__ int qn;
     const int cell = a.blk_cell[blockIdx.x];
     constexpr bool var = VAR;  // the replay's variants (a.var_x and the var_* arrays set)
-    if (threadIdx.x == 0) dev::load_ssa_consts<double>(cc, a.cs[cell]);
-    if (threadIdx.x == 32) {
-        dev::load_screen_consts(sk, a.cs[cell]);
-        qn = 0;
+    if (a.cc) {  // (one thread forming them takes longer than a small block's CRUs)
+        const uint2 *src = reinterpret_cast<const uint2 *>(a.cc + cell);
+        for (int i = (int)threadIdx.x; i < (int)(sizeof cc / 8); i += kBlk) reinterpret_cast<uint2 *>(&cc)[i] = src[i];
+        if (threadIdx.x < dev::SK_COUNT) sk[threadIdx.x] = a.sk[(int64_t)cell * dev::SK_COUNT + threadIdx.x];
+    } else {
+        if (threadIdx.x == 0) dev::load_ssa_consts<double>(cc, a.cs[cell]);
+        if (threadIdx.x == 32) dev::load_screen_consts(sk, a.cs[cell]);
     }
+    if (threadIdx.x == 32) qn = 0;
     if (threadIdx.x < kSvCount) {
         sv[threadIdx.x] = a.sv[(int64_t)cell * kSvCount + threadIdx.x];
         svf[threadIdx.x] = (float)sv[threadIdx.x];
@@ -334,7 +340,25 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
     // the next CRU; so every pass of the range runs with full lanes.
     int m = a.status[cell] == 0 ? -1 : -2;  // CRU of this lane; -1 none yet, -2 none left
     bool fresh = false;                      // no iteration of the lane's CRU has run yet
-    for (;;) {
+    // (a block of up to eight CRUs per warp takes four lanes for each: see SsaLane::begin_group)
+    const bool grouped = !VAR && span <= 8 * nw && m == -1;
+    if (grouped) {
+        const int mb = cursor + (lane >> 2), mg = min(mb, end - 1);
+        if (cursor < end) {
+            // (a group without a CRU holds, and computes along on, the range's last)
+            fetch(mg, true);
+            const bool last = L.surely_last_group(c, cc, sk, svf, rng, a.dt) && mb < end;
+            L.finish_group(last, c, cc, sv, rng, a.dt);
+            if (mb < end && (lane & 3) == 0) {
+                if (last)
+                    after(mg, dev::IterInfo<double>{}, 0u, 0u, true);
+                else
+                    q[atomicAdd(&qn, 1)] = mg;  // (at most 8 nw of them)
+            }
+        }
+    }
+    static_assert(8 * (kBlk / 32) <= kQCap, "the queue holds a grouped block's CRUs");
+    while (!grouped) {
         const unsigned need = __ballot_sync(0xffffffffu, m == -1);
         if (need) {
             const int nm = cursor + __popc(need & ((1u << lane) - 1u));
@@ -935,9 +959,11 @@ __global__ void __launch_bounds__(kGlobAdjBlk) k_global_adj(const GradArgs a, co
 }
 
 // SSA constants of every cell, for the kernels whose threads mix cells.
-__global__ void k_init_consts(const CellStatic *cs, dev::SsaConsts<double> *cc, int n_cells) {
+__global__ void k_init_consts(const CellStatic *cs, dev::SsaConsts<double> *cc, float *sk, int n_cells) {
     const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (c < n_cells) dev::load_ssa_consts<double>(cc[c], cs[c]);
+    if (c >= n_cells) return;
+    dev::load_ssa_consts<double>(cc[c], cs[c]);
+    dev::load_screen_consts(sk + (int64_t)c * dev::SK_COUNT, cs[c]);
 }
 
 int fail_to(std::string &err, int code, const char *fmt, ...) {
@@ -1025,7 +1051,7 @@ struct gw_grad {
     gw_grad_stats stats{};
     std::vector<double> G_final;
     // tables
-    Buf d_cs, d_prog, d_blk_cell, d_blk_lo, d_blk_hi, d_blk0, d_cru_cell, d_cru0, d_ncru, d_rng_cell, d_stim, d_cc;
+    Buf d_cs, d_prog, d_blk_cell, d_blk_lo, d_blk_hi, d_blk0, d_cru_cell, d_cru0, d_ncru, d_rng_cell, d_stim, d_cc, d_sk;
     // initial state
     Buf x_init, G_init, carry_init, sv_init;
     // state
@@ -1056,6 +1082,8 @@ struct gw_grad {
         GradArgs a{};
         a.prog = d_prog.as<OdeProgram>();
         a.cs = d_cs.as<CellStatic>();
+        a.cc = d_cc.as<dev::SsaConsts<double>>();
+        a.sk = d_sk.as<float>();
         a.blk_cell = d_blk_cell.as<int>();
         a.blk_lo = d_blk_lo.as<int>();
         a.blk_hi = d_blk_hi.as<int>();
@@ -1255,6 +1283,7 @@ int gw_grad_create(const gw_grad_desc *d, gw_grad **out) {
     up(g->ai_part, nullptr, sizeof(double) * kAdjIn * g->n_blocks);
     up(g->d_cru_cell, g->cru_cell.data(), sizeof(int) * N);
     up(g->d_cc, nullptr, sizeof(dev::SsaConsts<double>) * C);
+    up(g->d_sk, nullptr, sizeof(float) * dev::SK_COUNT * C);
     up(g->d_cru0, g->cru0.data(), sizeof(int64_t) * C);
     up(g->d_ncru, g->ncru.data(), sizeof(int) * C);
     up(g->d_rng_cell, rng_cell.data(), sizeof(int) * C);
@@ -1298,7 +1327,8 @@ int gw_grad_create(const gw_grad_desc *d, gw_grad **out) {
     if (!rc) rc = g->cuda(cudaEventCreate(&g->ev1), "gw_grad_create");
     if (!rc) {
         k_init_consts<<<(d->n_cells + 127) / 128, 128, 0, g->stream>>>(g->d_cs.as<CellStatic>(),
-                                                                      g->d_cc.as<dev::SsaConsts<double>>(), d->n_cells);
+                                                                      g->d_cc.as<dev::SsaConsts<double>>(),
+                                                                      g->d_sk.as<float>(), d->n_cells);
         rc = g->cuda(cudaGetLastError(), "gw_grad_create");
         if (!rc) rc = g->cuda(cudaStreamSynchronize(g->stream), "gw_grad_create");
     }
