@@ -747,7 +747,7 @@ __device__ int run_rec(const CruD &x0, const dev::SsaConsts<double> &cc, const d
 // one thread per listed CRU, slot0 + blockIdx.y the step's slot.  The step is re-run from its stored start state
 // (same draws, same trajectory); steps do not wait for one another here, as they do in the sweep, where
 // the re-run took two thirds of k_cru_busy's time (84 us per step for three small cells, 165 for 32 x
-// 5,000 CRUs; now 31 and 58, and 3 and 20 here).  A step of more than kRec sub-steps, or one that finds the pool full, is left to
+// 5,000 CRUs; now 27 and 50, and 3 and 20 here).  A step of more than kRec sub-steps, or one that finds the pool full, is left to
 // the sweep.
 __global__ void __launch_bounds__(kBusyBlk) k_busy_rec(const GradArgs a, const AdjArgs b, int64_t step0, int slot0) {
     const int slot = slot0 + (int)blockIdx.y, nb = a.busy_n[slot];
