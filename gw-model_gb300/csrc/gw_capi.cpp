@@ -234,13 +234,15 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
     if (need > C)
         return fail(c, GW_ERR_UNSUPPORTED, "a cell of %d CRUs needs %d CTAs of %d CRUs but the cluster has %d",
                     max_n, need, tile, C);
-    // SSA warps: one for 32 CRUs; FP32 where there is an SM for every CTA down to one for eight CRUs, which take
-    // four lanes each (a cell of 60 CRUs amid the release 3.8 us per step, with a warp for 32 4.3; but
-    // 256 cells of 100, two CTAs to an SM, 6.9 at rest and 9.9 amid the release against 9.2 and 13.9).
+    // SSA warps.  FP64: four (beside the leader's ODE warps; eight in the others), since a CRU takes four lanes
+    // and the registers leave an SM one CTA anyway (a cell of 64 CRUs over 2 CTAs, one and four: 15.7 and
+    // 13.5 us per step).  FP32: one for 32 CRUs; where there is an SM for every CTA down to one for eight
+    // (a cell of 60 CRUs amid the release 3.8 us per step, with a warp for 32 4.3; but 256 cells of 100, two
+    // CTAs to an SM, 6.9 at rest and 9.9 amid the release against 9.2 and 13.9).
     int64_t ctas = 0;
     for (int i = 0; i < c->n_cells; ++i) ctas += (c->ncru[i] + tile - 1) / tile;
-    const bool fp64 = c->precision == GW_PRECISION_FP64;
-    c->ssa_warps = std::min(fp64 ? kMaxSsaWarpsFp64 : kMaxSsaWarps, tile / (fp64 || ctas > kSms ? 32 : 8));
+    c->ssa_warps = c->precision == GW_PRECISION_FP64 ? kMaxSsaWarpsFp64
+                                                     : std::min(kMaxSsaWarps, tile / (ctas > kSms ? 32 : 8));
     c->tile_cap = tile;
     // Pack cells (first-fit decreasing on CTA count) into clusters of C CTAs.
     std::vector<int> order(c->n_cells);

@@ -1275,11 +1275,14 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                     continue;
                 }
                 const int nsw = n_ssa >> 5;
-                // This warp's CRUs [beg, end), four lanes each (grouped) or one, on no more warps than these fill.
+                // This warp's CRUs [beg, end), four lanes each (grouped) or one.
                 // (a leader takes CRUs on its first lead_warps SSA warps only, possibly none)
                 const bool grouped = w.cru_count <= kGroupCrusFp64;
                 const int per = grouped ? 8 : 32;
-                const int nse = max(1, min(v.leader ? w.lead_warps : nsw, (w.cru_count + per - 1) / per));
+                // (no more warps than the rounds take: they share the sub-partitions' FP64 pipes)
+                const int fills = (w.cru_count + per - 1) / per, nwu = max(1, v.leader ? w.lead_warps : nsw);
+                const int rounds = max(1, (fills + nwu - 1) / nwu);
+                const int nse = grouped ? max(1, (fills + rounds - 1) / rounds) : max(1, min(nwu, fills));
                 const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
                 const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
                 FluxAcc<FP64> acc;
@@ -1377,10 +1380,10 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                     // warps.
                     ssa_bar(n_ssa);
                     const int nq = min(*qn, kEngQCap);
-                    const int nwu = min(nsw, (nq + 7) >> 3);
-                    if (warp < nwu) {
-                        int qc = (int)((int64_t)nq * warp / nwu);
-                        const int qe = (int)((int64_t)nq * (warp + 1) / nwu);
+                    const int nw2 = min(nsw, (nq + 7) >> 3);
+                    if (warp < nw2) {
+                        int qc = (int)((int64_t)nq * warp / nw2);
+                        const int qe = (int)((int64_t)nq * (warp + 1) / nw2);
                         m = -1;  // the group's CRU
                         bool first = false;
                         for (;;) {
