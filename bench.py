@@ -65,15 +65,15 @@ METRIC = "CRU-steps/s and sim-ms/wall-s: batched vs plain GPU vs CPU, at KS/FP64
 # FP32 CRU state per CRU: LCC states 4 B, gate + ClCh bits 4 B, RyR counts 24 B, CaSS 16 B,
 # JLCC 16 B, CaJSR 4 B, CaJSR compensation 4 B = 72 B, read and written once per CRU-step.
 BYTES_PER_CRU_STEP = 2 * 72
-# From the ncu captures of the engine kernel on this workload (profiles/engine_kernel_cell12500.txt
-# and profiles/engine_kernel_cell12500_instmix.txt, the launch at 0-1 ms of the beat): DRAM bytes
+# From the ncu capture of the engine kernel on this workload (profiles/engine_kernel_cell12500.txt,
+# the launch at 0-1 ms of the beat): DRAM bytes
 # (read + write) of one 1000-step launch, and warp instructions issued per CRU-step.
-TRAFFIC_PER_LAUNCH = 1.05472e6
-WARP_INST_PER_CRU_STEP = 31.25
+TRAFFIC_PER_LAUNCH = 1.095424e6
+WARP_INST_PER_CRU_STEP = 22.27
 # The same for config 3's ensemble kernel (profiles/engine_kernel_batched256.txt, one 100-step launch
 # at 20 ms): DRAM bytes per launch and CRU, and warp instructions per CRU-step.
-BATCHED_TRAFFIC_PER_LAUNCH_CRU = 213.9e6 / 1870540
-BATCHED_WARP_INST_PER_CRU_STEP = 38.8
+BATCHED_TRAFFIC_PER_LAUNCH_CRU = 214.4e6 / 1870540
+BATCHED_WARP_INST_PER_CRU_STEP = 32.97
 CPU_PRE_NCRU = 1250   # the CPU's beat run, tiled x10 to 12,500 CRUs at each window start
 
 
