@@ -14,10 +14,12 @@
 // step; then it is stepped in reverse:
 //   k_cru_quiet   the CRUs without a jump in the step (most of them): their step is one sub-step of
 //                 length dt, reversed directly from the stored start state.
-//   k_cru_busy    the listed CRUs, densely packed: each re-runs its step from its stored start state
-//                 with the same draws (hence the same jump times and transitions), keeps the
-//                 sub-steps in blocks of kRec and walks them backwards through the adjoint of the
-//                 sub-step and event arithmetic.
+//   k_busy_rec    once per segment: the listed CRUs of all its steps re-run their step from its stored
+//                 start state with the same draws (hence the same jump times and transitions) and
+//                 record the sub-steps.
+//   k_cru_busy    the listed CRUs of a step, densely packed: each walks its sub-steps backwards through
+//                 the adjoint of the sub-step and event arithmetic (without records it re-runs the
+//                 step itself, in blocks of kRec sub-steps).
 //   Both write per CRU its adjoint state and its adjoints of the step inputs (Cai, CaNSR, the JLCC
 //   factors) and of rRyR and CSQN.
 //   k_global_adj  one block per cell: sums the cell's CRU rows in a fixed order, then the adjoint
@@ -227,7 +229,9 @@ __device__ __forceinline__ CruIn cru_in(const double *sv) {
 
 // Forward SSA of step `step`: block b takes CRUs [blk_lo, blk_hi) of cell blk_cell, split evenly
 // over its warps; each warp runs its range with lane refill (one SSA iteration per pass; a lane
-// whose CRU finished its step takes the warp's next CRU).  CRUs whose first iteration the FP32
+// whose CRU finished its step takes the warp's next CRU), or, in blocks of at most eight CRUs per warp, on
+// four lanes per CRU (three cells of 180 to 420 CRUs: 144 us for a whole step and its reverse, 153 with
+// one lane per CRU and the constants formed by one thread per block).  CRUs whose first iteration the FP32
 // screen declines (an event in the step) run after the ranges, packed into as few warps as they
 // fill, so that the FP64 rate evaluations run with full lanes.
 template <bool VAR>
