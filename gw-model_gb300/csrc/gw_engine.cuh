@@ -944,7 +944,7 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
         const int64_t r_idx = rec ? ri / a.record_every - a.rec_base : -1;
         const bool rec_ok = rec && r_idx >= 0 && r_idx < a.rec_cap;
         if (my_err & 2) continue;
-        // (as in split_steps; the first two warps wait, one entry of the rate table per lane)
+        // (as in split_steps; the first two warps, or the only one, wait and build the rate table)
         const uint32_t svm = v.mbar + 16u + 8u * (uint32_t)par;
         if (threadIdx.x == 0) mbar_arrive_expect_tx(svm, (uint32_t)(kSvCount * sizeof(float)));
         const float *sv = v.svbuf + par * kSvCount;
@@ -952,7 +952,7 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
         bool bad = false;
         if (warp < 2) {
             bad = !mbar_wait_warp(svm, (uint32_t)(s >> 1) & 1u);
-            for (int e = (int)threadIdx.x; e < kRateTab; e += 64) build_rate_entry<float>(rtab, cc, sv, e);
+            for (int e = (int)threadIdx.x; e < kRateTab; e += min(64, v.n_ssa)) build_rate_entry<float>(rtab, cc, sv, e);
         }
         if (bar_or(2, v.n_ssa, bad)) {
             my_err |= 2;
