@@ -114,6 +114,8 @@ __device__ __forceinline__ void cluster_wait() {
 __device__ __forceinline__ void ode_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kOdeLanes) : "memory"); }
 // barrier of a CTA's SSA warps (named barrier 2, n threads: the CTA's SSA threads 0 .. n-1)
 __device__ __forceinline__ void ssa_bar(int n) { asm volatile("bar.sync 2, %0;" ::"r"(n) : "memory"); }
+// barrier of a CTA's quiet warps after a record (split_steps; named barrier 3, n threads)
+__device__ __forceinline__ void rec_bar(int n) { asm volatile("bar.sync 3, %0;" ::"r"(n) : "memory"); }
 // named barrier `id` of n threads that also returns the OR of v over them: a decision that every
 // participating thread takes the same way (a bounded wait's outcome, which is per thread)
 __device__ __forceinline__ bool bar_or(int id, int n, bool v) {
@@ -1215,7 +1217,13 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
                 bad |= !mbar_wait_warp(bars + kEvent, ph);
                 const int beg = (int)((int64_t)n_crus * warp / nq), end = (int)((int64_t)n_crus * (warp + 1) / nq);
                 record_pass<float>(a, w, cell, r_idx, beg, end, lane, tile);
-                __syncwarp();
+                // The quiet warps meet again: one that takes events in step s + 1 is not in that step's bar_or,
+                // and nothing else keeps the first writes of step s + 1 (which come after warp 0's arrival there,
+                // those of event warps by m_clear) behind its reads.  All of them are here: the record step and
+                // the split are the same for the CTA's quiet warps.  A barrier of its own, since a warp that
+                // turns quiet may be waiting in the next bar_or already; no two uses of it overlap, because a
+                // warp comes to the next one only through a bar_or that warp 0 is in.
+                rec_bar(nq * 32);
             }
         }
         send_partial<false, ODE64>(a, v, par, pslot, acc.warp_total());
