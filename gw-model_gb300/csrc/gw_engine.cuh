@@ -31,17 +31,27 @@ template <>
 struct alignas(16) Partial<true> {
     double v[4];
 };
-// FP32: each sum in two integers, hi and lo 2^-23 of a unit (FluxUnit) below it; or, with flag set, three
-// floats in the hi fields.
+// FP32: each sum in three integers, of the cell's units (SsaConsts::flux_exp) and of 2^-23 and 2^-46 of them,
+// the latter two from 0 to 2^28; or, with the last one's top bit set, an FP64 number in the first two.
+// Jtr's last two words lie apart (CtaView::part_tail), which keeps the others' stride at 32 bytes.
 template <>
 struct alignas(16) Partial<false> {
-    int jh, jl, xh, xl;
-    int th, tl, cl, flag;
+    int jh;
+    uint32_t jl, jm;
+    int cl;
+    int xh;
+    uint32_t xl, xm;
+    int th;
 };
-// The units of the FP32 sums' hi parts: powers of two, 2^21 of them bound a CRU's term (1024, 256 and
-// 16 mM/ms for JLCC, Jxfer and Jtr; the model's terms stay below 100, 100 and 1).  kMaxSumCrus terms
-// fit 32 bits.
-constexpr int kUnitJ = -11, kUnitX = -13, kUnitT = -17;
+struct alignas(8) PartialTail {
+    uint32_t tl, tm;
+};
+constexpr uint32_t kWideSum = 0x80000000u;
+// Bytes of a warp's partial.
+template <bool FP64>
+constexpr int kPartBytes = (int)sizeof(Partial<FP64>) + (FP64 ? 0 : (int)sizeof(PartialTail));
+// A term has to stay below kMaxFluxUnits units; kMaxSumCrus terms fit 32 bits.
+constexpr float kMaxFluxUnits = 524288.f;
 constexpr int kMaxSumCrus = 500;
 
 struct OdeShared {
@@ -84,13 +94,13 @@ __host__ __device__ inline SmemLayout smem_layout(int tile_cap, int max_cta_cell
     L.rtab = o;  // the CTA's subunit rate tables (FP32 SSA), one per step parity
     o += align16((size_t)2 * kRateTab * sizeof(float2));
     L.part = o;  // [parity][rank in cell][warp]: warp partials (written by the cell's CTAs)
-    o += (size_t)2 * max_cta_cell * kMaxWarps * sizeof(Partial<sizeof(R) == 8>);
+    o += (size_t)2 * max_cta_cell * kMaxWarps * kPartBytes<sizeof(R) == 8>;
     L.mbar = o;  // mbarriers: the warp partials of steps of parity 0 and 1 (leader CTA), then the
     o += 80;     // per-step SSA values of parity 0 and 1 (every CTA); FP32: the quiet warps', the event
                  // warps' and the queue's of parity 0 and 1
     L.fq = o;    // the event queue: FP64: four counters, then kEngQCap tile indices; FP32: eight counters,
-                 // then three queues of a 16-bit tile index for every CRU of the CTA
-    o += sizeof(R) == 8 ? align16((size_t)(4 + kEngQCap) * sizeof(int)) : align16(32 + (size_t)6 * tile_cap);
+                 // then two queues of a 16-bit tile index for every CRU of the CTA
+    o += sizeof(R) == 8 ? align16((size_t)(4 + kEngQCap) * sizeof(int)) : align16(32 + (size_t)4 * tile_cap);
     L.tile = o;  // TileRec<R> per CRU
     o += align16((size_t)tile_cap * sizeof(TileRec<R>));
     L.total = o;
@@ -364,13 +374,20 @@ struct OdeLane {
 // Sums {JLCC, ClCh, Jtr, Jxfer} of the n warp partials of one slot (n <= 16 CTAs x kMaxWarps), quantity
 // `warp` by ODE warp `warp`.
 constexpr int kSlotsPerLane = 16 * kMaxWarps / 32;
-// FP32: 64-bit integer sums, the lanes' through REDUX in three pieces, hence exact, and rounded once to
-// FP64; u is the exponent of their unit.
-__device__ __forceinline__ double fixed_total(long long s, int u) {
+// FP32: integer sums, the lanes' through REDUX (s in three pieces), hence exact: s units of 2^-23 of the
+// flux unit 2^u, and f < 2^23 per lane of 2^-46 of it; rounded once to FP64 (sums of 2^40 and more of the
+// former, 2^17 flux units, without the latter: 2^-40 of them).
+__device__ __forceinline__ double fixed_total(long long s, uint32_t f, int u) {
     const uint32_t lo = (uint32_t)s;
     const int h = __reduce_add_sync(0xffffffffu, (int)(s >> 32));
     const uint32_t l1 = __reduce_add_sync(0xffffffffu, lo >> 16), l0 = __reduce_add_sync(0xffffffffu, lo & 0xFFFFu);
-    s = ((long long)h << 32) + ((long long)l1 << 16) + (long long)l0;
+    f = __reduce_add_sync(0xffffffffu, f);
+    s = ((long long)h << 32) + ((long long)l1 << 16) + (long long)l0 + (long long)(f >> 23);
+    u -= 23;
+    if ((unsigned long long)(s + (1ll << 40)) < (2ull << 40)) {
+        s = s * 8388608ll + (long long)(f & 0x7FFFFFu);
+        u -= 23;
+    }
     const unsigned long long m = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
     if (m == 0ull) return 0.0;
     const uint32_t mh = (uint32_t)(m >> 32);
@@ -379,40 +396,49 @@ __device__ __forceinline__ double fixed_total(long long s, int u) {
     return __longlong_as_double((long long)(s < 0 ? d | 0x8000000000000000ull : d));
 }
 template <typename T>
-__device__ __forceinline__ void reduce_partials(const Partial<false> *slot, int n, int warp, int lane, double *out, T *X) {
-    // field of {jh, jl, xh, xl, th, tl, cl, flag}, and its unit
-    const int at = warp == 0 ? 0 : (warp == 1 ? 6 : (warp == 2 ? 4 : 2));
-    const int unit = warp == 0 ? kUnitJ : (warp == 2 ? kUnitT : kUnitX);
-    int hi[kSlotsPerLane], lo[kSlotsPerLane], flag = 0;
-#pragma unroll
-    for (int k = 0; k < kSlotsPerLane; ++k) {
-        const int i = lane + 32 * k;
-        const int *f = reinterpret_cast<const int *>(slot + (i < n ? i : 0));
-        hi[k] = i < n ? f[at] : 0;
-        lo[k] = i < n && warp != 1 ? f[at + 1] : 0;
-        flag |= i < n ? f[7] : 0;
-    }
+__device__ __forceinline__ void reduce_partials(const Partial<false> *slot, const PartialTail *tail, const int *flux_exp,
+                                                int n, int warp, int lane, double *out, T *X) {
+    // the words of {jh, jl, jm, cl, xh, xl, xm, th} and {tl, tm} that are this warp's sum
+    const int *const first = reinterpret_cast<const int *>(slot) + (warp == 0 ? 0 : (warp == 1 ? 3 : (warp == 2 ? 7 : 4)));
+    const uint32_t *const next = reinterpret_cast<const uint32_t *>(warp == 2 ? reinterpret_cast<const int *>(tail) : first + 1);
+    const int step = warp == 2 ? 2 : 8;
     double r;
-    if (!__any_sync(0xffffffffu, flag)) {
-        long long s = 0;
-        const int up = warp == 1 ? 0 : 23;
+    if (warp == 1) {
+        int c = 0;
 #pragma unroll
-        for (int k = 0; k < kSlotsPerLane; ++k) s += ((long long)hi[k] << up) + lo[k];
-        r = fixed_total(s, warp == 1 ? 0 : unit - 23);
-    } else {
-        // some warp had a term beyond the fixed-point range (or a NaN): its sums are floats
-        r = 0.0;
         for (int k = 0; k < kSlotsPerLane; ++k) {
             const int i = lane + 32 * k;
-            if (i >= n) continue;
-            if (warp == 1)
-                r += (double)hi[k];
-            else
-                r += slot[i].flag ? (double)__int_as_float(hi[k])
-                                  : (double)(((long long)hi[k] << 23) + lo[k]) * ldexp(1.0, unit - 23);
+            c += i < n ? first[8 * i] : 0;
         }
+        r = (double)__reduce_add_sync(0xffffffffu, c);
+    } else {
+        const int unit = flux_exp[warp == 0 ? 0 : (warp == 2 ? 2 : 1)];
+        long long s = 0;
+        uint32_t l = 0, m = 0, any = 0;  // (the sums of eight slots fit)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        for (int k = 0; k < kSlotsPerLane; ++k) {
+            const int i = lane + 32 * k;
+            const uint32_t mi = i < n ? next[step * i + 1] : 0u;
+            s += i < n ? first[8 * i] : 0;
+            l += i < n ? next[step * i] : 0u;
+            m += mi;
+            any |= mi;
+        }
+        if (!__any_sync(0xffffffffu, any & kWideSum)) {
+            r = fixed_total(s * 8388608ll + (long long)(l + (m >> 23)), m & 0x7FFFFFu, unit);
+        } else {
+            // some warp had a term beyond the integers' range (or a NaN): FP64 sums
+            r = 0.0;
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32) {
+                const int h = first[8 * i];
+                const uint32_t l = next[step * i], m = next[step * i + 1];
+                r += m & kWideSum ? __hiloint2double(h, (int)l)
+                                  : ldexp((double)h + (double)l * 0x1p-23 + (double)m * 0x1p-46, unit);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        }
     }
     if (lane == 0) {
         out[warp] = r;
@@ -420,7 +446,8 @@ __device__ __forceinline__ void reduce_partials(const Partial<false> *slot, int 
     }
 }
 template <typename T>
-__device__ __forceinline__ void reduce_partials(const Partial<true> *slot, int n, int warp, int lane, double *out, T *X) {
+__device__ __forceinline__ void reduce_partials(const Partial<true> *slot, const PartialTail *, const int *, int n, int warp,
+                                                int lane, double *out, T *X) {
     const int src = warp == 0 ? 0 : (warp == 1 ? 3 : (warp == 2 ? 2 : 1));  // of {JLCC, Jxfer, Jtr, ClCh}
     const int nk = (n + 31) >> 5;
     double a = 0.0;
@@ -571,7 +598,7 @@ struct FluxAcc<true> {
         dtr += t;
         acl += cl;
     }
-    __device__ __forceinline__ Partial<true> warp_total() {
+    __device__ __forceinline__ Partial<true> warp_total(PartialTail &) {
         Partial<true> pv;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -588,59 +615,76 @@ struct FluxAcc<true> {
     }
 };
 // FP32: fixed-point sums, so that they do not depend on which lane of which warp took a CRU, or when (the
-// split between quiet and event warps depends on the launch's start).  A term v is rounded to a multiple
-// of its unit by adding 1.5 * 2^23 units, whose float's low bits are then the multiple (less the
-// constant's); what is left goes the same way to a unit 2^-23 of that.  Two exact subtractions and
-// integer adds; a term's rounding error is at most half the lower unit (2.9e-11, 7.3e-12 and 4.5e-13
-// mM/ms).  Terms out of range, or too many of them, set `big`, and the warp sends plain float sums.
+// split between quiet and event warps depends on the launch's start).  A term v is scaled to the cell's
+// units (SsaConsts::flux_scale, from its JLCC_const, rxfer and rtr) and rounded to a multiple of them by
+// adding 1.5 * 2^23, whose float's low bits are then the multiple (less the constant's); what is left goes
+// the same way to multiples of 2^-23 and 2^-46 of a unit.  All differences are exact.  So a term of 2^-23 units or
+// more is summed whole (at the model's parameters down to 2.3e-10, 3.7e-9 and 7.3e-12 mM/ms of JLCC, Jxfer and
+// Jtr, and in proportion to those three), a smaller one rounded to 2^-46 units.
+// (Two words, the last at 2^-34 to 2^-40 mM/ms whatever the parameters, took 15 fewer of ~710 instructions per
+// pass, but a warp's Jxfer sum at rest was off by up to 9.4e-8 of itself at rxfer = 200 and 3.5e-5 at 0.2, an FP32
+// tree's by 5.9e-8 and 1.2e-7; these by nothing.  1,024 cells 20.0 -> 20.8 ms per 50 steps, 256 amid the release
+// 11.4 -> 11.8 per 100, one 12,500-CRU cell 10.6 -> 10.8 per 1,000.  Not taken: the terms converted to 64-bit
+// integers, 21.8 ms; a branch on the range instead of the maximum and the float sums, 21.2.)
+// Terms out of range, or too many of them: the warp sends its plain float sums.
 template <>
 struct FluxAcc<false> {
-    int jh = 0, jl = 0, xh = 0, xl = 0, th = 0, tl = 0, acl = 0;
-    float jf = 0, xf = 0, tf = 0;
-    bool big = false;
-    __device__ __forceinline__ static constexpr float pow2(int e) { return e < 0 ? 1.f / (float)(1ull << -e) : (float)(1ull << e); }
-    template <int UNIT>
-    __device__ __forceinline__ void split(float v, int &hi, int &lo) {
-        constexpr float H = 12582912.f * pow2(UNIT), L = H * pow2(-23);
-        const float t = __fadd_rn(v, H);
-        const float u = __fadd_rn(__fsub_rn(v, __fsub_rn(t, H)), L);
-        hi += __float_as_int(t) - (0x4B400000 + UNIT * (1 << 23));
-        lo += __float_as_int(u) - (0x4B400000 + ((UNIT - 23) * (1 << 23)));
-        big |= !(fabsf(v) < 2097152.f * pow2(UNIT));
+    int jh = 0, jl = 0, jm = 0, xh = 0, xl = 0, xm = 0, th = 0, tl = 0, tm = 0, acl = 0;
+    float jf = 0.f, xf = 0.f, tf = 0.f;
+    float largest = 0.f;  // term, in its units
+    bool wide = false;    // too many terms
+    const SsaConsts<float> &c;
+    __device__ __forceinline__ explicit FluxAcc(const SsaConsts<float> &cc) : c(cc) {}
+    __device__ __forceinline__ static void split(float a, int &h, int &l, int &m) {
+        constexpr uint32_t Mb = 0x4B400000u;
+        constexpr float M = 12582912.f, S = 8388608.f;
+        const float t = __fadd_rn(a, M), r = __fsub_rn(a, __fsub_rn(t, M));
+        const float u = __fmaf_rn(r, S, M), w = __fmaf_rn(__fmaf_rn(r, S, __fsub_rn(M, u)), S, M);
+        h += (int)(__float_as_uint(t) - Mb);
+        l += (int)(__float_as_uint(u) - Mb);
+        m += (int)(__float_as_uint(w) - Mb);
+    }
+    // the largest of |a|, |b| and |c|, or NaN
+    __device__ __forceinline__ static float max3(float a, float b, float c) {
+        float r;
+        asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+        return r;
     }
     __device__ __forceinline__ void add(float j, float x, float t, int cl) {
-        split<kUnitJ>(j, jh, jl);
-        split<kUnitX>(x, xh, xl);
-        split<kUnitT>(t, th, tl);
+        const float aj = __fmul_rn(j, c.flux_scale[0]), ax = __fmul_rn(x, c.flux_scale[1]), at = __fmul_rn(t, c.flux_scale[2]);
+        largest = max3(max3(largest, aj, ax), at, at);
+        split(aj, jh, jl, jm);
+        split(ax, xh, xl, xm);
+        split(at, th, tl, tm);
         jf += j;
         xf += x;
         tf += t;
         acl += cl;
     }
-    __device__ __forceinline__ Partial<false> warp_total() {
-        Partial<false> pv;
-        pv.cl = __reduce_add_sync(0xffffffffu, acl);
-        pv.flag = __any_sync(0xffffffffu, big) ? 1 : 0;
-        if (pv.flag) {
+    // The warp's sum: the lower words' carries go up in every lane, which leaves them from 0 to 2^23.
+    __device__ __forceinline__ static void total(bool floats, float f, int &h, int &l, int &m) {
+        if (floats) {
+            double v = (double)f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                jf += __shfl_xor_sync(0xffffffffu, jf, o);
-                xf += __shfl_xor_sync(0xffffffffu, xf, o);
-                tf += __shfl_xor_sync(0xffffffffu, tf, o);
-            }
-            pv.jh = __float_as_int(jf);
-            pv.xh = __float_as_int(xf);
-            pv.th = __float_as_int(tf);
-            pv.jl = pv.xl = pv.tl = 0;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            h = __double2hiint(v);
+            l = __double2loint(v);
+            m = (int)kWideSum;
         } else {
-            pv.jh = __reduce_add_sync(0xffffffffu, jh);
-            pv.jl = __reduce_add_sync(0xffffffffu, jl);
-            pv.xh = __reduce_add_sync(0xffffffffu, xh);
-            pv.xl = __reduce_add_sync(0xffffffffu, xl);
-            pv.th = __reduce_add_sync(0xffffffffu, th);
-            pv.tl = __reduce_add_sync(0xffffffffu, tl);
+            l += m >> 23;
+            h = __reduce_add_sync(0xffffffffu, h + (l >> 23));
+            l = (int)__reduce_add_sync(0xffffffffu, (uint32_t)l & 0x7FFFFFu);
+            m = (int)__reduce_add_sync(0xffffffffu, (uint32_t)m & 0x7FFFFFu);
         }
-        return pv;
+    }
+    __device__ __forceinline__ Partial<false> warp_total(PartialTail &tail) {
+        const bool floats = __any_sync(0xffffffffu, wide || !(largest < kMaxFluxUnits));
+        total(floats, jf, jh, jl, jm);
+        total(floats, xf, xh, xl, xm);
+        total(floats, tf, th, tl, tm);
+        tail = PartialTail{(uint32_t)tl, (uint32_t)tm};
+        return Partial<false>{jh, (uint32_t)jl, (uint32_t)jm, (int)__reduce_add_sync(0xffffffffu, acl),
+                              xh, (uint32_t)xl, (uint32_t)xm, th};
     }
 };
 
@@ -660,9 +704,10 @@ struct CtaView {
     math64::Tables *M;
     void *svstage;
     Partial<FP64> *part;
+    PartialTail *part_tail;  // FP32
     float2 *rtab;
     int *fq;        // FP64: by parity, entries queued; FP32: by step mod 3, entries reserved << 16 | written, and
-                    // claimed, then the split by parity; then the queues
+                    // claimed, then the split by parity; then the queues, by parity
     uint32_t mbar;  // shared address of the partials' mbarrier of parity 0 (parity 1 at +8); the
                     // SSA values' mbarriers of parity 0 and 1 at +16 and +24; FP32: the quiet warps'
                     // at +32 and +40, the event warps' at +48 and +56, the queue's (cleared for the
@@ -690,6 +735,7 @@ struct CtaView {
         M = reinterpret_cast<math64::Tables *>(smem + L.math);
         svstage = smem + L.svs;
         part = reinterpret_cast<Partial<FP64> *>(smem + L.part);
+        part_tail = reinterpret_cast<PartialTail *>(part + 2 * a.max_cta_cell * kMaxWarps);
         rtab = reinterpret_cast<float2 *>(smem + L.rtab);
         fq = reinterpret_cast<int *>(smem + L.fq);
         mbar = smem_addr(smem + L.mbar);
@@ -780,7 +826,7 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
     push(0);
     // bytes of the cell's warp partials per step
     const uint32_t part_bytes =
-        (uint32_t)sizeof(Partial<FP64>) * (uint32_t)(v.nw + (v.w.n_cta_cell - 1) * (v.nw + kOdeWarps));
+        (uint32_t)kPartBytes<FP64> * (uint32_t)(v.nw + (v.w.n_cta_cell - 1) * (v.nw + kOdeWarps));
     bool stopped = false;  // a wait ran out (the same on every ODE thread)
     int s_stop = -1;       // the step whose wait (for the partials of step s_stop - 1) ran out
     for (int s = 0; s < a.n_steps; ++s) {
@@ -814,7 +860,8 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
             __syncwarp();
             // (a warp's lanes may find different outcomes; whatever is summed after a wait that ran out
             // is not used)
-            reduce_partials(v.part + (par ^ 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp, lane, os.sums, X);
+            reduce_partials(v.part + (par ^ 1) * pslot, v.part_tail + (par ^ 1) * pslot, v.cc->flux_exp,
+                            v.w.n_cta_cell * kMaxWarps, warp, lane, os.sums, X);
         }
         if (bar_or(1, kOdeLanes, !ok)) {  // the same decision on all ODE threads
             if (ot == 0) atomicCAS(&os.status, 0, (int)GW_ERR_SYNC_TIMEOUT);
@@ -856,7 +903,8 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         mbar_wait(v.mbar + 8u * (uint32_t)(s_stop & 1), (uint32_t)(s_stop >> 1) & 1u);
     }
     if (a.n_steps > 0)
-        reduce_partials(v.part + ((a.n_steps - 1) & 1) * pslot, v.w.n_cta_cell * kMaxWarps, warp, lane, os.sums, X);
+        reduce_partials(v.part + ((a.n_steps - 1) & 1) * pslot, v.part_tail + ((a.n_steps - 1) & 1) * pslot, v.cc->flux_exp,
+                        v.w.n_cta_cell * kMaxWarps, warp, lane, os.sums, X);
     ode_bar();
     CellDyn &d = a.dyn[cell];
     for (int i = ot; i < kNumGlobals; i += kOdeLanes) d.g[i] = os.g[i];
@@ -875,21 +923,24 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
 }
 
 // A warp's flux partial of a step of parity par, pushed by lane 0 straight into the leader's slot (rank,
-// warp) by 16-byte asynchronous stores that count themselves off the leader's mbarrier of this parity
+// warp) by asynchronous stores that count themselves off the leader's mbarrier of this parity
 // (the warp goes on without waiting for them to land); the leader sums the cell's warp partials.
 template <bool FP64, bool ODE64>
 __device__ __forceinline__ void send_partial(const KernelArgs &a, const CtaView<FP64, ODE64> &v, int par, int pslot,
-                                             const Partial<FP64> &pv) {
+                                             FluxAcc<FP64> &acc) {
+    PartialTail tail;
+    const Partial<FP64> pv = acc.warp_total(tail);
     if (v.lane != 0) return;
-    Partial<FP64> *dst = v.part + par * pslot + v.w.rank_in_cell * kMaxWarps + v.warp;
-    const uint32_t rd = map_rank(dst, (uint32_t)v.w.first);
+    const int slot = par * pslot + v.w.rank_in_cell * kMaxWarps + v.warp;
+    const uint32_t rd = map_rank(v.part + slot, (uint32_t)v.w.first);
     const uint32_t rm = map_rank_addr(v.mbar + 8u * (uint32_t)par, (uint32_t)v.w.first);
     if constexpr (FP64) {
         st_async(rd, make_uint4(lo_of(pv.v[0]), hi_of(pv.v[0]), lo_of(pv.v[1]), hi_of(pv.v[1])), rm);
         st_async(rd + 16u, make_uint4(lo_of(pv.v[2]), hi_of(pv.v[2]), lo_of(pv.v[3]), hi_of(pv.v[3])), rm);
     } else {
-        st_async(rd, make_uint4((uint32_t)pv.jh, (uint32_t)pv.jl, (uint32_t)pv.xh, (uint32_t)pv.xl), rm);
-        st_async(rd + 16u, make_uint4((uint32_t)pv.th, (uint32_t)pv.tl, (uint32_t)pv.cl, (uint32_t)pv.flag), rm);
+        st_async(rd, make_uint4((uint32_t)pv.jh, pv.jl, pv.jm, (uint32_t)pv.cl), rm);
+        st_async(rd + 16u, make_uint4((uint32_t)pv.xh, pv.xl, pv.xm, (uint32_t)pv.th), rm);
+        st_async8(map_rank(v.part_tail + slot, (uint32_t)v.w.first), make_uint2(tail.tl, tail.tm), rm);
     }
 }
 
@@ -961,8 +1012,8 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
             s_stop = s;
             continue;
         }
-        FluxAcc<false> acc;
-        acc.big = end - beg > kMaxSumCrus;
+        FluxAcc<false> acc(cc);
+        acc.wide = end - beg > kMaxSumCrus;
         int n = end - beg;
         if (!direct) {
             StepDraw draw;
@@ -1003,7 +1054,7 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
         __syncwarp();  // (the CRUs of this step are stored)
         if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr))
             record_pass<float>(a, w, cell, r_idx, beg, end, lane, tile);
-        send_partial<false, ODE64>(a, v, par, pslot, acc.warp_total());
+        send_partial<false, ODE64>(a, v, par, pslot, acc);
     }
 }
 
@@ -1027,8 +1078,9 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
 // by their tag at step s + 1 and taken last, in the queue's order, once the events of step s are through.
 // Buffers: the SSA values, the rate table and the split of step s are used until the warps send their
 // partials of step s, and rewritten for step s + 2, whose SSA values the leader sends only after those
-// partials.  The queue of step s, one of three, is used until the quiet passes of step s + 1 are through
-// (m_quiet), and cleared for step s + 3 after that.
+// partials.  The queue of step s is used by its events, and until the quiet passes of step s + 1 are through;
+// m_quiet of step s + 1 takes every warp's arrival from after both, so warp 0 has its counters, one of three
+// sets, cleared in step s + 2 (for step s + 3), and its entries, one of two arrays, rewritten from then on.
 // m_quiet(s): every warp arrives when its quiet passes of step s are through, its queue entries written;
 // m_event(s): when it finds no more events of step s.  Two of each, by parity: the phase of step s + 2
 // takes every warp's arrival in step s + 2, so a waiter is at most one phase behind and the parity tells
@@ -1071,10 +1123,10 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
         float2 *rtab = v.rtab + par * kRateTab;
         const uint32_t tag = (uint32_t)s + 2u;
         const int slot_prev = slot == 0 ? 2 : slot - 1, slot_next = slot == 2 ? 0 : slot + 1;
-        uint16_t *q = queues + slot * a.tile_cap;
+        uint16_t *q = queues + par * a.tile_cap;
         int *const q_put = v.fq + 2 * slot, *const q_got = q_put + 1;
         const bool quiet_warp = warp < nq;
-        FluxAcc<false> acc;
+        FluxAcc<false> acc(cc);
         int taken = 0;
         int nq_next;
         if (!quiet_warp) {
@@ -1122,7 +1174,7 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
             // The CTA's groups of 32, without the CRUs of step s-1's queue, then the groups of those, in turn
             // to the quiet warps.
             const int n_own = (n_crus + 31) >> 5, n_late = s > 0 ? v.fq[2 * slot_prev] & 0xFFFF : 0;
-            const uint16_t *q_prev = queues + slot_prev * a.tile_cap;
+            const uint16_t *q_prev = queues + (par ^ 1) * a.tile_cap;
             bool waited = false;
             for (int g = warp; g < n_own + ((n_late + 31) >> 5); g += nq) {
                 const bool late = g >= n_own;
@@ -1208,7 +1260,7 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bars + kEvent);
-        acc.big |= taken > kMaxSumCrus;
+        acc.wide = taken > kMaxSumCrus;
         const int64_t ri = a.run_step0 + s;
         if (quiet_warp && a.record_every > 0 && (ri % a.record_every) == 0 && (cell == a.tr_cell || a.tr_sums != nullptr)) {
             // records of this step, from the warp's part of the tile at the end of the step
@@ -1226,7 +1278,7 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
                 rec_bar(nq * 32);
             }
         }
-        send_partial<false, ODE64>(a, v, par, pslot, acc.warp_total());
+        send_partial<false, ODE64>(a, v, par, pslot, acc);
         nq = nq_next;
         slot = slot_next;
     }
@@ -1434,7 +1486,7 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                 // Records of this step, from the warp's part of the tile (now at the end of the step)
                 if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr))
                     record_pass<R>(a, w, cell, r_idx, beg, end, lane, tile);
-                send_partial<FP64, ODE64>(a, v, par, pslot, acc.warp_total());
+                send_partial<FP64, ODE64>(a, v, par, pslot, acc);
             }
         }
     } else if (v.active) {
@@ -1537,7 +1589,7 @@ __global__ void __launch_bounds__(FP64 ? kMaxThreadsFp64 : kMaxThreads, 1) engin
         // so); the cell's CTAs write them only after the first cluster barrier of the steps.
         if (v.leader) {
             uint4 *pz = reinterpret_cast<uint4 *>(v.part);
-            const int nz = 2 * a.max_cta_cell * kMaxWarps * (int)(sizeof(Partial<FP64>) / 16);
+            const int nz = 2 * a.max_cta_cell * kMaxWarps * kPartBytes<FP64> / 16;
             for (int i = (int)threadIdx.x; i < nz; i += (int)blockDim.x) pz[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         step0 = a.dyn[cell].step;

@@ -220,6 +220,12 @@ __device__ __forceinline__ void st_async(uint32_t addr, uint4 v, uint32_t mbar) 
                  "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mbar)
                  : "memory");
 }
+// The same for 8 bytes (addr 8-byte aligned).
+__device__ __forceinline__ void st_async8(uint32_t addr, uint2 v, uint32_t mbar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(v.x),
+                 "r"(v.y), "r"(mbar)
+                 : "memory");
+}
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
@@ -325,7 +331,19 @@ struct SsaConsts {
     uint32_t lcct[16];  // LCC rate table by state (lcc_word), in shared memory: no divergent branch
     uint32_t lccn[16];  // next LCC state by state: transition t in bits 4t..4t+3
     float2 pk[PK_COUNT];  // FP32 lane: constants duplicated into (value, value) pairs
+    // FP32 engine: units of the flux sums of JLCC, Jxfer and Jtr, as their exponents and as what a term is
+    // multiplied with (flux_exp_of)
+    int flux_exp[3];
+    float flux_scale[3];
 };
+
+// Exponent e of a flux sum's unit: 2^19 units are the power of two above |bound| (at most twice that), so
+// that a term up to the bound fits.  The bounds below stand for differences of concentrations of 16 mM in
+// each subunit (Jxfer) and 64 mM (Jtr), and for four open LCCs at -600 mV (JLCC).
+__device__ __forceinline__ int flux_exp_of(double bound) {
+    const int e = ((__double2hiint(bound) >> 20) & 0x7FF) - 1022;
+    return max(-60, min(60, e)) - 19;
+}
 
 template <typename R>
 __device__ void load_ssa_consts(SsaConsts<R> &c, const CellStatic &s) {
@@ -351,6 +369,11 @@ __device__ void load_ssa_consts(SsaConsts<R> &c, const CellStatic &s) {
                                 (float)(p.k56 + p.k54), (float)p.k52, (float)p.k65, (float)p.k54, (float)p.k56,
                                 (float)p.KBSR, (float)p.KBSL, (float)s.BSR_const, (float)s.BSL_const};
     for (int i = 0; i < PK_COUNT; ++i) c.pk[i] = make_float2(pv[i], pv[i]);
+    const double bound[3] = {64.0 * s.JLCC_const * (1.0 + s.Cao_scaled), 64.0 * p.rxfer, 64.0 * p.rtr};
+    for (int i = 0; i < 3; ++i) {
+        c.flux_exp[i] = flux_exp_of(bound[i]);
+        c.flux_scale[i] = __int_as_float((127 - c.flux_exp[i]) << 23);
+    }
     for (int st = 0; st < 16; ++st) {
         c.lcct[st] = lcc_table(st);
         c.lccn[st] = (uint32_t)lcc_next(st, 0) | ((uint32_t)lcc_next(st, 1) << 4) | ((uint32_t)lcc_next(st, 2) << 8);
