@@ -50,9 +50,13 @@ constexpr uint32_t kWideSum = 0x80000000u;
 // Bytes of a warp's partial.
 template <bool FP64>
 constexpr int kPartBytes = (int)sizeof(Partial<FP64>) + (FP64 ? 0 : (int)sizeof(PartialTail));
-// A term has to stay below kMaxFluxUnits units; kMaxSumCrus terms fit 32 bits.
-constexpr float kMaxFluxUnits = 524288.f;
-constexpr int kMaxSumCrus = 500;
+// A term has to stay below kMaxFluxUnits units.  Then 32 bits hold a warp's first words (2^19 a term, and
+// whatever warp takes how many, the CTA's CRUs once each) and a lane's other words (2^22 a term: at most two
+// quiet passes over all CRUs of the CTA, or one event in each batch of eight).
+constexpr int kMaxFluxUnits = 1 << 19;
+constexpr int kMostCtaCrus = 232448 / (int)(sizeof(TileRec<float>) + 4);  // in 227 KB of shared memory
+static_assert((int64_t)kMostCtaCrus * (kMaxFluxUnits + 1) < (1ll << 31) && (int64_t)(kMostCtaCrus / 8 + 1) * (1 << 22) < (1ll << 31) &&
+              2 * (kMostCtaCrus / 32 + 1) <= kMostCtaCrus / 8, "FP32 flux sums in 32 bits");
 
 struct OdeShared {
     double g[kNumGlobals];  // the cell's globals (FP64 state)
@@ -626,13 +630,12 @@ struct FluxAcc<true> {
 // tree's by 5.9e-8 and 1.2e-7; these by nothing.  1,024 cells 20.0 -> 20.8 ms per 50 steps, 256 amid the release
 // 11.4 -> 11.8 per 100, one 12,500-CRU cell 10.6 -> 10.8 per 1,000.  Not taken: the terms converted to 64-bit
 // integers, 21.8 ms; a branch on the range instead of the maximum and the float sums, 21.2.)
-// Terms out of range, or too many of them: the warp sends its plain float sums.
+// With a term out of range the warp sends its plain float sums.
 template <>
 struct FluxAcc<false> {
     int jh = 0, jl = 0, jm = 0, xh = 0, xl = 0, xm = 0, th = 0, tl = 0, tm = 0, acl = 0;
     float jf = 0.f, xf = 0.f, tf = 0.f;
     float largest = 0.f;  // term, in its units
-    bool wide = false;    // too many terms
     const SsaConsts<float> &c;
     __device__ __forceinline__ explicit FluxAcc(const SsaConsts<float> &cc) : c(cc) {}
     __device__ __forceinline__ static void split(float a, int &h, int &l, int &m) {
@@ -678,7 +681,7 @@ struct FluxAcc<false> {
         }
     }
     __device__ __forceinline__ Partial<false> warp_total(PartialTail &tail) {
-        const bool floats = __any_sync(0xffffffffu, wide || !(largest < kMaxFluxUnits));
+        const bool floats = __any_sync(0xffffffffu, !(largest < (float)kMaxFluxUnits));
         total(floats, jf, jh, jl, jm);
         total(floats, xf, xh, xl, xm);
         total(floats, tf, th, tl, tm);
@@ -1013,7 +1016,6 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
             continue;
         }
         FluxAcc<false> acc(cc);
-        acc.wide = end - beg > kMaxSumCrus;
         int n = end - beg;
         if (!direct) {
             StepDraw draw;
@@ -1127,7 +1129,6 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
         int *const q_put = v.fq + 2 * slot, *const q_got = q_put + 1;
         const bool quiet_warp = warp < nq;
         FluxAcc<false> acc(cc);
-        int taken = 0;
         int nq_next;
         if (!quiet_warp) {
             // (each of these waits for itself: they may be in different steps, the set changing with nq)
@@ -1198,7 +1199,6 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
                 const bool quiet = sl.quiet(c, cc, sv, rtab, draw.word((uint32_t)(w.cru_begin + m)), dt);
                 const bool done = valid && quiet, jumps = valid && !quiet;
                 if (done) tile_put_quiet(rec_m, c, late ? tag - 1u : 0u);
-                taken += 32;
                 acc.add(done ? c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3] : 0.f, done ? sl.jxfer_sum : 0.f,
                         done ? sl.jtr : 0.f, done ? __popc((c.flags >> 4) & 0xFu) : 0);
                 const unsigned em = __ballot_sync(0xffffffffu, jumps);
@@ -1245,7 +1245,6 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
             }
             if (h < 0) break;
             __threadfence_block();
-            taken += n;
             // (a group without a CRU holds, and computes along on, the batch's last)
             const int i = lane >> 2;
             int m = q[h + min(i, n - 1)];
@@ -1260,7 +1259,6 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bars + kEvent);
-        acc.wide = taken > kMaxSumCrus;
         const int64_t ri = a.run_step0 + s;
         if (quiet_warp && a.record_every > 0 && (ri % a.record_every) == 0 && (cell == a.tr_cell || a.tr_sums != nullptr)) {
             // records of this step, from the warp's part of the tile at the end of the step

@@ -83,3 +83,29 @@ def test_every_shape_gives_the_same_crus_fp64(n, shapes, busy):
         got = simulate(n, busy, precision="fp64", steps=1, cluster_ctas=cl, cta_crus=tile)
         for k in ("CaSS", "CaJSR", "LCC", "LCC_inactivation", "RyR", "ClCh", "events"):
             assert np.array_equal(want[k], got[k]), (k, cl, tile)
+
+
+def test_many_events_in_one_warp():
+    """A step in which an event warp takes more than 500 CRUs of a CTA (large steps, and more than a third of the
+    CRUs with a jump when the split still expects one in 32): the same bits in every shape, and again."""
+    from gwgb300 import engine
+
+    n, dt = 2080, 1.5e-2
+
+    def run(steps, **shape):
+        with engine.Ensemble([n], precision="fp32", seed=6, **shape) as e:
+            g = e.get_globals(0)
+            g[0], g[3], g[4] = 20.0, 4.0e-4, 0.88
+            e.set_globals(0, g)
+            e.set_crus(0, states(n, True))
+            e.run(dt, steps)
+            s = e.get_crus(0)
+            return ([np.array(getattr(s, k)) for k in ("CaSS", "CaJSR", "LCC", "RyR", "ClCh")] +
+                    [e.get_globals(0), np.array(e.get_flux_carry(0))]), e.stats()["events"]
+
+    assert run(1)[1] > 1200
+    want, _ = run(12)
+    for shape in (dict(cluster_ctas=1, cta_crus=2080), dict(cluster_ctas=1, cta_crus=2080), dict(cluster_ctas=2), dict(cluster_ctas=3)):
+        got, _ = run(12, **shape)
+        for a, b in zip(want, got):
+            assert np.array_equal(a, b), shape
