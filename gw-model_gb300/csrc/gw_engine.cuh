@@ -971,12 +971,19 @@ __device__ __forceinline__ void group_run(const KernelArgs &a, const SsaConsts<f
 // The FP32 SSA of a CTA with few CRUs (v.grouped), each warp with a contiguous range of them and nothing shared
 // between the warps.  With up to eight to a warp every CRU goes on four lanes at once: one pass, 2.0 k cycles
 // without an event and 5.3 k with one, and the global step beside it sets the time (3.2 us per step at rest
-// for a cell of 777 CRUs over 9 to 16 CTAs; 4.4 with one CRU per lane).  With more, a quiet pass of one CRU
-// per lane (SsaLane::quiet) comes first and those with a possible jump follow, eight at a time.
-// split_steps shares these between warps, which pays from 16 CRUs per warp on in a CTA of 16 warps (us per
-// step of 30 cells of 300 to 1,000 CRUs amid the release, line at 16 and 32: 6.5 and 7.1; at rest 4.6 and
-// 4.4), and not in smaller CTAs, where few warps are left for either part (100 cells of 50 to 200, 12 SSA
-// warps, line at 16 and 32 amid the release: 9.0 and 6.8; 256 of 100, 4 SSA warps: 13.0 and 9.9).
+// for a cell of 777 CRUs over 9 to 16 CTAs).  With more, up to 32, one CRU goes on each lane through all its
+// iterations (SsaLane::iterate): the warp runs as many as its CRU with the most jumps, the first one together
+// with the quiet CRUs' only one.  It is bound by latency: 2.7 k cycles an iteration, 5.5 k with an event in it,
+// most of it instruction fetch.  (A quiet pass first and then the CRUs with a jump eight at a time on four lanes did the
+// first iteration twice and kept more code in flight.  us per step at rest and amid the release, this and that,
+// and last a lane that takes the warp's next CRU, beside the global step of that time:
+// 300 cells of 20 to 60 CRUs, two SSA warps: 4.4 and 8.4; 7.0 and 10.1; 7.0 and 7.3 (a whole beat of 400 ms: this
+// 5.7, the last 7.0).
+// 256 cells of 100, four warps: 5.4 and 8.6; 7.1 and 10.0; 7.1 and 9.2.
+// 100 cells of 50 to 200, twelve warps: 4.2 and 6.6; 4.6 and 6.9; 6.2 and 6.6.)
+// split_steps shares quiet passes and events between warps, which pays from 16 CRUs per warp on in a CTA of 16
+// warps (30 cells of 300 to 1,000 CRUs amid the release, line at 16 and 32: 6.7 and 7.1; at rest 4.7 and 4.1),
+// and not in smaller CTAs, where few warps are left for either part.
 template <bool ODE64>
 __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<false, ODE64> &v, uint64_t step0,
                                             unsigned long long &my_events, int &my_err, int &s_stop) {
@@ -992,7 +999,6 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
     const int nse = direct ? max(1, (w.cru_count + 7) >> 3) : nwu;
     const int beg = warp < nse ? (int)((int64_t)w.cru_count * warp / nse) : w.cru_count;
     const int end = warp < nse ? (int)((int64_t)w.cru_count * (warp + 1) / nse) : w.cru_count;
-    uint16_t *const q = reinterpret_cast<uint16_t *>(v.fq + 8) + beg;
     for (int s = 0; s < a.n_steps; ++s) {
         const int par = s & 1;
         const int64_t ri = a.run_step0 + s;
@@ -1016,42 +1022,33 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
             continue;
         }
         FluxAcc<false> acc(cc);
-        int n = end - beg;
-        if (!direct) {
-            StepDraw draw;
-            draw.open(a.seed, rcell, step0 + s, 0);
-            n = 0;
-            for (int b = beg; b < end; b += 32) {
-                const int m = b + lane;
-                // (a lane without a CRU computes along on the range's last: no branch in the pass)
-                Cru<float> c;
-                SsaLane<float, false> sl;
-                TileRec<float> &rec_m = tile[min(m, end - 1)];
-                tile_get(c, rec_m);
-                sl.begin(c, cc);
-                const bool quiet = sl.quiet(c, cc, sv, rtab, draw.word((uint32_t)(w.cru_begin + m)), (float)a.dt);
-                const bool done = m < end && quiet, jumps = m < end && !quiet;
-                if (done) tile_put_quiet(rec_m, c, 0u);
-                acc.add(done ? c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3] : 0.f, done ? sl.jxfer_sum : 0.f,
-                        done ? sl.jtr : 0.f, done ? __popc((c.flags >> 4) & 0xFu) : 0);
-                const unsigned em = __ballot_sync(0xffffffffu, jumps);
-                if (jumps) q[n + __popc(em & ((1u << lane) - 1u))] = (uint16_t)m;
-                n += __popc(em);
-            }
-            __syncwarp();
-        }
-        for (int h = 0; h < n; h += 8) {
-            // (a group without a CRU holds, and computes along on, the batch's last)
-            const int i = h + (lane >> 2), k = min(i, n - 1);
-            int m = direct ? beg + k : (int)q[k];
+        if (beg < end) {
+            // (a group or lane without a CRU computes along on the range's last)
+            const int i = beg + (direct ? lane >> 2 : lane), m = min(i, end - 1);
             Cru<float> c;
             SsaLane<float, false> sl;
             Stream rng;
             tile_get(c, tile[m]);
             rng.open(a.seed, rcell, (uint32_t)(w.cru_begin + m), step0 + s, 0);
             sl.begin(c, cc);
-            if (i >= n) m = -1;
-            group_run(a, cc, tile, m, c, sl, rng, sv, rtab, 0u, acc, my_events, my_err);
+            if (direct) {
+                group_run(a, cc, tile, i < end ? m : -1, c, sl, rng, sv, rtab, 0u, acc, my_events, my_err);
+            } else {
+                StepDraw draw;
+                draw.open(a.seed, rcell, step0 + s, 0);
+                float u0 = Stream::u24_of(draw.word((uint32_t)(w.cru_begin + m)));
+                bool live = i < end;
+                int err = 0;
+                while (__any_sync(0xffffffffu, live))
+                    if (sl.iterate(live, c, cc, sv, rtab, rng, u0, (float)a.dt, a.event_cap, err)) live = false;
+                if (i < end) {
+                    tile_put(tile[m], c);
+                    my_events += (unsigned long long)sl.ev;
+                    my_err |= err;
+                    acc.add(c.jlcc[0] + c.jlcc[1] + c.jlcc[2] + c.jlcc[3], sl.jxfer_sum, sl.jtr,
+                            __popc((c.flags >> 4) & 0xFu));
+                }
+            }
         }
         __syncwarp();  // (the CRUs of this step are stored)
         if (rec_ok && (cell == a.tr_cell || a.tr_sums != nullptr))

@@ -1628,6 +1628,53 @@ struct SsaLane<float, false> {
         return last && !crossed;
     }
 
+    // The generic lane's iteration (same draws, same decisions) with one CRU per lane, the same results as
+    // iterate_group().  u0: the iteration's first draw; on return, after an event, the next one's.  All lanes of the
+    // warp call it together; one that is not live computes along and leaves its CRU as it is.
+    __device__ __forceinline__ bool iterate(bool live, Cru<float> &s, const SsaConsts<float> &c, const float *sv,
+                                            const float2 *tab, Stream &rng, float &u0, float dt, int cap, int &err) {
+        const float2 C[2] = {make_float2(s.cass[0], s.cass[1]), make_float2(s.cass[2], s.cass[3])};
+        float2 dss[2], jx[2], S[2], Y[2], tmp[2];
+        const float jtr0 = jtr;
+        const float total = totals(s, c, sv, tab, C, dss, jx, S, Y);
+        const float jump = -logf(u0) * rcp_approx(total);
+        const bool last = !live || !(t + jump < dt);
+        const float h = last ? (dt - t) : jump;
+        const bool crossed = cass_step(s, c, h, C, dss, jx, tmp);
+        if (!live) {
+            jtr = jtr0;
+            return false;
+        }
+        int kind[4] = {0, 0, 0, 0};
+        const uint32_t D = crossed ? crossing_kinds(s, C, tmp, kind) : 0u;
+        uint32_t kk = k + 1u + D;
+        int act = 0, aj = 0, atr = 0;
+        if (!last) {
+            t += jump;
+            const float sub[4] = {S[0].x, S[0].y, S[1].x, S[1].y}, ryr_sub[4] = {Y[0].x, Y[0].y, Y[1].x, Y[1].y};
+            float ua, ub, uc;
+            rng.u24x3(kk, ua, ub, uc);
+            select_event_f32(s, c, sv, sub, ryr_sub, total, ua, ub, uc, kk, act, aj, atr);
+        }
+        if (crossed) resplit_crossed<float>(s, c, kind, rng, k);
+        s.cass[0] = tmp[0].x;
+        s.cass[1] = tmp[0].y;
+        s.cass[2] = tmp[1].x;
+        s.cass[3] = tmp[1].y;
+        cajsr_step(s, c, h);
+        if (act != 0) apply_event<float>(s, c, sv, act, aj, atr, jrel);
+        const float2 jxs = add2(jx[0], jx[1]);
+        jxfer_sum = jxs.x + jxs.y;
+        k = kk;
+        if (last) return true;
+        if (++ev > cap) {
+            err = 1;
+            return true;
+        }
+        u0 = rng.u24<2>(k);
+        return false;
+    }
+
     // The generic lane's iteration (same draws, same decisions) by the four lanes of a group (lanes 4g ..
     // 4g+3 of the warp, every one holding the same CRU and lane state): lane j = lane & 3 evaluates subunit
     // j's total and CaSS update in scalar form (rounding as the packed form of quiet()) and one Philox block
