@@ -81,6 +81,11 @@ struct Buf {
         n = bytes;
         return dev_alloc(&p, bytes);
     }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        n = 0;
+    }
     template <typename T>
     T *as() const {
         return reinterpret_cast<T *>(p);
@@ -147,7 +152,7 @@ struct AdjArgs {
     double *ai_row;     // [n_crus][kAdjIn] each CRU's adjoints of its step inputs and parameters
     double *ai_part;    // [blocks][kAdjIn] each block's sums of its CRUs' rows
     const dev::SsaConsts<double> *cc;  // [n_cells] SSA constants (k_busy_rec, k_cru_busy)
-    Rec *pool;   // [pool_cap] the segment's recorded sub-steps, and how many are taken
+    Rec *pool;   // [pool_cap] the segment's recorded sub-steps, or null, and how many are taken
     int *pool_n;
     int pool_cap;
     int *rec_at;        // [slots][n_crus] where each listed CRU's are, or -1 where they did not fit
@@ -794,7 +799,7 @@ __global__ void __launch_bounds__(kBusyBlk) k_cru_busy(const GradArgs a, const A
         CruAdjIn ai{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         Rec rec[kRec];
         const uint32_t rc = (uint32_t)a.rng_cell[cell];
-        const Rec *const got = b.rec_at[at] >= 0 ? b.pool + b.rec_at[at] : nullptr;
+        const Rec *const got = b.pool && b.rec_at[at] >= 0 ? b.pool + b.rec_at[at] : nullptr;
         const int n = got ? got->n
                           : run_rec(x0, cc, sv, a.seed, rc, m, (uint64_t)step, a.dt, a.event_cap, 0, 1 << 30, rec);
         CruCont s1 = cont_of(x0);  // the state at the sub-step's end (CaSS and CaJSR): the next one's start
@@ -1318,8 +1323,6 @@ int gw_grad_create(const gw_grad_desc *d, gw_grad **out) {
     up(g->quiet, nullptr, sizeof(uint8_t) * N * S);
     up(g->busy, nullptr, sizeof(int) * N * S);
     up(g->busy_n, nullptr, sizeof(int) * S);
-    up(g->pool_n, nullptr, sizeof(int));
-    up(g->rec_at, nullptr, sizeof(int) * N * S);
     up(g->lam_x, nullptr, sizeof(double) * kLamX * N);
     up(g->lam_G, nullptr, sizeof(double) * kNumGlobals * C);
     up(g->lam_cy, nullptr, sizeof(double) * 3 * C);
@@ -1342,12 +1345,26 @@ int gw_grad_create(const gw_grad_desc *d, gw_grad **out) {
         return rc;
     }
     // The pool of recorded sub-steps, for a quarter of the segment's CRU-steps (amid the Ca release six in a
-    // hundred have a jump, and their steps 2.2 sub-steps); without the memory for it the sweep does without.
-    g->pool_cap = (int)std::min<int64_t>(std::max<int64_t>(N * S / 4, 4096), 1 << 26);
-    if (g->pool.alloc(sizeof(Rec) * (size_t)g->pool_cap) != (int)cudaSuccess) {
-        cudaGetLastError();
-        g->pool.n = 0;
-        g->pool_cap = 0;
+    // hundred have a jump, and their steps 2.2 sub-steps), with the index of each listed CRU's: of the memory that
+    // is left no more than a quarter, since the caller's other work on the device (the replay, torch) takes its own
+    // from there.  Without it the sweep re-runs the steps (three small cells 84 instead of 30 us per step).
+    {
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+            cudaGetLastError();
+            free_bytes = 0;
+        }
+        const int64_t spare = (int64_t)(free_bytes / 4) - (int64_t)sizeof(int) * N * S;
+        g->pool_cap = (int)std::min({std::max<int64_t>(N * S / 4, 4096), (int64_t)1 << 26,
+                                     std::max<int64_t>(spare, 0) / (int64_t)sizeof(Rec)});
+        if (g->pool_cap < 4096 || g->pool.alloc(sizeof(Rec) * (size_t)g->pool_cap) != (int)cudaSuccess ||
+            g->rec_at.alloc(sizeof(int) * N * S) != (int)cudaSuccess || g->pool_n.alloc(sizeof(int)) != (int)cudaSuccess) {
+            cudaGetLastError();
+            g->pool.release();
+            g->rec_at.release();
+            g->pool_n.release();
+            g->pool_cap = 0;
+        }
     }
     g->stats.checkpoint_bytes = (int64_t)(g->ck_x.n + g->ck_G.n + g->ck_carry.n + g->ck_t.n + g->ck_sv.n);
     g->stats.segment_bytes =
@@ -1477,10 +1494,12 @@ int gw_grad_backward(gw_grad *g, const double *dL_dV, double *sens) {
             k_ssa<false><<<g->n_blocks, kBlk, 0, g->stream>>>(a, s, (int)(s - s0));
             k_global<<<g->n_cells, kOdeLanes, 0, g->stream>>>(a, s, (int)(s - s0), 0);
         }
-        if ((rc = g->cuda(cudaMemsetAsync(g->pool_n.p, 0, g->pool_n.n, g->stream), "gw_grad_backward"))) return rc;
-        for (int64_t s = s0; s < s1; s += 32768)  // (the grid's y extent)
-            k_busy_rec<<<dim3(rgrid, (unsigned)std::min<int64_t>(s1 - s, 32768)), kBusyBlk, 0, g->stream>>>(a, b, s0,
-                                                                                                        (int)(s - s0));
+        if (g->pool_cap > 0) {
+            if ((rc = g->cuda(cudaMemsetAsync(g->pool_n.p, 0, g->pool_n.n, g->stream), "gw_grad_backward"))) return rc;
+            for (int64_t s = s0; s < s1; s += 32768)  // (the grid's y extent)
+                k_busy_rec<<<dim3(rgrid, (unsigned)std::min<int64_t>(s1 - s, 32768)), kBusyBlk, 0, g->stream>>>(
+                    a, b, s0, (int)(s - s0));
+        }
         for (int64_t s = s1 - 1; s >= s0; --s) {
             k_cru_busy<<<bgrid, kBusyBlk, 0, g->stream>>>(a, b, s, (int)(s - s0));
             k_cru_quiet<<<g->n_blocks, kBlk, 0, g->stream>>>(a, b, (int)(s - s0));
