@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
                     m = -1;
                     ran = false;
                 } else {  // the queue is full, or the CRU is past its first iteration
-                    done = L.iterate(c, cc, sv, nullptr, rng, a.dt, a.event_cap, err, var ? &f : nullptr);
+                    done = L.iterate(c, cc, sv, rng, a.dt, a.event_cap, err, var ? &f : nullptr);
                 }
             }
             fresh = false;
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kBlk, VAR ? 1 : kSsaBlocksPerSm) k_ssa(const G
                 }
                 const unsigned pm = __ballot_sync(0xffffffffu, pend);
                 if (pm && (qc >= qe || __popc(pm) >= dev::kDefer) && pend) {
-                    done = L.iterate(c, cc, sv, nullptr, rng, a.dt, a.event_cap, err, var ? &f : nullptr);
+                    done = L.iterate(c, cc, sv, rng, a.dt, a.event_cap, err, var ? &f : nullptr);
                     ran = true;
                     pend = false;
                 }
@@ -739,7 +739,7 @@ __device__ int run_rec(const CruD &x0, const dev::SsaConsts<double> &cc, const d
         }
         const uint32_t lcc0 = c.lcc, fl0 = c.flags;
         dev::IterInfo<double> f;
-        const bool done = L.iterate(c, cc, sv, nullptr, rng, dt, cap, err, &f);
+        const bool done = L.iterate(c, cc, sv, rng, dt, cap, err, &f);
         if (keep) {
             Rec &r = rec[k % kRec];
             r.s = s;

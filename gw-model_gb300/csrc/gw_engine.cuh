@@ -118,9 +118,6 @@ __device__ __forceinline__ bool finite_bits(double x) {
 __device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_arrive_relaxed() {
-    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
-}
 __device__ __forceinline__ void cluster_wait() {
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -1421,7 +1418,7 @@ __device__ __forceinline__ void ssa_warps(const KernelArgs &a, uint64_t step0) {
                                     q[qs] = m;
                                     m = -1;
                                 } else {  // the queue is full, or the CRU is past its first iteration
-                                    done = sl.iterate(c, cc, sv, rtab, rng, dt, a.event_cap, err);
+                                    done = sl.iterate(c, cc, sv, rng, dt, a.event_cap, err);
                                 }
                             }
                             fresh = false;

@@ -190,14 +190,6 @@ struct StepDraw {
 // ------------------------------------------------------------------------------------------
 // Cluster helpers (inline PTX).
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
 __device__ __forceinline__ uint32_t map_rank(const void *p, uint32_t rank) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
     uint32_t r;
@@ -641,29 +633,6 @@ __device__ __forceinline__ uint32_t rate_index_word(uint32_t lcc, uint32_t flags
     return lcc | (g << 4) | (k << 5);
 }
 
-// FP32 total outgoing rate of subunit j (used only to draw the jump time and the subunit; the
-// transition itself is drawn from the full rate list of subunit_rates): the table part plus the
-// RyR rates regrouped.
-template <typename R>
-__device__ __forceinline__ R subunit_total_fast(const Cru<R> &s, int j, R x, const SsaConsts<R> &c,
-                                                const float2 *tab, uint32_t iw) {
-    const float2 tv = tab[(iw >> (8 * j)) & 0x3Fu];
-    const R other = fmaf(tv.y, x, tv.x);
-    const R R0 = (R)byte_s(s.ryr[0], j), R1 = (R)byte_s(s.ryr[1], j), R2 = (R)byte_s(s.ryr[2], j);
-    const R R3 = (R)byte_s(s.ryr[3], j), R4 = (R)byte_s(s.ryr[4], j), R5 = (R)byte_s(s.ryr[5], j);
-    const R x2 = x * x;
-    R ryr = x2 * (R0 * c.k12 + R1 * c.k2325) + R1 * c.k21;
-    if (x > (R)3.685e-2)
-        ryr += (R2 + R3) * __fdividef((float)(c.k45k34 * x2 + c.k32k43), (float)(c.k34 * x2 + c.k43));
-    else
-        ryr += x2 * R2 * c.k34 + R3 * c.k4543 + R2 * c.k32;
-    if (x > (R)1.15e-4)
-        ryr += (R4 + R5) * __fdividef((float)(c.k65 * (c.k52 + c.k54 * x2)), (float)(c.k56 * x2 + c.k65));
-    else
-        ryr += x2 * R4 * c.k5654 + R4 * c.k52 + R5 * c.k65;
-    return other + ryr;
-}
-
 // sample_weights (common.hpp:49-59) with the draw already scaled: u = U * total.  In FP32 mode a
 // scan that runs past the last positive weight (possible when rounding makes the partial sums fall
 // short of u) is moved back to the last positive weight.
@@ -759,42 +728,35 @@ __device__ __forceinline__ int crossing(const Cru<R> &s, int j, R x, R x_new, ui
 // Event selection (sample_weights over subunits, sample_new_state) from the rates of the start of
 // the iteration with draws kk, kk+1, kk+2: act 1 LCC, 2 inactivation toggle, 3 RyR, 4 ClCh
 // toggle; aj the subunit, atr the transition.
-template <typename R, bool EXACT>
+template <typename R>
 __device__ __forceinline__ void select_transition(const Rates<R> &r, R subr, Stream &rng, uint32_t &kk, int &act,
                                                   int &atr);
-template <typename R, bool EXACT>
+template <typename R>
 __device__ __forceinline__ void select_event(const Cru<R> &s, const SsaConsts<R> &c, const R *sv, const R (&sub)[4],
                                              R total, Stream &rng, uint32_t &kk, int &act, int &aj, int &atr) {
     const R us = rng.uniform<R>(kk++) * total;
-    aj = scan_weights<R, 4, !EXACT>(sub, us);
+    aj = scan_weights<R, 4, false>(sub, us);
     Rates<R> r;
-    const R sr = subunit_rates<R>(s, aj, pick4(s.cass, aj), c, sv, r);
-    select_transition<R, EXACT>(r, EXACT ? pick4(sub, aj) : sr, rng, kk, act, atr);
+    subunit_rates<R>(s, aj, pick4(s.cass, aj), c, sv, r);
+    select_transition<R>(r, pick4(sub, aj), rng, kk, act, atr);
 }
 
 // sample_new_state's choice within subunit aj (SSA.tpp:262-283) from its rates r and total subr,
 // with draws kk, kk+1: act 1 LCC, 2 inactivation toggle, 3 RyR, 4 ClCh toggle; atr the transition.
-template <typename R, bool EXACT>
+template <typename R>
 __device__ __forceinline__ void select_transition(const Rates<R> &r, R subr, Stream &rng, uint32_t &kk, int &act,
                                                   int &atr) {
     const R sum_lcc = r.lcc[0] + r.lcc[1] + r.lcc[2];
-    R sum_ryr;
-    if (EXACT) {
-        sum_ryr = subr - (sum_lcc + r.inact + r.clch);
-    } else {
-        sum_ryr = (R)0;
-#pragma unroll
-        for (int q = 0; q < 12; ++q) sum_ryr += r.ryr[q];
-    }
+    const R sum_ryr = subr - (sum_lcc + r.inact + r.clch);
     const R u = rng.uniform<R>(kk++) * subr;
     if (u < sum_lcc) {
         act = 1;
-        atr = scan_weights<R, 3, !EXACT>(r.lcc, rng.uniform<R>(kk++) * sum_lcc);
+        atr = scan_weights<R, 3, false>(r.lcc, rng.uniform<R>(kk++) * sum_lcc);
     } else if (u < (sum_lcc + r.inact)) {
         act = 2;
     } else if (u < (sum_lcc + r.inact + sum_ryr)) {
         act = 3;
-        atr = scan_weights<R, 12, !EXACT>(r.ryr, rng.uniform<R>(kk++) * sum_ryr);
+        atr = scan_weights<R, 12, false>(r.ryr, rng.uniform<R>(kk++) * sum_ryr);
     } else {
         act = 4;
     }
@@ -986,8 +948,10 @@ __device__ __forceinline__ void screen_subunit(const Cru<R> &s, int j, float x, 
     }
 }
 
+// One CRU's step on a lane: the FP64 form, and below it the FP32 one (SsaLane<float, false>).
 template <typename R, bool EXACT>
 struct SsaLane {
+    static_assert(sizeof(R) == 8 && EXACT, "FP32 has its own form");
     R t;          // time reached within the global step
     uint32_t k;   // next draw index
     int ev;       // events so far in this step
@@ -1010,51 +974,32 @@ struct SsaLane {
     __device__ __forceinline__ void fluxes(const Cru<R> &s, const SsaConsts<R> &c, const R *sv, R (&jxfer)[4],
                                            R (&jiss)[4]) {
         const R Cai = sv[SV_CAI], CaNSR = sv[SV_CANSR];
-        const R Cai_lo = EXACT ? (R)0 : sv[SV_CAI_LO], CaNSR_lo = EXACT ? (R)0 : sv[SV_CANSR_LO];
-        if (EXACT) {
-            jtr = c.rtr * (CaNSR - s.cajsr);
-        } else {
-            jtr = c.rtr * ((CaNSR - s.cajsr) + (CaNSR_lo - (R)s.cajsr_lo));
-        }
+        jtr = c.rtr * (CaNSR - s.cajsr);
         const R odd = s.cass[1] + s.cass[3], even = s.cass[0] + s.cass[2];
         jiss[0] = c.riss * minus_twice(odd, s.cass[0]);
         jiss[1] = c.riss * minus_twice(even, s.cass[1]);
         jiss[2] = c.riss * minus_twice(odd, s.cass[2]);
         jiss[3] = c.riss * minus_twice(even, s.cass[3]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (EXACT)
-                jxfer[j] = c.rxfer * (s.cass[j] - Cai);
-            else
-                jxfer[j] = c.rxfer * ((s.cass[j] - Cai) - Cai_lo);
-        }
+        for (int j = 0; j < 4; ++j) jxfer[j] = c.rxfer * (s.cass[j] - Cai);
     }
 
     // One iteration of the event loop; true when the CRU's step is complete (the jump passed the
     // end of the step, or the event cap was exceeded, which sets err).
-    __device__ __forceinline__ bool iterate(Cru<R> &s, const SsaConsts<R> &c, const R *sv, const float2 *tab,
-                                            Stream &rng, R dt, int cap, int &err, IterInfo<R> *info = nullptr) {
+    __device__ __forceinline__ bool iterate(Cru<R> &s, const SsaConsts<R> &c, const R *sv, Stream &rng, R dt, int cap,
+                                            int &err, IterInfo<R> *info = nullptr) {
         R jxfer[4], jiss[4];
         fluxes(s, c, sv, jxfer, jiss);
         // update_rates (SSA.tpp:48-56): only the subunit totals are kept here.
         R sub[4];
-        const uint32_t iw = EXACT ? 0u : rate_index_word(s.lcc, s.flags);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (EXACT) {
-                Rates<R> r;
-                sub[j] = subunit_rates<R>(s, j, s.cass[j], c, sv, r);
-            } else {
-                sub[j] = subunit_total_fast<R>(s, j, s.cass[j], c, tab, iw);
-            }
+            Rates<R> r;
+            sub[j] = subunit_rates<R>(s, j, s.cass[j], c, sv, r);
         }
         const R total = sub[0] + sub[1] + sub[2] + sub[3];
         const R u0 = rng.uniform<R>(k);
-        R jump;
-        if (EXACT)
-            jump = quot(-log(u0), total);
-        else
-            jump = __fdividef(-logf((float)u0), (float)total);
+        const R jump = quot(-log(u0), total);
         const bool last = !(t + jump < dt);
         const R h = last ? (dt - t) : jump;
         return advance(s, c, sv, rng, h, last, jump, sub, total, jxfer, jiss, cap, err, info);
@@ -1079,15 +1024,8 @@ struct SsaLane {
         // (pick4: j may be a lane's own subunit, and a register array indexed by a value known only
         // at run time would go to local memory)
         const R x = pick4(s.cass, j);
-        R beta;
-        if (EXACT) {
-            const R u = c.KBSR + x, v = c.KBSL + x;
-            beta = quot((R)1.0, (R)1 + quot(c.BSR_const, u * u) + quot(c.BSL_const, v * v));
-        } else {
-            const R u = (c.KBSR + x) * (c.KBSR + x), v = (c.KBSL + x) * (c.KBSL + x);
-            const R uv = u * v;
-            beta = __fdividef((float)uv, (float)(uv + c.BSR_const * v + c.BSL_const * u));
-        }
+        const R u = c.KBSR + x, v = c.KBSL + x;
+        const R beta = quot((R)1.0, (R)1 + quot(c.BSR_const, u * u) + quot(c.BSL_const, v * v));
         const R d = h * (pick4(s.jlcc, j) + pick4(jrel, j) - jxfer_j + jiss_j) * beta;
         tmp_j = x + d;
         kind_j = crossing<R>(s, j, x, tmp_j, D);
@@ -1108,7 +1046,7 @@ struct SsaLane {
         int act = 0, aj = 0, atr = 0;
         if (!last) {
             t += jump;
-            select_event<R, EXACT>(s, c, sv, sub, total, rng, kk, act, aj, atr);
+            select_event<R>(s, c, sv, sub, total, rng, kk, act, aj, atr);
         }
         return conclude(s, c, sv, rng, h, last, tmp, kind, D, kk, act, aj, atr, jxfer, cap, err, info);
     }
@@ -1124,26 +1062,8 @@ struct SsaLane {
         for (int j = 0; j < 4; ++j) s.cass[j] = tmp[j];
         {
             const R x = s.cajsr;
-            R beta;
-            if (EXACT)
-                beta = quot((R)1.0, (R)1 + quot(c.CSQN_const, (c.KCSQN + x) * (c.KCSQN + x)));
-            else {
-                const R u = (c.KCSQN + x) * (c.KCSQN + x);
-                beta = __fdividef((float)u, (float)(u + c.CSQN_const));
-            }
-            const R d = h * beta * (jtr - c.VSS_VJSR * (jrel[0] + jrel[1] + jrel[2] + jrel[3]));
-            if (EXACT) {
-                s.cajsr += d;
-            } else {
-                // Fast2Sum into (hi, lo): near rest the per-step JSR increment is below half an
-                // ulp of CaJSR in FP32, and would otherwise be lost.
-                const float hi = (float)s.cajsr;
-                const float y = (float)d + s.cajsr_lo;
-                const float sum = hi + y;
-                const float err_ = y - (sum - hi);
-                s.cajsr = (R)sum;
-                s.cajsr_lo = err_;
-            }
+            const R beta = quot((R)1.0, (R)1 + quot(c.CSQN_const, (c.KCSQN + x) * (c.KCSQN + x)));
+            s.cajsr += h * beta * (jtr - c.VSS_VJSR * (jrel[0] + jrel[1] + jrel[2] + jrel[3]));
         }
         // Apply the transition to the updated state.
         if (act != 0) apply_event<R>(s, c, sv, act, aj, atr, jrel);
@@ -1161,7 +1081,7 @@ struct SsaLane {
     }
 
     // The same by the four lanes of a group (lanes 4g .. 4g+3 of the warp, every one holding the same CRU and lane
-    // state; EXACT, R = double): lane j = lane & 3 evaluates subunit j's flux, CaSS update and rates, the
+    // state): lane j = lane & 3 evaluates subunit j's flux, CaSS update and rates, the
     // group exchanges them by shuffles, and the rest runs on the four lanes alike.  Same expressions in the
     // same order as the one-lane functions, hence the same results on every lane; an FP64 warp instruction
     // takes its sub-partition's pipe for ~64 cycles whatever its active lanes, and a group's step without
@@ -1223,7 +1143,6 @@ struct SsaLane {
     }
     __device__ __forceinline__ bool iterate_group(bool live, Cru<R> &s, const SsaConsts<R> &c, const R *sv,
                                                   Stream &rng, R dt, int cap, int &err) {
-        static_assert(sizeof(R) == 8 && EXACT, "the group iteration is for the FP64 lane");
         constexpr unsigned kAll = 0xffffffffu;
         const int lane = (int)(threadIdx.x & 31u), j = lane & 3, base = lane & ~3;
         R jx, js;
@@ -1259,7 +1178,7 @@ struct SsaLane {
 #pragma unroll
             for (int q = 0; q < 12; ++q) r.ryr[q] = __shfl_sync(kAll, rj.ryr[q], src);
             r.clch = __shfl_sync(kAll, rj.clch, src);
-            if (!last) select_transition<R, true>(r, pick4(sub, aj), rng, kk, act, atr);
+            if (!last) select_transition<R>(r, pick4(sub, aj), rng, kk, act, atr);
         }
         R jxfer[4];
 #pragma unroll
@@ -1269,7 +1188,7 @@ struct SsaLane {
         return conclude(s, c, sv, rng, h, last, tmp, kind, D, kk, act, aj, atr, jxfer, cap, err, nullptr);
     }
 
-    // FP32 screen of the next FP64 iteration (EXACT, R = double): true only if that iteration is
+    // FP32 screen of the next FP64 iteration: true only if that iteration is
     // certainly the step's last, i.e. its jump -log(u0) / total passes dt - t.  An FP64 iteration
     // spends most of its FP64 instructions on the 68 rates and the log and division of the jump
     // time, which the last iteration does not otherwise use; an FP64 instruction takes a warp
@@ -1292,7 +1211,6 @@ struct SsaLane {
     // those margins, and on every iteration that has an event.
     __device__ __forceinline__ bool surely_last(const Cru<R> &s, const SsaConsts<R> &c, const float *sk,
                                                 const float *svf, Stream &rng, R dt) {
-        static_assert(sizeof(R) == 8 && EXACT, "the screen is for the FP64 lane");
         float T = 0.f, A = 0.f;
         bool ok = true;
 #pragma unroll
@@ -1495,7 +1413,8 @@ struct SsaLane<float, false> {
             dss[p] = fma2(K[PK_M2], C[p], oe);
             jx[p] = mul2(K[PK_RXFER], add2(add2(C[p], ncai), ncailo));
         }
-        // subunit totals (the FP32 regrouping of subunit_total_fast)
+        // subunit totals: the table part plus the RyR rates regrouped (they draw the jump time and the subunit; the
+        // transition itself is drawn from the full rate list)
         const uint32_t iw = rate_index_word(s.lcc, s.flags);
         const uint32_t b0 = s.ryr[0] ^ 0x80808080u, b1 = s.ryr[1] ^ 0x80808080u, b2 = s.ryr[2] ^ 0x80808080u;
         const uint32_t b3 = s.ryr[3] ^ 0x80808080u, b4 = s.ryr[4] ^ 0x80808080u, b5 = s.ryr[5] ^ 0x80808080u;
@@ -1586,7 +1505,8 @@ struct SsaLane<float, false> {
         return D;
     }
 
-    // update_CaJSR (SSA.hpp:68-71) over a sub-step h, Fast2Sum into (hi, lo) as in the generic lane
+    // update_CaJSR (SSA.hpp:68-71) over a sub-step h, Fast2Sum into (hi, lo): near rest the per-step
+    // JSR increment is below half an ulp of CaJSR in FP32, and would otherwise be lost
     __device__ __forceinline__ void cajsr_step(Cru<float> &s, const SsaConsts<float> &c, float h) const {
         const float x = s.cajsr;
         const float u = (c.KCSQN + x) * (c.KCSQN + x);

@@ -71,7 +71,7 @@ __global__ void screen_check_kernel(const CellStatic *cs, int n, const uint32_t 
     const bool sc = L.surely_last(c, cc, sk, svf, rng, dt[i]);
     IterInfo<double> f;
     int err = 0;
-    L.iterate(c, cc, svi, nullptr, rng, dt[i], 1 << 30, err, &f);
+    L.iterate(c, cc, svi, rng, dt[i], 1 << 30, err, &f);
     out[2 * (int64_t)i] = sc ? 1 : 0;
     out[2 * (int64_t)i + 1] = f.act == 0 ? 1 : 0;
     jump[i] = f.act == 0 ? 0.0 : f.h;

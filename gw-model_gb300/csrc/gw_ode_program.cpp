@@ -523,7 +523,6 @@ bool ode_program_build(const CellStatic &cs, bool pow_fast, OdeProgram *prog, do
                     kind = op->kind;
                 }
             }
-            prog->wkind[q][w] = (uint8_t)kind;
         }
     }
     prog->n_slots = v[0].next;

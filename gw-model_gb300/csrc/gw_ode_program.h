@@ -70,7 +70,6 @@ struct alignas(16) OdeProgram {
     int const_begin, n_consts;           // per-cell constants occupy X[const_begin, +n_consts)
     int n_alt;
     uint16_t sv_src[kSvCount];           // X slot of each sv value (XS_ZERO if not produced)
-    uint8_t wkind[kOdeMaxPhases][kOdeWarps];  // the one op kind of each warp in each phase (NOP: idle)
     uint8_t alt_idx[kOdeMaxOps];         // 255, or index of the op's variant in alt[regime-1]
     uint8_t sv_stage[kOdeMaxOps];        // 1 + the sv index an op's output is staged to for the push, or 0
     OdeOp ops[kOdeMaxOps];               // regime 0: V >= -40
