@@ -191,9 +191,10 @@ int byte_of(int v) { return v & 0xFF; }
 // Launch shape: cluster size C, CRU tile per CTA and SSA warps per CTA.  A cell needs
 // ceil(ncru / tile) <= C CTAs.
 // The size rule: cluster size C and CTA capacity (tile) for n_cells cells of at most max_n CRUs, from the
-// requested values (0 = derive).
+// requested values (0 = derive).  It depends on nothing else and needs no device, so that every share of an
+// ensemble can be given the whole one's shape (gw_default_shape); hence a constant for the CTAs that cells
+// are spread over, GB300's (152 SMs).
 constexpr int kSpreadCtas = 112;
-constexpr int kSms = 152;
 void shape_rule(int precision, int n_cells, int max_n, int cluster_req, int tile_req, int &C, int &tile) {
     C = cluster_req > 0 ? cluster_req : 0;
     tile = tile_req > 0 ? tile_req : 0;
@@ -236,13 +237,16 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
                     max_n, need, tile, C);
     // SSA warps.  FP64: four (beside the leader's ODE warps; eight in the others), since a CRU takes four lanes
     // and the registers leave an SM one CTA anyway (a cell of 64 CRUs over 2 CTAs, one and four: 15.7 and
-    // 13.5 us per step).  FP32: one for 32 CRUs; where there is an SM for every CTA down to one for eight
-    // (a cell of 60 CRUs amid the release 3.8 us per step, with a warp for 32 4.3; but 256 cells of 100, two
-    // CTAs to an SM, 6.9 at rest and 9.9 amid the release against 9.2 and 13.9).
+    // 13.5 us per step).  FP32, whose results do not depend on it: one for 32 CRUs; where there is an SM for every
+    // CTA down to one for eight (us per step at rest and amid the release, 152 cells of 20 to 60 CRUs: 3.7 and 6.3,
+    // with a warp for 32 4.1 and 6.5; but 256 cells of 100, two CTAs to an SM: 8.4 and 13.0, with a warp for 32
+    // 5.4 and 8.5).
     int64_t ctas = 0;
     for (int i = 0; i < c->n_cells; ++i) ctas += (c->ncru[i] + tile - 1) / tile;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) cudaGetLastError();
     c->ssa_warps = c->precision == GW_PRECISION_FP64 ? kMaxSsaWarpsFp64
-                                                     : std::min(kMaxSsaWarps, tile / (ctas > kSms ? 32 : 8));
+                                                     : std::min(kMaxSsaWarps, tile / (ctas > sms ? 32 : 8));
     c->tile_cap = tile;
     // Pack cells (first-fit decreasing on CTA count) into clusters of C CTAs.
     std::vector<int> order(c->n_cells);
