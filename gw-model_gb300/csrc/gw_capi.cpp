@@ -192,9 +192,20 @@ int byte_of(int v) { return v & 0xFF; }
 // ceil(ncru / tile) <= C CTAs.
 // The size rule: cluster size C and CTA capacity (tile) for n_cells cells of at most max_n CRUs, from the
 // requested values (0 = derive).  It depends on nothing else and needs no device, so that every share of an
-// ensemble can be given the whole one's shape (gw_default_shape); hence a constant for the CTAs that cells
-// are spread over, GB300's (152 SMs).
-constexpr int kSpreadCtas = 112;
+// ensemble can be given the whole one's shape (gw_default_shape); hence GB300's figures as constants.
+//
+// Clusters of C CTAs that are resident at once, with a CTA to an SM: 152, 76, 46, 36, 28, 23, 15, 15, 15, 13, 8, 8,
+// 7, 7, 7, 7 for C = 1 .. 16 by cudaOccupancyMaxActiveClusters (a cluster lies within a GPC); fewer of the small ones here, since
+// parts differ in the SMs that are off.  Cells spread over more than that run in two rounds (us per step at rest and
+// amid the release: 9 cells of 1,500 to 3,000 CRUs over 12 CTAs each 8.6 and 12.4, over 10 4.6 and 6.5; 16 of 600 to
+// 1,200 over 7 7.7 and 12.3, over 6 4.3 and 6.6).
+constexpr int kResident[kMaxClusterCtas + 1] = {0, 152, 56, 44, 32, 26, 21, 15, 15, 15, 11, 8, 8, 7, 7, 7, 7};
+// The largest cluster size at which n_cells clusters are resident together (0: none).
+int spread_ctas(int n_cells) {
+    int C = kMaxClusterCtas;
+    while (C > 0 && n_cells > kResident[C]) --C;
+    return C;
+}
 void shape_rule(int precision, int n_cells, int max_n, int cluster_req, int tile_req, int &C, int &tile) {
     C = cluster_req > 0 ? cluster_req : 0;
     tile = tile_req > 0 ? tile_req : 0;
@@ -205,18 +216,17 @@ void shape_rule(int precision, int n_cells, int max_n, int cluster_req, int tile
         // cell of 64 CRUs over 1 and 2 CTAs: 21.2, 10.4; of 200 over 3, 8: 18.6, 12.6; of 400 over 6, 16:
         // 19.0, 13.2; of 1,250 over 12, 16: 25.0, 19.8.
         C = std::min(kMaxClusterCtas, std::max(1, (max_n + 95) / 96));
-        C = std::max(C, std::min({kMaxClusterCtas, (max_n + 31) / 32, kSpreadCtas / n_cells}));
+        C = std::max(C, std::min({kMaxClusterCtas, (max_n + 31) / 32, spread_ctas(n_cells)}));
         tile = (max_n + C - 1) / C;
     } else if (C == 0 && tile == 0) {
         // Default FP32: one CRU per SSA thread where possible, at most 16 CTAs per cell.
         C = 1;
         while (C < kMaxClusterCtas && (max_n + C - 1) / C > 32 * kMaxSsaWarps) C *= 2;
         // Cells that leave SMs idle are spread further, down to 64 CRUs per CTA beside the leader's:
-        // with one CRU per four lanes in one pass (kGroupCrus) the step is the global step's.  Clusters of
-        // any size are all resident up to 112 CTAs (7 clusters of 16, 14 of 8, 64 of 2).  us per step of
+        // with one CRU per four lanes in one pass (kGroupCrus) the step is the global step's.  us per step of
         // one cell of 200 CRUs over 1, 3, 5 CTAs: 4.5, 3.1, 3.1; of 777 over 4, 9, 16: 4.6, 3.2, 3.2;
-        // of 3,000 over 8, 16: 5.4, 4.8; 16 cells of 777 over 4 and 8: 4.6, 7.0 (two rounds).
-        C = std::max(C, std::min({kMaxClusterCtas, (max_n + 63) / 64 + 1, kSpreadCtas / n_cells}));
+        // of 3,000 over 8, 16: 5.4, 3.9.
+        C = std::max(C, std::min({kMaxClusterCtas, (max_n + 63) / 64 + 1, spread_ctas(n_cells)}));
         tile = (max_n + C - 1) / C;
     } else if (C == 0) {
         C = std::max(1, (max_n + tile - 1) / tile);
