@@ -247,16 +247,17 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
                     max_n, need, tile, C);
     // SSA warps.  FP64: four (beside the leader's ODE warps; eight in the others), since a CRU takes four lanes
     // and the registers leave an SM one CTA anyway (a cell of 64 CRUs over 2 CTAs, one and four: 15.7 and
-    // 13.5 us per step).  FP32, whose results do not depend on it: one for 32 CRUs; where there is an SM for every
-    // CTA down to one for eight (us per step at rest and amid the release, 152 cells of 20 to 60 CRUs: 3.7 and 6.3,
-    // with a warp for 32 4.1 and 6.5; but 256 cells of 100, two CTAs to an SM: 8.4 and 13.0, with a warp for 32
-    // 5.4 and 8.5).
+    // 13.5 us per step).  FP32, whose results do not depend on it: one for 32 CRUs, which then go on a lane each
+    // (group_steps); where there is an SM for every CTA one for eight, up to a CTA of 96 that holds a whole cell,
+    // whose warps then take four lanes per CRU, or where cells have several CTAs.  us per step at rest and amid the
+    // release, a warp for eight and for 32: 152 cells of 20 to 60 CRUs 3.7 and 6.3, 4.1 and 6.5; but 95 cells of 86 to
+    // 115 3.8 and 6.0, 3.4 and 5.4; 256 cells of 100, two CTAs to an SM, 8.4 and 13.0, 5.4 and 8.5.
     int64_t ctas = 0;
     for (int i = 0; i < c->n_cells; ++i) ctas += (c->ncru[i] + tile - 1) / tile;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) cudaGetLastError();
     c->ssa_warps = c->precision == GW_PRECISION_FP64 ? kMaxSsaWarpsFp64
-                                                     : std::min(kMaxSsaWarps, tile / (ctas > sms ? 32 : 8));
+                                                     : std::min(kMaxSsaWarps, tile / (ctas > sms || (C == 1 && tile > 8 * kMaxSsaWarps) ? 32 : 8));
     c->tile_cap = tile;
     // Pack cells (first-fit decreasing on CTA count) into clusters of C CTAs.
     std::vector<int> order(c->n_cells);

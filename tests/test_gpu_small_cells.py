@@ -27,7 +27,7 @@ def _state(e, i):
 
 
 @pytest.mark.parametrize("busy", [False, True])
-@pytest.mark.parametrize("largest", [32, 60])
+@pytest.mark.parametrize("largest", [32, 60, 100])
 def test_each_cell_as_alone(largest, busy):
     from gwgb300 import engine
 
