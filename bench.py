@@ -68,12 +68,12 @@ BYTES_PER_CRU_STEP = 2 * 72
 # From the ncu capture of the engine kernel on this workload (profiles/engine_kernel_cell12500.txt,
 # the launch at 0-1 ms of the beat): DRAM bytes
 # (read + write) of one 1000-step launch, and warp instructions issued per CRU-step.
-TRAFFIC_PER_LAUNCH = 1.095424e6
-WARP_INST_PER_CRU_STEP = 22.27
+TRAFFIC_PER_LAUNCH = 1.10848e6
+WARP_INST_PER_CRU_STEP = 22.95
 # The same for config 3's ensemble kernel (profiles/engine_kernel_batched256.txt, one 100-step launch
 # at 20 ms): DRAM bytes per launch and CRU, and warp instructions per CRU-step.
-BATCHED_TRAFFIC_PER_LAUNCH_CRU = 214.4e6 / 1870540
-BATCHED_WARP_INST_PER_CRU_STEP = 32.97
+BATCHED_TRAFFIC_PER_LAUNCH_CRU = 214.3e6 / 1870540
+BATCHED_WARP_INST_PER_CRU_STEP = 33.58
 CPU_PRE_NCRU = 1250   # the CPU's beat run, tiled x10 to 12,500 CRUs at each window start
 
 

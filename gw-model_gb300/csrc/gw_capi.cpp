@@ -285,9 +285,10 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
     // ssa_warps + kOdeWarps, the leader ssa_warps, or none when the cell is spread over several
     // CTAs of under kLeaderFreeCrus CRUs each: the global step on the leader's SM then sets the step and
     // runs faster without SSA warps beside it.  (One 12,500-CRU cell over 16 CTAs, 782 CRUs each, line
-    // at 1024 and 300: 7.94 and 7.61 ms per 1,000 steps at rest, 10.7 and 10.5 amid the release; 24
-    // cells of 500 to 3,000: line at 500 and 300: 14.0 and 13.7; 200: the same.)
-    constexpr int64_t kLeaderFreeCrus = 300;
+    // at 1024 and 300: 7.94 and 7.61 ms per 1,000 steps at rest, 10.7 and 10.5 amid the release.  us per step at
+    // rest and amid the release, line at 300 and 200: 100 cells of 385 to 600 CRUs over two CTAs 9.7 and 15.0, 8.1
+    // and 13.4; 30 of 300 to 1,000 over four 4.2 and 7.2, 4.1 and 6.9.)
+    constexpr int64_t kLeaderFreeCrus = 200;
     const int64_t wo = c->ssa_warps + kOdeWarps;
     int max_count = 0;
     for (int q = 0; q < c->n_clusters; ++q) {

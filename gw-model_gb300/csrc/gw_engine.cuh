@@ -726,7 +726,7 @@ struct CtaView {
         leader = active && w.rank_in_cell == 0;
         ode_thread = leader && warp >= nw;
         n_ssa = (leader ? nw : nw + kOdeWarps) * 32;  // SSA threads of this CTA
-        grouped = !FP64 && w.cru_count <= (n_ssa == 32 * kMaxWarps ? kGroupCrus : 32) * (n_ssa >> 5);
+        grouped = !FP64 && w.cru_count <= kGroupCrus * (n_ssa >> 5);
         const SmemLayout L = smem_layout<R, T>(a.tile_cap, a.max_cta_cell);
         cc = reinterpret_cast<SsaConsts<R> *>(smem + L.cc);
         svbuf = reinterpret_cast<R *>(smem + L.sv);
@@ -978,9 +978,11 @@ __device__ __forceinline__ void group_run(const KernelArgs &a, const SsaConsts<f
 // 5.7, the last 7.0).
 // 256 cells of 100, four warps: 5.4 and 8.6; 7.1 and 10.0; 7.1 and 9.2.
 // 100 cells of 50 to 200, twelve warps: 4.2 and 6.6; 4.6 and 6.9; 6.2 and 6.6.)
-// split_steps shares quiet passes and events between warps, which pays from 16 CRUs per warp on in a CTA of 16
-// warps (30 cells of 300 to 1,000 CRUs amid the release, line at 16 and 32: 6.7 and 7.1; at rest 4.7 and 4.1),
-// and not in smaller CTAs, where few warps are left for either part.
+// split_steps shares quiet passes and events between warps.  With fewer CRUs that does not pay: one warp has the CTA's
+// few events, a batch of 8 to 10 k cycles after the quiet pass, and the next step's passes over those CRUs wait for
+// it.  us per step at rest and amid the release, CTAs of 16 warps split above 16 and above 32 CRUs per warp: 76
+// cells of 385 to 760 CRUs over two CTAs 7.4 and 11.3, 4.4 and 7.3; 198 of 373 to 711 19.0 and 29.2, 12.5 and 20.3;
+// 20 of 600 to 1,200 over six 4.4 and 6.6, 4.0 and 6.7; one of 5,000 over 16 5.0 and 6.8, 4.1 and 7.0.
 template <bool ODE64>
 __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<false, ODE64> &v, uint64_t step0,
                                             unsigned long long &my_events, int &my_err, int &s_stop) {
@@ -1066,7 +1068,7 @@ __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<f
 // (With both kinds in one loop, one or two lanes of a warp with an event made the other thirty walk
 // through the event code, in most passes: 17 of 32 lanes active during the release.  A pass takes 2.4 k
 // cycles beside eleven others, a batch 5.5 k to 8 k.  us per step, one loop before: a 12,500-CRU cell over 16
-// CTAs 6.7 at rest, 10.6 amid the release, now 5.9 and 8.9; 256 mixed cells amid the release 132, now 113.
+// CTAs 6.7 at rest, 10.6 amid the release, now 5.9 and 8.9; 256 mixed cells amid the release 132, now 116.
 // A queue per warp run at its end costs about as much as one loop, its few lanes' event code being as long
 // as all the quiet passes; one CRU per lane for the events takes twice the latency.)
 //

@@ -68,9 +68,8 @@ struct CellDyn {
     int64_t stim_n;
 };
 
-// FP32 engine: CTAs of kMaxWarps SSA warps with at most this many CRUs per warp keep each warp to its own CRUs
-// (group_steps).
-constexpr int kGroupCrus = 16;
+// FP32 engine: CTAs with at most this many CRUs per SSA warp, a lane each, keep each warp to its own CRUs (group_steps).
+constexpr int kGroupCrus = 32;
 // FP32 engine, larger CTAs: an event batch (eight CRUs) in quiet passes (32 CRUs).
 constexpr int kBatchCost = 4;
 

@@ -87,18 +87,21 @@ typedef struct gw_ensemble_desc {
     uint64_t seed;
     int device;               /* CUDA device ordinal */
     int event_cap;            /* max jumps per CRU per step; 0 -> 65536 */
-    int cluster_ctas;         /* CTAs per thread-block cluster; 0 -> FP32: the smallest power of two
-                                 that keeps a cell's CTAs at <= 384 CRUs, FP64: enough CTAs of at
-                                 most 96 CRUs; at most 16 either way (gw_autotune measures the best
-                                 choice instead) */
+    int cluster_ctas;         /* CTAs per thread-block cluster, at most 16; 0 -> enough for the largest
+                                 cell (FP32: the smallest power of two that keeps a CTA at <= 384 CRUs,
+                                 FP64: CTAs of at most 96 CRUs), and more while the clusters of all
+                                 n_cells cells are resident together, down to about 64 (FP32) or 32
+                                 (FP64) CRUs per CTA: one 777-CRU cell takes 14 CTAs, 256 take 4 each
+                                 (gw_autotune measures the best choice instead) */
     int cta_crus;             /* CRU capacity of one CTA; 0 -> derived from cluster_ctas */
     int steps_per_launch;     /* global steps fused in one launch; 0 -> 1000 */
     int ode_fp32_rhs;         /* GW_PRECISION_FP32 only: 1 evaluates the global right-hand side in
                                  FP32 (state and Euler update stay FP64); 0 (default) keeps it FP64 */
     int cell_base;            /* global index of this context's cell 0: cell i draws from the streams
                                  of cell cell_base + i, so an ensemble split into contexts (one per
-                                 GPU, contiguous shares) gives the results of one context holding all
-                                 its cells; 0 for a whole ensemble.  cell_base + n_cells <= 2^28 */
+                                 GPU, contiguous shares), each with the whole ensemble's shape
+                                 (gw_default_shape), gives the results of one context holding all its
+                                 cells; 0 for a whole ensemble.  cell_base + n_cells <= 2^28 */
 } gw_ensemble_desc;
 
 /* Optional recording for gw_run, mirroring record_state (pyGW.hpp:56-99): after step i of the
@@ -197,9 +200,11 @@ int gw_autotune(const gw_ensemble_desc *desc, int trial_steps, int *best_cluster
 
 /* No counterpart in the reference.  The launch shape gw_create derives for *desc (its size rule,
  * or desc's own cluster_ctas / cta_crus where set): CTAs per cluster and CTA capacity.  Needs no
- * device.  Results depend on the shape only through each cell's CRU split, so contexts that hold
- * shares of an ensemble (cell_base) and are created with the whole ensemble's shape reproduce the
- * one-context results bit for bit. */
+ * device.  FP64 results depend on the shape in the rounding of each cell's flux sums (its CRU split
+ * over CTAs); FP32 ones do not, their flux sums being exact (unless a flux term is out of range: a
+ * concentration difference above 16 mM).  So contexts that hold shares of an ensemble (cell_base) and
+ * are created with the whole ensemble's shape reproduce the one-context results bit for bit.  The rule
+ * looks at desc's n_cells, so a share's own default shape may be another one. */
 int gw_default_shape(const gw_ensemble_desc *desc, int *cluster_ctas, int *cta_crus);
 
 /* Replaces GW_model::set_initial_value (GW.tpp:6-10) for one cell.  JLCC may be NULL: the

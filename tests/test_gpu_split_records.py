@@ -1,5 +1,5 @@
 """Records and repeatability of the FP32 path of CTAs with many CRUs, whose warps are split between quiet passes and
-events: cells of 500 to 1,600 CRUs held by one CTA, amid the release, recorded every few steps while the split
+events: cells of 500 to 1,600 CRUs held by one or two CTAs, amid the release, recorded every few steps while the split
 follows the events, against the same run spread over CTAs of few CRUs (another path, same bits)."""
 import numpy as np
 import pytest
@@ -30,12 +30,12 @@ def _run(n, every, steps, cluster_ctas, dt=1e-3, codec=False):
         return tr, end
 
 
-@pytest.mark.parametrize("n,every", [(500, 1), (1100, 1), (1600, 3)])
-def test_records_equal_those_of_few_crus_per_cta(n, every):
+@pytest.mark.parametrize("n,every,ctas", [(500, 1, 1), (1100, 1, 1), (1600, 3, 1), (1100, 1, 2)])  # of 12, or 12 and 16 warps
+def test_records_equal_those_of_few_crus_per_cta(n, every, ctas):
     steps = 480
     a, end_a = _run(n, every, steps, 16)
-    b, end_b = _run(n, every, steps, 1)
-    c, _ = _run(n, every, steps, 1, codec=True)
+    b, end_b = _run(n, every, steps, ctas)
+    c, _ = _run(n, every, steps, ctas, codec=True)
     for k in end_a:
         np.testing.assert_array_equal(end_a[k], end_b[k], err_msg=k)
     np.testing.assert_array_equal(a.globals, b.globals)
