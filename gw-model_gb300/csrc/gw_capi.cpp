@@ -287,8 +287,8 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
     // runs faster without SSA warps beside it.  (One 12,500-CRU cell over 16 CTAs, 782 CRUs each, line
     // at 1024 and 300: 7.94 and 7.61 ms per 1,000 steps at rest, 10.7 and 10.5 amid the release.  us per step at
     // rest and amid the release, line at 300 and 200: 100 cells of 385 to 600 CRUs over two CTAs 9.7 and 15.0, 8.1
-    // and 13.4; 30 of 300 to 1,000 over four 4.2 and 7.2, 4.1 and 6.9.)
-    constexpr int64_t kLeaderFreeCrus = 200;
+    // and 13.4; 43 of 304 to 945 over four 5.2 and 7.1, 4.9 and 7.4.)
+    constexpr int64_t kLeaderFreeCrus = 300, kLeaderFreeCrusPair = 200;
     const int64_t wo = c->ssa_warps + kOdeWarps;
     int max_count = 0;
     for (int q = 0; q < c->n_clusters; ++q) {
@@ -296,7 +296,7 @@ int plan_shape(gw_ctx *c, int cluster_req, int tile_req) {
         for (int cell : members[q]) {
             const int64_t n = c->ncru[cell];
             const int k = std::max(1, (int)((n + tile - 1) / tile));
-            const int64_t wl = (k >= 2 && n < kLeaderFreeCrus * k) ? 0 : c->ssa_warps;
+            const int64_t wl = k >= 2 && n < (k == 2 ? kLeaderFreeCrusPair : kLeaderFreeCrus) * k ? 0 : c->ssa_warps;
             const int64_t W = wl + (k - 1) * wo;
             auto cum = [&](int r) -> int64_t { return r == 0 ? 0 : wl + (r - 1) * wo; };
             for (int r = 0; r < k; ++r) {

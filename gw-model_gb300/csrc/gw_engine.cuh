@@ -726,7 +726,7 @@ struct CtaView {
         leader = active && w.rank_in_cell == 0;
         ode_thread = leader && warp >= nw;
         n_ssa = (leader ? nw : nw + kOdeWarps) * 32;  // SSA threads of this CTA
-        grouped = !FP64 && w.cru_count <= kGroupCrus * (n_ssa >> 5);
+        grouped = !FP64 && w.cru_count <= (n_ssa == 32 * kMaxWarps && w.n_cta_cell > 2 ? kGroupCrusSpread : kGroupCrus) * (n_ssa >> 5);
         const SmemLayout L = smem_layout<R, T>(a.tile_cap, a.max_cta_cell);
         cc = reinterpret_cast<SsaConsts<R> *>(smem + L.cc);
         svbuf = reinterpret_cast<R *>(smem + L.sv);
@@ -978,11 +978,12 @@ __device__ __forceinline__ void group_run(const KernelArgs &a, const SsaConsts<f
 // 5.7, the last 7.0).
 // 256 cells of 100, four warps: 5.4 and 8.6; 7.1 and 10.0; 7.1 and 9.2.
 // 100 cells of 50 to 200, twelve warps: 4.2 and 6.6; 4.6 and 6.9; 6.2 and 6.6.)
-// split_steps shares quiet passes and events between warps.  With fewer CRUs that does not pay: one warp has the CTA's
-// few events, a batch of 8 to 10 k cycles after the quiet pass, and the next step's passes over those CRUs wait for
-// it.  us per step at rest and amid the release, CTAs of 16 warps split above 16 and above 32 CRUs per warp: 76
-// cells of 385 to 760 CRUs over two CTAs 7.4 and 11.3, 4.4 and 7.3; 198 of 373 to 711 19.0 and 29.2, 12.5 and 20.3;
-// 20 of 600 to 1,200 over six 4.4 and 6.6, 4.0 and 6.7; one of 5,000 over 16 5.0 and 6.8, 4.1 and 7.0.
+// split_steps shares quiet passes and events between warps.  It needs enough events: with few, one warp has them, a
+// batch of 8 to 10 k cycles after the quiet pass, and the next step's passes over those CRUs wait for it.  So CTAs of
+// fewer than 16 warps and those of cells over one or two CTAs are split above 32 CRUs per warp, the others above 16.
+// us per step at rest and amid the release, line at 16 and at 32: 76 cells of 385 to 760 CRUs over two CTAs 7.4 and
+// 11.3, 4.4 and 7.3; 198 of 373 to 711 19.0 and 29.2, 12.5 and 20.3; but 38 of 672 to 989 over four 8.4 and 11.9,
+// 7.8 and 13.3; one of 5,000 over 16 5.0 and 6.8, 4.1 and 7.0.
 template <bool ODE64>
 __device__ __forceinline__ void group_steps(const KernelArgs &a, const CtaView<false, ODE64> &v, uint64_t step0,
                                             unsigned long long &my_events, int &my_err, int &s_stop) {

@@ -68,8 +68,10 @@ struct CellDyn {
     int64_t stim_n;
 };
 
-// FP32 engine: CTAs with at most this many CRUs per SSA warp, a lane each, keep each warp to its own CRUs (group_steps).
+// FP32 engine: CTAs with at most this many CRUs per SSA warp, a lane each, keep each warp to its own CRUs (group_steps);
+// those of kMaxWarps SSA warps of cells over more than two CTAs, this many.
 constexpr int kGroupCrus = 32;
+constexpr int kGroupCrusSpread = 16;
 // FP32 engine, larger CTAs: an event batch (eight CRUs) in quiet passes (32 CRUs).
 constexpr int kBatchCost = 4;
 
