@@ -843,7 +843,7 @@ __device__ __noinline__ void ode_warps(const KernelArgs &a, uint64_t step0) {
         // step s-2's, completed before the wait of step s-1)
         if (ot == 0)
             mbar_arrive_expect_tx(v.mbar + 8u * (uint32_t)par,
-                                  part_bytes + (s == a.n_steps - 1 ? (uint32_t)a.test_extra_tx : 0u));
+                                  part_bytes + (s == (a.test_extra_first ? 0 : a.n_steps - 1) ? (uint32_t)a.test_extra_tx : 0u));
         if (ot == 0 && (not_positive(os.g[1]) || not_positive(os.g[2])) && os.status == 0)
             os.status = GW_ERR_NERNST;
         // the increments up to the flux sums (warps 0 and 1), the next stimulus (warp 2), and the sums of
@@ -1129,13 +1129,16 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
         int nq_next;
         if (!quiet_warp) {
             // (each of these waits for itself: they may be in different steps, the set changing with nq)
+            // Whether the CTA stops is warp 0's decision, passed on as a split of 0: a warp that gave up by its own
+            // clock while the quiet warps went on would be missing from a later step's bar_or.  So this wait is
+            // longer than all that warp 0 may wait through before it arrives (four waits).
             if (lane == 0) mbar_arrive(bars + kQuiet);
-            bad |= !mbar_wait_warp(bars + kClear, ph);
-            if (bad) {
-                my_err |= 2;  // the leader's wait for this warp's partial runs out in turn
+            const bool told = mbar_wait_warp(bars + kClear, ph, 8 * kWaitCycles);
+            nq_next = told ? v.fq[6 + (par ^ 1)] : 0;
+            if (nq_next == 0) {
+                my_err |= 2;
                 continue;
             }
-            nq_next = v.fq[6 + (par ^ 1)];
         } else {
             // The SSA values of step s arrive by st.async from the leader's ODE warps and complete this
             // CTA's mbarrier of parity par (thread 0 declares the bytes; that mbarrier's previous phase,
@@ -1158,15 +1161,17 @@ __device__ __forceinline__ void split_steps(const KernelArgs &a, const CtaView<f
                 if (lane == 0) v.fq[2 * slot_next] = v.fq[2 * slot_next + 1] = 0;
                 for (int e = lane; e < kRateTab; e += 32) build_rate_entry<float>(rtab, cc, sv, e);
             }
-            if (bar_or(2, nq * 32, bad)) {
+            const bool stop = bar_or(2, nq * 32, bad);
+            if (threadIdx.x == 0) {
+                if (stop) v.fq[6 + (par ^ 1)] = 0;
+                mbar_arrive(bars + kClear);  // to the event warps
+            }
+            if (stop) {
                 my_err |= 2;
                 s_stop = s;
                 continue;
             }
             nq_next = v.fq[6 + (par ^ 1)];
-            if (warp == 0) {
-                if (lane == 0) mbar_arrive(bars + kClear);  // to the event warps
-            }
             StepDraw draw;
             draw.open(a.seed, rcell, step0 + s, 0);
             // The CTA's groups of 32, without the CRUs of step s-1's queue, then the groups of those, in turn

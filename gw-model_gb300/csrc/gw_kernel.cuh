@@ -274,15 +274,20 @@ __device__ __forceinline__ bool mbar_poll(uint32_t mbar, uint32_t parity) {
         : "memory");
     return ok != 0u;
 }
-// Bounded wait: false if the phase did not complete within 2^31 cycles (about a second).  The clock is
-// read every 64th time only: the loop's instructions are issue slots that the SM's other warps lose.
+// Bounded wait: false if the phase did not complete within 2^31 cycles (about a second) and kLatePolls polls after
+// that: the clock also runs while the whole SM stands still (a context switch), and the warps that this one waits
+// for come back with it.  The clock is read every 64th time only: the loop's instructions are issue slots
+// that the SM's other warps lose.
+constexpr long long kWaitCycles = 1ll << 31;
+constexpr int kLatePolls = 4096;
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     const long long t0 = clock64();
+    int late = 0;
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 64; ++i)
             if (mbar_poll(mbar, parity)) return mbar_try_wait(mbar, parity);
-        if (clock64() - t0 > (1ll << 31)) return false;
+        if (clock64() - t0 > kWaitCycles && (late += 64) > kLatePolls) return false;
     }
 }
 
@@ -290,14 +295,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
 // mbar_wait by a whole warp, one outcome for its lanes.  Every lane polls, and the loop's branch is on a vote:
 // after a loop that one lane ran for the others the warp went on in parts, every instruction once for each
 // (a batch of events took 17 k cycles instead of 5.5 k).
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity, long long cycles = kWaitCycles) {
     const long long t0 = clock64();
+    int late = 0;
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 64; ++i)
             if (__all_sync(0xffffffffu, mbar_poll(mbar, parity)))
                 return __all_sync(0xffffffffu, mbar_try_wait(mbar, parity));
-        if (__any_sync(0xffffffffu, clock64() - t0 > (1ll << 31))) return false;
+        if (__any_sync(0xffffffffu, clock64() - t0 > cycles) && (late += 64) > kLatePolls) return false;
     }
 }
 
